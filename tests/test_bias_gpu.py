@@ -147,3 +147,41 @@ def test_fused_bias_same_bits_for_both_tile_widths():
         outs.append((rho, grad))
     assert plan.device_flags() == 0
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shells,np_range,nc_range,shift", [
+    ("s", (1, 3), (3, 3), 0),                  # one function per atom, fewer than 8 points
+    ("ssssppdd", (63, 65), (31, 33), 0),       # one function either side of a 32-wide chunk, 64-point passes
+    ("gggs", (100, 130), (84, 84), 0),         # 28 functions of one atom: two passes of 24
+    ("gggggggs", (60, 140), (190, 192), 1),    # 64 functions of one atom; odd wave offsets (8-byte copies)
+])
+def test_bias_pass_edges_match_oracle(shells, np_range, nc_range, shift):
+    """Edges of the passes: 24 functions, 64 points, 32-wide chunks, both copy
+    widths, 64- and 128-point work items.  The sums have at most 256 terms, so
+    1e-12 of the largest entry leaves a factor of about 40 over their rounding."""
+    import torch
+
+    from gpu_util import dev, host
+
+    p = synth.make_rho1_problem(T=4, seed=23, n_atoms=3, shells=shells, n_batches=9, np_range=np_range,
+                                nc_range=nc_range, pad_value=np.nan, n_active=3)
+    if shift:
+        p.wave = np.concatenate([np.full(shift, np.nan), p.wave])
+        p.gradient_wave = np.concatenate([np.full(3 * shift, np.nan), p.gradient_wave])
+        p.i_batch_2_wave_offset = (p.i_batch_2_wave_offset + shift).astype(np.int32)
+    dm = np.random.default_rng(8).normal(size=(p.n_basis, p.n_basis))
+    ref = oracle.rho_bias_part2(p, dm, j_coord=2)
+    plan = _lib.Rho1Plan(p)
+    for tile in (64, 128):
+        plan.set_tuning(fp64_tile_points=tile)
+        out = torch.full((p.n_max_batch_size * p.n_my_batches_work * 4,), 5.0, dtype=torch.float64, device="cuda")
+        plan.bias_part2(4, p.n_atoms, 1, 3, 2, dev(p.atom_valid_n_compute_c_batches, np.int32), dev(p.wave),
+                        dev(p.gradient_wave), dev(dm), out)
+        torch.cuda.synchronize()
+        got = host(out, ref.shape)
+        for b in range(p.n_my_batches_work):
+            n = p.n_point_batches[b]
+            assert np.max(np.abs(got[:n, b, :3] - ref[:n, b, :3])) < TOL * np.max(np.abs(ref))
+            assert np.all(got[n:, b, :] == 5.0) and np.all(got[:, b, 3] == 5.0)
+    assert plan.device_flags() == 0
