@@ -25,10 +25,13 @@
 //   loop.  The Horner degree is lam, specialised at compile time per warp-
 //   uniform lam (the l_max-specialised AOT kernels of the reference's
 //   task3_jit/version5, but derived from the runtime table rather than baked in).
-// * Near field.  Real Y_lm by the associated-Legendre recursion fused with the
-//   Hermite spline dot, read straight from the caller's
-//   (L^2, 2, n_hartree_grid, atom, t) table (the two grid nodes needed are one
-//   contiguous 4 L^2 run), so the reference's per-call transpose is not needed.
+// * Near field, in a launch of its own after the far field's.  Real Y_lm by the
+//   associated-Legendre recursion fused with the Hermite spline dot, read
+//   straight from the caller's (L^2, 2, n_hartree_grid, atom, t) table (the two
+//   grid nodes needed are one contiguous 4 L^2 run), so the reference's
+//   per-call transpose is not needed.
+// * Which pairs are near, far or skipped is decided for a warp's points at once
+//   wherever the box around them allows it (the points are in spatial order).
 // * Generic path.  When the fast path's preconditions do not hold (a
 //   centers_hartree_potential list that is not the identity, whose far field
 //   the reference evaluates with the loop slot as centre, :161-162/:183; or a
@@ -47,10 +50,8 @@
 namespace frpa {
 
 constexpr int SU_LMAX = FRPA_SUMUP_MAX_L;  // 8
-constexpr int SU_THREADS = 128;  // fast kernel: 5 CTAs per SM, 96 registers (no spills; measured against
-                                 // 3, 4 and 6 CTAs per SM and two centres per thread)
-constexpr int SU_PPT = 2;                  // points per thread (share coefficient loads)
-constexpr int SU_CHUNK = 16;               // centre records staged per shared-memory chunk
+constexpr int SU_THREADS = 128;
+constexpr int SU_CHUNK = 8;      // centre records per shared-memory chunk (two buffers)
 
 // Near-field constants: Y_lm = K[l][m] Q_l^m(z) {C_m, S_m}; recursion
 // Q_l^m = RA[l][m] z Q_{l-1}^m - RB[l][m] Q_{l-2}^m; DF[m] = (2m-1)!!.
@@ -59,17 +60,24 @@ __constant__ double c_Kcos[SU_LMAX + 1][SU_LMAX + 1];
 __constant__ double c_RA[SU_LMAX + 1][SU_LMAX + 1];
 __constant__ double c_RB[SU_LMAX + 1][SU_LMAX + 1];
 __constant__ double c_DF[SU_LMAX + 1];
+// the near-field kernel's copy of K, RA, RB, for threads that each read another entry
+__device__ double d_near_tables[3][SU_LMAX + 1][SU_LMAX + 1];
 __host__ __device__ constexpr int n_kelvin(int L) { return kelvin_count(L); }
 
 // record layout (doubles) for one (centre slot, t)
 enum : int {
-  R_X = 0, R_Y, R_Z, R_MRS, R_LAM0, R_ATOM, R_RGM, R_LINC, R_NGRID, R_OPR  // R_OPR .. R_OPR+L
+  R_X = 0, R_Y, R_Z, R_MRS, R_LAM0, R_ATOM, R_RGM, R_LINC, R_NGRID, R_SAFE, R_OPR  // R_OPR .. R_OPR+L
 };
-__host__ __device__ constexpr int rec_coef_off(int L) { return R_OPR + L + 1; }
-__host__ __device__ constexpr int rec_stride(int L) { return ((rec_coef_off(L) + n_kelvin(L)) + 1) & ~1; }
+__host__ __device__ constexpr int rec_coef_off(int L) { return (R_OPR + L + 2) & ~1; }
+// R_SAFE: no coefficient above SAFE_COEF and no far pair closer than
+// sqrt(SAFE_MRS), so that every partial sum of the far-field polynomial is
+// finite (165 terms of at most 1e100 x 1e20^8) and 0 x (partial sum) is 0
+constexpr double SAFE_COEF = 1e100, SAFE_MRS = 1e-40;
+__host__ __device__ constexpr int rec_stride(int L) { return rec_coef_off(L) + kelvin_slots(L); }
 
 struct SumupPlan {
   int device = 0;
+  std::vector<void *> owned;  // the device allocations behind the pointers below
   int T = 1, L = 0, L2 = 1, lma = 0, icc_dim0 = 0, mc_dim = 0, hfla = 0;
   int n_full_points = 0, n_valid_points = 0, n_centers = 0, n_chp = 0, n_atoms = 0, n_species = 0;
   int n_hartree_grid = 0;
@@ -77,26 +85,30 @@ struct SumupPlan {
   int n_coef = 0, rs = 0;
   // device const arrays
   int *d_map = nullptr;
-  int *d_order = nullptr;  // valid points in spatial (Morton) order, for warp-uniform branches
+  // valid points in spatial (Morton) order, for warp-uniform branches: their valid-point
+  // index, full index and coordinates (x, y, z rows of n_valid_points), so that the fast
+  // kernels' loads coalesce and none waits for an index
+  int *d_order = nullptr, *d_pfull = nullptr;
+  double *d_pxyz = nullptr;
   double *d_coord = nullptr;
   int *d_species = nullptr, *d_species_center = nullptr, *d_l_hartree = nullptr, *d_n_grid = nullptr;
   int *d_c2a = nullptr, *d_chp = nullptr, *d_icc = nullptr, *d_ncc = nullptr, *d_ijkmax = nullptr;
   int *d_icc_packed = nullptr;  // (i | j<<8 | k<<16 | nn<<24) per row
   double *d_cc = nullptr, *d_cc_xyz = nullptr, *d_rgm = nullptr, *d_linc = nullptr;
-  int *d_conv_ptr = nullptr, *d_conv_n = nullptr;
-  double *d_conv_f = nullptr;
-  int n_conv = 0;
+  int *d_slot = nullptr;                            // coefficient -> position in a record
+  int *d_conv_ptr = nullptr, *d_conv_lm = nullptr;  // Kelvin conversion (CSR by coefficient): (l, m) slot,
+  double2 *d_conv_fc = nullptr;                     // factor and cc of the table row
   // workspaces
   double *d_mc = nullptr;    // (mc_dim, n_atoms, T)
   double *d_recs = nullptr;  // (rs, n_chp, T)
+  double4 *d_heads = nullptr;  // (n_chp, T): centre and near radius^2, for the near-field launch's search
   int *d_err = nullptr;      // device-side input error flags
-  // adjoint: transpose of the Kelvin conversion (by table row) and workspaces
+  // adjoint: transpose of the Kelvin conversion (by table row; coefficients in
+  // the dQ kernels' order), the table rows of each (l, m), per point-block partial
+  // sums (n_coef, n_chp, T, adj_nz) and the slots of each atom (CSR, ascending)
   int *d_convT_ptr = nullptr, *d_convT_k = nullptr;
   double *d_convT_f = nullptr;
-  double *d_dcoef = nullptr;  // (n_coef, n_chp, T)
-  double *d_dmc = nullptr;    // (mc_dim, n_atoms, T)
-  // deterministic adjoint: per point-block partial sums (n_coef, n_chp, T,
-  // adj_nz), reduced in block order; slots of each atom (CSR, ascending)
+  int *d_lm_ptr = nullptr, *d_lm_row = nullptr;
   double *d_dcoef_part = nullptr;
   int adj_nz = 1, adj_pts = 4096;
   int *d_atom_slot_ptr = nullptr, *d_atom_slots = nullptr;
@@ -132,50 +144,95 @@ __global__ void sumup_multipole_c_kernel(int n_atoms, int L, int L2, int mc_dim,
   }
 }
 
+// The valid points' full indices and coordinates in the plan's spatial order.
+__global__ void sumup_gather_points_kernel(int n_valid, const int *__restrict__ map, const int *__restrict__ order,
+                                           const double *__restrict__ coord, int *__restrict__ pfull,
+                                           double *__restrict__ pxyz) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_valid; i += gridDim.x * blockDim.x) {
+    const int f = map[order[i]];
+    pfull[i] = f;
+    for (int c = 0; c < 3; ++c) pxyz[i + (long long)c * n_valid] = coord[3LL * f + c];
+  }
+}
+
 // Per (slot, t) record for the fast kernels: centre, radii, l_hartree, near
-// field parameters and the Kelvin coefficients (CSR contraction of multipole_c).
-__global__ void sumup_records_kernel(int L, int n_atoms, int n_chp, int mc_dim, int n_coef, int rs,
-                                     const int *__restrict__ chp, const int *__restrict__ c2a,
-                                     const int *__restrict__ species, const int *__restrict__ species_center,
-                                     const int *__restrict__ l_hartree, const int *__restrict__ n_grid,
-                                     const double *__restrict__ rgm, const double *__restrict__ linc,
-                                     const double *__restrict__ cc_xyz, const double *__restrict__ mrs,
-                                     const double *__restrict__ opr, const double *__restrict__ mc,
-                                     const int *__restrict__ conv_ptr, const int *__restrict__ conv_n,
-                                     const double *__restrict__ conv_f, double *__restrict__ recs) {
-  const int slot = blockIdx.x, t = blockIdx.y;
+// field parameters and the Kelvin coefficients (CSR contraction of
+// multipole_c = cc Q with the l cap and the 1e-10 threshold of
+// sum_up_whole_potential.cpp:357-378, formed on the way).  Also checks
+// l_hartree_max_far_distance of every atom, as sumup_multipole_c_kernel does.
+__global__ void __launch_bounds__(128)
+    sumup_prep_kernel(int L, int lma, int n_atoms, int n_chp, int n_coef, int rs, const int *__restrict__ chp,
+                      const int *__restrict__ c2a, const int *__restrict__ species,
+                      const int *__restrict__ species_center, const int *__restrict__ l_hartree,
+                      const int *__restrict__ n_grid, const double *__restrict__ rgm,
+                      const double *__restrict__ linc, const double *__restrict__ cc_xyz,
+                      const double *__restrict__ mrs, const double *__restrict__ opr,
+                      const int *__restrict__ lhmfd, const double *__restrict__ Q, const int *__restrict__ slot_of,
+                      const int *__restrict__ conv_ptr, const int *__restrict__ conv_lm, const double2 *__restrict__ conv_fc,
+                      double *__restrict__ recs, double4 *__restrict__ heads, int *__restrict__ err) {
+  __shared__ double q_kept[(SU_LMAX + 1) * (SU_LMAX + 1)];
+  const int slot = blockIdx.x, t = blockIdx.y, L2 = (L + 1) * (L + 1);
+  if (slot < n_atoms && threadIdx.x == 0) {
+    const int lh = lhmfd[slot + n_atoms * t];
+    if (lh < 0 || lh > L || lh > lma) atomicOr(err, 1);
+  }
+  if (slot >= n_chp) return;
   const int cur = chp[slot] - 1;
   const int atom = c2a[cur] - 1;
+  const long long at = atom + (long long)n_atoms * t;
+  const int lh = min(max(lhmfd[at], 0), L);
+  for (int lm = threadIdx.x; lm < L2; lm += blockDim.x) {
+    const double q = Q[lm + L2 * at];
+    q_kept[lm] = (lm < (lh + 1) * (lh + 1) && fabs(q) > 1e-10) ? q : 0.0;
+  }
   double *r = recs + (long long)rs * (slot + (long long)n_chp * t);
-  const double *m = mc + (long long)mc_dim * (atom + (long long)n_atoms * t);
+  for (int l = threadIdx.x; l <= L; l += blockDim.x) r[R_OPR + l] = opr[l + (L + 1) * at];
+  __syncthreads();
+  bool small = true;
+  for (int k = threadIdx.x; k < n_coef; k += blockDim.x) {
+    double s = 0.0;
+    const int e1 = conv_ptr[k + 1];
+#pragma unroll 4
+    for (int e = conv_ptr[k]; e < e1; ++e) {
+      const double q = q_kept[conv_lm[e]];
+      const double2 fc = conv_fc[e];
+      s += fc.x * (q != 0.0 ? fc.y * q : 0.0);
+    }
+    r[rec_coef_off(L) + slot_of[k]] = s;
+    small = small && fabs(s) <= SAFE_COEF;
+  }
+  const bool safe = __syncthreads_and(small);
   if (threadIdx.x == 0) {
     const int sp = species_center[cur] - 1;
+    const double m = mrs[at];
     r[R_X] = cc_xyz[3 * cur + 0];
     r[R_Y] = cc_xyz[3 * cur + 1];
     r[R_Z] = cc_xyz[3 * cur + 2];
-    r[R_MRS] = mrs[atom + (long long)n_atoms * t];
+    r[R_MRS] = m;
     r[R_LAM0] = (double)l_hartree[species[atom] - 1];
     r[R_ATOM] = (double)atom;
     r[R_RGM] = rgm[sp];
     r[R_LINC] = linc[sp];
     r[R_NGRID] = (double)n_grid[sp];
-  }
-  for (int l = threadIdx.x; l <= L; l += blockDim.x)
-    r[R_OPR + l] = opr[l + (long long)(L + 1) * (atom + (long long)n_atoms * t)];
-  for (int k = threadIdx.x; k < n_coef; k += blockDim.x) {
-    double s = 0.0;
-    for (int e = conv_ptr[k]; e < conv_ptr[k + 1]; ++e) s += conv_f[e] * m[conv_n[e]];
-    r[rec_coef_off(L) + k] = s;
+    r[R_SAFE] = safe && m >= SAFE_MRS ? 1.0 : 0.0;
+    heads[slot + (long long)n_chp * t] = make_double4(cc_xyz[3 * cur], cc_xyz[3 * cur + 1], cc_xyz[3 * cur + 2], m);
   }
 }
 
 // ------------------------------------------------------- device pieces ---
 
-// Near field for one pair (sum_up_whole_potential.cpp:411-477, spline :12-52):
-// trig values exactly as the reference forms them, then Y_lm by recursion
-// fused with the Hermite spline dot.
-__device__ double near_field(int lam, int L2, double dx, double dy, double dz, double d2, double rgm, double linc,
-                             int ngrid, const double *__restrict__ spl) {
+// Near-field geometry of one pair (sum_up_whole_potential.cpp:411-477, spline
+// :12-52): the trig values exactly as the reference forms them, the spline
+// interval and its four Hermite weights.
+struct NearGeom {
+  double x, y, z;         // unit vector
+  double ta, tb, tc, td;  // weights of (value, slope) at the interval's two nodes
+  int i_spl;              // interval, 1-based
+};
+
+__device__ __forceinline__ NearGeom near_geometry(double dx, double dy, double dz, double d2, double rgm, double linc,
+                                                  int ngrid) {
+  NearGeom G;
   const double dist = sqrt(d2);
   const double din0 = dx / dist, din1 = dy / dist, din2 = dz / dist;
   const double r_log = 1.0 + log(dist / rgm) / linc;
@@ -200,18 +257,30 @@ __device__ double near_field(int lam, int L2, double dx, double dy, double dz, d
     ct = 0.0;
     st = 1.0;
   }
-  const double x = st * cph, y = st * sph, z = ct;
+  G.x = st * cph;
+  G.y = st * sph;
+  G.z = ct;
   int i_spl = (int)r_log;
   i_spl = i_spl < 1 ? 1 : i_spl;
   i_spl = i_spl > ngrid - 1 ? ngrid - 1 : i_spl;
+  G.i_spl = i_spl;
   const double u = r_log - i_spl;
-  const double ta = (u - 1) * (u - 1) * (1 + 2 * u);
-  const double tb = (u - 1) * (u - 1) * u;
-  const double tc = u * u * (3 - 2 * u);
-  const double td = u * u * (u - 1);
-  const double *g0 = spl + (long long)2 * L2 * (i_spl - 1);
+  G.ta = (u - 1) * (u - 1) * (1 + 2 * u);
+  G.tb = (u - 1) * (u - 1) * u;
+  G.tc = u * u * (3 - 2 * u);
+  G.td = u * u * (u - 1);
+  return G;
+}
+
+// Near field of one pair by one thread (generic path): Y_lm by recursion fused
+// with the Hermite spline dot.
+__device__ double near_field(int lam, int L2, double dx, double dy, double dz, double d2, double rgm, double linc,
+                             int ngrid, const double *__restrict__ spl) {
+  const NearGeom G = near_geometry(dx, dy, dz, d2, rgm, linc, ngrid);
+  const double x = G.x, y = G.y, z = G.z;
+  const double *g0 = spl + (long long)2 * L2 * (G.i_spl - 1);
   const double *g1 = g0 + 2 * L2;
-  auto S = [&](int i) { return g0[i] * ta + g0[i + L2] * tb + g1[i] * tc + g1[i + L2] * td; };
+  auto S = [&](int i) { return g0[i] * G.ta + g0[i + L2] * G.tb + g1[i] * G.tc + g1[i + L2] * G.td; };
   double acc = 0.0;
   double C = 1.0, Sm = 0.0;
   for (int m = 0; m <= lam; ++m) {
@@ -237,142 +306,435 @@ __device__ double near_field(int lam, int L2, double dx, double dy, double dz, d
   return acc;
 }
 
-// 1/sqrt(x) for x > 0: the PTX approximation (relative error below 1e-6)
-// refined by two Newton-Raphson steps y <- y + y/2 (1 - x y^2), within about
-// one ulp of 1 / sqrt(x) (measured over x in [1e-4, 1e10]); cheaper than the
-// library's correctly rounded form.
-__device__ __forceinline__ double rsqrt_nr(double x) {
+// 1/sqrt(x) for x > 0: the PTX approximation y (relative error below 1e-6) with
+// one third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2: within about one
+// ulp of 1 / sqrt(x); cheaper than the library's correctly rounded form.
+__device__ __forceinline__ double rsqrt_refined(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const double e = fma(-(x * y), y, 1.0);
-    y = fma(0.5 * y, e, y);
-  }
-  return y;
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
-// --------------------------------------------------------- fast kernel ---
+// l_atom_max at squared distance d2 (sum_up_whole_potential.cpp:404-411).
+__device__ __forceinline__ int lam_at(const double *opr, int lam0, double d2) {
+  int l = lam0;
+  while (opr[l] < d2 && l > 0) --l;
+  return l;
+}
 
-__global__ void __launch_bounds__(SU_THREADS, 5)
-    sumup_fast_kernel(int n_valid, int n_full, const int *__restrict__ map, const int *__restrict__ order,
-                      const double *__restrict__ coord, int n_active, int n_chp, int n_atoms, int L,
-                      int n_hartree_grid, const double *__restrict__ recs, const double *__restrict__ spline,
-                      double *__restrict__ dv, unsigned char *__restrict__ codes) {
-  const int RS = rec_stride(L);
-  const int CO = rec_coef_off(L);
-  const int L2 = (L + 1) * (L + 1);
-  __shared__ __align__(16) double srec[SU_CHUNK * rec_stride(SU_LMAX)];
-  const int tid = threadIdx.x;
-  const unsigned FULL = 0xffffffffu;
+// --------------------------------------------------- far-field kernel ---
 
-  int vidx[SU_PPT], full[SU_PPT];
-  double px[SU_PPT], py[SU_PPT], pz[SU_PPT];
-  bool valid[SU_PPT];
+// Box around a warp's points (points that are not finite, and lanes without a
+// point, left out: every pair of theirs is skipped; an empty box is infinitely
+// far from everything).
+struct Box {
+  double lo[3], hi[3];
+};
+
+template <int N>
+__device__ __forceinline__ Box warp_box(const double *px, const double *py, const double *pz, const bool *live) {
+  Box b;
 #pragma unroll
-  for (int j = 0; j < SU_PPT; ++j) {
-    // a warp's points are neighbours in space when the plan gives an order,
-    // so its near / far / skip decisions for an atom mostly agree
-    const int slot = blockIdx.x * (SU_THREADS * SU_PPT) + j * SU_THREADS + tid;
-    valid[j] = slot < n_valid;
-    vidx[j] = valid[j] ? (order ? order[slot] : slot) : 0;
-    full[j] = valid[j] ? map[vidx[j]] : 0;
-    px[j] = valid[j] ? coord[3LL * full[j] + 0] : 0.0;
-    py[j] = valid[j] ? coord[3LL * full[j] + 1] : 0.0;
-    pz[j] = valid[j] ? coord[3LL * full[j] + 2] : 0.0;
+  for (int c = 0; c < 3; ++c) {
+    b.lo[c] = __longlong_as_double(0x7ff0000000000000LL);
+    b.hi[c] = -b.lo[c];
   }
-
-  for (int t = 0; t < n_active; ++t) {
-    double v[SU_PPT];
 #pragma unroll
-    for (int j = 0; j < SU_PPT; ++j) v[j] = valid[j] ? dv[full[j] + (long long)n_full * t] : 0.0;
-
-    for (int c0 = 0; c0 < n_chp; c0 += SU_CHUNK) {
-      const int nch = min(SU_CHUNK, n_chp - c0);
-      __syncthreads();
-      const double *src = recs + (long long)RS * (c0 + (long long)n_chp * t);
-      for (int e = tid; e < nch * RS; e += SU_THREADS) srec[e] = src[e];
-      __syncthreads();
-
-      for (int s = 0; s < nch; ++s) {
-        const double *rec = srec + s * RS;
-        const double cx = rec[R_X], cy = rec[R_Y], cz = rec[R_Z], mrs = rec[R_MRS];
-        const int lam0 = (int)rec[R_LAM0];
-        double dx[SU_PPT], dy[SU_PPT], dz[SU_PPT], d2[SU_PPT];
-        int lam[SU_PPT], br[SU_PPT];  // br: 0 skip, 1 near, 2 far
+  for (int j = 0; j < N; ++j)
+    if (live[j]) {
+      const double p[3] = {px[j], py[j], pz[j]};
 #pragma unroll
-        for (int j = 0; j < SU_PPT; ++j) {
-          dx[j] = sub_rn(px[j], cx);
-          dy[j] = sub_rn(py[j], cy);
-          dz[j] = sub_rn(pz[j], cz);
-          d2[j] = add_rn(add_rn(mul_rn(dx[j], dx[j]), mul_rn(dy[j], dy[j])), mul_rn(dz[j], dz[j]));
-          int l = lam0;
-          while (rec[R_OPR + l] < d2[j] && l > 0) --l;
-          lam[j] = l;
-          br[j] = !valid[j] ? 0 : (d2[j] < mrs ? 1 : (d2[j] < 1e8 ? 2 : 0));
-        }
-        if (codes) {
-#pragma unroll
-          for (int j = 0; j < SU_PPT; ++j)
-            if (valid[j])
-              codes[vidx[j] + (long long)n_valid * ((c0 + s) + (long long)n_chp * t)] =
-                  (unsigned char)(br[j] == 1 ? 1 + lam[j] : (br[j] == 2 ? 16 + lam[j] : 0));
-        }
-
-        // far field
-        bool mine = true;
-#pragma unroll
-        for (int j = 0; j < SU_PPT; ++j) mine = mine && br[j] == 2 && lam[j] == lam[0];
-        const int lam_lane0 = __shfl_sync(FULL, lam[0], 0);  // every lane, before the vote
-        const bool all_far_same = __all_sync(FULL, mine && lam[0] == lam_lane0);
-        if (all_far_same) {
-          double ux[SU_PPT], uy[SU_PPT], uz[SU_PPT], P[SU_PPT], rinv[SU_PPT];
-#pragma unroll
-          for (int j = 0; j < SU_PPT; ++j) {
-            rinv[j] = rsqrt_nr(d2[j]);
-            const double ir2 = rinv[j] * rinv[j];
-            ux[j] = dx[j] * ir2;
-            uy[j] = dy[j] * ir2;
-            uz[j] = dz[j] * ir2;
-          }
-          kelvin_eval<SU_PPT>(lam[0], rec + CO, ux, uy, uz, P);
-#pragma unroll
-          for (int j = 0; j < SU_PPT; ++j) v[j] += P[j] * rinv[j];
-        } else {
-#pragma unroll
-          for (int j = 0; j < SU_PPT; ++j) {
-            bool pend = br[j] == 2;
-            while (__any_sync(FULL, pend)) {
-              const int sel = __reduce_max_sync(FULL, pend ? lam[j] : -1);
-              if (pend && lam[j] == sel) {
-                double ux[1], uy[1], uz[1], P[1];
-                const double ri = rsqrt_nr(d2[j]);
-                const double ir2 = ri * ri;
-                ux[0] = dx[j] * ir2;
-                uy[0] = dy[j] * ir2;
-                uz[0] = dz[j] * ir2;
-                kelvin_eval_1(sel, rec + CO, ux, uy, uz, P);
-                v[j] += P[0] * ri;
-                pend = false;
-              }
-            }
-          }
-        }
-        // near field (rare)
-#pragma unroll
-        for (int j = 0; j < SU_PPT; ++j) {
-          if (br[j] == 1) {
-            const long long atom = (long long)rec[R_ATOM];
-            const double *spl = spline + (long long)2 * L2 * n_hartree_grid * (atom + (long long)n_atoms * t);
-            v[j] += near_field(lam[j], L2, dx[j], dy[j], dz[j], d2[j], rec[R_RGM], rec[R_LINC], (int)rec[R_NGRID], spl);
-          }
-        }
+      for (int c = 0; c < 3; ++c) {
+        b.lo[c] = fmin(b.lo[c], p[c]);
+        b.hi[c] = fmax(b.hi[c], p[c]);
       }
     }
 #pragma unroll
-    for (int j = 0; j < SU_PPT; ++j)
-      if (valid[j]) dv[full[j] + (long long)n_full * t] = v[j];
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      b.lo[c] = fmin(b.lo[c], __shfl_xor_sync(0xffffffffu, b.lo[c], o));
+      b.hi[c] = fmax(b.hi[c], __shfl_xor_sync(0xffffffffu, b.hi[c], o));
+    }
+  return b;
+}
+
+// Bounds of the squared distance from (cx, cy, cz) to the box's points, widened
+// by 1e-12 (the exactly rounded d2 of a pair is within 1e-15 of the true one).
+__device__ __forceinline__ void box_distance(const Box &b, double cx, double cy, double cz, double *near2,
+                                             double *far2) {
+  const double c[3] = {cx, cy, cz};
+  double n2 = 0.0, f2 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double gap = fmax(fmax(b.lo[k] - c[k], c[k] - b.hi[k]), 0.0);
+    const double span = fmax(fabs(b.lo[k] - c[k]), fabs(c[k] - b.hi[k]));
+    n2 = fma(gap, gap, n2);
+    f2 = fma(span, span, f2);
   }
+  *near2 = n2 * (1.0 - 1e-12);
+  *far2 = f2 * (1.0 + 1e-12);
+}
+
+constexpr int CLS_SKIP = -1, CLS_MIXED = SU_LMAX + 1;  // 0..SU_LMAX: every point far with that l_atom_max
+
+// One record for one warp's box.
+__device__ __forceinline__ int classify(const Box &b, const double *rec) {
+  double n2, f2;
+  box_distance(b, rec[R_X], rec[R_Y], rec[R_Z], &n2, &f2);
+  const double mrs = rec[R_MRS];
+  if (n2 >= 1e8 || f2 < mrs) return CLS_SKIP;  // beyond the far field, or all near (the near-field launch's)
+  if (!(n2 >= mrs) || !(f2 < 1e8)) return CLS_MIXED;
+  // l_atom_max does not grow with the distance
+  const int l0 = (int)rec[R_LAM0], l = lam_at(rec + R_OPR, l0, n2);
+  return l == lam_at(rec + R_OPR, l0, f2) ? l : CLS_MIXED;
+}
+
+// Far field of PPT points per thread, blockIdx.y = perturbation.  A warp owns
+// 32 PPT neighbouring points of the plan's spatial order and one of `slices`
+// interleaved parts of the records (1, 2 or 4; the parts' sums are added in
+// order at the end), so a small point set still fills the chip.
+//
+// The bound is the FP64 pipe (83 multiply-adds of the polynomial at l = 6 and
+// 16 operations of geometry per pair) and the registers' read ports, which hold
+// a multiply-add of three distinct operands to two thirds of the pipe: see
+// gen_kelvin.py for the order that gets round it, which is why a thread takes
+// four points where there are enough.  Everything else is decided once per
+// (warp, record): lane s classifies record s of a chunk against the box of the
+// warp's points, and a record that is far with one l_atom_max for all of them
+// runs without a comparison or a vote (the rule is exact: bounds widened by more
+// than the rounding of d2).  A record whose radii the box straddles takes the
+// exact per-pair decisions and, if it is safe, one pass per 32 points at the
+// largest l_atom_max present in which a lane's higher degrees are multiplied by
+// zero (kelvin_masked_eval); an unsafe one takes a pass per l_atom_max.  (A box
+// per 32 points as well was slower: 7.9 ms below, and 6% on truncated radii.)
+// CODES: every record per pair, with the branch codes written.
+// Measured, 500 atoms, 2 million points, l_max 6: 9.4 ms (two points per thread,
+// decisions per pair, near field inside) -> 7.7 ms, 70% of the FP64 peak (two
+// points per thread 8.7 ms, in the compiler's order 9.0 ms).
+template <int PPT, bool CODES>
+__global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
+    sumup_far_kernel(int n_valid, int n_full, const int *__restrict__ order, const int *__restrict__ pfull,
+                     const double *__restrict__ pxyz, int n_chp, int L, const double *__restrict__ recs, int slices,
+                     double *__restrict__ dv, unsigned char *__restrict__ codes) {
+  const int RS = rec_stride(L), CO = rec_coef_off(L);
+  __shared__ __align__(16) double srec[2][SU_CHUNK * rec_stride(SU_LMAX)];
+  __shared__ double part[SU_THREADS / 32][32 * PPT];
+  __shared__ Box boxes[SU_THREADS / 32];  // read by the classification only: not worth registers
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.y;
+  const unsigned FULL = 0xffffffffu;
+  const int slice = warp & (slices - 1);
+  const int base = (blockIdx.x * (SU_THREADS / 32) / slices + warp / slices) * (32 * PPT);
+
+  int vidx[PPT], full[PPT];
+  double px[PPT], py[PPT], pz[PPT], v[PPT];
+  bool valid[PPT], live[PPT];
+#pragma unroll
+  for (int j = 0; j < PPT; ++j) {
+    const int slot = base + j * 32 + lane;
+    valid[j] = slot < n_valid;
+    vidx[j] = CODES && valid[j] ? order[slot] : 0;
+    full[j] = valid[j] ? pfull[slot] : 0;
+    px[j] = valid[j] ? pxyz[slot] : 0.0;
+    py[j] = valid[j] ? pxyz[slot + (long long)n_valid] : 0.0;
+    pz[j] = valid[j] ? pxyz[slot + 2LL * n_valid] : 0.0;
+    live[j] = valid[j] && isfinite(px[j]) && isfinite(py[j]) && isfinite(pz[j]);
+    v[j] = 0.0;
+  }
+  {
+    const Box b = warp_box<PPT>(px, py, pz, live);
+    if (lane == 0) boxes[warp] = b;
+    __syncwarp();
+  }
+  bool any_live = false;
+#pragma unroll
+  for (int j = 0; j < PPT; ++j) any_live = any_live || live[j];
+  const bool work = CODES || __any_sync(FULL, any_live);
+
+  const double *src = recs + (long long)RS * n_chp * t;
+  auto load = [&](int c0, int buf) {  // records c0.. of this perturbation (RS is even: 16-byte copies)
+    const int n = min(SU_CHUNK, n_chp - c0) * RS / 2;
+    const double *from = src + (long long)RS * c0;
+    for (int e = tid; e < n; e += SU_THREADS) cp_async_16(&srec[buf][2 * e], from + 2 * e, 16);
+    cp_async_commit();
+  };
+  load(0, 0);
+  for (int c0 = 0, buf = 0; c0 < n_chp; c0 += SU_CHUNK, buf ^= 1) {
+    const int nch = min(SU_CHUNK, n_chp - c0);
+    cp_async_wait<0>();
+    __syncthreads();  // this chunk is there; every warp is done with the other buffer
+    if (c0 + SU_CHUNK < n_chp) load(c0 + SU_CHUNK, buf ^ 1);
+    if (!work) continue;
+    const double *chunk = srec[buf];
+    int cls_mine = CLS_MIXED;
+    if (!CODES) cls_mine = lane < nch ? classify(boxes[warp], chunk + lane * RS) : CLS_SKIP;
+    for (int s = slice; s < nch; s += slices) {
+      const double *rec = chunk + s * RS;
+      const int cls = CODES ? CLS_MIXED : __shfl_sync(FULL, cls_mine, s);
+      if (cls == CLS_SKIP) continue;
+      const double cx = rec[R_X], cy = rec[R_Y], cz = rec[R_Z];
+      if (cls < CLS_MIXED) {
+        double ux[PPT], uy[PPT], uz[PPT], P[PPT], rinv[PPT];
+#pragma unroll
+        for (int j = 0; j < PPT; ++j) {
+          const double dx = px[j] - cx, dy = py[j] - cy, dz = pz[j] - cz;
+          rinv[j] = rsqrt_refined(fma(dz, dz, fma(dy, dy, dx * dx)));
+          const double ir2 = rinv[j] * rinv[j];
+          ux[j] = dx * ir2;
+          uy[j] = dy * ir2;
+          uz[j] = dz * ir2;
+        }
+        kelvin_eval<PPT>(cls, rec + CO, ux, uy, uz, P);
+#pragma unroll
+        for (int j = 0; j < PPT; ++j) v[j] = fma(P[j], rinv[j], v[j]);
+        continue;
+      }
+      const double mrs = rec[R_MRS];
+      const int lam0 = (int)rec[R_LAM0];
+      const bool safe = rec[R_SAFE] != 0.0;
+#pragma unroll 1
+      for (int j = 0; j < PPT; ++j) {  // one body for all points: selects instead of indexed registers
+        double x = px[0], y = py[0], z = pz[0];
+        bool val = valid[0];
+        int vi = vidx[0];
+#pragma unroll
+        for (int i = 1; i < PPT; ++i)
+          if (j == i) {
+            x = px[i];
+            y = py[i];
+            z = pz[i];
+            val = valid[i];
+            vi = vidx[i];
+          }
+        const double dx = sub_rn(x, cx), dy = sub_rn(y, cy), dz = sub_rn(z, cz);
+        const double d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+        const int lam = lam_at(rec + R_OPR, lam0, d2);
+        const bool is_near = val && d2 < mrs, is_far = val && !is_near && d2 < 1e8;
+        if (CODES && val)
+          codes[vi + (long long)n_valid * ((c0 + s) + (long long)n_chp * t)] =
+              (unsigned char)(is_near ? 1 + lam : (is_far ? 16 + lam : 0));
+        const double ri = is_far ? rsqrt_refined(d2) : 0.0;
+        const double ir2 = ri * ri;
+        const double ux = is_far ? dx * ir2 : 0.0, uy = is_far ? dy * ir2 : 0.0, uz = is_far ? dz * ir2 : 0.0;
+        double P = 0.0, sum = 0.0;
+        bool pend = is_far;
+        while (__any_sync(FULL, pend)) {
+          const int top = __reduce_max_sync(FULL, pend ? lam : -1);
+          kelvin_masked_eval(top, rec + CO, &ux, &uy, &uz, min(lam, top), &P);
+          if (pend && (safe || lam == top)) {
+            sum = P * ri;
+            pend = false;
+          }
+        }
+        if (is_far) {
+#pragma unroll
+          for (int i = 0; i < PPT; ++i)
+            if (j == i) v[i] += sum;
+        }
+      }
+    }
+  }
+  if (slices > 1) {
+#pragma unroll
+    for (int j = 0; j < PPT; ++j) part[warp][j * 32 + lane] = v[j];
+    __syncthreads();
+    if (slice != 0) return;
+#pragma unroll
+    for (int j = 0; j < PPT; ++j)
+      for (int k = 1; k < slices; ++k) v[j] += part[warp + k][j * 32 + lane];
+  }
+#pragma unroll
+  for (int j = 0; j < PPT; ++j)
+    if (live[j]) dv[full[j] + (long long)n_full * t] += v[j];
+}
+
+// -------------------------------------------------- near-field kernel ---
+
+constexpr int NF_THREADS = 128;
+constexpr int NF_MAX_SLICES = 8;  // warps that may share 32 points
+constexpr int NF_PAIRS = 32;      // pairs evaluated together, one per lane
+
+struct NearWarp {
+  double x[NF_PAIRS], y[NF_PAIRS], z[NF_PAIRS];  // unit vectors
+  double h[NF_PAIRS][4];                         // Hermite weights
+  const double *run[NF_PAIRS];                   // the 4 (L + 1)^2 spline values of the interval
+  double val[NF_PAIRS];
+  int lam[NF_PAIRS];
+  int owner[2 * NF_PAIRS], slot[2 * NF_PAIRS];  // pairs found: lane of the point, centre slot
+  unsigned touched;
+};
+
+// Near field of 32 neighbouring points per warp, blockIdx.y = perturbation.  The
+// lanes test the centres against the box of the points, 32 at a time; only the
+// few that can be near are looked at per point (exact d2), and the near pairs go
+// to a queue that is evaluated 32 pairs at a time, so that sparse hits cost no
+// more than dense ones.  The geometry (square roots, divisions, a logarithm)
+// takes one lane per pair; the sum over (l, m) eight lanes, lane m the orders +-m
+// (lane 0 also +-8): for every l their loads are one contiguous stretch of the
+// pair's run of 4 (L + 1)^2 values and none waits for the recursion.
+// What bounds it is L1 (85% busy): a pair reads 1.6 KB of spline (l_max 6).  Whole
+// warps along a run, with the harmonics in shared memory, had fewer L1 lookups but
+// were slower (1.57 ms against 0.94 ms on 2 million points, 500 atoms).  Where the
+// points are few, 2 to 8 warps share 32 points and take the candidate centres in
+// turn (2,000 points, 20 atoms: 76 us with one).  Every sum has a fixed order.
+template <int L>
+__global__ void __launch_bounds__(32 * NF_MAX_SLICES)
+    sumup_near_kernel(int n_valid, int n_full, const int *__restrict__ pfull, const double *__restrict__ pxyz,
+                      int n_chp, int n_atoms, int n_hartree_grid, int slices,
+                      const double *__restrict__ recs, const double4 *__restrict__ heads,
+                      const double *__restrict__ spline, double *__restrict__ dv) {
+  constexpr int RS = rec_stride(L), L2 = (L + 1) * (L + 1);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double s_ra[L2], s_rb[L2], s_k[L2];  // (l, m) at l (L + 1) + m
+  const unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.y;
+  NearWarp &W = reinterpret_cast<NearWarp *>(smem_raw)[warp];
+  for (int e = tid; e < L2; e += blockDim.x) {
+    const int l = e / (L + 1), m = e % (L + 1);
+    s_k[e] = d_near_tables[0][l][m];
+    s_ra[e] = d_near_tables[1][l][m];
+    s_rb[e] = d_near_tables[2][l][m];
+  }
+  __syncthreads();
+  const int slice = warp & (slices - 1);
+  const int pt = ((blockIdx.x * (blockDim.x >> 5) + warp) / slices) * 32 + lane;
+  const bool valid = pt < n_valid;
+  const int full = valid ? pfull[pt] : 0;
+  const double px = valid ? pxyz[pt] : 0.0, py = valid ? pxyz[pt + (long long)n_valid] : 0.0,
+               pz = valid ? pxyz[pt + 2LL * n_valid] : 0.0;
+  const bool live = valid && isfinite(px) && isfinite(py) && isfinite(pz);
+  const Box box = warp_box<1>(&px, &py, &pz, &live);
+  const int m8 = lane & 7, grp = lane >> 3;
+  double v = 0.0;
+  bool touched = false;
+
+  auto evaluate = [&](int n) {  // the first n (<= 32) pairs of the queue
+    __syncwarp();
+    {
+      const bool has = lane < n;
+      const int o = has ? W.owner[lane] : lane;
+      const double x = __shfl_sync(FULL, px, o), y = __shfl_sync(FULL, py, o), z = __shfl_sync(FULL, pz, o);
+      if (has) {
+        const double *rec = recs + (long long)RS * (W.slot[lane] + (long long)n_chp * t);
+        const double dx = sub_rn(x, rec[R_X]), dy = sub_rn(y, rec[R_Y]), dz = sub_rn(z, rec[R_Z]);
+        const double d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+        const NearGeom G = near_geometry(dx, dy, dz, d2, rec[R_RGM], rec[R_LINC], (int)rec[R_NGRID]);
+        W.x[lane] = G.x;
+        W.y[lane] = G.y;
+        W.z[lane] = G.z;
+        W.h[lane][0] = G.ta;
+        W.h[lane][1] = G.tb;
+        W.h[lane][2] = G.tc;
+        W.h[lane][3] = G.td;
+        W.lam[lane] = lam_at(rec + R_OPR, (int)rec[R_LAM0], d2);
+        W.run[lane] = spline + (long long)2 * L2 *
+                                   (n_hartree_grid * ((long long)rec[R_ATOM] + (long long)n_atoms * t) + G.i_spl - 1);
+      }
+    }
+    __syncwarp();
+    for (int k0 = 0; k0 < n; k0 += 4) {
+      const int k = k0 + grp;
+      double acc = 0.0;
+      if (k < n) {
+        const double *run = W.run[k];
+        const double z = W.z[k], ta = W.h[k][0], tb = W.h[k][1], tc = W.h[k][2], td = W.h[k][3];
+        const int lam = W.lam[k];
+        auto S = [&](int i) {
+          return __ldg(run + i) * ta + __ldg(run + i + L2) * tb + __ldg(run + i + 2 * L2) * tc +
+                 __ldg(run + i + 3 * L2) * td;
+        };
+        // (x + i y)^m8 and ^8 by squaring
+        double C = 1.0, Sn = 0.0, bc = W.x[k], bs = W.y[k];
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1) {
+          if (m8 & bit) {
+            const double c2 = C * bc - Sn * bs;
+            Sn = C * bs + Sn * bc;
+            C = c2;
+          }
+          const double b2 = bc * bc - bs * bs;
+          bs = 2.0 * bc * bs;
+          bc = b2;
+        }
+        if (m8 & 1) C = -C;  // the cosine terms carry (-1)^m
+        double q = 0.0, q1 = 0.0;
+#pragma unroll
+        for (int l = 0; l <= L; ++l) {
+          if (m8 <= l && l <= lam) {
+            const int e = l * (L + 1) + m8;
+            const double qn = l == m8 ? c_DF[m8] : s_ra[e] * z * q - s_rb[e] * q1;
+            q1 = q;
+            q = qn;
+            double term = C * S(l * l + l + m8);
+            if (m8 > 0) term += Sn * S(l * l + l - m8);
+            acc += s_k[e] * q * term;
+          }
+        }
+        if (L >= 8 && m8 == 0 && lam >= 8) acc += c_K[8][8] * c_DF[8] * (bc * S(80) + bs * S(64));
+      }
+#pragma unroll
+      for (int o = 4; o; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+      if (m8 == 0 && k < n) W.val[k] = acc;
+    }
+    __syncwarp();
+    for (int k = 0; k < n; ++k)
+      if (W.owner[k] == lane) {
+        v += W.val[k];
+        touched = true;
+      }
+    __syncwarp();
+  };
+
+  int queued = 0, seen = 0;
+  for (int c0 = 0; c0 < n_chp; c0 += 32) {
+    bool cand = false;
+    if (c0 + lane < n_chp) {
+      const double4 h = heads[c0 + lane + (long long)n_chp * t];
+      double n2, f2;
+      box_distance(box, h.x, h.y, h.z, &n2, &f2);
+      cand = n2 < h.w;
+    }
+    for (unsigned todo = __ballot_sync(FULL, cand); todo; todo &= todo - 1) {
+      if ((seen++ & (slices - 1)) != slice) continue;
+      const int s = c0 + __ffs(todo) - 1;
+      const double4 h = heads[s + (long long)n_chp * t];
+      const double dx = sub_rn(px, h.x), dy = sub_rn(py, h.y), dz = sub_rn(pz, h.z);
+      const double d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+      const bool is_near = valid && d2 < h.w;
+      const unsigned nm = __ballot_sync(FULL, is_near);
+      if (is_near) {
+        const int at = queued + __popc(nm & ((1u << lane) - 1));
+        W.owner[at] = lane;
+        W.slot[at] = s;
+      }
+      queued += __popc(nm);
+      if (queued >= NF_PAIRS) {
+        evaluate(NF_PAIRS);
+        queued -= NF_PAIRS;
+        if (lane < queued) {  // the rest moves up
+          W.owner[lane] = W.owner[NF_PAIRS + lane];
+          W.slot[lane] = W.slot[NF_PAIRS + lane];
+        }
+      }
+    }
+  }
+  if (queued > 0) evaluate(queued);
+  if (slices > 1) {
+    W.val[lane] = v;
+    const unsigned any = __ballot_sync(FULL, touched);
+    if (lane == 0) W.touched = any;
+    __syncthreads();
+    if (slice != 0) return;
+    for (int k = 1; k < slices; ++k) {
+      const NearWarp &O = reinterpret_cast<NearWarp *>(smem_raw)[warp + k];
+      if (O.touched >> lane & 1) {
+        v += O.val[lane];
+        touched = true;
+      }
+    }
+  }
+  if (touched) dv[full + (long long)n_full * t] += v;
 }
 
 // ------------------------------------------------------ generic kernel ---
@@ -449,201 +811,294 @@ __global__ void __launch_bounds__(SU_THREADS)
   }
 }
 
-int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *dv, unsigned char *codes,
-                cudaStream_t stream) {
-  const int per_block = SU_THREADS * SU_PPT;
-  const int grid = (P.n_valid_points + per_block - 1) / per_block;
-  sumup_fast_kernel<<<grid, SU_THREADS, 0, stream>>>(P.n_valid_points, P.n_full_points, P.d_map, P.d_order,
-                                                     P.d_coord,
-                                                     n_active, P.n_chp, P.n_atoms, P.L, P.n_hartree_grid, P.d_recs,
-                                                     spline, dv, codes);
+int launch_prep(const SumupPlan &P, int n_active, const int *lhmfd, const double *mrs, const double *opr,
+                const double *Q, cudaStream_t stream) {
+  sumup_prep_kernel<<<dim3(std::max(P.n_chp, P.n_atoms), n_active), 128, 0, stream>>>(
+      P.L, P.lma, P.n_atoms, P.n_chp, P.n_coef, P.rs, P.d_chp, P.d_c2a, P.d_species, P.d_species_center,
+      P.d_l_hartree, P.d_n_grid, P.d_rgm, P.d_linc, P.d_cc_xyz, mrs, opr, lhmfd, Q, P.d_slot, P.d_conv_ptr,
+      P.d_conv_lm, P.d_conv_fc, P.d_recs, P.d_heads, P.d_err);
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
+}
+
+int launch_near(const SumupPlan &P, int n_active, const double *spline, double *dv, cudaStream_t stream) {
+  int n_sm = 148;
+  FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, P.device));
+  const int groups = ceil_div(P.n_valid_points, 32);
+  // candidate centres split over up to 8 warps until the warps fill the chip (16 per SM)
+  int slices = 1, threads = NF_THREADS;
+  while ((long long)groups * n_active * slices < 16LL * n_sm && slices < NF_MAX_SLICES) slices *= 2;
+  if (32 * slices > threads) threads = 32 * slices;
+  const dim3 grid(ceil_div(groups, threads / 32 / slices), n_active);
+  const size_t smem = (threads / 32) * sizeof(NearWarp);
+  switch (P.L) {
+#define FRPA_NEAR_CASE(LL)                                                                                           \
+  case LL:                                                                                                           \
+    sumup_near_kernel<LL><<<grid, threads, smem, stream>>>(P.n_valid_points, P.n_full_points, P.d_pfull, P.d_pxyz,    \
+                                                           P.n_chp, P.n_atoms, P.n_hartree_grid, slices, P.d_recs,   \
+                                                           P.d_heads, spline, dv);                                   \
+    break;
+    FRPA_NEAR_CASE(0) FRPA_NEAR_CASE(1) FRPA_NEAR_CASE(2) FRPA_NEAR_CASE(3) FRPA_NEAR_CASE(4)
+    FRPA_NEAR_CASE(5) FRPA_NEAR_CASE(6) FRPA_NEAR_CASE(7) FRPA_NEAR_CASE(8)
+#undef FRPA_NEAR_CASE
+    default:
+      return fail(FRPA_ERR_UNSUPPORTED, "sum-up: l_pot_max %d above %d", P.L, SU_LMAX);
+  }
+  FRPA_LAUNCH_CHECK();
+  return FRPA_OK;
+}
+
+template <int PPT, bool CODES>
+int launch_far(const SumupPlan &P, int n_active, int slices, double *dv, unsigned char *codes, cudaStream_t stream) {
+  const int groups = SU_THREADS / 32 / slices;  // point groups per CTA
+  const dim3 grid(ceil_div(ceil_div(P.n_valid_points, 32 * PPT), groups), n_active);
+  sumup_far_kernel<PPT, CODES><<<grid, SU_THREADS, 0, stream>>>(P.n_valid_points, P.n_full_points, P.d_order,
+                                                                P.d_pfull, P.d_pxyz, P.n_chp, P.L, P.d_recs, slices, dv, codes);
+  FRPA_LAUNCH_CHECK();
+  return FRPA_OK;
+}
+
+int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *dv, unsigned char *codes,
+                cudaStream_t stream) {
+  if (codes) {
+    FRPA_TRY((launch_far<2, true>(P, n_active, 1, dv, codes, stream)));
+    return launch_near(P, n_active, spline, dv, stream);
+  }
+  int n_sm = 148;
+  FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, P.device));
+  // four points per thread share every coefficient load; the fewer warps that
+  // leaves, the more the records are split (over 2, then 4 warps), then the
+  // fewer points a thread takes, until the warps fill the chip twice (16 per SM)
+  const long long want = 2LL * 16 * n_sm;
+  int ppt = 4, slices = 1;
+  auto warps = [&] { return (long long)ceil_div(P.n_valid_points, 32 * ppt) * n_active * slices; };
+  while (warps() < want && slices < 4 && P.n_chp >= 4 * slices) slices *= 2;
+  while (warps() < want && ppt > 1) ppt /= 2;
+  if (ppt == 4)
+    FRPA_TRY((launch_far<4, false>(P, n_active, slices, dv, nullptr, stream)));
+  else if (ppt == 2)
+    FRPA_TRY((launch_far<2, false>(P, n_active, slices, dv, nullptr, stream)));
+  else
+    FRPA_TRY((launch_far<1, false>(P, n_active, slices, dv, nullptr, stream)));
+  return launch_near(P, n_active, spline, dv, stream);
 }
 
 
 // -------------------------------------------------------- adjoint (dQ) ---
 
-constexpr int ADJ_KCH = 32;
-
-// Exponents (a, b, c) of coefficient slot k in the degree-graded packing
-// (the inverse of kelvin_index), for compile-time use.
-struct Abc {
-  int a, b, c;
+// The coefficients with x exponent in [A0, A1) for degrees <= L: how many, and
+// the position of (a, b, c) among them.
+template <int L, int A0, int A1>
+struct CoefRange {
+  static constexpr int before(int a) {  // coefficients with x exponent in [A0, a)
+    int n = 0;
+    for (int q = A0; q < a; ++q) n += (L - q + 1) * (L - q + 2) / 2;
+    return n;
+  }
+  static constexpr int count = before(A1);
+  static constexpr int index(int a, int b, int c) {
+    int n = before(a);
+    for (int q = 0; q < b; ++q) n += L - a - q + 1;
+    return n + c;
+  }
 };
-__host__ __device__ constexpr Abc kelvin_abc(int k) {
-  int d = 0;
-  while ((d + 1) * (d + 2) * (d + 3) / 6 <= k) ++d;
-  int r = k - d * (d + 1) * (d + 2) / 6, a = 0;
-  while (r >= d + 1 - a) {
-    r -= d + 1 - a;
-    ++a;
-  }
-  return Abc{a, r, d - a - r};
-}
-__host__ __device__ constexpr bool kelvin_abc_inverts_index() {
-  for (int k = 0; k < kelvin_count(SU_LMAX); ++k) {
-    const Abc m = kelvin_abc(k);
-    if (kelvin_index(m.a, m.b, m.c) != k) return false;
-  }
-  return true;
-}
-static_assert(kelvin_abc_inverts_index(), "kelvin_abc is the inverse of kelvin_index");
 
-// acc[I] += w ux^a uy^b uz^c for the chunk's slots K0 + I of degree <= lam
-// (exponents are compile-time constants: the power arrays stay in registers)
-template <int L, int K0, int... I>
-__device__ __forceinline__ void dcoef_terms(std::integer_sequence<int, I...>, double *acc, double w, const double *pa,
-                                            const double *pb, const double *pc, int lam) {
-  auto term = [&](auto ic) {
-    constexpr int k = K0 + decltype(ic)::value;
-    if constexpr (k < kelvin_count(L)) {
-      constexpr Abc m = kelvin_abc(k);
-      if (m.a + m.b + m.c <= lam) acc[decltype(ic)::value] += w * pa[m.a] * pb[m.b] * pc[m.c];
+// acc(a, b, c) += w x^a y^b z^c for the range's coefficients of degree <= LAM
+template <int L, int A0, int A1, int LAM>
+__device__ __forceinline__ void dcoef_add(double *acc, double w, double x, double y, const double *zp) {
+  using R = CoefRange<L, A0, A1>;
+  double wa = w;
+#pragma unroll
+  for (int a = 0; a < A1 && a <= LAM; ++a) {
+    if (a >= A0) {
+      double wab = wa;
+#pragma unroll
+      for (int b = 0; a + b <= LAM; ++b) {
+#pragma unroll
+        for (int c = 0; a + b + c <= LAM; ++c) acc[R::index(a, b, c)] = fma(wab, zp[c], acc[R::index(a, b, c)]);
+        wab *= y;
+      }
     }
-  };
-  (term(std::integral_constant<int, I>{}), ...);
+    wa *= x;
+  }
 }
 
-// One chunk of ADJ_KCH coefficient slots starting at K0: every point of the
-// block once, then the block's partial sums (warp shuffles, then the warps in
-// order) to part[k, slot, t, z].
-template <int L, int K0>
-__device__ __forceinline__ void dcoef_chunk(int n_full, const int *__restrict__ map,
-                                            const double *__restrict__ coord, const double *__restrict__ rec,
-                                            const double *__restrict__ g, int t, int p_begin, int p_end,
-                                            double (&red)[SU_THREADS / 32][ADJ_KCH], double *__restrict__ part) {
+template <int L, int A0, int A1, int... LAM>
+__device__ __forceinline__ void dcoef_switch(std::integer_sequence<int, LAM...>, int lam, double *acc, double w,
+                                             double x, double y, const double *zp) {
+  ((lam == LAM ? dcoef_add<L, A0, A1, LAM>(acc, w, x, y, zp) : (void)0), ...);
+}
+
+// One pass over a block's points for the coefficients with x exponent in
+// [A0, A1): each thread adds its points in registers, then the block's sums go
+// to part[] (recursive halving over the lanes, the warps in order).
+template <int L, int A0, int A1>
+__device__ __forceinline__ void dcoef_pass(int n_valid, const int *__restrict__ pfull,
+                                           const double *__restrict__ pxyz, const double *__restrict__ rec,
+                                           const double *__restrict__ gt, int p_begin, int p_end, double *red,
+                                           double *__restrict__ part) {
+  using R = CoefRange<L, A0, A1>;
+  constexpr int N = R::count, NP = (N + 31) / 32 * 32;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double cx = rec[R_X], cy = rec[R_Y], cz = rec[R_Z], mrs = rec[R_MRS];
   const int lam0 = (int)rec[R_LAM0];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double acc[ADJ_KCH];
+  double acc[NP];
 #pragma unroll
-  for (int kk = 0; kk < ADJ_KCH; ++kk) acc[kk] = 0.0;
-  for (int iv = p_begin + threadIdx.x; iv < p_end; iv += SU_THREADS) {
-    const int f = map[iv];
-    const double dx = sub_rn(coord[3LL * f], cx), dy = sub_rn(coord[3LL * f + 1], cy),
-                 dz = sub_rn(coord[3LL * f + 2], cz);
+  for (int k = 0; k < NP; ++k) acc[k] = 0.0;
+  // a point's loads are issued one turn ahead, its full index two turns
+  struct Point {
+    double x, y, z, g;
+  };
+  const int first = p_begin + warp * 32 + lane;
+  auto index = [&](int iv) { return iv < p_end ? __ldg(pfull + iv) : 0; };
+  auto fetch = [&](int iv, int f) {
+    Point P{0.0, 0.0, 0.0, 0.0};
+    if (iv < p_end) {
+      P.x = __ldg(pxyz + iv);
+      P.y = __ldg(pxyz + iv + (long long)n_valid);
+      P.z = __ldg(pxyz + iv + 2LL * n_valid);
+      P.g = __ldg(gt + f);
+    }
+    return P;
+  };
+  Point next = fetch(first, index(first));
+  int f_next = index(first + SU_THREADS);
+  for (int iv = first; iv - lane < p_end; iv += SU_THREADS) {
+    const bool in = iv < p_end;
+    const Point P = next;
+    next = fetch(iv + SU_THREADS, f_next);
+    f_next = index(iv + 2 * SU_THREADS);
+    const double dx = sub_rn(P.x, cx), dy = sub_rn(P.y, cy), dz = sub_rn(P.z, cz);
     const double d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
-    if (d2 < mrs || !(d2 < 1e8)) continue;
-    int lam = lam0;
-    while (rec[R_OPR + lam] < d2 && lam > 0) --lam;
-    const double ri = rsqrt(d2), ir2 = ri * ri;
+    const bool is_far = in && !(d2 < mrs) && d2 < 1e8;
+    unsigned todo = __ballot_sync(FULL, is_far);
+    if (!todo) continue;
+    const int lam = lam_at(rec + R_OPR, lam0, d2);
+    const double ri = is_far ? rsqrt_refined(d2) : 0.0, ir2 = ri * ri;
+    const double gw = is_far ? P.g * ri : 0.0;
     const double ux = dx * ir2, uy = dy * ir2, uz = dz * ir2;
-    double pa[L + 1], pb[L + 1], pc[L + 1];
-    pa[0] = pb[0] = pc[0] = 1.0;
+    // neighbouring points mostly share l_atom_max; each value present is one
+    // pass, the other lanes adding zeros
+    while (todo) {
+      const int sel = __shfl_sync(FULL, lam, __ffs(todo) - 1);
+      const bool mine = is_far && lam == sel;
+      todo &= ~__ballot_sync(FULL, mine);
+      const double z = mine ? uz : 0.0;
+      double zp[L + 1];
+      zp[0] = 1.0;
 #pragma unroll
-    for (int e = 1; e <= L; ++e) {
-      pa[e] = pa[e - 1] * ux;
-      pb[e] = pb[e - 1] * uy;
-      pc[e] = pc[e - 1] * uz;
+      for (int e = 1; e <= L; ++e) zp[e] = zp[e - 1] * z;
+      dcoef_switch<L, A0, A1>(std::make_integer_sequence<int, L + 1>{}, sel, acc, mine ? gw : 0.0, mine ? ux : 0.0,
+                              mine ? uy : 0.0, zp);
     }
-    const double w = g[f + (long long)n_full * t] * ri;
-    dcoef_terms<L, K0>(std::make_integer_sequence<int, ADJ_KCH>{}, acc, w, pa, pb, pc, lam);
   }
 #pragma unroll
-  for (int kk = 0; kk < ADJ_KCH; ++kk) {
-    double v = acc[kk];
+  for (int k0 = 0; k0 < NP; k0 += 32) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane == 0) red[warp][kk] = v;
+    for (int o = 16; o; o >>= 1) {
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const double keep = upper ? acc[k0 + i + o] : acc[k0 + i], give = upper ? acc[k0 + i] : acc[k0 + i + o];
+        acc[k0 + i] = keep + __shfl_xor_sync(FULL, give, o);
+      }
+    }
+    red[warp * NP + k0 + lane] = acc[k0];  // lane holds coefficient k0 + lane
   }
   __syncthreads();
-  constexpr int NK = kelvin_count(L);
-  if (threadIdx.x < ADJ_KCH && K0 + (int)threadIdx.x < NK) {
+  for (int k = threadIdx.x; k < N; k += SU_THREADS) {
     double v = 0.0;
-    for (int w = 0; w < SU_THREADS / 32; ++w) v += red[w][threadIdx.x];
-    part[K0 + threadIdx.x] = v;  // this point block's partial, summed over the blocks in order later
+    for (int w = 0; w < SU_THREADS / 32; ++w) v += red[w * NP + k];
+    part[CoefRange<L, 0, L + 1>::before(A0) + k] = v;
   }
   __syncthreads();
 }
 
-template <int L, int... C>
-__device__ __forceinline__ void dcoef_chunks(std::integer_sequence<int, C...>, int n_full, const int *map,
-                                             const double *coord, const double *rec, const double *g, int t,
-                                             int p_begin, int p_end, double (&red)[SU_THREADS / 32][ADJ_KCH],
-                                             double *part) {
-  (dcoef_chunk<L, C * ADJ_KCH>(n_full, map, coord, rec, g, t, p_begin, p_end, red, part), ...);
-}
+// x exponents of the second pass on: one pass up to l_max 6 (84 sums in
+// registers), two above (64 + 56 and 81 + 84)
+__host__ __device__ constexpr int dcoef_split(int L) { return L <= 6 ? L + 1 : 2; }
 
-// part[k, slot, t, z] = sum over point block z's points of g(p, t) u^k / r
-// for far-field pairs with deg(k) <= lam (the derivative of the fast path's
-// Horner sum with respect to its coefficients), one instance per l_max; each
-// block sums its points in a fixed order, and sumup_dcoef_reduce_kernel adds
-// the blocks in order, so the result is the same on every run.
+// part[z, t, slot, (a, b, c)] = sum over point block z of g(p, t) u^(a,b,c) / r
+// over the far-field pairs whose l_atom_max reaches the degree (the derivative of
+// the far field's polynomial with respect to its coefficients), in a fixed order.
+// The bound is the FP64 pipe: a multiply-add per coefficient, a multiplication per
+// (a, b) and the geometry, about 140 operations a pair at l_max 6 (the first form
+// walked the points once per 32 coefficients, with two multiplications and a
+// multiply-add each: 1.05 ms on 100 atoms and 200,000 points, now 0.37 ms).
 template <int L>
-__global__ void __launch_bounds__(SU_THREADS)
-    sumup_dcoef_kernel(int n_valid, int n_full, const int *__restrict__ map, const double *__restrict__ coord,
+__global__ void __launch_bounds__(SU_THREADS, 2)
+    sumup_dcoef_kernel(int n_valid, int n_full, const int *__restrict__ pfull, const double *__restrict__ pxyz,
                        int n_chp, const double *__restrict__ recs, const double *__restrict__ g, int pts_per_block,
-                       double *__restrict__ dcoef) {
-  constexpr int NK = kelvin_count(L), NCH = (NK + ADJ_KCH - 1) / ADJ_KCH;
-  __shared__ double red[SU_THREADS / 32][ADJ_KCH];
+                       double *__restrict__ part) {
+  constexpr int NK = kelvin_count(L), A1 = dcoef_split(L);
+  __shared__ double red[SU_THREADS / 32 * 96];
   const int slot = blockIdx.x, t = blockIdx.y;
-  const int p_begin = blockIdx.z * pts_per_block;
-  const int p_end = min(n_valid, p_begin + pts_per_block);
+  const int p_begin = blockIdx.z * pts_per_block, p_end = min(n_valid, p_begin + pts_per_block);
   const double *rec = recs + (long long)rec_stride(L) * (slot + (long long)n_chp * t);
-  double *part = dcoef + (long long)NK * (slot + (long long)n_chp * (t + (long long)gridDim.y * blockIdx.z));
-  dcoef_chunks<L>(std::make_integer_sequence<int, NCH>{}, n_full, map, coord, rec, g, t, p_begin, p_end, red, part);
+  double *out = part + (long long)NK * (slot + (long long)n_chp * (t + (long long)gridDim.y * blockIdx.z));
+  const double *gt = g + (long long)n_full * t;
+  dcoef_pass<L, 0, A1>(n_valid, pfull, pxyz, rec, gt, p_begin, p_end, red, out);
+  if constexpr (A1 <= L)
+    dcoef_pass<L, A1, L + 1>(n_valid, pfull, pxyz, rec, gt, p_begin, p_end, red, out);
 }
 
-// dcoef[k, slot, t] = sum over the point blocks z, in order, of part[k, slot, t, z]
-__global__ void sumup_dcoef_reduce_kernel(long long n, int nz, const double *__restrict__ part,
-                                          double *__restrict__ dcoef) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int z = 0; z < nz; ++z) s += part[e + n * z];
-    dcoef[e] = s;
+// dQ of one atom and perturbation: its slots' coefficient gradients (point blocks
+// in order, then slots), back through the Kelvin conversion and cc to (l, m),
+// where the forward kept the moment (l <= l_hartree_max_far_distance,
+// |Q| > 1e-10).  A warp per (l, m), lanes over its table rows.  Perturbations
+// past n_active get zeros.
+__global__ void __launch_bounds__(256)
+    sumup_dq_kernel(int n_atoms, int L, int n_chp, int n_coef, int n_active, int nz, const int *__restrict__ slot_ptr,
+                    const int *__restrict__ slots, const int *__restrict__ lm_ptr, const int *__restrict__ lm_row,
+                    const int *__restrict__ convT_ptr, const int *__restrict__ convT_k,
+                    const double *__restrict__ convT_f, const double *__restrict__ cc, const int *__restrict__ lhmfd,
+                    const double *__restrict__ Q, const double *__restrict__ part, double *__restrict__ dQ) {
+  __shared__ double dc[(SU_LMAX + 1) * (SU_LMAX + 2) * (SU_LMAX + 3) / 6];
+  const int a = blockIdx.x, t = blockIdx.y, L2 = (L + 1) * (L + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double *out = dQ + (long long)L2 * (a + (long long)n_atoms * t);
+  if (t >= n_active) {
+    for (int lm = threadIdx.x; lm < L2; lm += blockDim.x) out[lm] = 0.0;
+    return;
   }
-}
-
-// dmc[n, atom, t] = sum over the atom's slots, in ascending order, of
-// sum_k conv[k, n] dcoef[k, slot, t] (a gather: no two threads add into one
-// entry, so the result is the same on every run)
-__global__ void sumup_dmc_kernel(int n_chp, int n_atoms, int mc_dim, int n_coef, const int *__restrict__ slot_ptr,
-                                 const int *__restrict__ slots, const int *__restrict__ convT_ptr,
-                                 const int *__restrict__ convT_k, const double *__restrict__ convT_f,
-                                 const double *__restrict__ dcoef, double *__restrict__ dmc) {
-  const int atom = blockIdx.x, t = blockIdx.y;
-  for (int n = threadIdx.x; n < mc_dim; n += blockDim.x) {
+  const long long stride = (long long)n_coef * n_chp * n_active;
+  for (int k = threadIdx.x; k < n_coef; k += blockDim.x) {
     double s = 0.0;
-    for (int q = slot_ptr[atom]; q < slot_ptr[atom + 1]; ++q) {
-      const double *dc = dcoef + (long long)n_coef * (slots[q] + (long long)n_chp * t);
-      for (int e = convT_ptr[n]; e < convT_ptr[n + 1]; ++e) s += convT_f[e] * dc[convT_k[e]];
+    for (int q = slot_ptr[a]; q < slot_ptr[a + 1]; ++q) {
+      const double *p = part + k + (long long)n_coef * (slots[q] + (long long)n_chp * t);
+#pragma unroll 8
+      for (int z = 0; z < nz; ++z) s += p[stride * z];
     }
-    dmc[n + (long long)mc_dim * (atom + (long long)n_atoms * t)] = s;
+    dc[k] = s;
   }
-}
-
-// dQ[lm, atom, t] = sum over rows n with (l, m) of cc[n] dmc[n] where the
-// forward kept the moment (l <= l_hartree_max_far_distance, |Q| > 1e-10).
-__global__ void sumup_dq_kernel(int n_atoms, int L, int L2, int mc_dim, int icc_dim0, const int *__restrict__ icc,
-                                const int *__restrict__ ncc, const double *__restrict__ cc,
-                                const int *__restrict__ lhmfd, const double *__restrict__ Q,
-                                const double *__restrict__ dmc, double *__restrict__ dQ) {
-  const int a = blockIdx.x, t = blockIdx.y;
-  int lh = lhmfd[a + n_atoms * t];
-  lh = lh < 0 ? 0 : (lh > L ? L : lh);
-  const int nmax = ncc[lh];
-  const double *dm = dmc + (long long)mc_dim * (a + (long long)n_atoms * t);
-  for (int lm = threadIdx.x; lm < L2; lm += blockDim.x) {
-    const long long qi = lm + (long long)L2 * (a + (long long)n_atoms * t);
-    const double q = Q[qi];
+  __syncthreads();
+  const int lh = min(max(lhmfd[a + n_atoms * t], 0), L);
+  for (int lm = warp; lm < L2; lm += blockDim.x / 32) {
     double s = 0.0;
-    for (int n = 0; n < nmax; ++n) {
-      const int l = icc[n], m = icc[n + icc_dim0];
-      if (l * l + l + m == lm && l <= lh && fabs(q) > 1e-10) s += cc[n] * dm[n];
+    if (lm < (lh + 1) * (lh + 1) && fabs(Q[lm + (long long)L2 * (a + (long long)n_atoms * t)]) > 1e-10) {
+      for (int r = lm_ptr[lm] + lane; r < lm_ptr[lm + 1]; r += 32) {
+        const int n = lm_row[r];
+        double m = 0.0;
+        for (int e = convT_ptr[n]; e < convT_ptr[n + 1]; ++e) m += convT_f[e] * dc[convT_k[e]];
+        s += cc[n] * m;
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     }
-    dQ[qi] = s;
+    if (lane == 0) out[lm] = s;
   }
 }
 
-int launch_dcoef(const SumupPlan &P, int n_active, const double *g, cudaStream_t stream) {
+int launch_dq(const SumupPlan &P, int n_active, const int *lhmfd, const double *Q, const double *g, double *dQ,
+              cudaStream_t stream) {
   const dim3 grid(P.n_chp, n_active, P.adj_nz);
   switch (P.L) {
-#define FRPA_DCOEF_CASE(LL)                                                                                  \
-  case LL:                                                                                                   \
-    sumup_dcoef_kernel<LL><<<grid, SU_THREADS, 0, stream>>>(P.n_valid_points, P.n_full_points, P.d_map,       \
-                                                             P.d_coord, P.n_chp, P.d_recs, g, P.adj_pts,       \
-                                                             P.d_dcoef_part);                                  \
+#define FRPA_DCOEF_CASE(LL)                                                                                       \
+  case LL:                                                                                                        \
+    sumup_dcoef_kernel<LL><<<grid, SU_THREADS, 0, stream>>>(P.n_valid_points, P.n_full_points, P.d_pfull,           \
+                                                             P.d_pxyz, P.n_chp, P.d_recs, g, P.adj_pts,            \
+                                                             P.d_dcoef_part);                                      \
     break;
     FRPA_DCOEF_CASE(0) FRPA_DCOEF_CASE(1) FRPA_DCOEF_CASE(2) FRPA_DCOEF_CASE(3) FRPA_DCOEF_CASE(4)
     FRPA_DCOEF_CASE(5) FRPA_DCOEF_CASE(6) FRPA_DCOEF_CASE(7) FRPA_DCOEF_CASE(8)
@@ -652,9 +1107,9 @@ int launch_dcoef(const SumupPlan &P, int n_active, const double *g, cudaStream_t
       return fail(FRPA_ERR_UNSUPPORTED, "sum-up adjoint: l_pot_max %d above %d", P.L, SU_LMAX);
   }
   FRPA_LAUNCH_CHECK();
-  const long long n = (long long)P.n_coef * P.n_chp * n_active;
-  sumup_dcoef_reduce_kernel<<<(int)std::min<long long>(4096, (n + 255) / 256), 256, 0, stream>>>(
-      n, P.adj_nz, P.d_dcoef_part, P.d_dcoef);
+  sumup_dq_kernel<<<dim3(P.n_atoms, P.T), 256, 0, stream>>>(
+      P.n_atoms, P.L, P.n_chp, P.n_coef, n_active, P.adj_nz, P.d_atom_slot_ptr, P.d_atom_slots, P.d_lm_ptr, P.d_lm_row,
+      P.d_convT_ptr, P.d_convT_k, P.d_convT_f, P.d_cc, lhmfd, Q, P.d_dcoef_part, dQ);
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
 }
@@ -663,9 +1118,56 @@ int launch_dcoef(const SumupPlan &P, int n_active, const double *g, cudaStream_t
 
 // ------------------------------------------------------------ host side ---
 
-static int upload(void **dst, const void *src, size_t bytes) {
-  FRPA_CUDA_TRY(cudaMalloc(dst, bytes > 0 ? bytes : 8));
-  if (bytes) FRPA_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+// A plan's device memory: arrays up to 1 MiB (and all uninitialised workspaces)
+// share one allocation and one copy, larger ones are copied from where they
+// are.  (One allocation and copy per array made creating a small plan mostly
+// driver calls.)
+struct PlanMemory {
+  struct Part {
+    void **dst;
+    size_t off;
+  };
+  std::vector<Part> parts;
+  std::vector<unsigned char> host;
+  size_t tail = 0;  // workspaces, after the copied bytes
+
+  static size_t padded(size_t n) { return (std::max<size_t>(n, 8) + 255) / 256 * 256; }
+  void array(void **dst, const void *src, size_t bytes) {
+    parts.push_back({dst, host.size()});
+    host.resize(host.size() + padded(bytes));
+    if (bytes) memcpy(host.data() + parts.back().off, src, bytes);
+  }
+  struct Space {
+    void **dst;
+    size_t bytes;
+  };
+  std::vector<Space> spaces;
+  void space(void **dst, size_t bytes) {
+    spaces.push_back({dst, bytes});
+    tail += padded(bytes);
+  }
+  int commit(void **base) {
+    if (cudaMalloc(base, padded(host.size() + tail)) != cudaSuccess) {
+      *base = nullptr;
+      return fail(FRPA_ERR_OOM, "sumup: allocation of %zu bytes failed", host.size() + tail);
+    }
+    unsigned char *d = static_cast<unsigned char *>(*base);
+    for (const Part &p : parts) *p.dst = d + p.off;
+    size_t off = host.size();
+    for (const Space &w : spaces) {
+      *w.dst = d + off;
+      off += padded(w.bytes);
+    }
+    if (!host.empty()) FRPA_CUDA_TRY(cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice));
+    return FRPA_OK;
+  }
+};
+constexpr size_t PLAN_SMALL = 1 << 20;
+
+static int upload_large(std::vector<void *> *owned, void **dst, const void *src, size_t bytes) {
+  if (cudaMalloc(dst, bytes) != cudaSuccess) return fail(FRPA_ERR_OOM, "sumup: allocation of %zu bytes failed", bytes);
+  owned->push_back(*dst);
+  FRPA_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
   return FRPA_OK;
 }
 
@@ -696,6 +1198,9 @@ static int sumup_upload_constants_once() {
   FRPA_CUDA_TRY(cudaMemcpyToSymbol(c_RA, RA, sizeof(RA)));
   FRPA_CUDA_TRY(cudaMemcpyToSymbol(c_RB, RB, sizeof(RB)));
   FRPA_CUDA_TRY(cudaMemcpyToSymbol(c_DF, DF, sizeof(DF)));
+  FRPA_CUDA_TRY(cudaMemcpyToSymbol(d_near_tables, K, sizeof(K), 0));
+  FRPA_CUDA_TRY(cudaMemcpyToSymbol(d_near_tables, RA, sizeof(RA), sizeof(K)));
+  FRPA_CUDA_TRY(cudaMemcpyToSymbol(d_near_tables, RB, sizeof(RB), 2 * sizeof(K)));
   return FRPA_OK;
 }
 
@@ -708,13 +1213,7 @@ int sumup_upload_constants(int device) {
 
 void sumup_plan_free(SumupPlan *P) {
   if (!P) return;
-  void *ptrs[] = {P->d_map, P->d_order, P->d_coord, P->d_species, P->d_species_center, P->d_l_hartree, P->d_n_grid,
-                  P->d_c2a, P->d_chp, P->d_icc, P->d_ncc, P->d_ijkmax, P->d_icc_packed, P->d_cc, P->d_cc_xyz,
-                  P->d_rgm, P->d_linc, P->d_conv_ptr, P->d_conv_n, P->d_conv_f, P->d_mc, P->d_recs, P->d_err,
-                  P->d_convT_ptr, P->d_convT_k, P->d_convT_f, P->d_dcoef, P->d_dmc, P->d_dcoef_part,
-                  P->d_atom_slot_ptr, P->d_atom_slots};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
+  for (void *p : P->owned) cudaFree(p);
   delete P;
 }
 
@@ -805,28 +1304,40 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
         conv[kelvin_index(i + 2 * s1, j + 2 * s2, k + 2 * s3)].push_back({n, fnn * multi});
       }
   }
-  std::vector<int> conv_ptr(n_kelvin(L) + 1, 0), conv_n;
-  std::vector<double> conv_f;
+  std::vector<int> conv_ptr(n_kelvin(L) + 1, 0), conv_lm;
+  std::vector<double2> conv_fc;
   for (int q = 0; q < n_kelvin(L); ++q) {
     for (auto &e : conv[q]) {
-      conv_n.push_back(e.first);
-      conv_f.push_back(e.second);
+      const int l = D->index_cc[e.first], m = D->index_cc[e.first + icc_dim0];
+      conv_lm.push_back(l * l + l + m);
+      conv_fc.push_back(make_double2(e.second, D->cc[e.first]));
     }
-    conv_ptr[q + 1] = (int)conv_n.size();
+    conv_ptr[q + 1] = (int)conv_lm.size();
   }
-  // transpose (by table row) for the adjoint
+  // transpose (by table row) for the adjoint, and the rows of each (l, m)
   std::vector<int> convT_ptr(std::max(1, mc_dim) + 1, 0), convT_k;
   std::vector<double> convT_f;
+  std::vector<int> lm_ptr((L + 1) * (L + 1) + 1, 0), lm_row;
   {
     std::vector<std::vector<std::pair<int, double>>> byrow(std::max(1, mc_dim));
-    for (int q = 0; q < n_kelvin(L); ++q)
-      for (auto &e : conv[q]) byrow[e.first].push_back({q, e.second});
+    int at = 0;  // the dQ kernels keep the coefficients by a, b, c
+    for (int a = 0; a <= L; ++a)
+      for (int b = 0; a + b <= L; ++b)
+        for (int c = 0; a + b + c <= L; ++c, ++at)
+          for (auto &e : conv[kelvin_index(a, b, c)]) byrow[e.first].push_back({at, e.second});
     for (size_t n = 0; n < byrow.size(); ++n) {
       for (auto &e : byrow[n]) {
         convT_k.push_back(e.first);
         convT_f.push_back(e.second);
       }
       convT_ptr[n + 1] = (int)convT_k.size();
+    }
+    for (int lm = 0; lm < (L + 1) * (L + 1); ++lm) {
+      for (int n = 0; n < mc_dim; ++n) {
+        const int l = D->index_cc[n], m = D->index_cc[n + icc_dim0];
+        if (l * l + l + m == lm) lm_row.push_back(n);
+      }
+      lm_ptr[lm + 1] = (int)lm_row.size();
     }
   }
   std::vector<int> packed(std::max(1, icc_dim0), 0);
@@ -853,10 +1364,13 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
   P->fast = fast ? 1 : 0;
   P->n_coef = n_kelvin(L);
   P->rs = rec_stride(L);
-  P->n_conv = (int)conv_n.size();
   int st = FRPA_OK;
-#define UP(field, src, bytes) \
-  if (st == FRPA_OK) st = upload((void **)&P->field, (src), (bytes));
+  PlanMemory mem;
+#define UP(field, src, bytes)                                                                     \
+  if ((size_t)(bytes) <= PLAN_SMALL)                                                              \
+    mem.array((void **)&P->field, (src), (bytes));                                                \
+  else if (st == FRPA_OK)                                                                         \
+    st = upload_large(&P->owned, (void **)&P->field, (src), (bytes));
   UP(d_map, D->i_valid_point_2_i_full_points_map, sizeof(int) * (size_t)D->n_valid_points);
   {
     // Morton order of the valid points (21 bits per axis over their bounding box)
@@ -910,25 +1424,27 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
   UP(d_cc_xyz, D->coords_center, sizeof(double) * 3 * (size_t)D->n_centers);
   UP(d_rgm, D->r_grid_min, sizeof(double) * D->n_species);
   UP(d_linc, D->log_r_grid_inc, sizeof(double) * D->n_species);
+  std::vector<int> slot_of(n_kelvin(L));
+  for (int a = 0; a <= L; ++a)
+    for (int b = 0; a + b <= L; ++b)
+      for (int c = 0; a + b + c <= L; ++c) slot_of[kelvin_index(a, b, c)] = kelvin_slot(a, b, c);
+  UP(d_slot, slot_of.data(), sizeof(int) * slot_of.size());
   UP(d_conv_ptr, conv_ptr.data(), sizeof(int) * conv_ptr.size());
-  UP(d_conv_n, conv_n.data(), sizeof(int) * conv_n.size());
-  UP(d_conv_f, conv_f.data(), sizeof(double) * conv_f.size());
+  UP(d_conv_lm, conv_lm.data(), sizeof(int) * conv_lm.size());
+  UP(d_conv_fc, conv_fc.data(), sizeof(double2) * conv_fc.size());
+  UP(d_lm_ptr, lm_ptr.data(), sizeof(int) * lm_ptr.size());
+  UP(d_lm_row, lm_row.data(), sizeof(int) * lm_row.size());
   UP(d_convT_ptr, convT_ptr.data(), sizeof(int) * convT_ptr.size());
   UP(d_convT_k, convT_k.data(), sizeof(int) * convT_k.size());
   UP(d_convT_f, convT_f.data(), sizeof(double) * convT_f.size());
-#undef UP
-  if (st == FRPA_OK &&
-      cudaMalloc((void **)&P->d_dcoef, sizeof(double) * (size_t)n_kelvin(L) * std::max(1, P->n_chp) * T) != cudaSuccess)
-    st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
-  if (st == FRPA_OK &&
-      cudaMalloc((void **)&P->d_dmc, sizeof(double) * (size_t)P->mc_dim * P->n_atoms * T) != cudaSuccess)
-    st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
-  // adjoint: at most 64 point blocks per (slot, t), partials reduced in order
-  P->adj_pts = std::max(4096, (P->n_valid_points + 63) / 64);
-  P->adj_nz = std::max(1, (P->n_valid_points + P->adj_pts - 1) / P->adj_pts);
-  if (st == FRPA_OK && cudaMalloc((void **)&P->d_dcoef_part, sizeof(double) * (size_t)n_kelvin(L) *
-                                                                 std::max(1, P->n_chp) * T * P->adj_nz) != cudaSuccess)
-    st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
+  // adjoint: point blocks of 512 to 4096 points (more past 262,144 points, at most
+  // 64 blocks there), as small as still gives about 2,400 blocks; partials added in order
+  {
+    const long long pairs = (long long)P->n_valid_points * P->n_chp * T;
+    const long long most = std::max(4096, ceil_div(P->n_valid_points, 64));
+    P->adj_pts = (int)((std::min(most, std::max(512LL, pairs / 2400)) + 127) / 128 * 128);
+    P->adj_nz = std::max(1, ceil_div(P->n_valid_points, P->adj_pts));
+  }
   {
     std::vector<int> cnt(P->n_atoms + 1, 0), slots(std::max(1, P->n_chp));
     std::vector<int> atom_of(std::max(1, P->n_chp));
@@ -939,22 +1455,30 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
     for (int a = 0; a < P->n_atoms; ++a) cnt[a + 1] += cnt[a];
     std::vector<int> fill(cnt.begin(), cnt.end() - 1);
     for (int q = 0; q < P->n_chp; ++q) slots[fill[atom_of[q]]++] = q;  // ascending within each atom
-    if (st == FRPA_OK && (cudaMalloc((void **)&P->d_atom_slot_ptr, sizeof(int) * cnt.size()) != cudaSuccess ||
-                          cudaMalloc((void **)&P->d_atom_slots, sizeof(int) * slots.size()) != cudaSuccess))
-      st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
-    if (st == FRPA_OK &&
-        (cudaMemcpy(P->d_atom_slot_ptr, cnt.data(), sizeof(int) * cnt.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-         cudaMemcpy(P->d_atom_slots, slots.data(), sizeof(int) * slots.size(), cudaMemcpyHostToDevice) != cudaSuccess))
-      st = fail(FRPA_ERR_CUDA, "sumup: upload failed");
+    UP(d_atom_slot_ptr, cnt.data(), sizeof(int) * cnt.size());
+    UP(d_atom_slots, slots.data(), sizeof(int) * slots.size());
   }
-  if (st == FRPA_OK && cudaMalloc((void **)&P->d_mc, sizeof(double) * (size_t)P->mc_dim * P->n_atoms * T) != cudaSuccess)
-    st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
-  if (st == FRPA_OK &&
-      cudaMalloc((void **)&P->d_recs, sizeof(double) * (size_t)P->rs * std::max(1, P->n_chp) * T) != cudaSuccess)
-    st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
-  if (st == FRPA_OK && cudaMalloc((void **)&P->d_err, sizeof(int)) != cudaSuccess)
-    st = fail(FRPA_ERR_OOM, "sumup: workspace allocation failed");
-  if (st == FRPA_OK) st = cudaMemset(P->d_err, 0, sizeof(int)) == cudaSuccess ? FRPA_OK : fail(FRPA_ERR_CUDA, "memset");
+  const int no_flags = 0;
+  UP(d_err, &no_flags, sizeof(int));
+#undef UP
+  const size_t chp = std::max(1, P->n_chp);
+  mem.space((void **)&P->d_pfull, sizeof(int) * (size_t)P->n_valid_points);
+  mem.space((void **)&P->d_pxyz, sizeof(double) * 3 * (size_t)P->n_valid_points);
+  mem.space((void **)&P->d_mc, sizeof(double) * (size_t)P->mc_dim * P->n_atoms * T);
+  mem.space((void **)&P->d_recs, sizeof(double) * (size_t)P->rs * chp * T);
+  mem.space((void **)&P->d_heads, sizeof(double4) * chp * T);
+  mem.space((void **)&P->d_dcoef_part, sizeof(double) * (size_t)n_kelvin(L) * chp * T * P->adj_nz);
+  if (st == FRPA_OK) {
+    void *base = nullptr;
+    st = mem.commit(&base);
+    if (base) P->owned.push_back(base);
+  }
+  if (st == FRPA_OK && P->n_valid_points > 0) {
+    sumup_gather_points_kernel<<<std::min(1184, ceil_div(P->n_valid_points, 256)), 256>>>(
+        P->n_valid_points, P->d_map, P->d_order, P->d_coord, P->d_pfull, P->d_pxyz);
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess)
+      st = fail(FRPA_ERR_CUDA, "sumup: point ordering failed");
+  }
   if (st == FRPA_OK) st = sumup_upload_constants(P->device);
   if (st != FRPA_OK) {
     sumup_plan_free(P);
@@ -971,18 +1495,14 @@ int sumup_execute(const SumupPlan *P, int n_active, int force_generic, const int
                   cudaStream_t stream) {
   FRPA_CHECK_ARG(n_active >= 0 && n_active <= P->T, "sumup: %d active perturbations > tile %d", n_active, P->T);
   if (n_active == 0 || P->n_valid_points == 0 || P->n_chp == 0) return FRPA_OK;
+  if (P->fast && !force_generic) {
+    FRPA_TRY(launch_prep(*P, n_active, lhmfd, mrs, opr, Q, stream));
+    return launch_fast(*P, n_active, spline, dv, codes, stream);
+  }
   sumup_multipole_c_kernel<<<dim3(P->n_atoms, n_active), 128, 0, stream>>>(
       P->n_atoms, P->L, P->L2, P->mc_dim, P->icc_dim0, P->lma, P->d_icc, P->d_ncc, P->d_cc, lhmfd, Q, P->d_mc,
       P->d_err);
   FRPA_LAUNCH_CHECK();
-  if (P->fast && !force_generic) {
-    sumup_records_kernel<<<dim3(P->n_chp, n_active), 128, 0, stream>>>(
-        P->L, P->n_atoms, P->n_chp, P->mc_dim, P->n_coef, P->rs, P->d_chp, P->d_c2a, P->d_species,
-        P->d_species_center, P->d_l_hartree, P->d_n_grid, P->d_rgm, P->d_linc, P->d_cc_xyz, mrs, opr, P->d_mc,
-        P->d_conv_ptr, P->d_conv_n, P->d_conv_f, P->d_recs);
-    FRPA_LAUNCH_CHECK();
-    return launch_fast(*P, n_active, spline, dv, codes, stream);
-  }
   const int grid = (P->n_valid_points + SU_THREADS - 1) / SU_THREADS;
   sumup_generic_kernel<<<grid, SU_THREADS, 0, stream>>>(
       P->n_valid_points, P->n_full_points, P->d_map, P->d_coord, n_active, P->n_chp, P->n_atoms, P->L, P->L2,
@@ -1006,28 +1526,12 @@ int sumup_adjoint_q(const SumupPlan *P, int n_active, const int *lhmfd, const do
                 "sumup adjoint: dQ is implemented for the fast path only (identity centers_hartree_potential and a "
                 "homogeneous multipole table); this plan uses the generic far-field kernel");
   FRPA_CHECK_ARG(n_active >= 0 && n_active <= P->T, "sumup adjoint: n_active %d", n_active);
-  FRPA_CUDA_TRY(cudaMemsetAsync(dQ, 0, sizeof(double) * (size_t)P->L2 * P->n_atoms * P->T, stream));
-  if (n_active == 0 || P->n_chp == 0 || P->n_valid_points == 0) return FRPA_OK;
-  sumup_multipole_c_kernel<<<dim3(P->n_atoms, n_active), 128, 0, stream>>>(
-      P->n_atoms, P->L, P->L2, P->mc_dim, P->icc_dim0, P->lma, P->d_icc, P->d_ncc, P->d_cc, lhmfd, Q, P->d_mc,
-      P->d_err);
-  FRPA_LAUNCH_CHECK();
-  sumup_records_kernel<<<dim3(P->n_chp, n_active), 128, 0, stream>>>(
-      P->L, P->n_atoms, P->n_chp, P->mc_dim, P->n_coef, P->rs, P->d_chp, P->d_c2a, P->d_species,
-      P->d_species_center, P->d_l_hartree, P->d_n_grid, P->d_rgm, P->d_linc, P->d_cc_xyz, mrs, opr, P->d_mc,
-      P->d_conv_ptr, P->d_conv_n, P->d_conv_f, P->d_recs);
-  FRPA_LAUNCH_CHECK();
-  int st = FRPA_OK;
-  st = launch_dcoef(*P, n_active, g, stream);
-  if (st != FRPA_OK) return st;
-  sumup_dmc_kernel<<<dim3(P->n_atoms, n_active), 128, 0, stream>>>(
-      P->n_chp, P->n_atoms, P->mc_dim, P->n_coef, P->d_atom_slot_ptr, P->d_atom_slots, P->d_convT_ptr, P->d_convT_k,
-      P->d_convT_f, P->d_dcoef, P->d_dmc);
-  FRPA_LAUNCH_CHECK();
-  sumup_dq_kernel<<<dim3(P->n_atoms, n_active), 64, 0, stream>>>(P->n_atoms, P->L, P->L2, P->mc_dim, P->icc_dim0,
-                                                                  P->d_icc, P->d_ncc, P->d_cc, lhmfd, Q, P->d_dmc, dQ);
-  FRPA_LAUNCH_CHECK();
-  return FRPA_OK;
+  if (n_active == 0 || P->n_chp == 0 || P->n_valid_points == 0) {
+    FRPA_CUDA_TRY(cudaMemsetAsync(dQ, 0, sizeof(double) * (size_t)P->L2 * P->n_atoms * P->T, stream));
+    return FRPA_OK;
+  }
+  FRPA_TRY(launch_prep(*P, n_active, lhmfd, mrs, opr, Q, stream));
+  return launch_dq(*P, n_active, lhmfd, Q, g, dQ, stream);
 }
 
 }  // namespace frpa

@@ -136,3 +136,33 @@ def test_dQ_on_the_generic_path_is_reported_unsupported():
     with pytest.raises(_lib.FrpaError) as e:
         plan.adjoint_q(1, *args, dev(p.delta_v_hartree), dQ)
     assert e.value.status == _lib.FRPA_ERR_UNSUPPORTED and "fast path" in e.value.message
+
+
+@pytest.mark.parametrize("L,T,points", [(0, 1, 31), (3, 2, 513), (6, 1, 1300), (7, 1, 1300), (8, 2, 700)])
+def test_dQ_equals_unit_moment_potentials(L, T, points):
+    """dL/dQ_lm of L = sum g delta_v is sum g v(unit moment lm): the potential is
+    linear in Q.  One and two coefficient passes (l_max up to 6, above), several
+    point blocks, truncated radii; entries the forward drops are zero."""
+    p = synth.make_sumup_problem(n_atoms=7, n_points=points, l_pot_max=L, T=T, seed=40 + L, outer_radius=5.0,
+                                 l_hartree_per_species=[L, max(0, L - 1), L, L], extra_full_points=9)
+    rng = np.random.default_rng(L)
+    g = rng.normal(size=(p.n_full_points, T))
+    plan = _lib.SumupPlan(p)
+    dQ = torch.empty(p.multipole_moments.size, dtype=torch.float64, device="cuda")
+    plan.adjoint_q(T, dev(p.l_hartree_max_far_distance, np.int32), dev(p.multipole_radius_sq),
+                   dev(p.outer_potential_radius), dev(p.multipole_moments), dev(g), dQ)
+    torch.cuda.synchronize()
+    got = host(dQ, p.multipole_moments.shape)
+    Q = p.multipole_moments.copy()
+    p.spline[:] = 0.0  # the far field only
+    p.delta_v_hartree[:] = 0.0
+    scale = np.max(np.abs(got))
+    l_of = np.floor(np.sqrt(np.arange((L + 1) ** 2))).astype(int)
+    kept = (np.abs(Q) > 1e-10) & (l_of[:, None, None] <= p.l_hartree_max_far_distance[None, :, :])
+    assert np.all(got[~kept] == 0.0)
+    for lm, a, t in rng.permutation(np.argwhere(kept))[:25]:
+        p.multipole_moments = np.zeros_like(Q)
+        p.multipole_moments[lm, a, t] = 1.0
+        v = oracle.sumup(p)
+        # 1,300 terms of at most |g| |v| each, one rounding per operation
+        assert abs(got[lm, a, t] - np.sum(g[:, t] * v[:, t])) < 1e-12 * scale

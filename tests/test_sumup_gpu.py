@@ -98,3 +98,46 @@ def test_sumup_session_cu_host_matches_oracle():
         out2 = s.sumup(delta_v=out)
         ref2 = oracle.sumup(p, delta_v=ref)
         assert delta_rel(out2, ref2, p.delta_v_hartree) < TOL
+
+
+@pytest.mark.parametrize("atoms,points,T,L,outer", [
+    (1, 1, 1, 0, None),         # one record, one point
+    (7, 33, 1, 3, 6.0),         # one record less than a chunk, a warp and one lane
+    (8, 129, 1, 4, 6.0),        # a whole chunk
+    (9, 1000, 2, 8, 5.0),       # a chunk and one record; one point per thread, records over 4 warps
+    (20, 20_000, 4, 6, 6.0),    # two points per thread
+    (16, 40_001, 4, 5, 6.0),    # four points per thread, records over 4 warps
+    (3, 152_001, 4, 2, None),   # four points per thread, all records in one warp
+])
+def test_sumup_dispatch_edges_match_oracle(atoms, points, T, L, outer):
+    """Sizes at the edges of the far- and near-field launches' rules."""
+    p = synth.make_sumup_problem(n_atoms=atoms, n_points=points, l_pot_max=L, T=T, seed=90 + atoms, outer_radius=outer,
+                                 l_hartree_per_species=[L, max(0, L - 1), L, max(0, L - 2)], extra_full_points=5)
+    out = run(_lib.SumupPlan(p), p)
+    ref = oracle.sumup(p, n_threads=8)
+    assert delta_rel(out, ref, p.delta_v_hartree) < TOL
+    untouched = np.setdiff1d(np.arange(p.n_full_points), p.i_valid_point_2_i_full_points_map)
+    assert np.array_equal(out[untouched], p.delta_v_hartree[untouched])
+
+
+@pytest.mark.parametrize("points", [700, 40_000])
+def test_sumup_extreme_records_match_generic_kernel(points):
+    """Moments too large (or infinite) at an l that only near-by points reach, a
+    vanishing near radius and a point without finite coordinates: the same
+    points stay finite as in the table loop, with the same values."""
+    p = synth.make_sumup_problem(n_atoms=12, n_points=points, l_pot_max=6, T=4, seed=33, outer_radius=4.0)
+    p.multipole_moments[40, 0, :] = np.inf       # l = 6
+    p.multipole_moments[30, 1, 1:] = 1e200       # l = 5
+    p.multipole_radius_sq[2, :] = 1e-50          # every point far
+    bad = int(p.i_valid_point_2_i_full_points_map[3])
+    p.coord_points[1, bad] = np.nan
+    p.coord_points[0, int(p.i_valid_point_2_i_full_points_map[5])] = np.inf
+    plan = _lib.SumupPlan(p)
+    fast, generic = run(plan, p), run(plan, p, generic=True)
+    assert np.array_equal(fast[bad], p.delta_v_hartree[bad])
+    ok = np.isfinite(generic)
+    assert np.array_equal(ok, np.isfinite(fast)) and ok.mean() > 0.5
+    small = ok & (np.abs(generic) < 1e6)
+    assert np.max(np.abs(fast - generic)[small]) < TOL * np.max(np.abs(generic[small]))
+    big = ok & ~small
+    assert np.all(np.abs(fast - generic)[big] < TOL * np.abs(generic[big]) * 1e2)
