@@ -66,8 +66,7 @@ static void rho1_plan_free(Rho1Plan *P) {
   cudaFree(P->d_ib);
   cudaFree(P->d_map);
   cudaFree(P->d_counter);
-  cudaFree(P->d_adj_items);
-  cudaFree(P->d_h1_items_sym);
+  cudaFree(P->d_h1_items);
   cudaFree(P->d_h1_acc);
   cudaFree(P->d_items_split);
   cudaFree(P->d_rowmax);
@@ -180,21 +179,9 @@ static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D) {
   const int zero = 0;
   up((void **)&P->d_counter, &zero, sizeof(int));
   {
-    std::vector<int> ncb(nb), npb(nb), preb(nb);
-    std::vector<long long> offb(nb);
-    for (int b = 0; b < nb; ++b) {
-      ncb[b] = D->n_compute_c_batches[b];
-      npb[b] = D->n_point_batches[b];
-      preb[b] = D->n_point_batches_prefix_sum[b];
-      offb[b] = D->i_batch_2_wave_offset[b];
-    }
-    std::vector<unsigned char> adj, sym;
-    rho1_h1_build_items(ncb.data(), npb.data(), ib_off.data(), preb.data(), offb.data(), nb, T, false, &adj);
-    P->n_adj_items = (int)(adj.size() / rho1_h1_item_size());
-    up(&P->d_adj_items, adj.data(), adj.size());
-    rho1_h1_build_items(ncb.data(), npb.data(), ib_off.data(), preb.data(), offb.data(), nb, T, true, &sym);
-    P->n_h1_items_sym = (int)(sym.size() / rho1_h1_item_size());
-    up(&P->d_h1_items_sym, sym.data(), sym.size());
+    std::vector<unsigned char> h1;
+    rho1_h1_build_items(batches, &h1, &P->h1_groups, &P->h1_a_len);
+    up(&P->d_h1_items, h1.data(), h1.size());
   }
   if (st == FRPA_OK) {
     P->grid_fp64 = rho1_fp64_grid(P->device);

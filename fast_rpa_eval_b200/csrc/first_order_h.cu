@@ -17,23 +17,40 @@
 // With g_rho = w v and no g_grad the adjoint is the first-order H with every
 // exchange-correlation term zero.
 //
-// Work: one CTA per 64 x 64 (i, j) tile of one batch and perturbation on the
-// FP64 MMA (mma.sync m8n8k4, the only FP64 tensor instruction of sm_100a),
-// A and phi staged in shared memory as the point dimension streams; the
-// symmetric H computes the tiles with j >= i only, each from both products.
+// Work, two passes per perturbation.  The first is bound by memory: it reads phi,
+// grad phi (and the Hessian rows of atom j) once, writes A in phi's layout to a
+// scratch array and finds the bound of the contributions that fixes the
+// accumulation's scale (below), which needs a pass over the inputs anyway.  The
+// second is one CTA per (i, j) tile of at most 64 x 64 of one batch: a plain
+// product of A and phi on the FP64 MMA (mma.sync m8n8k4, the only FP64 tensor
+// instruction of sm_100a), both streamed by asynchronous copies three or four
+// stages of 16 points ahead, because batches are small (tens to some hundred
+// functions) and what counts is latency.  A batch's rows are split evenly into
+// tiles whose widths are multiples of 8, and the 8-row blocks of a tile go round
+// the warps, so that a narrow tile loads all four tensor pipes.  The symmetric H
+// computes the tiles with j >= i only, each from both products.  Where A would
+// take more than H1_A_BYTES, the first pass only finds the bound, and groups of
+// batches that fit are then combined and multiplied in turn.  Measured, 1,600
+// batches of 100-200 points, n_compute 40-120, n_basis 4,000 (one B200): first-order
+// H 1.60 ms (A rebuilt in every tile from synchronous loads, 128-bit sums with a
+// carry) -> 0.59 ms; adjoint 1.21 -> 0.48 ms, of it first pass 0.16 (60% of the HBM
+// bandwidth), tiles 0.25, last pass 0.05.
 //
 // Determinism.  Batches overlap in the output, so tiles of different batches
-// add into the same entries.  Every contribution is added as a 128-bit
-// fixed-point integer (two 64-bit words, the low word's carry propagated by
-// the thread that produced it), and integer addition does not depend on the
-// order: two runs give bit-identical results.  The fixed-point scale 2^s is
-// fixed per call before any addition from a bound of the inputs (a pass over
+// add into the same entries.  Every contribution is added as a 100-bit
+// fixed-point integer held in two 64-bit words of one 16-byte entry (a high and
+// a low part, both signed, each summed with its own no-return atomic: the low
+// word has room for the sum over every batch, so no carry and no wait for
+// another thread's sum; both parts come from the addition of 1.5 2^52, which
+// leaves an integer in the mantissa), and integer addition does not depend
+// on the order: two runs give bit-identical results.  The fixed-point scale 2^s
+// is fixed per call before any addition from a bound of the inputs (a pass over
 // phi, grad phi, Hessian and the per-point coefficients): every single
 // contribution is below 2^emax, at most 2 n_batches contributions meet in one
 // entry, so with s = 100 - emax - ceil(log2(2 n_batches)) every partial sum
 // stays below 2^100 and each contribution is represented to 2^-s, about 2^-80
-// of the largest one.  A last pass converts each entry to FP64 (one rounding)
-// and adds it to the output.
+// of the largest one.  A last pass converts each entry to FP64 (one rounding),
+// adds it to the output and leaves the accumulator zero for the next call.
 #include <climits>
 #include <cstring>
 #include <vector>
@@ -43,17 +60,17 @@
 namespace frpa {
 namespace {
 
-constexpr int BM = 64, BN = 64, KC = 16, THREADS = 256;
-constexpr int COEF_PTS = 128;  // points whose coefficients are staged together (a multiple of KC)
-static_assert(COEF_PTS % KC == 0, "coefficient stage holds whole K chunks");
-constexpr int LDA = BM + 4;  // As[k = point][m = i]
-constexpr int LDB = KC + 4;  // Bs[n = j][k = point]
+constexpr int TILE = 64, KC = 16, THREADS = 256;
+constexpr int LD = TILE + 4;  // [k = point][row]: stride = 4 (mod 16) doubles, conflict-free fragment loads
+constexpr long long H1_A_BYTES = 512LL << 20;  // scratch for A
 constexpr int EMAX_EMPTY = -2139062144;  // 0x80808080: no non-zero bound seen
 constexpr int H1_FLAG_NONFINITE = 16;    // device flag: a non-finite input reached the accumulation
 
 struct H1Item {
-  int batch, nc, np, ib_off, prefix, m0, n0, t;
+  int batch, nc, np, ib_off, prefix, t;
+  int m0, n0, mw, nw;  // first row and rows of the tile along i and j (m0, n0 multiples of 8)
   long long wave_off;
+  long long a_off;        // the batch's A in the scratch of its group
 };
 
 // Per-point inputs of the first-order H, reference layouts
@@ -72,9 +89,11 @@ struct H1Args {
   const double *wave, *gwave;
   const double *g_rho, *g_grad;  // adjoint mode
   H1Inputs h;                     // first-order H mode
-  unsigned long long *acc;        // (2, n_basis, n_basis, T): low words, then high words
-  long long n_entries;            // n_basis^2 T
-  int *emax;
+  ulonglong2 *acc;                // (n_basis, n_basis, T): low part, high part
+  double *A;                      // scratch: A(i, p) at a_off + p ncp + i
+  int *emax;                      // per perturbation
+  int grad;       // grad phi enters A (always, except an adjoint without g_grad)
+  int aligned16;  // phi, grad phi rows start on 16-byte boundaries
   int *err;
 };
 
@@ -131,19 +150,6 @@ __device__ __forceinline__ int hess_component(int k, int j_coord) {
   return k == 0 ? r : (k == 1 ? (r == 0 ? 1 : (r == 1 ? 3 : 4)) : (r == 0 ? 2 : (r == 1 ? 4 : 5)));
 }
 
-// A(i, p) from the point's coefficients; i < nc.
-__device__ __forceinline__ double a_value(const PointCoef &c, const double *phi, const double *gph,
-                                          const double *hph, int i, int ncp, bool in_range, int j_coord) {
-  double v = c.c_phi * phi[i];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) v = fma(c.c_grad[k], gph[i + k * ncp], v);
-  if (in_range) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) v = fma(c.c_hess[k], hph[i + hess_component(k, j_coord) * ncp], v);
-  }
-  return v;
-}
-
 // Compute-function range [vs, ve) of atom j_atom_begin + t in batch b
 // (atom_valid_n_compute_c_batches, evaluate_first_order_H.cpp:131-133),
 // clipped to the batch's compute functions; a range that leaves them sets
@@ -164,56 +170,109 @@ __device__ __forceinline__ void atom_range(const H1Args &a, int b, int t, int nc
 
 // ---------------------------------------------------------------- bound
 
-// One block per (batch, t): bound_b = sum_p max_i |A(i, p)| max_j |phi_j(p)|
-// (twice that for the symmetric H), then atomicMax of its binary exponent.
-__global__ void __launch_bounds__(THREADS) h1_bound_kernel(const H1Item *__restrict__ items, int n_items,
-                                                           H1Args a) {
-  __shared__ double red[THREADS / 32];
-  const int it = blockIdx.x;
-  const H1Item W = items[it];
-  if (W.m0 != 0 || W.n0 != 0) return;  // one block per (batch, t): its first tile
-  const int t = W.t;
-  if (a.mode == 1 && t >= a.n_active) return;
-  const int nc = W.nc, np = W.np, ncp = (nc + 3) & ~3;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// The largest |x| of a warp as an upper bound that is exact to 2^-20: the high
+// words are reduced (one instruction), a non-zero value counts as at least 1.
+__device__ __forceinline__ unsigned magnitude(double x) {
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return h | (h == 0 && __double2loint(x) != 0 ? 1u : 0u);
+}
+__device__ __forceinline__ double upper_bound(unsigned h) {
+  return h == 0 ? 0.0 : (h >= 0x7ff00000u ? __hiloint2double(0x7ff00000, 0) : __hiloint2double((int)h + 1, 0));
+}
+
+// One block per batch of the list, perturbation t: A(i, p) to the scratch (WRITE)
+// and, unless the scale is already known (BOUND), bound_b = sum_p max_i |A(i, p)|
+// max_j |phi_j(p)| (twice that for the symmetric H), of which the binary exponent
+// goes to an atomicMax.  The points' coefficients come first, a thread each; then
+// half a warp per point, 16-byte loads (a whole warp leaves most lanes idle in the
+// last 64 rows of a small batch).  gridDim.y blocks share a batch's points; each
+// bounds its own part and counts it gridDim.y times.
+template <bool WRITE, bool BOUND>
+__global__ void __launch_bounds__(THREADS) h1_combine_kernel(const H1Item *__restrict__ items, int t, H1Args a) {
+  __shared__ double red[THREADS / 16];
+  __shared__ PointCoef s_c[THREADS];
+  const H1Item W = items[blockIdx.x];
+  const int nc = W.nc, ncp = (nc + 3) & ~3;
+  const int part = (W.np + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int p_first = blockIdx.y * part, np = min(W.np, p_first + part);
+  const int half = threadIdx.x >> 4, lane = threadIdx.x & 15;
+  const unsigned members = 0xffffu << (threadIdx.x & 16);  // this half warp
   int vs = 0, ve = 0;
-  if (a.mode == 1) atom_range(a, W.batch, t, nc, &vs, &ve, true);
+  if (a.mode == 1) atom_range(a, W.batch, t, nc, &vs, &ve, BOUND);
   double sum = 0.0;
   bool finite = true;
-  for (int p = warp; p < np; p += THREADS / 32) {
-    const PointCoef c = point_coef(a, W.batch, p, W.prefix, t);
-    const double *phi = a.wave + W.wave_off + (long long)p * ncp;
-    const double *gph = a.gwave + 3 * W.wave_off + 3LL * p * ncp;
-    const double *hph = a.mode == 1 ? a.h.hessian + 6 * W.wave_off + 6LL * p * ncp : nullptr;
-    double mp = 0.0, mg = 0.0, mh = 0.0;
-    for (int i = lane; i < nc; i += 32) {
-      mp = fmax(mp, fabs(phi[i]));
+  for (int p0 = p_first; p0 < np; p0 += THREADS) {
+    __syncthreads();
+    if (p0 + (int)threadIdx.x < np) s_c[threadIdx.x] = point_coef(a, W.batch, p0 + threadIdx.x, W.prefix, t);
+    __syncthreads();
+    const int pe = min(np, p0 + THREADS);
+    for (int p = p0 + half; p < pe; p += THREADS / 16) {
+      const PointCoef c = s_c[p - p0];
+      const double *phi = a.wave + W.wave_off + (long long)p * ncp;
+      const double *gph = a.gwave + 3 * W.wave_off + 3LL * p * ncp;
+      const double *hph = a.mode == 1 ? a.h.hessian + 6 * W.wave_off + 6LL * p * ncp : nullptr;
+      double *A = a.A + W.a_off + (long long)p * ncp;
+      unsigned mp = 0, ma = 0;
+      // two rows at a time (i even): a vector that starts below n_compute ends by ncp
+#pragma unroll 2
+      for (int i = 2 * lane; i < nc; i += 32) {
+        double f[2], g[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        if (a.aligned16) {
+          const double2 x = __ldg(reinterpret_cast<const double2 *>(phi + i));
+          f[0] = x.x;
+          f[1] = x.y;
+          if (a.grad) {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) mg = fmax(mg, fabs(gph[i + k * ncp]));
-      if (hph && i >= vs && i < ve) {
+            for (int k = 0; k < 3; ++k) {
+              const double2 y = __ldg(reinterpret_cast<const double2 *>(gph + i + k * ncp));
+              g[k][0] = y.x;
+              g[k][1] = y.y;
+            }
+          }
+        } else {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) mh = fmax(mh, fabs(hph[i + hess_component(k, a.h.j_coord) * ncp]));
+          for (int e = 0; e < 2; ++e) {
+            f[e] = __ldg(phi + i + e);
+            if (a.grad) {
+#pragma unroll
+              for (int k = 0; k < 3; ++k) g[k][e] = __ldg(gph + i + e + k * ncp);
+            }
+          }
+        }
+        double v[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          v[e] = c.c_phi * f[e];
+          if (a.grad) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[e] = fma(c.c_grad[k], g[k][e], v[e]);
+          }
+          if (i + e >= vs && i + e < ve) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              v[e] = fma(c.c_hess[k], __ldg(hph + i + e + hess_component(k, a.h.j_coord) * ncp), v[e]);
+          }
+          if (i + e >= nc) v[e] = f[e] = 0.0;  // row padding
+          mp = max(mp, magnitude(f[e]));
+          ma = max(ma, magnitude(v[e]));
+        }
+        if (WRITE) *reinterpret_cast<double2 *>(A + i) = make_double2(v[0], v[1]);
+      }
+      if (BOUND) {
+        const double term =
+            upper_bound(__reduce_max_sync(members, ma)) * upper_bound(__reduce_max_sync(members, mp));
+        if (!(term <= 1.0e300)) finite = false;  // NaN, Inf or beyond what the bound can carry
+        if (lane == 0) sum += term;
       }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      mp = fmax(mp, __shfl_xor_sync(0xffffffffu, mp, o));
-      mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-      mh = fmax(mh, __shfl_xor_sync(0xffffffffu, mh, o));
-    }
-    const double ca = fabs(c.c_phi) * mp +
-                      (fabs(c.c_grad[0]) + fabs(c.c_grad[1]) + fabs(c.c_grad[2])) * mg +
-                      (fabs(c.c_hess[0]) + fabs(c.c_hess[1]) + fabs(c.c_hess[2])) * mh;
-    const double term = ca * mp;
-    if (!(term <= 1.0e300)) finite = false;  // NaN, Inf or beyond what the bound can carry
-    if (lane == 0) sum += term;
   }
-  if (lane == 0) red[warp] = finite ? sum : -1.0;
+  if (!BOUND) return;
+  if (lane == 0) red[half] = finite ? sum : -1.0;
   __syncthreads();
   if (threadIdx.x == 0) {
     double s = 0.0;
     bool ok = true;
-    for (int w = 0; w < THREADS / 32; ++w) {
+    for (int w = 0; w < THREADS / 16; ++w) {
       if (red[w] < 0.0) ok = false;
       s += red[w];
     }
@@ -221,170 +280,227 @@ __global__ void __launch_bounds__(THREADS) h1_bound_kernel(const H1Item *__restr
       atomicOr(a.err, H1_FLAG_NONFINITE);
       return;
     }
-    if (a.mode == 1) s *= 2.0;
+    s *= (a.mode == 1 ? 2.0 : 1.0) * gridDim.y;
     if (s > 0.0) {
       int e = 0;
       frexp(s, &e);  // s < 2^e
-      atomicMax(a.emax, e);
+      atomicMax(a.emax + t, e);
     }
   }
 }
 
-__device__ __forceinline__ int ceil_log2(long long n) {
+__host__ __device__ __forceinline__ int ceil_log2(long long n) {
   int k = 0;
   while ((1LL << k) < n) ++k;
   return k;
 }
 
+// The split of the fixed-point integer x = high 2^low + lowpart, |lowpart| <= 2^(low - 1):
+// the sum of 2 n_batches low parts stays below 2^62 and the sum of the high parts
+// below 2^62 (`bits` of the whole: 100 up to 2^23 batches); of a single
+// contribution both parts are below 2^51.
+struct FixedPoint {
+  int low, bits;
+};
+__host__ __device__ __forceinline__ FixedPoint fixed_point(int n_batches) {
+  const int c = ceil_log2(2LL * (n_batches > 0 ? n_batches : 1));
+  const int low = c <= 13 ? 50 : 63 - c;
+  return FixedPoint{low, low + 62 < 100 ? low + 62 : 100};
+}
 // The fixed-point exponent of this call (see the file comment).
 __device__ __forceinline__ int fixed_scale(int emax, int n_batches) {
-  return 100 - emax - ceil_log2(2LL * (n_batches > 0 ? n_batches : 1));
+  return fixed_point(n_batches).bits - emax - ceil_log2(2LL * (n_batches > 0 ? n_batches : 1));
 }
 
-// v 2^s (|v 2^s| < 2^100) rounded to an integer, added to the 128-bit entry
-// (lo, hi).  Modular two's-complement arithmetic: the carry out of the low
-// word is exactly the one of this addition, whatever other threads add.
-__device__ __forceinline__ void add_fixed(unsigned long long *lo, unsigned long long *hi, double v, int s) {
-  if (v == 0.0) return;
-  const double V = rint(ldexp(v, s));
-  const double A = trunc(ldexp(V, -52));
-  const double B = V - ldexp(A, 52);  // exact, |B| < 2^52
-  const __int128 x = ((__int128)(long long)A << 52) + (__int128)(long long)B;
-  const unsigned long long xl = (unsigned long long)x;
-  const unsigned long long xh = (unsigned long long)(x >> 64);
-  const unsigned long long old = atomicAdd(lo, xl);
-  const unsigned long long carry = (old + xl < old) ? 1ull : 0ull;
-  atomicAdd(hi, xh + carry);
+// Powers of two that take a value to its fixed-point parts.
+struct FixedScale {
+  double s1, s2;        // 2^s as a product (s can exceed the exponent range)
+  double low, inv_low;  // 2^low, 2^-low
+  double limit;         // 2^(bits - ceil(log2(2 n_batches))): above every contribution
+};
+__device__ __forceinline__ FixedScale make_scale(int emax, int n_batches) {
+  const FixedPoint f = fixed_point(n_batches);
+  const int s = fixed_scale(emax, n_batches);
+  return FixedScale{ldexp(1.0, s / 2), ldexp(1.0, s - s / 2), ldexp(1.0, f.low), ldexp(1.0, -f.low),
+                    ldexp(1.0, s + emax)};
+}
+
+// v 2^s rounded to an integer, in two parts; false for a value the scale cannot
+// hold (a non-finite input, flagged by the bound).
+__device__ __forceinline__ bool to_fixed(double v, const FixedScale &f, long long *lo, long long *hi) {
+  const double V = v * f.s1 * f.s2, magic = 6755399441055744.0;  // 1.5 2^52
+  const double th = fma(V, f.inv_low, magic);
+  const double tl = fma(magic - th, f.low, V) + magic;  // the difference is exact, the sum rounds to an integer
+  *hi = __double_as_longlong(th) - __double_as_longlong(magic);
+  *lo = __double_as_longlong(tl) - __double_as_longlong(magic);
+  return fabs(V) < f.limit;
+}
+
+__device__ __forceinline__ void add_fixed(ulonglong2 *entry, long long lo, long long hi) {
+  if (lo) atomicAdd(&entry->x, (unsigned long long)lo);
+  if (hi) atomicAdd(&entry->y, (unsigned long long)hi);
 }
 
 // ----------------------------------------------------------------- tiles
 
+// One chunk's products of a warp: CM of the tile's 8-row blocks along i (stride 2
+// blocks, the warps' round), CN along j (stride 4 blocks).
+template <int CM, int CN>
+__device__ __forceinline__ void tile_mma(double (&acc)[4][2][2], const double *X, const double *Y) {
+#pragma unroll
+  for (int ks = 0; ks < KC / 4; ++ks) {
+    double fa[CM], fb[CN];
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi) fa[mi] = X[ks * 4 * LD + mi * 16];
+#pragma unroll
+    for (int ni = 0; ni < CN; ++ni) fb[ni] = Y[ks * 4 * LD + ni * 32];
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < CN; ++ni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], fa[mi], fb[ni]);
+  }
+}
+__device__ __forceinline__ void tile_mma_any(int shape, double (&acc)[4][2][2], const double *X, const double *Y) {
+  switch (shape) {  // 2 CM + CN, uniform over the warp
+    case 2 * 4 + 2: tile_mma<4, 2>(acc, X, Y); break;
+    case 2 * 3 + 2: tile_mma<3, 2>(acc, X, Y); break;
+    case 2 * 2 + 2: tile_mma<2, 2>(acc, X, Y); break;
+    case 2 * 1 + 2: tile_mma<1, 2>(acc, X, Y); break;
+    case 2 * 4 + 1: tile_mma<4, 1>(acc, X, Y); break;
+    case 2 * 3 + 1: tile_mma<3, 1>(acc, X, Y); break;
+    case 2 * 2 + 1: tile_mma<2, 1>(acc, X, Y); break;
+    case 2 * 1 + 1: tile_mma<1, 1>(acc, X, Y); break;
+    default: break;
+  }
+}
+
 template <bool SYM>
-__global__ void __launch_bounds__(THREADS, 2) h1_tile_kernel(const H1Item *__restrict__ items, int n_items, H1Args a) {
-  __shared__ __align__(16) double As[KC * LDA];  // A(m0 + m, k)
-  __shared__ __align__(16) double Bs[BN * LDB];  // phi(n0 + n, k)
-  __shared__ __align__(16) double Ps[SYM ? KC * LDA : 1];  // phi(m0 + m, k)
-  __shared__ __align__(16) double Qs[SYM ? BN * LDB : 1];  // A(n0 + n, k)
-  __shared__ PointCoef coef[COEF_PTS];  // the per-point coefficients of COEF_PTS points at a time
+struct TileShape {
+  static constexpr int STAGES = SYM ? 3 : 4, ARRAYS = SYM ? 4 : 2, CTAS = SYM ? 2 : 3;
+  static constexpr int SMEM = (int)sizeof(double) * STAGES * ARRAYS * KC * LD;
+};
+
+template <bool SYM>
+__global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
+    h1_tile_kernel(const H1Item *__restrict__ items, int n_items, int t, H1Args a) {
+  // a stage: A of the tile's i rows and phi of its j rows; if SYM, phi of the i rows and A of the j rows
+  constexpr int STAGES = TileShape<SYM>::STAGES, ARRAYS = TileShape<SYM>::ARRAYS, BUF = KC * LD;
+  extern __shared__ __align__(16) double smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 2, wn = warp & 3, g = lane >> 2, q = lane & 3;
-  const long long nb2 = (long long)a.n_basis * a.n_basis;
-  const int emax = *a.emax;
+  const int emax = a.emax[t];
   if (emax == EMAX_EMPTY) return;  // every contribution is zero
-  const int s = fixed_scale(emax, a.n_batches);
-  unsigned long long *acc_lo = a.acc, *acc_hi = a.acc + a.n_entries;
+  const FixedScale scale = make_scale(emax, a.n_batches);
+  ulonglong2 *entries = a.acc + (long long)a.n_basis * a.n_basis * t;
 
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const H1Item W = items[it];
-    const int nc = W.nc, np = W.np, t = W.t, ncp = (nc + 3) & ~3;
-    if (a.mode == 1 && t >= a.n_active) continue;
-    const double *phi = a.wave + W.wave_off;
-    const double *gph = a.gwave + 3 * W.wave_off;
-    const double *hph = a.mode == 1 ? a.h.hessian + 6 * W.wave_off : nullptr;
-    int vs = 0, ve = 0;
-    if (a.mode == 1) atom_range(a, W.batch, t, nc, &vs, &ve, false);
+    const int nc = W.nc, np = W.np, ncp = (nc + 3) & ~3;
+    const bool diag = W.m0 == W.n0;
+    const double *phi = a.wave + W.wave_off, *amat = a.A + W.a_off;
     double acc[4][2][2];
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
       for (int y = 0; y < 2; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
 
-    for (int k0 = 0; k0 < np; k0 += KC) {
-      if (k0 % COEF_PTS == 0) {  // every thread, one point each (the loads of many points in flight)
-        for (int e = tid; e < COEF_PTS && k0 + e < np; e += THREADS) coef[e] = point_coef(a, W.batch, k0 + e, W.prefix, t);
-      }
-      __syncthreads();
-      {
-        // thread -> one point k of the chunk and four consecutive rows: the
-        // point's coefficients are read once, the rows' loads coalesce
-        constexpr int RPT = (BM * KC) / THREADS;  // rows per thread (4)
-        const int k = tid / (BM / RPT), r0 = (tid % (BM / RPT)) * RPT, p = k0 + k;
-        const bool pok = p < np;
-        const long long pc = (long long)(pok ? p : 0) * ncp;
-        const PointCoef c = coef[(k0 % COEF_PTS) + k];
-        const int jc = a.mode == 1 ? a.h.j_coord : 1;
-        const double *ph = phi + pc, *gp = gph + 3 * pc, *hp = hph ? hph + 6 * pc : nullptr;
+    const int nmi = (W.mw + 7) / 8, nni = (W.nw + 7) / 8;  // 8-row blocks of the tile
+    // Copies: lane -> two rows of the tile, warp -> points warp and warp + 8 of a
+    // chunk.  Rows past n_compute (up to whole blocks) and points past the batch
+    // are zero.
+    const int r = 2 * lane;
+    auto copy = [&](double *dst, const double *src, int i0, int blocks, int k0, bool wide) {
+      if (r >= blocks * 8) return;
+      const int i = i0 + r, left = nc - i;
 #pragma unroll
-        for (int rr = 0; rr < RPT; ++rr) {
-          const int i = W.m0 + r0 + rr;
-          double va = 0.0, vp = 0.0;
-          if (pok && i < nc) {
-            va = a_value(c, ph, gp, hp, i, ncp, hp != nullptr && i >= vs && i < ve, jc);
-            if (SYM) vp = ph[i];
+      for (int j = 0; j < KC / 8; ++j) {
+        const int k = warp + 8 * j, p = k0 + k;
+        const double *from = src + (long long)p * ncp + i;
+        double *to = dst + k * LD + r;
+        if (wide) {
+          const int bytes = p < np ? (left > 1 ? 16 : (left > 0 ? 8 : 0)) : 0;
+          cp_async_16(to, bytes ? from : src, bytes);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const bool ok = p < np && left > e;
+            cp_async_8(to + e, ok ? from + e : src, ok ? 8 : 0);
           }
-          As[k * LDA + r0 + rr] = va;
-          if (SYM) Ps[k * LDA + r0 + rr] = vp;
-        }
-#pragma unroll
-        for (int rr = 0; rr < RPT; ++rr) {
-          const int jj = W.n0 + r0 + rr;
-          double vb = 0.0, vq = 0.0;
-          if (pok && jj < nc) {
-            vb = ph[jj];
-            if (SYM) vq = a_value(c, ph, gp, hp, jj, ncp, hp != nullptr && jj >= vs && jj < ve, jc);
-          }
-          Bs[(r0 + rr) * LDB + k] = vb;
-          if (SYM) Qs[(r0 + rr) * LDB + k] = vq;
         }
       }
-      __syncthreads();
-#pragma unroll
-      for (int ks = 0; ks < KC / 4; ++ks) {
-        double fa[4], fb[2];
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi) fa[mi] = As[(ks * 4 + q) * LDA + wm * 32 + mi * 8 + g];
-#pragma unroll
-        for (int ni = 0; ni < 2; ++ni) fb[ni] = Bs[(wn * 16 + ni * 8 + g) * LDB + ks * 4 + q];
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < 2; ++ni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], fa[mi], fb[ni]);
-        if (SYM) {
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi) fa[mi] = Ps[(ks * 4 + q) * LDA + wm * 32 + mi * 8 + g];
-#pragma unroll
-          for (int ni = 0; ni < 2; ++ni) fb[ni] = Qs[(wn * 16 + ni * 8 + g) * LDB + ks * 4 + q];
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 2; ++ni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], fa[mi], fb[ni]);
-        }
+    };
+    auto load = [&](int c) {
+      double *S = smem + (c % STAGES) * ARRAYS * BUF;
+      const int k0 = c * KC;
+      copy(S, amat, W.m0, nmi, k0, true);
+      copy(S + BUF, phi, W.n0, nni, k0, a.aligned16);
+      if (SYM && !diag) {  // a diagonal tile has both on both sides
+        copy(S + 2 * BUF, phi, W.m0, nmi, k0, a.aligned16);
+        copy(S + 3 * BUF, amat, W.n0, nni, k0, true);
       }
-      __syncthreads();
+    };
+    const int nch = (np + KC - 1) / KC;
+    __syncthreads();  // the last item's stages are consumed
+#pragma unroll
+    for (int c = 0; c < STAGES - 1; ++c) {
+      if (c < nch) load(c);
+      cp_async_commit();
     }
+    const int cm = (nmi - wm + 1) / 2, cn = (nni - wn + 3) / 4;  // this warp's blocks
+    const int shape = cm > 0 && cn > 0 ? 2 * cm + cn : 0;
+    const int off_m = q * LD + g + wm * 8, off_n = q * LD + g + wn * 8;
+    for (int c = 0; c < nch; ++c) {
+      cp_async_wait<STAGES - 2>();
+      __syncthreads();
+      if (c + STAGES - 1 < nch) load(c + STAGES - 1);
+      cp_async_commit();
+      const double *S = smem + (c % STAGES) * ARRAYS * BUF;
+      tile_mma_any(shape, acc, S + off_m, S + BUF + off_n);
+      if (SYM) tile_mma_any(shape, acc, (diag ? S + BUF : S + 2 * BUF) + off_m, (diag ? S : S + 3 * BUF) + off_n);
+    }
+    cp_async_wait<0>();
     // add the tile (and, for an off-diagonal symmetric tile, its transpose)
+    long long col[2][2];
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        const int j = (ni * 4 + wn) * 8 + 2 * q + hh;
+        col[ni][hh] = j < W.nw && W.n0 + j < nc ? __ldg(a.ib_all + W.ib_off + W.n0 + j) - 1 : -1;
+      }
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi) {
-      const int i = W.m0 + wm * 32 + mi * 8 + g;
-      if (i >= nc) continue;
-      const long long row = a.ib_all[W.ib_off + i] - 1;
+      const int i = (mi * 2 + wm) * 8 + g;
+      if (i >= W.mw || W.m0 + i >= nc) continue;
+      const long long row = __ldg(a.ib_all + W.ib_off + W.m0 + i) - 1;
 #pragma unroll
       for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-          const int jj = W.n0 + wn * 16 + ni * 8 + 2 * q + hh;
-          if (jj >= nc) continue;
-          const long long col = a.ib_all[W.ib_off + jj] - 1;
-          const double v = acc[mi][ni][hh];
-          const long long e1 = row + col * a.n_basis + t * nb2;
-          add_fixed(acc_lo + e1, acc_hi + e1, v, s);
-          if (SYM && W.n0 != W.m0) {
-            const long long e2 = col + row * a.n_basis + t * nb2;
-            add_fixed(acc_lo + e2, acc_hi + e2, v, s);
-          }
+          const long long c = col[ni][hh];
+          long long lo, hi;
+          if (c < 0 || !to_fixed(acc[mi][ni][hh], scale, &lo, &hi)) continue;
+          add_fixed(entries + row + c * a.n_basis, lo, hi);
+          if (SYM && !diag) add_fixed(entries + c + row * a.n_basis, lo, hi);
         }
     }
   }
 }
 
-// out(e) += (the 128-bit entry) 2^-s, one rounding; entries no tile touched add 0.
-__global__ void h1_finalize_kernel(long long n, const unsigned long long *__restrict__ acc, const int *emax_p,
-                                   int n_batches, double *__restrict__ out) {
-  const int emax = *emax_p;
+// out(e) += (the entry) 2^-s, one rounding; entries no tile touched add 0.  The
+// entries are zeroed for the next call.
+__global__ void h1_finalize_kernel(long long n, ulonglong2 *__restrict__ acc_all, const int *emax_p, int n_batches,
+                                   double *__restrict__ out_all) {
+  const int t = blockIdx.y, emax = emax_p[t];
+  ulonglong2 *acc = acc_all + n * t;
+  double *out = out_all + n * t;
   if (emax == EMAX_EMPTY) return;
-  const int s = fixed_scale(emax, n_batches);
+  const int s = fixed_scale(emax, n_batches), low = fixed_point(n_batches).low;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const __int128 x = (__int128)(((unsigned __int128)acc[n + e] << 64) | acc[e]);
+    const ulonglong2 w = acc[e];
+    if ((w.x | w.y) == 0) continue;
+    acc[e] = make_ulonglong2(0, 0);
+    const __int128 x = (__int128)(long long)w.y * ((__int128)1 << low) + (__int128)(long long)w.x;
     if (x == 0) continue;
     // magnitude as two unsigned words of one sign: no cancellation, the
     // result within 2 ulp, and the same bits on every run
@@ -396,28 +512,62 @@ __global__ void h1_finalize_kernel(long long n, const unsigned long long *__rest
 
 }  // namespace
 
-size_t rho1_h1_item_size() { return sizeof(H1Item); }
-
-// Packs (batch, i tile, j tile, t) items; `sym` keeps the tiles with j >= i.
-void rho1_h1_build_items(const int *nc_b, const int *np_b, const int *ib_off, const int *prefix,
-                         const long long *wave_off, int n_batches, int T, bool sym,
-                         std::vector<unsigned char> *host) {
+// Groups of batches, in locality order (`key`, then cost, so that the entries
+// neighbouring batches share are added to while they are in L2), whose A fits
+// H1_A_BYTES; per group its batches (one item each, for the first pass), its
+// tiles and its tiles with j >= i.
+void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *host,
+                         std::vector<H1Group> *groups, long long *a_len) {
+  std::vector<Rho1WorkItem> order;
+  for (const Rho1WorkItem &b : batches)
+    if (b.nc > 0 && b.np > 0) order.push_back(b);
+  rho1_order_items(&order, 2);
   std::vector<H1Item> v;
-  for (int b = 0; b < n_batches; ++b) {
-    if (nc_b[b] <= 0 || np_b[b] <= 0) continue;
-    for (int t = 0; t < T; ++t)
-      for (int m0 = 0; m0 < nc_b[b]; m0 += BM)
-        for (int n0 = sym ? m0 : 0; n0 < nc_b[b]; n0 += BN)
-          v.push_back(H1Item{b, nc_b[b], np_b[b], ib_off[b], prefix[b], m0, n0, t, wave_off[b]});
+  groups->clear();
+  *a_len = 0;
+  for (size_t b0 = 0; b0 < order.size();) {
+    std::vector<H1Item> first, tiles, upper;
+    long long len = 0;
+    size_t b1 = b0;
+    for (; b1 < order.size(); ++b1) {
+      const Rho1WorkItem &b = order[b1];
+      const long long need = (long long)((b.nc + 3) & ~3) * b.np;
+      if (b1 > b0 && (len + need) * (long long)sizeof(double) > H1_A_BYTES) break;
+      const int parts = ceil_div(b.nc, TILE), w = (ceil_div(b.nc, parts) + 7) / 8 * 8;
+      H1Item it{b.batch, b.nc, b.np, b.ib_off, b.prefix, 0, 0, 0, 0, 0, b.wave_off, len};
+      first.push_back(it);
+      for (it.m0 = 0; it.m0 < b.nc; it.m0 += w)
+        for (it.n0 = 0; it.n0 < b.nc; it.n0 += w) {
+          it.mw = std::min(w, b.nc - it.m0);
+          it.nw = std::min(w, b.nc - it.n0);
+          tiles.push_back(it);
+          if (it.n0 >= it.m0) upper.push_back(it);
+        }
+      len += need;
+    }
+    const int at = (int)v.size(), n1 = (int)first.size(), n2 = (int)tiles.size(), n3 = (int)upper.size();
+    groups->push_back(H1Group{at, n1, at + n1, n2, at + n1 + n2, n3});
+    for (const std::vector<H1Item> *part : {&first, &tiles, &upper}) v.insert(v.end(), part->begin(), part->end());
+    *a_len = std::max(*a_len, len);
+    b0 = b1;
   }
   host->resize(v.size() * sizeof(H1Item));
   if (!v.empty()) memcpy(host->data(), v.data(), host->size());
 }
 
-// Accumulator scratch: two words per entry of (n_basis, n_basis, T), plus the
-// exponent word; allocated by the first call (outside stream capture).
+// Scratch: the accumulator, two words per entry of (n_basis, n_basis, T), zero
+// between calls (the finalize pass clears what the tiles touched), the exponent
+// words, and A of one group; allocated by the first call (outside stream capture).
 static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
   if (plan.d_h1_acc) return FRPA_OK;
+  static PerDeviceOnce configured;
+  FRPA_TRY(configured.run(plan.device, []() -> int {
+    FRPA_CUDA_TRY(cudaFuncSetAttribute(h1_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       TileShape<true>::SMEM));
+    FRPA_CUDA_TRY(cudaFuncSetAttribute(h1_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       TileShape<false>::SMEM));
+    return FRPA_OK;
+  }));
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   FRPA_CUDA_TRY(cudaStreamIsCapturing(stream, &cap));
   if (cap != cudaStreamCaptureStatusNone)
@@ -425,27 +575,38 @@ static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
                 "first-order H / adjoint: the accumulator is allocated by the first call; call once before "
                 "capturing a graph");
   const size_t n = (size_t)plan.n_basis * plan.n_basis * plan.T;
-  if (cudaMalloc((void **)&plan.d_h1_acc, 2 * n * sizeof(unsigned long long) + 256) != cudaSuccess) {
+  const size_t words = 2 * sizeof(unsigned long long) * n, flags = (sizeof(int) * plan.T + 255) / 256 * 256;
+  const size_t bytes = words + flags + sizeof(double) * (size_t)plan.h1_a_len;
+  if (cudaMalloc((void **)&plan.d_h1_acc, bytes) != cudaSuccess) {
     plan.d_h1_acc = nullptr;
-    return fail(FRPA_ERR_OOM, "first-order H / adjoint: %zu bytes of accumulator could not be allocated",
-                2 * n * sizeof(unsigned long long) + 256);
+    return fail(FRPA_ERR_OOM, "first-order H / adjoint: %zu bytes of scratch could not be allocated", bytes);
   }
+  plan.h1_clean = false;
   return FRPA_OK;
 }
 
-// mode 0: the adjoint over the full tile list; mode 1: the first-order H over
-// the symmetric one.  `out` (n_basis, n_basis, T) is accumulated into.
+template <bool SYM>
+static int h1_tiles(const Rho1Plan &plan, const H1Item *items, int n_items, int t, const H1Args &a, int n_sm,
+                    cudaStream_t stream) {
+  const int grid = std::min(n_items, n_sm * TileShape<SYM>::CTAS);
+  h1_tile_kernel<SYM><<<grid, THREADS, TileShape<SYM>::SMEM, stream>>>(items, n_items, t, a);
+  FRPA_LAUNCH_CHECK();
+  return FRPA_OK;
+}
+
+// mode 0: the adjoint over all tiles; mode 1: the first-order H over the tiles
+// with j >= i.  `out` (n_basis, n_basis, T) is accumulated into.
 static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, const double *gwave,
                   const double *g_rho, const double *g_grad, const H1Inputs *h, double *out, cudaStream_t stream) {
-  const void *items = mode == 1 ? plan.d_h1_items_sym : plan.d_adj_items;
-  const int n_items = mode == 1 ? plan.n_h1_items_sym : plan.n_adj_items;
-  if (n_items == 0) return FRPA_OK;
+  if (plan.h1_groups.empty()) return FRPA_OK;
   FRPA_TRY(h1_scratch(plan, stream));
-  const size_t n = (size_t)plan.n_basis * plan.n_basis * plan.T;
-  unsigned long long *acc = plan.d_h1_acc;
-  int *emax = reinterpret_cast<int *>(acc + 2 * n);
-  FRPA_CUDA_TRY(cudaMemsetAsync(acc, 0, 2 * n * sizeof(unsigned long long), stream));
-  FRPA_CUDA_TRY(cudaMemsetAsync(emax, 0x80, sizeof(int), stream));
+  const size_t nb2 = (size_t)plan.n_basis * plan.n_basis, n = nb2 * plan.T;
+  ulonglong2 *acc = reinterpret_cast<ulonglong2 *>(plan.d_h1_acc);
+  int *emax = reinterpret_cast<int *>(acc + n);
+  // zero already unless this is the first call or an earlier one failed half-way
+  if (!plan.h1_clean) FRPA_CUDA_TRY(cudaMemsetAsync(acc, 0, n * sizeof(ulonglong2), stream));
+  plan.h1_clean = false;
+  FRPA_CUDA_TRY(cudaMemsetAsync(emax, 0x80, sizeof(int) * plan.T, stream));
   H1Args a{};
   a.mode = mode;
   a.n_active = n_active;
@@ -461,22 +622,41 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
   a.g_grad = g_grad;
   if (h) a.h = *h;
   a.acc = acc;
-  a.n_entries = (long long)n;
+  a.A = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(emax) + (sizeof(int) * plan.T + 255) / 256 * 256);
   a.emax = emax;
   a.err = plan.d_err;
-  const H1Item *it = static_cast<const H1Item *>(items);
-  h1_bound_kernel<<<n_items, THREADS, 0, stream>>>(it, n_items, a);
-  FRPA_LAUNCH_CHECK();
+  a.grad = mode == 1 || g_grad != nullptr;
+  a.aligned16 = plan.wave_aligned16 && !(((uintptr_t)wave | (uintptr_t)gwave) & 15);
+  const H1Item *items = static_cast<const H1Item *>(plan.d_h1_items);
   int n_sm = 148;
   FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, plan.device));
-  const int grid = std::min(n_items, n_sm * 4);
-  if (mode == 1)
-    h1_tile_kernel<true><<<grid, THREADS, 0, stream>>>(it, n_items, a);
-  else
-    h1_tile_kernel<false><<<grid, THREADS, 0, stream>>>(it, n_items, a);
-  FRPA_LAUNCH_CHECK();
-  h1_finalize_kernel<<<n_sm * 8, 256, 0, stream>>>((long long)n, acc, emax, plan.n_batches, out);
-  FRPA_LAUNCH_CHECK();
+  const bool one_group = plan.h1_groups.size() == 1;
+  // the adjoint's g_grad covers every perturbation, everything else the active ones
+  const int n_t = mode == 0 && g_grad ? plan.T : std::max(0, n_active);
+  for (int t = 0; t < n_t; ++t) {
+    if (!one_group) {
+      for (const H1Group &g : plan.h1_groups) {
+        h1_combine_kernel<false, true><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
+        FRPA_LAUNCH_CHECK();
+      }
+    }
+    for (const H1Group &g : plan.h1_groups) {
+      if (one_group)
+        h1_combine_kernel<true, true><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
+      else
+        h1_combine_kernel<true, false><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
+      FRPA_LAUNCH_CHECK();
+      if (mode == 1)
+        FRPA_TRY(h1_tiles<true>(plan, items + g.upper, g.n_upper, t, a, n_sm, stream));
+      else
+        FRPA_TRY(h1_tiles<false>(plan, items + g.tiles, g.n_tiles, t, a, n_sm, stream));
+    }
+  }
+  if (n_t > 0) {
+    h1_finalize_kernel<<<dim3(n_sm * 8, n_t), 256, 0, stream>>>((long long)nb2, acc, emax, plan.n_batches, out);
+    FRPA_LAUNCH_CHECK();
+  }
+  plan.h1_clean = true;
   return FRPA_OK;
 }
 

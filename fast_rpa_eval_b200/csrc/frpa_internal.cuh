@@ -151,6 +151,12 @@ struct I8Group {
   int sa_len, sb_len;
 };
 
+// Adjoint / first-order H: ranges of the work list for a group of batches (its
+// batches, its (i, j) tiles, those with j >= i).
+struct H1Group {
+  int first, n_first, tiles, n_tiles, upper, n_upper;
+};
+
 struct Rho1Plan {
   int device = 0;
   int T = 1;
@@ -170,13 +176,13 @@ struct Rho1Plan {
   int *d_map = nullptr;       // i_valid_point_2_i_full_points_map
   int *d_counter = nullptr;   // persistent scheduler cursor
   int grid_fp64 = 0;
-  // adjoint work list (batch, i tile, j tile, t), built with the plan, and
-  // the first-order H's list of the tiles with j >= i; their 128-bit
-  // fixed-point accumulator (allocated by the first call)
-  void *d_adj_items = nullptr;
-  int n_adj_items = 0;
-  void *d_h1_items_sym = nullptr;
-  int n_h1_items_sym = 0;
+  // adjoint and first-order H: work list in groups (first_order_h.cu), built
+  // with the plan, and the scratch that the first call allocates: fixed-point
+  // accumulator (zero between calls while h1_clean) and A of one group
+  void *d_h1_items = nullptr;
+  std::vector<H1Group> h1_groups;
+  long long h1_a_len = 0;
+  bool h1_clean = false;
   unsigned long long *d_h1_acc = nullptr;
   // split-BF16 path: <= 128-point tiles, per-row P1 scales, device error flags
   Rho1WorkItem *d_items_split = nullptr;
@@ -256,9 +262,8 @@ int rho1_bias_part2_launch(const Rho1Plan &plan, const int *h_atom_valid, const 
                            const double *gwave, const double *dm, double *bias, cudaStream_t stream);
 // First-order H and the rho1 adjoint (first_order_h.cu): deterministic
 // fixed-point accumulation into an (n_basis, n_basis, T) output.
-size_t rho1_h1_item_size();
-void rho1_h1_build_items(const int *nc_b, const int *np_b, const int *ib_off, const int *prefix,
-                         const long long *wave_off, int n_batches, int T, bool sym, std::vector<unsigned char> *host);
+void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *host,
+                         std::vector<H1Group> *groups, long long *a_len);
 int rho1_adjoint_run(Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *g_rho,
                      const double *g_grad, double *dP1, cudaStream_t stream);
 int rho1_first_order_h_run(Rho1Plan &plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,

@@ -106,3 +106,82 @@ def test_first_order_h_flags_a_range_outside_its_batch():
     torch.cuda.synchronize()
     assert plan.device_flags() & 8
     assert torch.isfinite(H).all()
+
+
+@pytest.mark.parametrize("nc,np_range,shift,T", [
+    (1, (1, 3), 0, 1),        # one function, fewer points than a chunk
+    (63, (15, 17), 0, 2),     # one tile, either side of a 16-point chunk
+    (66, (31, 64), 1, 1),     # two tiles of 40 and 26 rows; odd wave offsets (8-byte copies)
+    (130, (257, 260), 0, 1),  # three tiles of 48, 48 and 34; points past one coefficient stage
+])
+def test_tile_edges_match_oracle(nc, np_range, shift, T):
+    """Adjoint (g_rho only, both, g_grad only) and first-order H at the edges of
+    tiles, chunks and copy widths.  Sums of at most 260 x 12 terms a batch."""
+    p = synth.make_rho1_problem(T=T, seed=200 + nc, n_atoms=8, n_batches=12, np_range=np_range, nc_range=(nc, nc),
+                                pad_value=np.nan, with_bias=True)
+    xc = synth.first_order_h_inputs(p, seed=5, pad_value=np.nan)
+    if shift:
+        p.wave = np.concatenate([np.full(shift, np.nan), p.wave])
+        p.gradient_wave = np.concatenate([np.full(3 * shift, np.nan), p.gradient_wave])
+        xc["hessian_wave"] = np.concatenate([np.full(6 * shift, np.nan), xc["hessian_wave"]])
+        p.i_batch_2_wave_offset = (p.i_batch_2_wave_offset + shift).astype(np.int32)
+    rng = np.random.default_rng(nc)
+    v = np.asfortranarray(rng.normal(size=(p.n_full_points, T)))
+    plan = _lib.Rho1Plan(p)
+    d, vd, pt, av = _device_inputs(p, xc, v)
+    w, gw, n = dev(p.wave), dev(p.gradient_wave), p.n_basis * p.n_basis * T
+    H = torch.zeros(n, dtype=torch.float64, device="cuda")
+    plan.first_order_h(T, p.n_atoms, 1, 2, av, w, gw, d["hessian_wave"], d, vd, pt, H)
+    ref = oracle.first_order_h(p, v, use_reference=oracle.ref_available(T), xc=xc, j_coord=2)
+    assert normwise_rel(host(H, ref.shape), ref) < TOL
+    # the adjoint, per batch in numpy
+    gr = rng.normal(size=(p.n_full_points, T))
+    gg = rng.normal(size=(3, p.n_max_batch_size, p.n_my_batches_work, T))
+    for use_r, use_g in ((True, False), (True, True), (False, True)):
+        want = np.zeros((p.n_basis, p.n_basis, T))
+        for b in range(p.n_my_batches_work):
+            o, npb, ncp = int(p.i_batch_2_wave_offset[b]), int(p.n_point_batches[b]), (nc + 3) // 4 * 4
+            phi = p.wave[o:o + ncp * npb].reshape(npb, ncp)[:, :nc]
+            gphi = p.gradient_wave[3 * o:3 * (o + ncp * npb)].reshape(npb, 3, ncp)[:, :, :nc]
+            pre = p.n_point_batches_prefix_sum[b]
+            ib = p.i_basis_batches[:nc, b] - 1
+            for t in range(T):
+                a = np.zeros((npb, nc))
+                if use_r:
+                    a += gr[p.i_valid_point_2_i_full_points_map[pre:pre + npb], t][:, None] * phi
+                if use_g:
+                    a += 2.0 * np.einsum("kp,pki->pi", gg[:, :npb, b, t], gphi)
+                want[np.ix_(ib, ib, [t])] += (a.T @ phi)[:, :, None]
+        dP1 = torch.zeros(n, dtype=torch.float64, device="cuda")
+        plan.adjoint_p1(T, w, gw, dev(gr) if use_r else None, dev(gg) if use_g else None, dP1)
+        assert normwise_rel(host(dP1, want.shape), want) < TOL
+    assert plan.device_flags() == 0
+
+
+def test_adjoint_over_several_scratch_groups_equals_the_sum_of_its_parts():
+    """A problem whose A(i, p) exceeds the scratch (several groups of batches)
+    against its two halves, each within it."""
+    from fast_rpa_eval_b200 import parallel
+
+    p = synth.config2(seed=3, n_batches=1250)
+    assert 8 * p.wave_len > (512 << 20)
+    n = p.n_basis * p.n_basis
+    rng = np.random.default_rng(1)
+    g_rho = dev(rng.normal(size=p.n_full_points))
+
+    def run(q):
+        w = torch.empty(q.wave_len, dtype=torch.float64, device="cuda")
+        gw = torch.empty(3 * q.wave_len, dtype=torch.float64, device="cuda")
+        _lib.synth_basis_values(q, dev(np.asfortranarray(q.valid_points_xyz.T)), w, gw)
+        plan, out = _lib.Rho1Plan(q), torch.zeros(n, dtype=torch.float64, device="cuda")
+        for _ in range(2):  # the second call starts from the accumulator the first one left
+            plan.adjoint_p1(1, w, gw, g_rho, None, out)
+        assert plan.device_flags() == 0
+        return out
+
+    whole = run(p)
+    halves = [parallel.select_batches(p, np.arange(a, b)) for a, b in ((0, 600), (600, 1250))]
+    assert all(8 * h.wave_len < (512 << 20) for h in halves)
+    parts = run(halves[0]) + run(halves[1])
+    assert float((whole - parts).abs().max()) < 1e-13 * float(parts.abs().max())
+    assert float(parts.abs().max()) > 0
