@@ -43,7 +43,7 @@ constexpr int STAGES = 2;    // cp.async pipeline depth (double buffering)
 constexpr int LDA = BM + 4;  // As[k][m]: stride = 4 (mod 16) doubles -> conflict-free fragment loads
 constexpr int LDB = KC + 4;  // Bs[n][k]: stride = 4 (mod 16) doubles, rows 16-byte aligned
 constexpr int MAX_NC = FRPA_MAX_N_COMPUTE;
-constexpr int WM = BM / 32;  // warps along M (warp tile 32 x 16)
+constexpr int RG = 4;        // warps along the rows, one per SM sub-partition
 // Epilogue staging: a finished 64-row work1 tile is written to the stage that
 // its last K chunk used (rows 0-31 in A's buffer, rows 32-63 in B's), 64
 // points per round, each point's 32 rows at a stride of LDW doubles
@@ -52,18 +52,24 @@ constexpr int LDW = 34;
 static_assert(BM == 64, "the epilogue staging assumes 64-row tiles");
 static_assert(64 * LDW <= KC * LDA && 64 * LDW <= 64 * LDB, "a 64-point work1 half-tile fits a stage buffer");
 
-// Tile shapes: BN points per work item, 2 warps along M x BN / 16 along N,
-// warp tile 32 x 16, 32-wide K chunks.  BN = 64: 256 threads, 2 CTAs per SM
-// (84 KB of shared memory each, up to 128 registers); BN = 128: 512 threads,
-// one CTA per SM, each gathered P1c tile serving twice the points.
+// Tile shapes: BN points per work item, 4 warps along the rows x BN / 32 along the
+// points, 32-wide K chunks.  BN = 64: 256 threads, 2 CTAs per SM (84 KB of shared
+// memory each, up to 128 registers); BN = 128: 512 threads, one CTA per SM, each
+// gathered P1c tile serving twice the points.
+// A warp's 16 x 32 tile is two 8-row blocks, RG apart, by four 8-point blocks,
+// BN / 32 apart.  The four warps of one column group are the SM's four
+// sub-partitions, each with a tensor pipe of its own: dealing the row blocks out
+// to them in turn loads the pipes equally whatever the tile's width and up to 8
+// rows in n_compute (with sub-partitions along the points, a tile of 50 points
+// left one pipe half idle and one of 32 points two of them, in every CTA alike).
 // The loop is issue-bound, not MMA-bound, when its bookkeeping is heavy: every
 // step advances its (t, row tile, K chunk) position by increments (no integer
-// division), and warps whose 32 x 16 tile and K chunk are complete run an
-// unpredicated MMA loop.
+// division), and each warp runs an MMA loop for its number of blocks without
+// predicates.
 template <int BN, bool BIAS>
 struct Fp64Shape {
-  static constexpr int WN = BN / 16;
-  static constexpr int THREADS = 32 * WM * WN;
+  static constexpr int CG = BN / 32;  // warps along the points
+  static constexpr int THREADS = 32 * RG * CG;
   static constexpr int MIN_BLOCKS = (BN == 64 && BM == 64) ? 2 : 1;
 };
 
@@ -71,7 +77,7 @@ template <int BN>
 struct Smem {
   double A[STAGES][KC * LDA];
   double B[STAGES][BN * LDB];
-  double red[WM][4][BN];
+  double red[4][BN];
   int ib[MAX_NC];
   int rs[FRPA_MAX_ATOM_TILE], re[FRPA_MAX_ATOM_TILE];  // fused bias: each perturbation's compute range
   int nkb;                                             // fused bias: K chunks per row tile
@@ -97,6 +103,45 @@ __device__ __forceinline__ void step_advance(int &kk, int &mt, int &t, int nKs, 
   }
 }
 
+// One chunk's products of a warp: CM of its row blocks, CN of its point blocks,
+// nks steps of 4 along K.
+template <int CM, int CN, int CG>
+__device__ __forceinline__ void chunk_mma(double (&acc)[2][4][2], const double *A, const double *B, int nks) {
+  auto step = [&](int ks) {
+    double a[CM], b[CN];
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi) a[mi] = A[ks * 4 * LDA + mi * RG * 8];
+#pragma unroll
+    for (int ni = 0; ni < CN; ++ni) b[ni] = B[ni * CG * 8 * LDB + ks * 4];
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < CN; ++ni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
+  };
+  if (nks == KC / 4) {
+#pragma unroll
+    for (int ks = 0; ks < KC / 4; ++ks) step(ks);
+  } else {
+#pragma unroll 1
+    for (int ks = 0; ks < nks; ++ks) step(ks);
+  }
+}
+template <int CG>
+__device__ __forceinline__ void chunk_mma_any(int shape, double (&acc)[2][4][2], const double *A, const double *B,
+                                              int nks) {
+  switch (shape) {  // 4 (CM - 1) + CN, uniform over the warp; 0: nothing
+    case 1: chunk_mma<1, 1, CG>(acc, A, B, nks); break;
+    case 2: chunk_mma<1, 2, CG>(acc, A, B, nks); break;
+    case 3: chunk_mma<1, 3, CG>(acc, A, B, nks); break;
+    case 4: chunk_mma<1, 4, CG>(acc, A, B, nks); break;
+    case 5: chunk_mma<2, 1, CG>(acc, A, B, nks); break;
+    case 6: chunk_mma<2, 2, CG>(acc, A, B, nks); break;
+    case 7: chunk_mma<2, 3, CG>(acc, A, B, nks); break;
+    case 8: chunk_mma<2, 4, CG>(acc, A, B, nks); break;
+    default: break;
+  }
+}
+
 template <int BN, bool BIAS>
 __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BIAS>::MIN_BLOCKS)
     rho1_fp64_kernel(const Rho1WorkItem *__restrict__ items, int n_items, int *__restrict__ counter,
@@ -105,13 +150,12 @@ __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BI
                      const double *__restrict__ gwave, const double *__restrict__ P1,
                      const double *__restrict__ bias, const double *__restrict__ gbias, double *__restrict__ rho,
                      double *__restrict__ grad, int aligned16, FusedBias fb) {
-  constexpr int THREADS = Fp64Shape<BN, BIAS>::THREADS, WN = Fp64Shape<BN, BIAS>::WN;
+  constexpr int THREADS = Fp64Shape<BN, BIAS>::THREADS, CG = Fp64Shape<BN, BIAS>::CG;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem<BN> &S = *reinterpret_cast<Smem<BN> *>(smem_raw);
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const int wm = warp / WN, wn = warp % WN;
-  const int col_w = wn * 16;  // this warp's first point in the tile
+  const int rg = warp % RG, cg = warp / RG;  // row blocks rg, rg + RG; point blocks cg, cg + CG, ...
   const int g = lane >> 2, q = lane & 3;
   const long long nb2 = (long long)n_basis * n_basis;
 
@@ -224,11 +268,11 @@ __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BI
       }
     };
 
-    double acc[4][2][2];
+    double acc[2][4][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+      for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
     // per-point sums: after each row tile's epilogue lane l of warp w holds the
     // sum (over rows so far) of component c = (l % NV) / PPW (rho1, d/dx, d/dy,
     // d/dz) of point w PPW + (l % NV) % PPW of each 64-point round
@@ -251,14 +295,14 @@ __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BI
 #pragma unroll
         for (int r = 0; r < ROUNDS; ++r) {
           const int idx = lane & (NV - 1);
-          S.red[0][idx / PPW][r * 64 + warp * PPW + idx % PPW] = tot[r];
+          S.red[idx / PPW][r * 64 + warp * PPW + idx % PPW] = tot[r];
           tot[r] = 0.0;
         }
       }
       __syncthreads();
       if (tid < pn) {
         const int p = W.p0 + tid;
-        const double r = S.red[0][0][tid], gx = S.red[0][1][tid], gy = S.red[0][2][tid], gz = S.red[0][3][tid];
+        const double r = S.red[0][tid], gx = S.red[1][tid], gy = S.red[2][tid], gz = S.red[3][tid];
         const long long bidx = p + (long long)n_max_batch_size * (W.batch + (long long)n_batches * t);
         const long long gi = 3 * bidx;
         grad[gi + 0] = gx * 2 - gbias[gi + 0];
@@ -281,15 +325,16 @@ __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BI
       __syncthreads();  // every warp's MMAs are done with this stage's operands
 #pragma unroll
       for (int round = 0; round < ROUNDS; ++round) {
-        if (col_w / 64 == round) {
-          double *Wh = wm == 0 ? Wa : Wb;
 #pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
+        for (int mi = 0; mi < 2; ++mi) {
+          double *Wh = mi == 0 ? Wa : Wb;
 #pragma unroll
-            for (int ni = 0; ni < 2; ++ni)
+          for (int ni = 0; ni < 4; ++ni)
+            if (ni * CG / 8 == round) {
 #pragma unroll
               for (int h = 0; h < 2; ++h)
-                Wh[((col_w & 63) + ni * 8 + 2 * q + h) * LDW + mi * 8 + g] = acc[mi][ni][h];
+                Wh[(((ni * CG + cg) * 8 + 2 * q + h) & 63) * LDW + rg * 8 + g] = acc[mi][ni][h];
+            }
         }
         __syncthreads();
         double v[NV];
@@ -341,11 +386,12 @@ __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BI
         if (round + 1 < ROUNDS) __syncthreads();  // the next round rewrites the staging
       }
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
+      for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+        for (int ni = 0; ni < 4; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
     };
 
+    const int cn = ((pn + 7) / 8 - cg + CG - 1) / CG;  // this warp's point blocks (0..4)
     int kk = 0, mt = 0, t = 0;
     for (int s = 0; s < steps; ++s) {
       cp_async_wait<STAGES - 2>();
@@ -354,43 +400,12 @@ __global__ void __launch_bounds__(Fp64Shape<BN, BIAS>::THREADS, Fp64Shape<BN, BI
       cp_async_commit();
 
       const int m0 = mt * BM;
-      const double *As = S.A[s % STAGES];
-      const double *Bs = S.B[s % STAGES];
-      const int row_w = m0 + wm * 32;
       // valid K extent of this chunk: the compute functions, or the bias range
       const int klim = (!BIAS || kk < nKc) ? nc - kk * KC : (S.re[t] - S.rs[t]) - (kk - nKc) * KC;
-      if (row_w + 32 <= nc && col_w + 16 <= pn && klim >= KC) {
-        // complete warp tile and chunk: no predicates
-#pragma unroll
-        for (int ks = 0; ks < KC / 4; ++ks) {
-          double a[4], b[2];
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi) a[mi] = As[(ks * 4 + q) * LDA + wm * 32 + mi * 8 + g];
-#pragma unroll
-          for (int ni = 0; ni < 2; ++ni) b[ni] = Bs[(col_w + ni * 8 + g) * LDB + ks * 4 + q];
-#pragma unroll
-          for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 2; ++ni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
-        }
-      } else if (row_w < nc && col_w < pn) {
-        const int nmi = min(4, (nc - row_w + 7) / 8), nni = min(2, (pn - col_w + 7) / 8);
-#pragma unroll
-        for (int ks = 0; ks < KC / 4; ++ks) {
-          if (ks * 4 < klim) {
-            double a[4], b[2];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi) a[mi] = As[(ks * 4 + q) * LDA + wm * 32 + mi * 8 + g];
-#pragma unroll
-            for (int ni = 0; ni < 2; ++ni) b[ni] = Bs[(col_w + ni * 8 + g) * LDB + ks * 4 + q];
-#pragma unroll
-            for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-              for (int ni = 0; ni < 2; ++ni)
-                if (mi < nmi && ni < nni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
-          }
-        }
-      }
+      const int blocks = min(BM / 8, (nc - m0 + 7) / 8);
+      const int cm = (blocks - rg + RG - 1) / RG;  // this warp's row blocks (0..2)
+      chunk_mma_any<CG>(cm > 0 && cn > 0 ? 4 * (cm - 1) + cn : 0, acc, S.A[s % STAGES] + q * LDA + rg * 8 + g,
+                        S.B[s % STAGES] + (cg * 8 + g) * LDB + q, min(KC / 4, (klim + 3) / 4));
 
       if (kk == nKc - 1) {
         tile_epilogue(s % STAGES, m0, false);  // work1 tile: contract with phi and grad phi
@@ -540,8 +555,7 @@ int rho1_locality_key(const int *ib, int nc) {
   return (int)best;
 }
 
-// Work items of <= tile_points points (a batch's points split evenly, widths a
-// multiple of 8), grouped into FP64_CHUNKS ranges of consecutive batches, each
+// Work items of <= tile_points points (a batch's 8-point blocks split evenly), grouped into FP64_CHUNKS ranges of consecutive batches, each
 // range in the given order.  The ranges hold 6%, 44%, 44% and 6% of the cost
 // (nc^2 np): the host-buffer entry waits for the first range's biases before
 // any compute and for the last range's outputs after it, so those are small.
@@ -570,12 +584,13 @@ void rho1_fp64_build_items(const std::vector<Rho1WorkItem> &batches, int tile_po
     std::vector<Rho1WorkItem> part;
     for (const Rho1WorkItem &b : batches) {
       if (b.np == 0 || b.batch < bounds[c] || b.batch >= bounds[c + 1]) continue;
-      const int tiles = (b.np + tile_points - 1) / tile_points;
-      int w = (b.np + tiles - 1) / tiles;
-      w = std::min(tile_points, (w + 7) & ~7);
-      for (int p0 = 0; p0 < b.np; p0 += w)
+      const int blocks = (b.np + 7) / 8, tiles = (b.np + tile_points - 1) / tile_points;
+      for (int k = 0, p0 = 0; k < tiles; ++k) {  // the 8-point blocks dealt out evenly
+        const int w = 8 * (blocks / tiles + (k < blocks % tiles ? 1 : 0));
         part.push_back(Rho1WorkItem{b.batch, b.nc, b.np, p0, std::min(w, b.np - p0), b.ib_off, b.prefix, b.key,
                                     b.wave_off});
+        p0 += w;
+      }
     }
     rho1_order_items(&part, order);
     out->insert(out->end(), part.begin(), part.end());
