@@ -62,20 +62,21 @@ int synth_basis_values(const frpa_rho1_desc *D, const double *points, int n_atom
 
 static void rho1_plan_free(Rho1Plan *P) {
   if (!P) return;
-  cudaFree(P->d_items);
-  cudaFree(P->d_ib);
-  cudaFree(P->d_map);
-  cudaFree(P->d_counter);
-  cudaFree(P->d_h1_items);
+  for (void *p : {(void *)P->d_items, (void *)P->d_items_small, (void *)P->d_items_split}) P->release(p);
   cudaFree(P->d_h1_acc);
-  cudaFree(P->d_items_split);
-  cudaFree(P->d_rowmax);
-  cudaFree(P->d_err);
+  cudaFree(P->arena);
   rho1_i8_free(P);
   delete P;
 }
 
-static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D) {
+// What a plan is for: the drop-ins, which make one per call, build no lists of
+// other paths.
+enum : unsigned { PLAN_RHO1 = 1, PLAN_SPLIT = 2, PLAN_I8 = 4, PLAN_H1 = 8, PLAN_ALL = 15 };
+unsigned plan_use(int mode) {
+  return PLAN_RHO1 | (mode == FRPA_RHO1_SPLIT_BF16 ? PLAN_SPLIT : mode == FRPA_RHO1_SPLIT_I8 ? PLAN_I8 : 0);
+}
+
+static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D, unsigned use = PLAN_ALL) {
   *out = nullptr;
   FRPA_CHECK_ARG(D != nullptr, "rho1: null descriptor");
   const int T = D->atom_tile_size, nb = D->n_my_batches_work;
@@ -151,38 +152,36 @@ static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D) {
   P->fp64_chunk_items = chunk_items;
   P->fp64_chunk_batches = chunk_batches;
   int st = FRPA_OK;
-  auto up = [&](void **dst, const void *src, size_t bytes) {
-    if (st != FRPA_OK) return;
-    if (cudaMalloc(dst, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-      st = fail(FRPA_ERR_OOM, "rho1: plan allocation of %zu bytes failed", bytes);
-      return;
-    }
-    if (bytes && cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess)
-      st = fail(FRPA_ERR_CUDA, "rho1: plan upload failed");
-  };
-  up((void **)&P->d_items, items.data(), sizeof(Rho1WorkItem) * items.size());
+  PlanMemory mem;
+  std::vector<Rho1WorkItem> small, split;
+  std::vector<unsigned char> h1_items, h1_tiles;
+  mem.array((void **)&P->d_items, items.data(), sizeof(Rho1WorkItem) * items.size());
   P->h_batches = batches;
   P->h_ib = ibc;
-  {
-    std::vector<Rho1WorkItem> split;
+  if (nc_max <= SMALL_MAX_NC && !items.empty()) {
+    rho1_small_build_items(batches, P->order, &small);
+    P->n_items_small = (int)small.size();
+    mem.array((void **)&P->d_items_small, small.data(), sizeof(Rho1WorkItem) * small.size());
+    st = rho1_small_configure(P->device);
+  }
+  if (use & PLAN_SPLIT) {
     rho1_split_build_items(batches, P->split_tile_points, P->order, &split);
     P->n_items_split = (int)split.size();
-    up((void **)&P->d_items_split, split.data(), sizeof(Rho1WorkItem) * split.size());
-    std::vector<double> zeros((size_t)D->n_basis * T, 0.0);
-    up((void **)&P->d_rowmax, zeros.data(), sizeof(double) * zeros.size());
-    const int z = 0;
-    up((void **)&P->d_err, &z, sizeof(int));
+    mem.array((void **)&P->d_items_split, split.data(), sizeof(Rho1WorkItem) * split.size());
   }
-  if (st == FRPA_OK) st = rho1_i8_build(P);
-  up((void **)&P->d_ib, ibc.data(), sizeof(int) * ibc.size());
-  up((void **)&P->d_map, D->i_valid_point_2_i_full_points_map, sizeof(int) * (size_t)map_len);
+  if (use & PLAN_H1) {
+    rho1_h1_build_items(batches, &h1_items, &h1_tiles, &P->h1_groups, &P->h1_a_len);
+    mem.array(&P->d_h1_items, h1_items.data(), h1_items.size());
+    mem.array(&P->d_h1_tiles, h1_tiles.data(), h1_tiles.size());
+  }
   const int zero = 0;
-  up((void **)&P->d_counter, &zero, sizeof(int));
-  {
-    std::vector<unsigned char> h1;
-    rho1_h1_build_items(batches, &h1, &P->h1_groups, &P->h1_a_len);
-    up(&P->d_h1_items, h1.data(), h1.size());
-  }
+  mem.array((void **)&P->d_err, &zero, sizeof(int));
+  mem.array((void **)&P->d_counter, &zero, sizeof(int));
+  mem.array((void **)&P->d_ib, ibc.data(), sizeof(int) * ibc.size());
+  mem.array((void **)&P->d_map, D->i_valid_point_2_i_full_points_map, sizeof(int) * (size_t)map_len);
+  mem.space((void **)&P->d_rowmax, sizeof(double) * (size_t)D->n_basis * T);
+  if (st == FRPA_OK) st = mem.commit(&P->arena, &P->arena_bytes);
+  if (st == FRPA_OK && (use & PLAN_I8)) st = rho1_i8_build(P);
   if (st == FRPA_OK) {
     P->grid_fp64 = rho1_fp64_grid(P->device);
     if (P->grid_fp64 <= 0) st = fail(FRPA_ERR_CUDA, "rho1: kernel attribute / occupancy query failed");
@@ -496,7 +495,7 @@ int frpa_rho1_device_flags(const frpa_rho1_plan *plan, int *flags) {
 }
 
 // Re-uploads a work list (synchronous; not inside a stream capture).
-static int replace_items(Rho1WorkItem **dst, int *count, const std::vector<Rho1WorkItem> &items) {
+static int replace_items(const Rho1Plan &P, Rho1WorkItem **dst, int *count, const std::vector<Rho1WorkItem> &items) {
   Rho1WorkItem *d = nullptr;
   FRPA_CUDA_TRY(cudaMalloc(&d, sizeof(Rho1WorkItem) * std::max<size_t>(items.size(), 1)));
   if (!items.empty() &&
@@ -504,7 +503,7 @@ static int replace_items(Rho1WorkItem **dst, int *count, const std::vector<Rho1W
     cudaFree(d);
     return fail(FRPA_ERR_CUDA, "rho1: work-list upload failed");
   }
-  cudaFree(*dst);
+  P.release(*dst);
   *dst = d;
   *count = (int)items.size();
   return FRPA_OK;
@@ -542,8 +541,12 @@ int frpa_rho1_plan_set_tuning(frpa_rho1_plan *plan, int key, int value) {
   rho1_fp64_build_items(P.h_batches, P.fp64_tile_points, P.order, P.n_batches, &items, &P.fp64_chunk_items,
                         &P.fp64_chunk_batches);
   rho1_split_build_items(P.h_batches, P.split_tile_points, P.order, &split);
-  FRPA_TRY(replace_items(&P.d_items, &P.n_items, items));
-  FRPA_TRY(replace_items(&P.d_items_split, &P.n_items_split, split));
+  FRPA_TRY(replace_items(P, &P.d_items, &P.n_items, items));
+  if (P.n_items_small > 0) {
+    rho1_small_build_items(P.h_batches, P.order, &items);
+    FRPA_TRY(replace_items(P, &P.d_items_small, &P.n_items_small, items));
+  }
+  FRPA_TRY(replace_items(P, &P.d_items_split, &P.n_items_split, split));
   return FRPA_OK;
 }
 
@@ -681,7 +684,8 @@ void evaluate_first_order_rho_reduce_memory_c_v3_batches_atoms_(
                                        i_valid_point_2_i_full_points_map, n_compute_c_batches, i_basis_batches,
                                        i_batch_2_wave_offset);
   Rho1Plan *P = nullptr;
-  if (rho1_plan_build(&P, &d) != FRPA_OK) return;
+  const int mode = g_rho1_mode;
+  if (rho1_plan_build(&P, &d, plan_use(mode)) != FRPA_OK) return;
   const int nb = d.n_my_batches_work;
   const size_t wl = (size_t)P->wave_len, nb2 = (size_t)d.n_basis * d.n_basis * T;
   const size_t nbias = (size_t)d.n_max_batch_size * nb * T, nrho = (size_t)d.n_full_points * T;
@@ -696,7 +700,7 @@ void evaluate_first_order_rho_reduce_memory_c_v3_batches_atoms_(
   if (st == FRPA_OK) st = ensure(5, sizeof(double) * nrho, (void **)&r);
   if (st == FRPA_OK) st = ensure(6, sizeof(double) * 3 * nbias, (void **)&g);
   if (st == FRPA_OK)
-    st = rho1_run(*P, g_rho1_mode, *j_atom_end - *j_atom_begin + 1, w, gw, p1, bi, gb, r, g, s);
+    st = rho1_run(*P, mode, *j_atom_end - *j_atom_begin + 1, w, gw, p1, bi, gb, r, g, s);
   if (st == FRPA_OK && cudaMemcpyAsync(first_order_rho, r, sizeof(double) * nrho, cudaMemcpyDeviceToHost, s) != cudaSuccess)
     st = fail(FRPA_ERR_CUDA, "rho1: download failed");
   if (st == FRPA_OK &&
@@ -740,7 +744,7 @@ void evaluate_first_order_h_reduce_memory_c_v2_(
                                        i_valid_point_2_i_full_points_map, n_compute_c_batches, i_basis_batches,
                                        i_batch_2_wave_offset);
   Rho1Plan *P = nullptr;
-  if (rho1_plan_build(&P, &d) != FRPA_OK) return;
+  if (rho1_plan_build(&P, &d, PLAN_H1) != FRPA_OK) return;
   const int nb = d.n_my_batches_work, nmb = d.n_max_batch_size, nf = d.n_full_points;
   const size_t wl = (size_t)P->wave_len, nH = (size_t)d.n_basis * d.n_basis * T;
   const size_t nav = (size_t)(*n_atoms + 1) * nb, nbt = (size_t)nmb * nb;
@@ -816,7 +820,7 @@ void generate_first_order_rho_bias_part2_(
                                        n_point_batches, pre.data(), ident.data(), n_compute_c_batches,
                                        i_basis_batches, i_batch_2_wave_offset);
   Rho1Plan *P = nullptr;
-  if (rho1_plan_build(&P, &d) != FRPA_OK) return;
+  if (rho1_plan_build(&P, &d, PLAN_RHO1) != FRPA_OK) return;
   const size_t wl = (size_t)P->wave_len, nbias = (size_t)d.n_max_batch_size * nb * T;
   const size_t nav = (size_t)(*n_atoms + 1) * nb, ndm = (size_t)d.n_basis * d.n_basis;
   double *w = nullptr, *gw = nullptr, *dm = nullptr, *bi = nullptr;

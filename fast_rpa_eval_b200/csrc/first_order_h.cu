@@ -66,11 +66,15 @@ constexpr long long H1_A_BYTES = 512LL << 20;  // scratch for A
 constexpr int EMAX_EMPTY = -2139062144;  // 0x80808080: no non-zero bound seen
 constexpr int H1_FLAG_NONFINITE = 16;    // device flag: a non-finite input reached the accumulation
 
+// One batch of a group; its (i, j) tiles are w rows wide (the last one less).
 struct H1Item {
-  int batch, nc, np, ib_off, prefix, t;
-  int m0, n0, mw, nw;  // first row and rows of the tile along i and j (m0, n0 multiples of 8)
+  int batch, nc, np, ib_off, prefix, w;
   long long wave_off;
-  long long a_off;        // the batch's A in the scratch of its group
+  long long a_off;  // the batch's A in the scratch of its group
+};
+struct H1Tile {
+  int item;               // the batch
+  unsigned short m0, n0;  // first row along i and j (multiples of 8)
 };
 
 // Per-point inputs of the first-order H, reference layouts
@@ -382,7 +386,7 @@ struct TileShape {
 
 template <bool SYM>
 __global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
-    h1_tile_kernel(const H1Item *__restrict__ items, int n_items, int t, H1Args a) {
+    h1_tile_kernel(const H1Item *__restrict__ items, const H1Tile *__restrict__ tiles, int n_tiles, int t, H1Args a) {
   // a stage: A of the tile's i rows and phi of its j rows; if SYM, phi of the i rows and A of the j rows
   constexpr int STAGES = TileShape<SYM>::STAGES, ARRAYS = TileShape<SYM>::ARRAYS, BUF = KC * LD;
   extern __shared__ __align__(16) double smem[];
@@ -393,10 +397,13 @@ __global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
   const FixedScale scale = make_scale(emax, a.n_batches);
   ulonglong2 *entries = a.acc + (long long)a.n_basis * a.n_basis * t;
 
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const H1Item W = items[it];
+  H1Tile tile = tiles[blockIdx.x];
+  for (int it = blockIdx.x; it < n_tiles; it += gridDim.x) {
+    const H1Item W = items[tile.item];
+    const int m0 = tile.m0, n0 = tile.n0, mw = min(W.w, W.nc - m0), nw = min(W.w, W.nc - n0);
+    if (it + (int)gridDim.x < n_tiles) tile = tiles[it + gridDim.x];
     const int nc = W.nc, np = W.np, ncp = (nc + 3) & ~3;
-    const bool diag = W.m0 == W.n0;
+    const bool diag = m0 == n0;
     const double *phi = a.wave + W.wave_off, *amat = a.A + W.a_off;
     double acc[4][2][2];
 #pragma unroll
@@ -404,7 +411,7 @@ __global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
 #pragma unroll
       for (int y = 0; y < 2; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
 
-    const int nmi = (W.mw + 7) / 8, nni = (W.nw + 7) / 8;  // 8-row blocks of the tile
+    const int nmi = (mw + 7) / 8, nni = (nw + 7) / 8;  // 8-row blocks of the tile
     // Copies: lane -> two rows of the tile, warp -> points warp and warp + 8 of a
     // chunk.  Rows past n_compute (up to whole blocks) and points past the batch
     // are zero.
@@ -432,11 +439,11 @@ __global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
     auto load = [&](int c) {
       double *S = smem + (c % STAGES) * ARRAYS * BUF;
       const int k0 = c * KC;
-      copy(S, amat, W.m0, nmi, k0, true);
-      copy(S + BUF, phi, W.n0, nni, k0, a.aligned16);
+      copy(S, amat, m0, nmi, k0, true);
+      copy(S + BUF, phi, n0, nni, k0, a.aligned16);
       if (SYM && !diag) {  // a diagonal tile has both on both sides
-        copy(S + 2 * BUF, phi, W.m0, nmi, k0, a.aligned16);
-        copy(S + 3 * BUF, amat, W.n0, nni, k0, true);
+        copy(S + 2 * BUF, phi, m0, nmi, k0, a.aligned16);
+        copy(S + 3 * BUF, amat, n0, nni, k0, true);
       }
     };
     const int nch = (np + KC - 1) / KC;
@@ -466,13 +473,13 @@ __global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int j = (ni * 4 + wn) * 8 + 2 * q + hh;
-        col[ni][hh] = j < W.nw && W.n0 + j < nc ? __ldg(a.ib_all + W.ib_off + W.n0 + j) - 1 : -1;
+        col[ni][hh] = j < nw && n0 + j < nc ? __ldg(a.ib_all + W.ib_off + n0 + j) - 1 : -1;
       }
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi) {
       const int i = (mi * 2 + wm) * 8 + g;
-      if (i >= W.mw || W.m0 + i >= nc) continue;
-      const long long row = __ldg(a.ib_all + W.ib_off + W.m0 + i) - 1;
+      if (i >= mw || m0 + i >= nc) continue;
+      const long long row = __ldg(a.ib_all + W.ib_off + m0 + i) - 1;
 #pragma unroll
       for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
@@ -514,45 +521,48 @@ __global__ void h1_finalize_kernel(long long n, ulonglong2 *__restrict__ acc_all
 
 // Groups of batches, in locality order (`key`, then cost, so that the entries
 // neighbouring batches share are added to while they are in L2), whose A fits
-// H1_A_BYTES; per group its batches (one item each, for the first pass), its
-// tiles and its tiles with j >= i.
-void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *host,
-                         std::vector<H1Group> *groups, long long *a_len) {
+// H1_A_BYTES: one item per batch (for the first pass), and per group its tiles,
+// those with j >= i first (the symmetric H takes only them).
+void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *items,
+                         std::vector<unsigned char> *tile_list, std::vector<H1Group> *groups, long long *a_len) {
   std::vector<Rho1WorkItem> order;
+  order.reserve(batches.size());
   for (const Rho1WorkItem &b : batches)
     if (b.nc > 0 && b.np > 0) order.push_back(b);
   rho1_order_items(&order, 2);
   std::vector<H1Item> v;
+  std::vector<H1Tile> tiles, lower;
+  v.reserve(order.size());
   groups->clear();
   *a_len = 0;
   for (size_t b0 = 0; b0 < order.size();) {
-    std::vector<H1Item> first, tiles, upper;
+    H1Group g{(int)v.size(), 0, (int)tiles.size(), 0, 0};
+    lower.clear();
     long long len = 0;
     size_t b1 = b0;
     for (; b1 < order.size(); ++b1) {
       const Rho1WorkItem &b = order[b1];
       const long long need = (long long)((b.nc + 3) & ~3) * b.np;
       if (b1 > b0 && (len + need) * (long long)sizeof(double) > H1_A_BYTES) break;
-      const int parts = ceil_div(b.nc, TILE), w = (ceil_div(b.nc, parts) + 7) / 8 * 8;
-      H1Item it{b.batch, b.nc, b.np, b.ib_off, b.prefix, 0, 0, 0, 0, 0, b.wave_off, len};
-      first.push_back(it);
-      for (it.m0 = 0; it.m0 < b.nc; it.m0 += w)
-        for (it.n0 = 0; it.n0 < b.nc; it.n0 += w) {
-          it.mw = std::min(w, b.nc - it.m0);
-          it.nw = std::min(w, b.nc - it.n0);
-          tiles.push_back(it);
-          if (it.n0 >= it.m0) upper.push_back(it);
-        }
+      const int w = (ceil_div(b.nc, ceil_div(b.nc, TILE)) + 7) / 8 * 8;
+      for (int m0 = 0; m0 < b.nc; m0 += w)
+        for (int n0 = 0; n0 < b.nc; n0 += w)
+          (n0 >= m0 ? tiles : lower).push_back(H1Tile{(int)v.size(), (unsigned short)m0, (unsigned short)n0});
+      v.push_back(H1Item{b.batch, b.nc, b.np, b.ib_off, b.prefix, w, b.wave_off, len});
       len += need;
     }
-    const int at = (int)v.size(), n1 = (int)first.size(), n2 = (int)tiles.size(), n3 = (int)upper.size();
-    groups->push_back(H1Group{at, n1, at + n1, n2, at + n1 + n2, n3});
-    for (const std::vector<H1Item> *part : {&first, &tiles, &upper}) v.insert(v.end(), part->begin(), part->end());
+    g.n_first = (int)v.size() - g.first;
+    g.n_upper = (int)tiles.size() - g.tiles;
+    tiles.insert(tiles.end(), lower.begin(), lower.end());
+    g.n_tiles = (int)tiles.size() - g.tiles;
+    groups->push_back(g);
     *a_len = std::max(*a_len, len);
     b0 = b1;
   }
-  host->resize(v.size() * sizeof(H1Item));
-  if (!v.empty()) memcpy(host->data(), v.data(), host->size());
+  items->resize(v.size() * sizeof(H1Item));
+  if (!v.empty()) memcpy(items->data(), v.data(), items->size());
+  tile_list->resize(tiles.size() * sizeof(H1Tile));
+  if (!tiles.empty()) memcpy(tile_list->data(), tiles.data(), tile_list->size());
 }
 
 // Scratch: the accumulator, two words per entry of (n_basis, n_basis, T), zero
@@ -586,10 +596,10 @@ static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
 }
 
 template <bool SYM>
-static int h1_tiles(const Rho1Plan &plan, const H1Item *items, int n_items, int t, const H1Args &a, int n_sm,
+static int h1_tiles(const H1Item *items, const H1Tile *tiles, int n_tiles, int t, const H1Args &a, int n_sm,
                     cudaStream_t stream) {
-  const int grid = std::min(n_items, n_sm * TileShape<SYM>::CTAS);
-  h1_tile_kernel<SYM><<<grid, THREADS, TileShape<SYM>::SMEM, stream>>>(items, n_items, t, a);
+  const int grid = std::min(n_tiles, n_sm * TileShape<SYM>::CTAS);
+  h1_tile_kernel<SYM><<<grid, THREADS, TileShape<SYM>::SMEM, stream>>>(items, tiles, n_tiles, t, a);
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
 }
@@ -628,6 +638,7 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
   a.grad = mode == 1 || g_grad != nullptr;
   a.aligned16 = plan.wave_aligned16 && !(((uintptr_t)wave | (uintptr_t)gwave) & 15);
   const H1Item *items = static_cast<const H1Item *>(plan.d_h1_items);
+  const H1Tile *tiles = static_cast<const H1Tile *>(plan.d_h1_tiles);
   int n_sm = 148;
   FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, plan.device));
   const bool one_group = plan.h1_groups.size() == 1;
@@ -647,9 +658,9 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
         h1_combine_kernel<true, false><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
       FRPA_LAUNCH_CHECK();
       if (mode == 1)
-        FRPA_TRY(h1_tiles<true>(plan, items + g.upper, g.n_upper, t, a, n_sm, stream));
+        FRPA_TRY(h1_tiles<true>(items, tiles + g.tiles, g.n_upper, t, a, n_sm, stream));
       else
-        FRPA_TRY(h1_tiles<false>(plan, items + g.tiles, g.n_tiles, t, a, n_sm, stream));
+        FRPA_TRY(h1_tiles<false>(items, tiles + g.tiles, g.n_tiles, t, a, n_sm, stream));
     }
   }
   if (n_t > 0) {

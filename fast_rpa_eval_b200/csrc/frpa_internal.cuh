@@ -3,9 +3,11 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -99,6 +101,53 @@ __device__ __forceinline__ void cp_async_wait() {
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 
+// ---------------------------------------------------------- plan memory --
+
+// A plan's device memory, one allocation: arrays up to 256 KiB go up in one
+// copy, larger ones each from where they are (their sources have to live until
+// commit), workspaces are left as they come.  (One allocation and copy per array
+// made creating a small plan mostly driver calls.)
+struct PlanMemory {
+  static constexpr size_t STAGED = 256 << 10;
+  struct Part {
+    void **dst;
+    const void *src;  // nullptr: staged
+    size_t off, bytes;
+  };
+  std::vector<Part> staged, tail;
+  std::vector<unsigned char> host;
+  size_t tail_bytes = 0;
+
+  static size_t padded(size_t n) { return (std::max<size_t>(n, 8) + 255) / 256 * 256; }
+  void array(void **dst, const void *src, size_t bytes) {
+    if (bytes > STAGED) {
+      tail.push_back({dst, src, tail_bytes, bytes});
+      tail_bytes += padded(bytes);
+      return;
+    }
+    staged.push_back({dst, nullptr, host.size(), bytes});
+    host.resize(host.size() + padded(bytes));
+    if (bytes) memcpy(host.data() + staged.back().off, src, bytes);
+  }
+  void space(void **dst, size_t bytes) {
+    tail.push_back({dst, nullptr, tail_bytes, bytes});
+    tail_bytes += padded(bytes);
+  }
+  int commit(unsigned char **base, size_t *bytes) {
+    *bytes = padded(host.size() + tail_bytes);
+    if (cudaMalloc((void **)base, *bytes) != cudaSuccess) {
+      *base = nullptr;
+      return fail(FRPA_ERR_OOM, "plan: allocation of %zu bytes failed", *bytes);
+    }
+    for (const Part &p : staged) *p.dst = *base + p.off;
+    for (const Part &p : tail) *p.dst = *base + host.size() + p.off;
+    if (!host.empty()) FRPA_CUDA_TRY(cudaMemcpy(*base, host.data(), host.size(), cudaMemcpyHostToDevice));
+    for (const Part &p : tail)
+      if (p.src) FRPA_CUDA_TRY(cudaMemcpy(*p.dst, p.src, p.bytes, cudaMemcpyHostToDevice));
+    return FRPA_OK;
+  }
+};
+
 // ------------------------------------------------------------ rho1 plan --
 
 // One unit of rho1 work: a point tile of one non-empty grid batch
@@ -151,14 +200,22 @@ struct I8Group {
   int sa_len, sb_len;
 };
 
-// Adjoint / first-order H: ranges of the work list for a group of batches (its
-// batches, its (i, j) tiles, those with j >= i).
+// Adjoint / first-order H: ranges of the work lists for a group of batches: its
+// batches, and its (i, j) tiles, the n_upper of them with j >= i first.
 struct H1Group {
-  int first, n_first, tiles, n_tiles, upper, n_upper;
+  int first, n_first, tiles, n_tiles, n_upper;
 };
 
 struct Rho1Plan {
   int device = 0;
+  // one allocation holds the arrays made with the plan; a list replaced later
+  // (a tuning) has its own
+  unsigned char *arena = nullptr;
+  size_t arena_bytes = 0;
+  void release(void *p) const {
+    const unsigned char *c = static_cast<const unsigned char *>(p);
+    if (c && (c < arena || c >= arena + arena_bytes)) cudaFree(p);
+  }
   int T = 1;
   int n_batches = 0;
   int n_full_points = 0;
@@ -176,10 +233,14 @@ struct Rho1Plan {
   int *d_map = nullptr;       // i_valid_point_2_i_full_points_map
   int *d_counter = nullptr;   // persistent scheduler cursor
   int grid_fp64 = 0;
+  // plans whose batches have at most SMALL_MAX_NC functions: the list of
+  // rho1_fp64_small.cu (empty otherwise)
+  Rho1WorkItem *d_items_small = nullptr;
+  int n_items_small = 0;
   // adjoint and first-order H: work list in groups (first_order_h.cu), built
   // with the plan, and the scratch that the first call allocates: fixed-point
   // accumulator (zero between calls while h1_clean) and A of one group
-  void *d_h1_items = nullptr;
+  void *d_h1_items = nullptr, *d_h1_tiles = nullptr;
   std::vector<H1Group> h1_groups;
   long long h1_a_len = 0;
   bool h1_clean = false;
@@ -239,6 +300,11 @@ int rho1_fp64_launch_chunk(const Rho1Plan &plan, int chunk, int n_active, const 
                            const double *P1, const double *bias, const double *gbias, double *rho, double *grad,
                            cudaStream_t stream);
 int rho1_fp64_grid(int device);
+constexpr int SMALL_MAX_NC = 120;  // P1c, two phi tiles and a work1 tile fit one SM's shared memory
+void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int order, std::vector<Rho1WorkItem> *out);
+int rho1_small_configure(int device);
+int rho1_small_launch(const Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *P1,
+                      const double *bias, const double *gbias, double *rho, double *grad, cudaStream_t stream);
 int rho1_fp64_fused_bias_launch(const Rho1Plan &plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,
                                 const int *atom_valid, const double *density_matrix, const double *wave,
                                 const double *gwave, const double *P1, const double *bias, const double *gbias,
@@ -262,8 +328,8 @@ int rho1_bias_part2_launch(const Rho1Plan &plan, const int *h_atom_valid, const 
                            const double *gwave, const double *dm, double *bias, cudaStream_t stream);
 // First-order H and the rho1 adjoint (first_order_h.cu): deterministic
 // fixed-point accumulation into an (n_basis, n_basis, T) output.
-void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *host,
-                         std::vector<H1Group> *groups, long long *a_len);
+void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *items,
+                         std::vector<unsigned char> *tile_list, std::vector<H1Group> *groups, long long *a_len);
 int rho1_adjoint_run(Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *g_rho,
                      const double *g_grad, double *dP1, cudaStream_t stream);
 int rho1_first_order_h_run(Rho1Plan &plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,

@@ -441,6 +441,20 @@ int fp64_grid(int device, int ctas_per_sm) {
   return per_sm * n_sm;
 }
 
+// 16-byte loads need even batch offsets (the plan) and 16-byte aligned arrays
+int rows_aligned16(const Rho1Plan &plan, const double *wave, const double *gwave) {
+  return plan.wave_aligned16 && !(((uintptr_t)wave | (uintptr_t)gwave) & 15);
+}
+
+// Zeros both outputs and the cursor.
+__global__ void clear_outputs_kernel(long long n_rho, double *__restrict__ rho, long long n_grad,
+                                     double *__restrict__ grad, int *__restrict__ counter) {
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if (first == 0) *counter = 0;
+  for (long long e = first; e < n_rho; e += step) rho[e] = 0.0;
+  for (long long e = first; e < n_grad; e += step) grad[e] = 0.0;
+}
+
 // items [item0, item0 + n_items) of the plan's list; the cursor must be zero
 template <int BN, bool BIAS>
 int fp64_launch(const Rho1Plan &plan, int item0, int n_items, int n_active, const double *wave, const double *gwave,
@@ -452,8 +466,7 @@ int fp64_launch(const Rho1Plan &plan, int item0, int n_items, int n_active, cons
   if (grid <= 0) return FRPA_OK;
   FusedBias fb{};
   if (fused) fb = *fused;
-  // 16-byte loads need even batch offsets (the plan) and 16-byte aligned arrays
-  const int aligned16 = plan.wave_aligned16 && !(((uintptr_t)wave | (uintptr_t)gwave) & 15);
+  const int aligned16 = rows_aligned16(plan, wave, gwave);
   rho1_fp64_kernel<BN, BIAS><<<grid, Fp64Shape<BN, BIAS>::THREADS, sizeof(Smem<BN>), stream>>>(
       plan.d_items + item0, n_items, plan.d_counter, plan.d_ib, plan.d_map, plan.T, n_active, plan.n_basis,
       plan.n_full_points, plan.n_max_batch_size, plan.n_batches, wave, gwave, P1, bias, gbias, rho, grad,
@@ -476,12 +489,14 @@ int rho1_fp64_grid(int device) {
 static int fp64_run(const Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *P1,
                     const double *bias, const double *gbias, double *rho, double *grad, const FusedBias *fused,
                     cudaStream_t stream) {
-  // evaluate_first_order_rho.cpp:113-114 zeroes both outputs before the batch loop
-  FRPA_CUDA_TRY(cudaMemsetAsync(rho, 0, sizeof(double) * (size_t)plan.n_full_points * plan.T, stream));
-  FRPA_CUDA_TRY(cudaMemsetAsync(
-      grad, 0, sizeof(double) * 3 * (size_t)plan.n_max_batch_size * plan.n_batches * plan.T, stream));
+  // evaluate_first_order_rho.cpp:113-114 zeroes both outputs before the batch
+  // loop; one launch instead of a memset each and one of the cursor
+  const long long n_rho = (long long)plan.n_full_points * plan.T;
+  const long long n_grad = 3LL * plan.n_max_batch_size * plan.n_batches * plan.T;
+  const int grid = (int)std::min<long long>(1184, ceil_div_ll(std::max({n_rho, n_grad, 1LL}), 512));
+  clear_outputs_kernel<<<grid, 256, 0, stream>>>(n_rho, rho, n_grad, grad, plan.d_counter);
+  FRPA_LAUNCH_CHECK();
   if (plan.n_items == 0) return FRPA_OK;
-  FRPA_CUDA_TRY(cudaMemsetAsync(plan.d_counter, 0, sizeof(int), stream));
   if (fused) {
     if (plan.fp64_tile_points == 128)
       return fp64_launch<128, true>(plan, 0, plan.n_items, n_active, wave, gwave, P1, bias, gbias, rho, grad, fused,
@@ -489,6 +504,8 @@ static int fp64_run(const Rho1Plan &plan, int n_active, const double *wave, cons
     return fp64_launch<64, true>(plan, 0, plan.n_items, n_active, wave, gwave, P1, bias, gbias, rho, grad, fused,
                                  stream);
   }
+  if (plan.n_items_small > 0 && rows_aligned16(plan, wave, gwave))
+    return rho1_small_launch(plan, n_active, wave, gwave, P1, bias, gbias, rho, grad, stream);
   if (plan.fp64_tile_points == 128)
     return fp64_launch<128, false>(plan, 0, plan.n_items, n_active, wave, gwave, P1, bias, gbias, rho, grad, nullptr,
                                    stream);

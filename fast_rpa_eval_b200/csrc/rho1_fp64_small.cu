@@ -1,0 +1,325 @@
+// Plain FP64 first-order density (rho1) and its gradient for plans whose batches
+// all have at most SMALL_MAX_NC compute functions and 16-byte aligned phi rows
+// (rho1_fp64.cu has the semantics and the kernel for everything else; the sums are
+// formed in the same order, so both give the same bits).
+//
+// Such batches are short: the general kernel takes a handful of 32-wide K chunks
+// per row tile, each a memory latency behind a barrier, gathers P1c once per 64
+// points and reads phi again for every row tile and in the epilogue.  Here a CTA
+// (one per SM) gathers the whole P1c of a batch into shared memory once, and its
+// two groups of 8 warps run over the batch's points 16 at a time, each with its own
+// barrier: one group's epilogue overlaps the other's MMAs.  phi of a group's next
+// pass is copied while this one is multiplied, the MMA loop goes through all of K
+// without a barrier, the epilogue takes phi from shared memory, and grad phi (read
+// once) is loaded into registers before the MMAs.
+// Bound: latency (two barriers per pass, one P1c gather per batch), then the FP64
+// tensor pipe.
+#include <algorithm>
+#include <vector>
+
+#include "frpa_internal.cuh"
+
+namespace frpa {
+namespace {
+
+constexpr int THREADS = 512, WARPS = THREADS / 32;
+constexpr int GROUPS = 2, GW = WARPS / GROUPS;  // groups of 8 warps
+constexpr int PTS = 16;                         // points per pass of a group: two 8-point blocks
+constexpr int RG = GW;                          // a group's warps go along the 8-row blocks
+constexpr int LDW = 2 * 64 + 2;  // W[point][row]: 2 (mod 8) doubles, conflict-free fragment stores
+static_assert(SMALL_MAX_NC <= 2 * RG * 8 && PTS == 2 * GW, "two row blocks and two points per warp");
+
+// Leading dimension of the P1c and phi tiles: 4 (mod 16) doubles (conflict-free
+// fragment loads), at least nc rounded up to whole 8-row blocks.
+__host__ __device__ __forceinline__ int small_ld(int nc) { return ((nc + 7) / 8 * 8 + 11) / 16 * 16 + 4; }
+size_t small_smem(int nc_max) {
+  const size_t ld = small_ld(nc_max), rows = (nc_max + 3) & ~3;
+  return sizeof(double) * (rows * ld + GROUPS * (2 * PTS * ld + PTS * LDW));
+}
+
+struct SmallParams {
+  const Rho1WorkItem *items;
+  int n_items, T, n_active, n_basis, n_full_points, n_max_batch_size, n_batches, nc_max;
+  int *counter;
+  const int *ib_all, *map;
+  const double *wave, *gwave, *P1, *bias, *gbias;
+  double *rho, *grad;
+};
+
+// The fragments of step ks + 1 are loaded before the MMAs of step ks: with two
+// warps per sub-partition nothing else covers a shared-memory load.
+template <int CM, int CN>
+__device__ __forceinline__ void small_mma(double (&acc)[2][2][2], const double *A, const double *B, int ld, int nks) {
+  double a[CM], b[CN];
+  auto load = [&](int ks, double (&x)[CM], double (&y)[CN]) {
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi) x[mi] = A[ks * 4 * ld + mi * RG * 8];
+#pragma unroll
+    for (int ni = 0; ni < CN; ++ni) y[ni] = B[ni * 8 * ld + ks * 4];
+  };
+  load(0, a, b);
+#pragma unroll 4
+  for (int ks = 0; ks < nks; ++ks) {
+    double x[CM], y[CN];
+    load(min(ks + 1, nks - 1), x, y);
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < CN; ++ni) dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
+#pragma unroll
+    for (int mi = 0; mi < CM; ++mi) a[mi] = x[mi];
+#pragma unroll
+    for (int ni = 0; ni < CN; ++ni) b[ni] = y[ni];
+  }
+}
+
+// Halves 2 N values over lanes 4 N apart: lanes with that bit keep the upper ones.
+template <int N>
+__device__ __forceinline__ void fold(double (&v)[8], int lane) {
+  const bool upper = (lane & (4 * N)) != 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double keep = upper ? v[i + N] : v[i], give = upper ? v[i] : v[i + N];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * N);
+  }
+}
+
+__global__ void __launch_bounds__(THREADS, 1) rho1_small_kernel(const SmallParams P) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int s_ib[SMALL_MAX_NC], s_next;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = warp / GW, gw = warp % GW;  // gw: this warp's pair of points in the epilogue
+  // first of its row blocks: the second group starts two sub-partitions further, so
+  // that the blocks left over by rounds of 8 fall on different tensor pipes
+  const int rb = (gw + 2 * group) % RG;
+  const int g = lane >> 2, q = lane & 3;
+  const int ld = small_ld(P.nc_max);
+  // As[k][m]; per group Bs[2][n][k] and Ws[n][m]
+  double *As = smem, *Bs = As + ((P.nc_max + 3) & ~3) * ld + group * (2 * PTS * ld + PTS * LDW), *Ws = Bs + 2 * PTS * ld;
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory"); };
+  const long long nb2 = (long long)P.n_basis * P.n_basis;
+
+  for (int it = blockIdx.x; it < P.n_items;) {
+    const Rho1WorkItem W = P.items[it];
+    const int nc = W.nc, ncp = (nc + 3) & ~3, nb = (nc + 7) / 8, nMt = (nc + 63) / 64;
+    const int passes = (W.pn + PTS - 1) / PTS;
+    const int cm = (nb - rb + RG - 1) / RG;  // this warp's row blocks (0..2)
+    if (tid == 0) s_next = (int)gridDim.x + atomicAdd(P.counter, 1);
+    if (tid < nc) s_ib[tid] = __ldg(P.ib_all + W.ib_off + tid) - 1;
+    const double *phi = P.wave + W.wave_off + (long long)W.p0 * ncp;
+    const double *gph = P.gwave + 3 * W.wave_off + 3LL * W.p0 * ncp;
+    // phi of pass j into buffer `buf`: warp -> points, lanes -> 16-byte pieces of a row; zero past n_compute
+    auto load_phi = [&](int j, int buf) {
+      double *B = Bs + buf * PTS * ld;
+      const int left = W.pn - j * PTS;
+#pragma unroll
+      for (int r = 0; r < PTS / GW; ++r) {
+        const int n = gw + r * GW;
+        if (n >= left) break;
+        const double *row = phi + (long long)(j * PTS + n) * ncp;
+        for (int k = 2 * lane; k < ncp; k += 64) {
+          const int bytes = k + 1 < nc ? 16 : (k < nc ? 8 : 0);
+          cp_async_16(B + n * ld + k, bytes ? row + k : row, bytes);
+        }
+      }
+    };
+    for (int t = 0; t < P.T; ++t) {
+      __syncthreads();  // the list is there; the last perturbation's (or item's) tiles are consumed
+      {
+        // P1c(i, k) = P1(ib_i, ib_k): warp -> columns k, lanes -> rows; zero up to whole blocks
+        const double *P1t = P.P1 + t * nb2;
+        for (int k = warp; k < ncp; k += WARPS) {
+          const double *col = P1t + (long long)s_ib[k < nc ? k : 0] * P.n_basis;
+          for (int m = lane; m < nb * 8; m += 32) {
+            const bool ok = m < nc && k < nc;
+            cp_async_8(As + k * ld + m, ok ? col + s_ib[m] : P1t, ok ? 8 : 0);
+          }
+        }
+      }
+      if (group < passes) load_phi(group, 0);
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();  // all of P1c is there
+      for (int j = group, buf = 0; j < passes; j += GROUPS, buf ^= 1) {
+        const int left = min(PTS, W.pn - j * PTS);
+        // this warp's two points of the pass: grad phi rows, bias and map entries
+        const int p_warp = 2 * gw;
+        double2 gx[2][3];  // [point][component], of one 64-row tile
+        auto load_grad = [&](int mt) {
+          const int r0 = mt * 64 + 2 * lane;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const double *src = gph + 3LL * (j * PTS + p_warp + i) * ncp + r0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              gx[i][c] = r0 < ncp && p_warp + i < left ? __ldg(reinterpret_cast<const double2 *>(src + c * ncp))
+                                                       : make_double2(0.0, 0.0);
+          }
+        };
+        load_grad(0);
+        // after the sums lane 4 (2 c + i) holds component c of point i
+        const int c_out = lane >> 3, p_out = p_warp + (lane >> 2 & 1);
+        const bool out = (lane & 3) == 0 && p_out < left;
+        const int pp = W.p0 + j * PTS + p_out;
+        const long long bidx = pp + (long long)P.n_max_batch_size * (W.batch + (long long)P.n_batches * t);
+        double offset = 0.0;
+        int full = 0;
+        if (out) {
+          offset = c_out == 0 ? __ldg(P.bias + bidx) : __ldg(P.gbias + 3 * bidx + c_out - 1);
+          if (c_out == 0) full = __ldg(P.map + W.prefix + pp);
+        }
+        cp_async_wait<0>();
+        group_sync();  // phi of this pass is there; the group is done with its last pass
+        if (j + GROUPS < passes) load_phi(j + GROUPS, buf ^ 1);
+        cp_async_commit();
+        const double *B = Bs + buf * PTS * ld;
+        double acc[2][2][2] = {};
+        const int cn = left > 8 ? 2 : 1;  // point blocks
+        const double *a0 = As + q * ld + rb * 8 + g, *b0 = B + g * ld + q;
+        if (cm == 2 && cn == 2)
+          small_mma<2, 2>(acc, a0, b0, ld, ncp / 4);
+        else if (cm == 2 && cn == 1)
+          small_mma<2, 1>(acc, a0, b0, ld, ncp / 4);
+        else if (cm == 1 && cn == 2)
+          small_mma<1, 2>(acc, a0, b0, ld, ncp / 4);
+        else if (cm == 1 && cn == 1)
+          small_mma<1, 1>(acc, a0, b0, ld, ncp / 4);
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi)
+          if (mi < cm) {
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                Ws[(ni * 8 + 2 * q + h) * LDW + (mi * RG + rb) * 8 + g] = acc[mi][ni][h];
+          }
+        group_sync();
+        // Two points per warp: lane l takes rows 2 l, 2 l + 1 of each 64-row tile; the
+        // eight sums (component, point) go over the lanes, the tiles in order.
+        double tot = 0.0;
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          if (mt >= nMt) break;
+          const int r0 = mt * 64 + 2 * lane;
+          const bool in_block = r0 < ncp, ok0 = r0 < nc, ok1 = r0 + 1 < nc;
+          double v[8];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int p = p_warp + i;
+            const bool live = in_block && p < left;
+            double2 w = make_double2(0.0, 0.0), f = w;
+            if (live) {
+              w = *reinterpret_cast<const double2 *>(Ws + p * LDW + r0);
+              f = *reinterpret_cast<const double2 *>(B + p * ld + r0);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const double2 x = c == 0 ? f : gx[i][c > 0 ? c - 1 : 0];
+              v[2 * c + i] = live ? fma(ok1 ? x.y : 0.0, w.y, (ok0 ? x.x : 0.0) * w.x) : 0.0;
+            }
+          }
+          if (mt == 0 && nMt > 1) load_grad(1);
+          fold<4>(v, lane);
+          fold<2>(v, lane);
+          fold<1>(v, lane);
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+          tot += v[0];
+        }
+        if (out) {
+          if (c_out > 0)
+            P.grad[3 * bidx + c_out - 1] = tot * 2 - offset;
+          else if (t < P.n_active)
+            P.rho[full + (long long)P.n_full_points * t] = tot + offset;
+        }
+      }
+    }
+    it = s_next;      // written before the first barrier
+    __syncthreads();  // read by everyone before the next item's first thread writes it
+  }
+}
+
+}  // namespace
+
+constexpr int STEP = GROUPS * PTS;  // points of a pass of both groups
+
+// Measured times of an item's parts, in microseconds: its start with the P1c
+// gather, and a pass of both groups (the MMA part is nc^2 x 32 points at one SM's
+// 250 GFLOP/s of FP64 MMAs).
+static double item_time(int nc, int passes) { return 3.5 + passes * (1.5 + 2.6e-4 * nc * nc); }
+
+// Work items: whole batches where those are many; otherwise every batch in equal
+// parts of at most a time limit, the limit that makes the launch shortest (with no
+// more items than SMs the longest item, else the mean load of an SM and half the
+// longest item), taken largest first.
+void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int order, std::vector<Rho1WorkItem> *out) {
+  constexpr int SMS = 148;
+  auto parts_of = [](const Rho1WorkItem &b, double limit) {
+    const int steps = ceil_div(b.np, STEP);
+    int parts = 1;
+    while (parts < steps && item_time(b.nc, ceil_div(steps, parts)) > limit) ++parts;
+    return parts;
+  };
+  double limit = 1e30;
+  const bool few = batches.size() <= 4 * SMS;
+  if (few) {
+    double best = 1e30;
+    for (double l = 5.0; l < 300.0; l *= 1.4) {
+      double sum = 0.0, longest = 0.0;
+      int n = 0;
+      bool cut = false;
+      for (const Rho1WorkItem &b : batches) {
+        if (b.np == 0) continue;
+        const int parts = parts_of(b, l);
+        cut = cut || parts > 1;
+        const double t = item_time(b.nc, ceil_div(ceil_div(b.np, STEP), parts));
+        sum += parts * t;
+        longest = std::max(longest, t);
+        n += parts;
+      }
+      const double launch = n <= SMS ? longest : sum / SMS + 0.5 * longest;
+      if (launch < best) {
+        best = launch;
+        limit = l;
+      }
+      if (!cut) break;
+    }
+  }
+  out->clear();
+  for (const Rho1WorkItem &b : batches) {
+    if (b.np == 0) continue;
+    const int steps = ceil_div(b.np, STEP), parts = parts_of(b, limit);
+    for (int k = 0, p0 = 0; k < parts; ++k) {  // the 32-point steps dealt out evenly
+      const int w = STEP * (steps / parts + (k < steps % parts ? 1 : 0));
+      out->push_back(Rho1WorkItem{b.batch, b.nc, b.np, p0, std::min(w, b.np - p0), b.ib_off, b.prefix, b.key,
+                                  b.wave_off});
+      p0 += w;
+    }
+  }
+  rho1_order_items(out, few ? 0 : order);
+}
+
+// Shared-memory attribute of the kernel, once per device (outside any capture).
+int rho1_small_configure(int device) {
+  static PerDeviceOnce configured;
+  return configured.run(device, []() -> int {
+    FRPA_CUDA_TRY(cudaFuncSetAttribute(rho1_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)small_smem(SMALL_MAX_NC)));
+    return FRPA_OK;
+  });
+}
+
+// The whole plan; the cursor must be zero.
+int rho1_small_launch(const Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *P1,
+                      const double *bias, const double *gbias, double *rho, double *grad, cudaStream_t stream) {
+  int n_sm = 148;
+  FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, plan.device));
+  const SmallParams P{plan.d_items_small, plan.n_items_small, plan.T, n_active, plan.n_basis, plan.n_full_points,
+                      plan.n_max_batch_size, plan.n_batches, plan.n_max_compute, plan.d_counter, plan.d_ib, plan.d_map,
+                      wave, gwave, P1, bias, gbias, rho, grad};
+  rho1_small_kernel<<<std::min(n_sm, plan.n_items_small), THREADS, small_smem(plan.n_max_compute), stream>>>(P);
+  FRPA_LAUNCH_CHECK();
+  return FRPA_OK;
+}
+
+}  // namespace frpa

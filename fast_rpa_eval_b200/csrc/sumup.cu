@@ -77,7 +77,8 @@ __host__ __device__ constexpr int rec_stride(int L) { return rec_coef_off(L) + k
 
 struct SumupPlan {
   int device = 0;
-  std::vector<void *> owned;  // the device allocations behind the pointers below
+  unsigned char *arena = nullptr;  // the device allocation behind the pointers below
+  size_t arena_bytes = 0;
   int T = 1, L = 0, L2 = 1, lma = 0, icc_dim0 = 0, mc_dim = 0, hfla = 0;
   int n_full_points = 0, n_valid_points = 0, n_centers = 0, n_chp = 0, n_atoms = 0, n_species = 0;
   int n_hartree_grid = 0;
@@ -1118,59 +1119,6 @@ int launch_dq(const SumupPlan &P, int n_active, const int *lhmfd, const double *
 
 // ------------------------------------------------------------ host side ---
 
-// A plan's device memory: arrays up to 1 MiB (and all uninitialised workspaces)
-// share one allocation and one copy, larger ones are copied from where they
-// are.  (One allocation and copy per array made creating a small plan mostly
-// driver calls.)
-struct PlanMemory {
-  struct Part {
-    void **dst;
-    size_t off;
-  };
-  std::vector<Part> parts;
-  std::vector<unsigned char> host;
-  size_t tail = 0;  // workspaces, after the copied bytes
-
-  static size_t padded(size_t n) { return (std::max<size_t>(n, 8) + 255) / 256 * 256; }
-  void array(void **dst, const void *src, size_t bytes) {
-    parts.push_back({dst, host.size()});
-    host.resize(host.size() + padded(bytes));
-    if (bytes) memcpy(host.data() + parts.back().off, src, bytes);
-  }
-  struct Space {
-    void **dst;
-    size_t bytes;
-  };
-  std::vector<Space> spaces;
-  void space(void **dst, size_t bytes) {
-    spaces.push_back({dst, bytes});
-    tail += padded(bytes);
-  }
-  int commit(void **base) {
-    if (cudaMalloc(base, padded(host.size() + tail)) != cudaSuccess) {
-      *base = nullptr;
-      return fail(FRPA_ERR_OOM, "sumup: allocation of %zu bytes failed", host.size() + tail);
-    }
-    unsigned char *d = static_cast<unsigned char *>(*base);
-    for (const Part &p : parts) *p.dst = d + p.off;
-    size_t off = host.size();
-    for (const Space &w : spaces) {
-      *w.dst = d + off;
-      off += padded(w.bytes);
-    }
-    if (!host.empty()) FRPA_CUDA_TRY(cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice));
-    return FRPA_OK;
-  }
-};
-constexpr size_t PLAN_SMALL = 1 << 20;
-
-static int upload_large(std::vector<void *> *owned, void **dst, const void *src, size_t bytes) {
-  if (cudaMalloc(dst, bytes) != cudaSuccess) return fail(FRPA_ERR_OOM, "sumup: allocation of %zu bytes failed", bytes);
-  owned->push_back(*dst);
-  FRPA_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
-  return FRPA_OK;
-}
-
 static int sumup_upload_constants_once() {
   double K[SU_LMAX + 1][SU_LMAX + 1] = {}, Kc[SU_LMAX + 1][SU_LMAX + 1] = {};
   double RA[SU_LMAX + 1][SU_LMAX + 1] = {}, RB[SU_LMAX + 1][SU_LMAX + 1] = {}, DF[SU_LMAX + 1] = {};
@@ -1213,7 +1161,7 @@ int sumup_upload_constants(int device) {
 
 void sumup_plan_free(SumupPlan *P) {
   if (!P) return;
-  for (void *p : P->owned) cudaFree(p);
+  cudaFree(P->arena);
   delete P;
 }
 
@@ -1366,16 +1314,12 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
   P->rs = rec_stride(L);
   int st = FRPA_OK;
   PlanMemory mem;
-#define UP(field, src, bytes)                                                                     \
-  if ((size_t)(bytes) <= PLAN_SMALL)                                                              \
-    mem.array((void **)&P->field, (src), (bytes));                                                \
-  else if (st == FRPA_OK)                                                                         \
-    st = upload_large(&P->owned, (void **)&P->field, (src), (bytes));
+#define UP(field, src, bytes) mem.array((void **)&P->field, (src), (bytes));
   UP(d_map, D->i_valid_point_2_i_full_points_map, sizeof(int) * (size_t)D->n_valid_points);
+  // Morton order of the valid points (21 bits per axis over their bounding box)
+  const int nv = D->n_valid_points;
+  std::vector<int> ord(nv);
   {
-    // Morton order of the valid points (21 bits per axis over their bounding box)
-    const int nv = D->n_valid_points;
-    std::vector<int> ord(nv);
     if (nv > 0) {
       double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
       for (int i = 0; i < nv; ++i)
@@ -1445,8 +1389,8 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
     P->adj_pts = (int)((std::min(most, std::max(512LL, pairs / 2400)) + 127) / 128 * 128);
     P->adj_nz = std::max(1, ceil_div(P->n_valid_points, P->adj_pts));
   }
+  std::vector<int> cnt(P->n_atoms + 1, 0), slots(std::max(1, P->n_chp));
   {
-    std::vector<int> cnt(P->n_atoms + 1, 0), slots(std::max(1, P->n_chp));
     std::vector<int> atom_of(std::max(1, P->n_chp));
     for (int q = 0; q < P->n_chp; ++q) {
       atom_of[q] = D->center_to_atom[D->centers_hartree_potential[q] - 1] - 1;
@@ -1455,9 +1399,9 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
     for (int a = 0; a < P->n_atoms; ++a) cnt[a + 1] += cnt[a];
     std::vector<int> fill(cnt.begin(), cnt.end() - 1);
     for (int q = 0; q < P->n_chp; ++q) slots[fill[atom_of[q]]++] = q;  // ascending within each atom
-    UP(d_atom_slot_ptr, cnt.data(), sizeof(int) * cnt.size());
-    UP(d_atom_slots, slots.data(), sizeof(int) * slots.size());
   }
+  UP(d_atom_slot_ptr, cnt.data(), sizeof(int) * cnt.size());
+  UP(d_atom_slots, slots.data(), sizeof(int) * slots.size());
   const int no_flags = 0;
   UP(d_err, &no_flags, sizeof(int));
 #undef UP
@@ -1468,11 +1412,7 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
   mem.space((void **)&P->d_recs, sizeof(double) * (size_t)P->rs * chp * T);
   mem.space((void **)&P->d_heads, sizeof(double4) * chp * T);
   mem.space((void **)&P->d_dcoef_part, sizeof(double) * (size_t)n_kelvin(L) * chp * T * P->adj_nz);
-  if (st == FRPA_OK) {
-    void *base = nullptr;
-    st = mem.commit(&base);
-    if (base) P->owned.push_back(base);
-  }
+  if (st == FRPA_OK) st = mem.commit(&P->arena, &P->arena_bytes);
   if (st == FRPA_OK && P->n_valid_points > 0) {
     sumup_gather_points_kernel<<<std::min(1184, ceil_div(P->n_valid_points, 256)), 256>>>(
         P->n_valid_points, P->d_map, P->d_order, P->d_coord, P->d_pfull, P->d_pxyz);

@@ -148,3 +148,31 @@ def test_synth_generator_matches_host_basis_values():
     torch.cuda.synchronize()
     assert normwise_rel(w.cpu().numpy(), p.wave) < 1e-13
     assert normwise_rel(gw.cpu().numpy(), p.gradient_wave) < 1e-13
+
+
+@pytest.mark.parametrize("nc_range,np_range,n_batches,T,n_active", [
+    ((1, 3), (1, 9), 5, 1, 1),         # one row block, part of a pass
+    ((15, 18), (31, 34), 7, 2, 1),     # either side of two row blocks and of a 32-point pass
+    ((63, 66), (95, 98), 6, 3, 3),     # one and two row tiles, items of several passes
+    ((119, 120), (150, 200), 40, 2, 2),  # the largest this kernel takes, more items than SMs
+    ((20, 120), (1, 300), 1500, 1, 1),   # whole batches as items, many rounds
+    ((100, 121), (60, 70), 9, 1, 1),   # one batch above the limit: the general kernel
+])
+def test_rho1_small_batches_match_oracle_and_the_general_kernel(nc_range, np_range, n_batches, T, n_active):
+    """Plans of batches with at most 120 functions: against the oracle, and bit
+    for bit against the general kernel, which the same problem takes when its
+    phi blocks start at odd offsets.  Padding rows hold NaN."""
+    p = synth.make_rho1_problem(T=T, seed=70 + nc_range[1], n_atoms=10, n_batches=n_batches, np_range=np_range,
+                                nc_range=nc_range, with_bias=True, extra_full_points=13, empty_batches=2,
+                                pad_value=np.nan, n_active=n_active)
+    p.first_order_density_matrix = np.asfortranarray(  # not symmetric: rows and columns both matter
+        p.first_order_density_matrix + 0.1 * np.random.default_rng(1).normal(size=p.first_order_density_matrix.shape))
+    r, g = rho1_device_run(_lib.Rho1Plan(p), p)
+    r_o, g_o = oracle.rho1(p, n_threads=8)
+    assert normwise_rel(r, r_o) < TOL_FP64 and normwise_rel(g, g_o) < TOL_FP64
+    assert np.array_equal(r_o == 0, r == 0) and np.array_equal(g_o == 0, g == 0)
+    p.wave = np.concatenate([[np.nan], p.wave])
+    p.gradient_wave = np.concatenate([[np.nan] * 3, p.gradient_wave])
+    p.i_batch_2_wave_offset = (p.i_batch_2_wave_offset + 1).astype(np.int32)
+    r1, g1 = rho1_device_run(_lib.Rho1Plan(p), p)
+    assert np.array_equal(r, r1) and np.array_equal(g, g1)
