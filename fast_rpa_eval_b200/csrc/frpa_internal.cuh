@@ -188,10 +188,10 @@ static_assert(sizeof(I8Item) == 80, "I8Item layout");
 // One N tile of one batch and perturbation, packed by one CTA.
 struct I8BTile {
   int ib_off, nc, jn, t;
-  int n_rows, n_kc, sb_off, pad_;  // rows of this tile (32; rows past n_compute are zero)
+  int n_kc, sb_off;  // K chunks; first per-row scale of the tile
   long long b_off;                 // bytes of the tile's first chunk
 };
-static_assert(sizeof(I8BTile) == 40, "I8BTile layout");
+static_assert(sizeof(I8BTile) == 32, "I8BTile layout");
 
 struct I8Group {
   int item0, item1;   // items [item0, item1)

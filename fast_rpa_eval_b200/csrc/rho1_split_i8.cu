@@ -21,23 +21,33 @@
 // operand rounding in a CPU emulation of these steps).
 //
 // Data flow, three launches per group of batches:
-//   1. pack A: one CTA per work item (<= 128 points of one batch) finds the
-//      per-point scales and writes phi's five digit planes in the tcgen05
-//      shared-memory tile image (K-major, no swizzle, 8 x 16-byte core
-//      matrices), one 32-wide K chunk after another, 16 points at a time;
+//   1. pack A: one CTA per eight points of a work item (<= 128 points of one
+//      batch) finds the per-point scales and writes phi's five digit planes in
+//      the tcgen05 shared-memory tile image (K-major, no swizzle, 8 x 16-byte
+//      core matrices), one 32-wide K chunk after another;
 //   2. pack B: one CTA per (batch, perturbation, N tile of 32 rows, the last
 //      one zero-padded) gathers P1c = P1[ib, ib] (lanes along P1's contiguous
 //      rows) and writes its digit planes the same way;
-//   3. contract: one persistent CTA per SM.  A loader thread moves each
-//      stage's A and B chunks into a 4-stage shared-memory ring with bulk
-//      copies; an MMA thread issues a stage's 19 digit products as five
+//   3. contract: one persistent CTA per SM.  A loader warp moves each stage's
+//      (two K chunks') A and B planes into a 3-stage shared-memory ring with
+//      two bulk copies; an MMA warp issues a chunk's 19 digit products as five
 //      tcgen05.mma.kind::i8 (M = 128 points, K = 32; the digit levels run
-//      along N: A plane s times B planes 0..5-s, N = 32 (6 - s) rows, into
-//      the six level accumulators from level s on) in one of two sets
-//      (2 x 192 of 512 TMEM columns); 8 epilogue warps read a
-//      finished set (tcgen05.ld), recombine in FP64 and contract with phi and
-//      grad phi (FP64, 256-bit loads from global memory issued a chunk ahead)
-//      while the MMAs of the next tile fill the other set.
+//      along N: A plane s times B planes 0..min(4, 5-s), into the level
+//      accumulators from level s on) in one of two sets (2 x 192 of 512 TMEM
+//      columns); 8 epilogue warps read a finished set (tcgen05.ld), recombine
+//      in FP64 and contract with phi and grad phi (FP64, 256-bit loads from
+//      global memory issued four columns ahead) while the MMAs of the next
+//      tile fill the other set.
+// What bounds the contraction (8,000 batches of 100-600 functions, 7.1 ms): a
+// chunk's MMAs take 304 cycles, but their operands are 40 KB and its copies
+// 21 KB through the 128 bytes a cycle of shared memory (~480 cycles, measured
+// with the epilogue's loads and sums left out), and with the 10 KB of phi and
+// grad phi the SMs draw ~10 TB/s from L2 (620 cycles).  Issue used to bound
+// it (660 cycles): six copies, two waits and two commits per 32-wide chunk from
+// single threads, and waiting warps that polled a global timer.  Not kept,
+// all slower or equal: 8 stages (26 KB of L1 left for the epilogue's loads),
+// 4 chunks a stage, sixteen epilogue warps (spills), a second set of phi
+// registers under setmaxnreg, smaller groups of batches.
 // The packed operands cost a write and a read of ~5 bytes per P1c and phi
 // element, in exchange the contraction has no gathers, no conversions and
 // no register-staged loads on its critical path.  Every mbarrier wait is
@@ -56,20 +66,21 @@ using namespace sm100;
 
 constexpr int I8_M = 128;      // points per work item (TMEM lanes)
 constexpr int I8_N = 32;       // rows i per N tile (accumulator columns per level)
-constexpr int I8_KC = 32;      // K per stage: one kind::i8 instruction
+constexpr int I8_KC = 32;      // K per chunk: one kind::i8 instruction
 constexpr int I8_LEVELS = 6;   // digit levels s + u = 0..5
 constexpr int I8_SLICES = 5;   // digit planes per operand
 constexpr int I8_SETS = 2;     // accumulator sets: a tile's epilogue overlaps the next tile's MMAs
-constexpr int I8_STAGES = 4;
+constexpr int I8_CHUNKS = 2;   // chunks per stage
+constexpr int I8_STAGES = 3;
 constexpr int I8_EPI_WARPS = 8;  // warps 0..7: lane quarter w % 4, column half w / 4; warp 0 owns TMEM
 constexpr int I8_COLS = I8_N / 2;  // 16 accumulator columns per epilogue warp
-constexpr int I8_LOAD_WARP = 8;  // lane 0 issues the bulk copies
-constexpr int I8_MMA_WARP = 9;   // lane 0 issues the MMAs
+constexpr int EPI_BUFS = 2;        // four-column steps whose phi and grad phi are in registers
+constexpr int I8_LOAD_WARP = 8;  // issues the bulk copies
+constexpr int I8_MMA_WARP = 9;   // issues the MMAs
 constexpr int I8_THREADS = 32 * 10;
 constexpr int I8_ROWB = I8_KC;                         // bytes per tile row of one plane
 constexpr int I8_A_PLANE = I8_M * I8_ROWB;             // 4096
-constexpr int I8_B_STAGE = I8_SLICES * I8_N * I8_ROWB;  // 5120: the five planes of a stage's B chunk
-constexpr int I8_B_SLOT = I8_B_STAGE + I8_N * I8_ROWB;  // 6144: plus a zero plane (see mma_role)
+constexpr int I8_B_CHUNK = I8_SLICES * I8_N * I8_ROWB;  // 5120: the five planes of a B chunk
 constexpr uint32_t I8_LBO = 128;                       // K-adjacent core matrices
 constexpr uint32_t I8_SBO = 256;                       // 8-row groups
 constexpr int I8_TMEM_COLS = 512;
@@ -94,10 +105,6 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate));
 }
 
-// Every N tile has 32 rows; the last one of a batch is padded with zero rows
-// (the B planes of all tiles then share one layout: plane u at rows 32 u).
-__host__ __device__ __forceinline__ int tile_rows(int, int, int) { return I8_N; }
-
 // Byte offset of (row r, K half kg) inside one plane of a tile.
 __device__ __forceinline__ int plane_off(int r, int kg) { return (r >> 3) * (int)I8_SBO + kg * 128 + (r & 7) * 16; }
 
@@ -115,40 +122,39 @@ __device__ __forceinline__ void digit_scale(double m, double *sc39, double *s23)
   *s23 = ldexp(1.0, e - 23);
 }
 
-// Sixteen consecutive values of one row as five 16-byte digit planes.
+// The digits of one value.
 //   t = fma(x, sc39, 1.5 2^52) holds X = rint(x sc39) in its mantissa, so
 //   bits(t) - 0x4338000000000000 = X exactly; X + 0x80808080 = a0 2^32 + sum
 //   c_s 2^(8 (4 - s)) with bytes c_s in [0, 255], i.e. the balanced digits
 //   a_s = c_s - 128 (= c_s ^ 0x80 as a signed byte) and a0 the high word.
-__device__ __forceinline__ void digits16(const double (&x)[16], double sc39, uint4 (&plane)[I8_SLICES]) {
-  int hi[16];
-  uint32_t lo[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const double t = fma(x[j], sc39, 6755399441055744.0);
-    const long long xp = __double_as_longlong(t) + (0x80808080LL - 0x4338000000000000LL);
-    hi[j] = (int)(xp >> 32);
-    lo[j] = (uint32_t)xp;
-  }
-  uint32_t w[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint32_t t1 = __byte_perm((uint32_t)hi[4 * q], (uint32_t)hi[4 * q + 1], 0x40);
-    const uint32_t t2 = __byte_perm((uint32_t)hi[4 * q + 2], (uint32_t)hi[4 * q + 3], 0x40);
-    w[q] = __byte_perm(t1, t2, 0x5410);
-  }
-  plane[0] = make_uint4(w[0], w[1], w[2], w[3]);
+__device__ __forceinline__ void digit_bits(double x, double sc39, int *hi, uint32_t *lo) {
+  const double t = fma(x, sc39, 6755399441055744.0);
+  const long long xp = __double_as_longlong(t) + (0x80808080LL - 0x4338000000000000LL);
+  *hi = (int)(xp >> 32);
+  *lo = (uint32_t)xp;
+}
+
+// Four values' digits as one word per plane.
+__device__ __forceinline__ void digit_words(const int *hi, const uint32_t *lo, uint32_t (&plane)[I8_SLICES]) {
+  plane[0] = __byte_perm(__byte_perm((uint32_t)hi[0], (uint32_t)hi[1], 0x40),
+                         __byte_perm((uint32_t)hi[2], (uint32_t)hi[3], 0x40), 0x5410);
 #pragma unroll
   for (int s = 1; s < I8_SLICES; ++s) {
     const uint32_t b = (uint32_t)(4 - s), sel = b | ((b + 4) << 4);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t t1 = __byte_perm(lo[4 * q], lo[4 * q + 1], sel);
-      const uint32_t t2 = __byte_perm(lo[4 * q + 2], lo[4 * q + 3], sel);
-      w[q] = __byte_perm(t1, t2, 0x5410) ^ 0x80808080u;
-    }
-    plane[s] = make_uint4(w[0], w[1], w[2], w[3]);
+    plane[s] = __byte_perm(__byte_perm(lo[0], lo[1], sel), __byte_perm(lo[2], lo[3], sel), 0x5410) ^ 0x80808080u;
   }
+}
+
+// Sixteen consecutive values of one row as five 16-byte digit planes.
+__device__ __forceinline__ void digits16(const double (&x)[16], double sc39, uint4 (&plane)[I8_SLICES]) {
+  int hi[16];
+  uint32_t lo[16], w[4][I8_SLICES];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) digit_bits(x[j], sc39, &hi[j], &lo[j]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) digit_words(hi + 4 * q, lo + 4 * q, w[q]);
+#pragma unroll
+  for (int s = 0; s < I8_SLICES; ++s) plane[s] = make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]);
 }
 
 // ------------------------------------------------------------ pack kernels
@@ -160,119 +166,145 @@ __device__ __forceinline__ void ld4(const double *p, double *v) {
                : "l"(p));
 }
 
-constexpr int PA_THREADS = 256;
-constexpr int PA_GROUP = 16;  // points per pass: their rows are re-read from L2, not DRAM
+constexpr int PA_ROWS = 8;  // rows (points) per CTA: one 8-row group of the tile image
+constexpr int PA_GROUPS = I8_M / PA_ROWS;
+constexpr int PA_WARPS = 8;
+constexpr int PA_THREADS = 32 * PA_WARPS;
 
-// phi of one work item -> A scratch: chunk kc, plane s at
+// Four values of one row -> one 32-bit word of each digit plane (see digit_bits).
+__device__ __forceinline__ void digits4(const double (&x)[4], double sc39, uint32_t (&plane)[I8_SLICES]) {
+  int hi[4];
+  uint32_t lo[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) digit_bits(x[j], sc39, &hi[j], &lo[j]);
+  digit_words(hi, lo, plane);
+}
+
+// phi of eight points of one work item -> A scratch: chunk kc, plane s at
 // a_off + (5 kc + s) rows8 32 bytes; rows pn..rows8-1 and k >= nc are zero.
-// Sixteen points at a time: their scales (one warp per point, lanes along the
-// row), then their digits (one thread per row and 16-wide K group; a warp's
-// stores cover 512 contiguous bytes of a plane).
-__global__ void __launch_bounds__(PA_THREADS) i8_pack_a_kernel(const I8Item *__restrict__ items,
+// Memory bound: phi is read (for the digits a second time, from L2) and five
+// bytes a value are written.  Lane (row r = lane / 4, quarter q = lane % 4) of
+// warp w takes the values 16 kg + 4 q..+3 of row r for kg = w, w + 8, ...: a
+// warp's load covers 128 contiguous bytes of each of its eight rows and its
+// stores 128 contiguous bytes of a plane.  A CTA lives for one chain of
+// latencies, so what counts is how many of them an SM holds: with all 2048
+// threads and the second read 1.52 ms for 8,000 batches of 100-600 functions
+// (7.3 GB in and out), with the values kept in registers between the maximum
+// and the digits 2.31 ms (three CTAs an SM), and 1.86 ms for sixteen points at
+// a time in a CTA per item.
+__global__ void __launch_bounds__(PA_THREADS, 2048 / PA_THREADS) i8_pack_a_kernel(const I8Item *__restrict__ items,
                                                                const double *__restrict__ wave,
                                                                unsigned char *__restrict__ a_scr,
                                                                double *__restrict__ sa, int vec) {
-  __shared__ double s_sc[PA_GROUP];
-  const I8Item W = items[blockIdx.x];
-  const int nc = W.nc, pn = W.pn, rows8 = W.rows8, ncp = (nc + 3) & ~3;
-  const double *phi = wave + W.wave_off + (long long)W.p0 * ncp;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long chunk = (long long)I8_SLICES * rows8 * I8_ROWB;
-  for (int g0 = 0; g0 < rows8; g0 += PA_GROUP) {
-    const int gn = min(PA_GROUP, rows8 - g0);  // 8 or 16
-    for (int r = warp; r < gn; r += PA_THREADS / 32) {
-      const int p = g0 + r;
-      double m = 0.0;
-      if (p < pn) {
-        const double *row = phi + (long long)p * ncp;
-        for (int k = lane; k < nc; k += 32) m = fmax(m, fabs(__ldg(row + k)));
-      }
+  __shared__ double s_max[PA_WARPS][PA_ROWS];
+  const I8Item &W = items[blockIdx.x / PA_GROUPS];
+  const int row0 = (int)(blockIdx.x % PA_GROUPS) * PA_ROWS;
+  if (row0 >= W.rows8) return;
+  const int nc = W.nc, ncp = (nc + 3) & ~3, n_kg = 2 * W.n_kc;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+  const int p = row0 + r;
+  const bool live = p < W.pn;
+  const double *row = wave + W.wave_off + (long long)(W.p0 + (live ? p : 0)) * ncp + 4 * q;
+  const int kend = live ? nc - 4 * q : 0;  // values of this lane's row from its quarter on
+  auto load = [&](int kg, double (&x)[4]) {
+    const int k = 16 * kg;
+    if (vec) {  // rows start on 32-byte boundaries; a vector that starts below nc ends by ncp
+      if (k < kend) {
+        ld4(row + k, x);
 #pragma unroll
-      for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (lane == 0) {
-        double sc39, s23;
-        digit_scale(m, &sc39, &s23);
-        s_sc[r] = sc39;
-        sa[W.sa_off + p] = s23;
-      }
-    }
-    __syncthreads();
-    const int units = W.n_kc * 2 * gn;
-    for (int u = threadIdx.x; u < units; u += PA_THREADS) {
-      const int r = u % gn, kg = (u / gn) & 1, kc = u / (2 * gn), p = g0 + r;
-      const int k0 = kc * I8_KC + kg * 16;
-      const double *row = phi + (long long)(p < pn ? p : 0) * ncp;
-      double x[16];
-      if (vec) {  // rows start on 32-byte boundaries; a vector that starts below nc ends by ncp
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          if (p < pn && k0 + 4 * v < nc) {
-            ld4(row + k0 + 4 * v, &x[4 * v]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) x[4 * v + e] = 0.0;
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = k0 + j < nc ? x[j] : 0.0;  // the row padding
+        for (int j = 1; j < 4; ++j) x[j] = k + j < kend ? x[j] : 0.0;  // the row padding
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = (p < pn && k0 + j < nc) ? __ldg(row + k0 + j) : 0.0;
+        for (int j = 0; j < 4; ++j) x[j] = 0.0;
       }
-      uint4 plane[I8_SLICES];
-      digits16(x, s_sc[r], plane);
-      unsigned char *dst = a_scr + W.a_off + kc * chunk + plane_off(p, kg);
+    } else {
 #pragma unroll
-      for (int s = 0; s < I8_SLICES; ++s) *reinterpret_cast<uint4 *>(dst + s * rows8 * I8_ROWB) = plane[s];
+      for (int j = 0; j < 4; ++j) x[j] = k + j < kend ? __ldg(row + k + j) : 0.0;
     }
-    __syncthreads();  // s_sc is rewritten by the next group
+  };
+  double m = 0.0;
+#pragma unroll 2
+  for (int kg = warp; kg < n_kg; kg += PA_WARPS) {
+    double x[4];
+    load(kg, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m = fmax(m, fabs(x[j]));
+  }
+  m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  if (q == 0) s_max[warp][r] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < PA_WARPS; ++w) m = fmax(m, s_max[w][r]);
+  double sc39, s23;
+  digit_scale(m, &sc39, &s23);
+  if (warp == 0 && q == 0) sa[W.sa_off + p] = s23;
+  const long long plane_bytes = (long long)W.rows8 * I8_ROWB;
+  unsigned char *dst = a_scr + W.a_off + plane_off(p, 0) + 4 * q;
+#pragma unroll 2
+  for (int kg = warp; kg < n_kg; kg += PA_WARPS) {
+    double x[4];
+    uint32_t w[I8_SLICES];
+    load(kg, x);
+    digits4(x, sc39, w);
+    unsigned char *d = dst + (kg >> 1) * I8_SLICES * plane_bytes + (kg & 1) * I8_LBO;
+#pragma unroll
+    for (int s = 0; s < I8_SLICES; ++s) *reinterpret_cast<uint32_t *>(d + s * plane_bytes) = w[s];
   }
 }
 
-constexpr int PB_THREADS = 2 * I8_N;  // 32 rows x two 16-wide halves of a K chunk
+constexpr int PB_WARPS = 4;
+constexpr int PB_THREADS = 32 * PB_WARPS;
 
 // P1c rows of one N tile -> B scratch: chunk kc, plane s at
-// b_off + kc 5 n_rows 32 + s n_rows 32; rows >= nc and k >= nc are zero.
+// b_off + (5 kc + s) 1024 bytes; rows >= nc and k >= nc are zero.  Lane = row
+// (P1's contiguous index), warp w takes the 16-wide K groups w, w + 4, ...; a
+// group's sixteen column indices come from shared memory as four 128-bit
+// broadcasts, and its sixteen gathers are in flight together.
 __global__ void __launch_bounds__(PB_THREADS) i8_pack_b_kernel(const I8BTile *__restrict__ tiles,
                                                                const int *__restrict__ ib_all,
                                                                const double *__restrict__ P1,
                                                                const double *__restrict__ rowmax, int n_basis,
                                                                unsigned char *__restrict__ b_scr,
                                                                double *__restrict__ sb) {
-  __shared__ int s_ib[FRPA_MAX_N_COMPUTE];
+  __shared__ __align__(16) int s_ib[(FRPA_MAX_N_COMPUTE + 31) / 32 * 32];
   const I8BTile B = tiles[blockIdx.x];
-  const int nc = B.nc, N = B.n_rows;
-  for (int i = threadIdx.x; i < nc; i += PB_THREADS) s_ib[i] = __ldg(ib_all + B.ib_off + i) - 1;
+  const int nc = B.nc;
+  for (int i = threadIdx.x; i < B.n_kc * I8_KC; i += PB_THREADS) s_ib[i] = i < nc ? __ldg(ib_all + B.ib_off + i) - 1 : 0;
   __syncthreads();
-  const int r = threadIdx.x % I8_N, kg = threadIdx.x / I8_N;
-  if (r >= N) return;
+  const int r = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = B.jn * I8_N + r;
   const bool rok = i < nc;
   const int ibr = rok ? s_ib[i] : 0;
-  const double *P1t = P1 + (long long)n_basis * n_basis * B.t;
+  const double *col = P1 + (long long)n_basis * n_basis * B.t + ibr;
   double sc39, s23;
   digit_scale(rok ? __ldg(rowmax + ibr + (long long)n_basis * B.t) : 0.0, &sc39, &s23);
-  if (kg == 0) sb[B.sb_off + r] = rok ? s23 * 0.00390625 : 0.0;  // 2^(e - 31): the recombination sums 256 S
-  const long long chunk = (long long)I8_SLICES * N * I8_ROWB;
-  for (int kc = 0; kc < B.n_kc; ++kc) {
-    const int k0 = kc * I8_KC + kg * 16;
+  if (warp == 0) sb[B.sb_off + r] = rok ? s23 * 0.00390625 : 0.0;  // 2^(e - 31): the recombination sums 256 S
+  unsigned char *dst = b_scr + B.b_off + plane_off(r, 0);
+  for (int kg = warp; kg < 2 * B.n_kc; kg += PB_WARPS) {
+    const int k0 = kg * 16, kn = rok ? nc - k0 : 0;
     double x[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      x[j] = (rok && k0 + j < nc) ? __ldg(P1t + ibr + (long long)s_ib[k0 + j] * n_basis) : 0.0;
+    for (int v = 0; v < 4; ++v) {
+      const int4 id = *reinterpret_cast<const int4 *>(s_ib + k0 + 4 * v);
+      x[4 * v + 0] = 4 * v + 0 < kn ? __ldg(col + (long long)id.x * n_basis) : 0.0;
+      x[4 * v + 1] = 4 * v + 1 < kn ? __ldg(col + (long long)id.y * n_basis) : 0.0;
+      x[4 * v + 2] = 4 * v + 2 < kn ? __ldg(col + (long long)id.z * n_basis) : 0.0;
+      x[4 * v + 3] = 4 * v + 3 < kn ? __ldg(col + (long long)id.w * n_basis) : 0.0;
+    }
     uint4 plane[I8_SLICES];
     digits16(x, sc39, plane);
-    unsigned char *dst = b_scr + B.b_off + kc * chunk + plane_off(r, kg);
+    unsigned char *d = dst + (kg >> 1) * I8_B_CHUNK + (kg & 1) * I8_LBO;
 #pragma unroll
-    for (int s = 0; s < I8_SLICES; ++s) *reinterpret_cast<uint4 *>(dst + s * N * I8_ROWB) = plane[s];
+    for (int s = 0; s < I8_SLICES; ++s) *reinterpret_cast<uint4 *>(d + s * I8_N * I8_ROWB) = plane[s];
   }
 }
 
 // ------------------------------------------------------ contraction kernel
 
 struct I8Smem {
-  unsigned char A[I8_STAGES][I8_SLICES][I8_A_PLANE];
-  unsigned char B[I8_STAGES][I8_B_SLOT];  // planes 0..4 (32 rows each), then a zero plane
+  unsigned char A[I8_STAGES][I8_CHUNKS * I8_SLICES * I8_A_PLANE];  // chunks and planes at their packed distance
+  unsigned char B[I8_STAGES][I8_CHUNKS * I8_B_CHUNK];
   double partial[2][4][I8_M];              // upper column half's per-point sums
   unsigned long long full[I8_STAGES];
   unsigned long long empty[I8_STAGES];
@@ -298,29 +330,39 @@ struct I8Params {
   int wave_vec;  // every phi / grad phi row starts on a 32-byte boundary: 256-bit loads
 };
 
-// Lane 0 of the loader warp: every stage's A planes (5 copies of rows8 x 32
-// bytes) and B planes (one copy of 5 x n_rows x 32 bytes) into the ring.
+// A warp-uniform value as the compiler can see it (uniform registers feed the
+// descriptors and loop bounds of the issuing warps).
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+// The loader warp (converged, one elected lane issues): every stage's A planes
+// and B planes, one bulk copy each, into the ring.  The planes of an A chunk
+// keep their packed distance of rows8 x 32 bytes, so that they are one copy:
+// issuing a copy takes ~70 cycles, and one per plane kept the loader busy for
+// 460 of a chunk's 660 cycles.
 __device__ void loader_role(const I8Params &P, I8Smem &S) {
   volatile int *abort_flag = &S.abort_flag;
   uint32_t fill = 0;
   for (int it = blockIdx.x; it < P.n_items; it += gridDim.x) {
-    const I8Item W = P.items[it];
-    const uint32_t a_bytes = (uint32_t)W.rows8 * I8_ROWB;
-    for (int t = 0; t < P.T; ++t)
-      for (int jn = 0; jn < W.n_nt; ++jn) {
-        const int N = tile_rows(W.nc, jn, W.n_nt);
-        const uint32_t b_bytes = (uint32_t)(I8_SLICES * N * I8_ROWB);
-        const unsigned char *bsrc = P.b_scr + W.b_off + t * W.b_tstride + (long long)jn * W.n_kc * I8_B_STAGE;
-        for (int kc = 0; kc < W.n_kc; ++kc, ++fill) {
+    const I8Item &W = P.items[it];
+    const int n_kc = uniform(W.n_kc), n_nt = uniform(W.n_nt);
+    const uint32_t a_bytes = (uint32_t)(uniform(W.rows8) * I8_SLICES * I8_ROWB);
+    const unsigned char *asrc = P.a_scr + W.a_off;
+    for (int t = 0; t < P.T; ++t) {
+      const unsigned char *bsrc = P.b_scr + W.b_off + t * W.b_tstride;  // the tiles' chunks, back to back
+      for (int jn = 0; jn < n_nt; ++jn)
+        for (int kc = 0; kc < n_kc; kc += I8_CHUNKS, ++fill) {
           const int st = fill % I8_STAGES;
-          if (!mbar_wait(&S.empty[st], ((fill / I8_STAGES) & 1) ^ 1, abort_flag, P.err)) goto out;
-          mbar_arrive_expect_tx(&S.full[st], I8_SLICES * a_bytes + b_bytes);
-          const unsigned char *a = P.a_scr + W.a_off + (long long)kc * I8_SLICES * a_bytes;
-#pragma unroll
-          for (int s = 0; s < I8_SLICES; ++s) bulk_g2s(S.A[st][s], a + s * a_bytes, a_bytes, &S.full[st]);
-          bulk_g2s(S.B[st], bsrc + (long long)kc * b_bytes, b_bytes, &S.full[st]);
+          const uint32_t n = (uint32_t)min(I8_CHUNKS, n_kc - kc);
+          if (!warp_wait_all(&S.empty[st], ((fill / I8_STAGES) & 1) ^ 1, abort_flag, P.err)) goto out;
+          if (elect_one()) {
+            mbar_arrive_expect_tx(&S.full[st], n * (a_bytes + I8_B_CHUNK));
+            bulk_g2s(S.A[st], asrc + (long long)kc * a_bytes, n * a_bytes, &S.full[st]);
+            bulk_g2s(S.B[st], bsrc, n * I8_B_CHUNK, &S.full[st]);
+          }
+          __syncwarp();
+          bsrc += n * I8_B_CHUNK;
         }
-      }
+    }
   }
 out:
   // the copies of the last (up to) I8_STAGES fills land before the CTA exits
@@ -329,79 +371,92 @@ out:
     if (!mbar_wait_quiet(&S.full[f % I8_STAGES], (f / I8_STAGES) & 1)) atomicOr(P.err, 4);
 }
 
-// Lane 0 of the MMA warp: per N tile, all K chunks' 19 digit products into
-// the six level accumulators of the tile's set (sets alternate by tile), five
-// MMA instructions per stage (one ~50-cycle issue each, so that issuing no
-// longer outlasts the tensor work of a stage).
+// One K chunk's 19 digit products (five MMAs; six in a tile's first chunk).
+// Digit levels run along N: B planes 0..m of a chunk are one contiguous matrix
+// of 32 (m + 1) rows, so A plane s times planes 0..min(4, 5-s), written from
+// accumulator column 32 s on, puts product (s, u) into the columns of level
+// s + u.  In the first chunk A plane 1 starts levels 1..5 and plane 0 level 0.
+template <bool FIRST>
+__device__ __forceinline__ void chunk_mmas(uint32_t dcol, uint64_t adesc, uint32_t plane, uint64_t bdesc) {
+  if (FIRST) {
+    umma_i8(dcol + I8_N, adesc + plane, bdesc, idesc_n(5 * I8_N), 0u);
+    umma_i8(dcol, adesc, bdesc, idesc_n(I8_N), 0u);
+    umma_i8(dcol + I8_N, adesc, bdesc + (I8_N * I8_ROWB >> 4), idesc_n(4 * I8_N), 1u);
+  } else {
+    umma_i8(dcol, adesc, bdesc, idesc_n(5 * I8_N), 1u);
+    umma_i8(dcol + I8_N, adesc + plane, bdesc, idesc_n(5 * I8_N), 1u);
+  }
+  umma_i8(dcol + 2 * I8_N, adesc + 2 * plane, bdesc, idesc_n(4 * I8_N), 1u);
+  umma_i8(dcol + 3 * I8_N, adesc + 3 * plane, bdesc, idesc_n(3 * I8_N), 1u);
+  umma_i8(dcol + 4 * I8_N, adesc + 4 * plane, bdesc, idesc_n(2 * I8_N), 1u);
+}
+
+// The MMA warp (converged, one elected lane issues): per N tile, all K chunks
+// into the six level accumulators of the tile's set (sets alternate by tile).
+// Rows rows8..127 of an A plane are the next plane's bytes: they only reach
+// TMEM lanes that no epilogue thread uses.
 __device__ void mma_role(const I8Params &P, I8Smem &S, uint32_t tmem) {
   volatile int *abort_flag = &S.abort_flag;
   uint32_t fill = 0, tile_ctr = 0;
-  bool issued = false;
   for (int it = blockIdx.x; it < P.n_items; it += gridDim.x) {
-    const I8Item W = P.items[it];
-    for (int t = 0; t < P.T; ++t)
-      for (int jn = 0; jn < W.n_nt; ++jn, ++tile_ctr) {
-        const int set = tile_ctr & 1;
-        const uint32_t dcol = tmem + (uint32_t)(set * I8_SET_COLS);
-        if (!mbar_wait(&S.acc_empty[set], ((tile_ctr >> 1) & 1) ^ 1, abort_flag, P.err)) goto out;
+    const I8Item &W = P.items[it];
+    const int n_kc = uniform(W.n_kc), n_tiles = uniform(W.n_nt) * P.T;
+    const uint32_t plane = (uint32_t)(uniform(W.rows8) * I8_ROWB) >> 4;  // descriptor units
+    for (int j = 0; j < n_tiles; ++j, ++tile_ctr) {
+      const int set = tile_ctr & 1;
+      const uint32_t dcol = tmem + (uint32_t)(set * I8_SET_COLS);
+      if (!warp_wait_all(&S.acc_empty[set], ((tile_ctr >> 1) & 1) ^ 1, abort_flag, P.err)) goto out;
+      for (int kc = 0; kc < n_kc; kc += I8_CHUNKS, ++fill) {
+        const int st = fill % I8_STAGES;
+        if (!warp_wait_all(&S.full[st], (fill / I8_STAGES) & 1, abort_flag, P.err)) goto out;
         tc_fence_after();
-        for (int kc = 0; kc < W.n_kc; ++kc, ++fill) {
-          const int st = fill % I8_STAGES;
-          if (!mbar_wait(&S.full[st], (fill / I8_STAGES) & 1, abort_flag, P.err)) goto out;
-          tc_fence_after();
-          // Digit levels along N: B planes 0..m of a stage are one contiguous
-          // matrix of 32 (m + 1) rows, so A plane s times planes 0..5-s, written
-          // from accumulator column 32 s on, puts product (s, u) into the
-          // columns of level s + u.  Plane s = 0 also multiplies the zero plane
-          // (rows 160..191), so its MMA covers all six levels and alone starts
-          // the accumulation of a tile; the other four always accumulate.
+        if (elect_one()) {
+          const uint64_t adesc = smem_desc<I8_LBO, I8_SBO>(smem_u32(S.A[st]));
           const uint64_t bdesc = smem_desc<I8_LBO, I8_SBO>(smem_u32(S.B[st]));
+          if (kc == 0)
+            chunk_mmas<true>(dcol, adesc, plane, bdesc);
+          else
+            chunk_mmas<false>(dcol, adesc, plane, bdesc);
 #pragma unroll
-          for (int s = 0; s < I8_SLICES; ++s) {
-            const int n_mma = I8_N * (s == 0 ? I8_LEVELS : I8_LEVELS - s);  // 192, 160, 128, 96, 64
-            umma_i8(dcol + (uint32_t)(s * I8_N), smem_desc<I8_LBO, I8_SBO>(smem_u32(S.A[st][s])), bdesc,
-                    idesc_n(n_mma), (s > 0 || kc > 0) ? 1u : 0u);
-          }
+          for (int q = 1; q < I8_CHUNKS; ++q)
+            if (kc + q < n_kc)
+              chunk_mmas<false>(dcol, adesc + q * I8_SLICES * plane, plane, bdesc + q * (I8_B_CHUNK >> 4));
           umma_commit(&S.empty[st]);
-          issued = true;
+          if (kc + I8_CHUNKS >= n_kc) umma_commit(&S.acc_full[set]);
         }
-        umma_commit(&S.acc_full[set]);
+        __syncwarp();
       }
+    }
   }
 out:
   // no MMA may be in flight when TMEM is released
-  if (issued) {
-    umma_commit(&S.drain);
-    if (!mbar_wait_quiet(&S.drain, 0)) atomicOr(P.err, 4);
-  }
+  if (elect_one()) umma_commit(&S.drain);
+  __syncwarp();
+  if (!mbar_wait_quiet(&S.drain, 0)) atomicOr(P.err, 4);
 }
 
-// FP64 operands of one 8-column chunk of the epilogue: phi and grad phi at
-// rows i0..i0+7 of one point's column.  Values at rows >= n_compute (the
-// row padding, possibly garbage) are masked where they are used.
+// FP64 operands of one four-column step of an epilogue warp: phi and
+// grad phi at rows i0..i0+3 of one point's column.  Values at rows >=
+// n_compute (the row padding, possibly garbage) are masked where they are used.
 struct EpiRegs {
-  double f[8], gx[8], gy[8], gz[8];
+  double f[4], gx[4], gy[4], gz[4];
 };
 
 __device__ __forceinline__ void epi_load(EpiRegs &E, const double *__restrict__ phi, const double *__restrict__ gph,
                                          int ncp, int nc, int i0, bool live, bool vec) {
   if (vec) {  // 32-byte loads: i0 and the row starts are multiples of 4, rows end at ncp >= i0 + 4
+    if (live && i0 < nc) {
+      ld4(phi + i0, E.f);
+      ld4(gph + i0, E.gx);
+      ld4(gph + ncp + i0, E.gy);
+      ld4(gph + 2 * ncp + i0, E.gz);
+    } else {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c = i0 + 4 * h;
-      if (live && c < nc) {
-        ld4(phi + c, &E.f[4 * h]);
-        ld4(gph + c, &E.gx[4 * h]);
-        ld4(gph + ncp + c, &E.gy[4 * h]);
-        ld4(gph + 2 * ncp + c, &E.gz[4 * h]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) E.f[4 * h + e] = E.gx[4 * h + e] = E.gy[4 * h + e] = E.gz[4 * h + e] = 0.0;
-      }
+      for (int e = 0; e < 4; ++e) E.f[e] = E.gx[e] = E.gy[e] = E.gz[e] = 0.0;
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 4; ++j) {
       const bool ok = live && i0 + j < nc;
       E.f[j] = ok ? __ldg(phi + i0 + j) : 0.0;
       E.gx[j] = ok ? __ldg(gph + i0 + j) : 0.0;
@@ -411,14 +466,36 @@ __device__ __forceinline__ void epi_load(EpiRegs &E, const double *__restrict__ 
   }
 }
 
+// Four columns of a tile: recombine the six levels in FP64 and contract with
+// phi and grad phi; rows at or past `lim` are outside n_compute.
+__device__ __forceinline__ void epi_step(const EpiRegs &E, uint32_t acc, const double *__restrict__ sbv, int lim,
+                                            double &r, double &gx, double &gy, double &gz) {
+  uint32_t v[I8_LEVELS][4];
+#pragma unroll
+  for (int l = 0; l < I8_LEVELS; ++l) tmem_ld4(acc + (uint32_t)(l * I8_N), v[l]);
+  tmem_wait_ld();
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    // 256 S = (L0 256 + L1) 2^32 + (L2 256 + L3) 2^16 + (L4 256 + L5), each pair exact in int64
+    const long long hi = (long long)(int)v[0][e] * 256 + (int)v[1][e];
+    const long long mid = (long long)(int)v[2][e] * 256 + (int)v[3][e];
+    const long long lo = (long long)(int)v[4][e] * 256 + (int)v[5][e];
+    const double w = fma((double)hi, 4294967296.0, fma((double)mid, 65536.0, (double)lo)) * __ldg(sbv + e);
+    const bool ok = e < lim;
+    r = fma(ok ? E.f[e] : 0.0, w, r);
+    gx = fma(ok ? E.gx[e] : 0.0, w, gx);
+    gy = fma(ok ? E.gy[e] : 0.0, w, gy);
+    gz = fma(ok ? E.gz[e] : 0.0, w, gz);
+  }
+}
+
 // Epilogue warp w reads TMEM lanes 32 (w % 4).. (its points) and columns
-// 16 (w / 4)..+15 of each level accumulator of the tile's set, recombines the
-// six levels in FP64 and contracts with phi and grad phi; the loads of each
-// 8-column chunk are issued one chunk ahead (the first chunk of a tile
-// before its accumulators are waited for).  The set is released after the
-// last chunk; meanwhile the MMAs of the next tile fill the other set.  The
-// two warps of a lane quarter add their partial sums through shared memory
-// at each perturbation's end.
+// 16 (w / 4)..+15 of each level accumulator of the tile's set, four at a time.
+// The phi / grad phi registers of a four-column step are loaded again as soon
+// as the step is done, two steps ahead of their use and across the tiles of an
+// item.  The set is released after its last read; meanwhile the MMAs of the
+// next tile fill the other set.  The two warps of a lane quarter add their
+// partial sums through shared memory at each perturbation's end.
 __device__ void epilogue_role(const I8Params &P, I8Smem &S, uint32_t tmem, int warp, int lane) {
   int *err = P.err;
   volatile int *abort_flag = &S.abort_flag;
@@ -429,56 +506,37 @@ __device__ void epilogue_role(const I8Params &P, I8Smem &S, uint32_t tmem, int w
   const bool vec = P.wave_vec != 0;
   uint32_t tile_ctr = 0, sum_ctr = 0;
   for (int it = blockIdx.x; it < P.n_items; it += gridDim.x) {
-    const I8Item W = P.items[it];
-    const int nc = W.nc, ncp = (nc + 3) & ~3;
+    const I8Item &W = P.items[it];
+    const int nc = W.nc, ncp = (nc + 3) & ~3, n_nt = W.n_nt;
     const bool live = p < W.pn;
     const long long pt = W.p0 + (live ? p : 0);
     const double *phi = P.wave + W.wave_off + pt * ncp;
     const double *gph = P.gwave + 3 * W.wave_off + 3 * pt * ncp;
+    EpiRegs E[EPI_BUFS];
+#pragma unroll
+    for (int q = 0; q < EPI_BUFS; ++q) epi_load(E[q], phi, gph, ncp, nc, cbase + 4 * q, live, vec);
     for (int t = 0; t < P.T; ++t) {
       double r = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-      const double *sbt = P.sb + W.sb_off + (long long)t * W.sb_tstride;
-      for (int jn = 0; jn < W.n_nt; ++jn, ++tile_ctr) {
-        const int N = tile_rows(nc, jn, W.n_nt);
-        const int ncols = min(I8_COLS, N - cbase);  // warp-uniform, a multiple of 8 (or <= 0)
-        const int ibase = jn * I8_N + cbase;
+      const double *sbv = P.sb + W.sb_off + (long long)t * W.sb_tstride + cbase;
+      for (int jn = 0; jn < n_nt; ++jn, ++tile_ctr, sbv += I8_N) {
         const int set = tile_ctr & 1;
         const uint32_t acc = lane_base + (uint32_t)(set * I8_SET_COLS + cbase);
-        const double *sbv = sbt + ibase;
-        EpiRegs E;
-        if (ncols > 0) epi_load(E, phi, gph, ncp, nc, ibase, live, vec);  // before the wait
+        const int lim = live ? nc - (jn * I8_N + cbase) : 0;  // rows from this column on inside n_compute
+        const int next = (jn + 1 < n_nt ? (jn + 1) * I8_N : (t + 1 < P.T ? 0 : nc)) + cbase;
         if (!warp_wait(&S.acc_full[set], (tile_ctr >> 1) & 1, abort_flag, err, lane)) return;
         tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < ncols; c += 8) {
-          const int lim = live ? nc - (ibase + c) : 0;  // rows of this chunk inside n_compute
 #pragma unroll
-          for (int hq = 0; hq < 8; hq += 4) {
-            uint32_t v[I8_LEVELS][4];
-#pragma unroll
-            for (int l = 0; l < I8_LEVELS; ++l) tmem_ld4(acc + (uint32_t)(l * I8_N + c + hq), v[l]);
-            tmem_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int j = hq + e;
-              // 256 S = (L0 256 + L1) 2^32 + (L2 256 + L3) 2^16 + (L4 256 + L5), each pair exact in int64
-              const long long hi = (long long)(int)v[0][e] * 256 + (int)v[1][e];
-              const long long mid = (long long)(int)v[2][e] * 256 + (int)v[3][e];
-              const long long lo = (long long)(int)v[4][e] * 256 + (int)v[5][e];
-              const double w = fma((double)hi, 4294967296.0, fma((double)mid, 65536.0, (double)lo)) *
-                               __ldg(sbv + c + j);
-              const bool ok = j < lim;
-              r = fma(ok ? E.f[j] : 0.0, w, r);
-              gx = fma(ok ? E.gx[j] : 0.0, w, gx);
-              gy = fma(ok ? E.gy[j] : 0.0, w, gy);
-              gz = fma(ok ? E.gz[j] : 0.0, w, gz);
-            }
+        for (int q = 0; q < I8_COLS / 4; ++q) {
+          epi_step(E[q % EPI_BUFS], acc + 4 * q, sbv + 4 * q, lim - 4 * q, r, gx, gy, gz);
+          if (q == I8_COLS / 4 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.acc_empty[set]);
           }
-          if (c + 8 < ncols) epi_load(E, phi, gph, ncp, nc, ibase + c + 8, live, vec);
+          const int ahead = 4 * (q + EPI_BUFS);
+          epi_load(E[q % EPI_BUFS], phi, gph, ncp, nc,
+                   ahead < I8_COLS ? jn * I8_N + cbase + ahead : next + ahead - I8_COLS, live, vec);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&S.acc_empty[set]);
       }
       // combine the two column halves of this point and write
       const int sp = sum_ctr & 1;
@@ -532,13 +590,6 @@ __global__ void __launch_bounds__(I8_THREADS, 1) rho1_i8_kernel(const I8Params P
     S.abort_flag = 0;
     mbar_init_fence();
   }
-  // the zero B plane of every stage (never written by the copies), made
-  // visible to the tensor core's (async proxy) reads
-  for (int e = tid; e < I8_STAGES * I8_N * I8_ROWB / 16; e += I8_THREADS) {
-    const int st = e / (I8_N * I8_ROWB / 16), o = e % (I8_N * I8_ROWB / 16);
-    reinterpret_cast<uint4 *>(S.B[st] + I8_B_STAGE)[o] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  fence_proxy_async_smem();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem_base)),
                  "r"(I8_TMEM_COLS));
@@ -553,10 +604,10 @@ __global__ void __launch_bounds__(I8_THREADS, 1) rho1_i8_kernel(const I8Params P
     epilogue_role(P, S, tmem, warp, lane);
     __syncwarp();
   } else if (warp == I8_LOAD_WARP) {
-    if (lane == 0) loader_role(P, S);
+    loader_role(P, S);
     __syncwarp();
   } else if (warp == I8_MMA_WARP) {
-    if (lane == 0) mma_role(P, S, tmem);
+    mma_role(P, S, tmem);
     __syncwarp();
   }
 
@@ -595,8 +646,7 @@ int rho1_i8_build(Rho1Plan *plan) {
   for (const Rho1WorkItem &bt : batches) {
     if (bt.np == 0) continue;
     const int nc = bt.nc, n_nt = ceil_div(nc, I8_N), n_kc = ceil_div(nc, I8_KC);
-    const int n_last = tile_rows(nc, n_nt - 1, n_nt);
-    const long long b_t = (long long)(n_nt - 1) * n_kc * I8_B_STAGE + (long long)n_kc * I8_SLICES * n_last * I8_ROWB;
+    const long long b_t = (long long)n_nt * n_kc * I8_B_CHUNK;  // the last N tile is padded with zero rows
     const int ntiles = ceil_div(bt.np, I8_M), width = ceil_div(bt.np, ntiles);
     long long a_need = 0;
     for (int p0 = 0; p0 < bt.np; p0 += width) {
@@ -612,9 +662,8 @@ int rho1_i8_build(Rho1Plan *plan) {
     const int sb_off = g.sb_len;
     for (int t = 0; t < T; ++t)
       for (int jn = 0; jn < n_nt; ++jn)
-        tiles.push_back(I8BTile{bt.ib_off, nc, jn, t, tile_rows(nc, jn, n_nt), n_kc,
-                                sb_off + t * n_nt * I8_N + jn * I8_N, 0,
-                                b_off + t * b_t + (long long)jn * n_kc * I8_B_STAGE});
+        tiles.push_back(I8BTile{bt.ib_off, nc, jn, t, n_kc, sb_off + t * n_nt * I8_N + jn * I8_N,
+                                b_off + t * b_t + (long long)jn * n_kc * I8_B_CHUNK});
     for (int p0 = 0; p0 < bt.np; p0 += width) {
       const int pn = std::min(width, bt.np - p0), rows8 = ((pn + 7) / 8) * 8;
       I8Item it{};
@@ -774,7 +823,7 @@ int rho1_i8_launch(Rho1Plan &plan, int n_active, const double *wave, const doubl
     const I8Group &g = plan.i8_groups[gi];
     const int k = gi % sets, ni = g.item1 - g.item0, nt = g.tile1 - g.tile0;
     if (gi >= sets) FRPA_CUDA_TRY(cudaStreamWaitEvent(plan.i8_side, plan.i8_ev_done[k], 0));
-    i8_pack_a_kernel<<<ni, PA_THREADS, 0, plan.i8_side>>>(plan.d_i8_items + g.item0, wave, plan.d_i8_a[k],
+    i8_pack_a_kernel<<<ni * PA_GROUPS, PA_THREADS, 0, plan.i8_side>>>(plan.d_i8_items + g.item0, wave, plan.d_i8_a[k],
                                                           plan.d_i8_sa[k], P.wave_vec);
     FRPA_LAUNCH_CHECK();
     i8_pack_b_kernel<<<nt, PB_THREADS, 0, plan.i8_side>>>(plan.d_i8_tiles + g.tile0, plan.d_ib, P1, plan.d_rowmax,

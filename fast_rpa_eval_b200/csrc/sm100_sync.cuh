@@ -39,26 +39,36 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, u
                : "memory");
 }
 
+// One poll; the thread may be suspended until the phase completes or
+// SUSPEND_NS have passed, so that waiting roles leave the issue slots and the
+// load/store unit to the working ones.
+constexpr uint32_t SUSPEND_NS = 20000;
+
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(SUSPEND_NS)
       : "memory");
   return ok != 0;
 }
 
 // Bounded wait: false (and error bit 2 set) if the phase does not complete
-// within WAIT_NS or another role has already given up.
+// within WAIT_NS or another role has already given up.  The abort flag and the
+// (slow) global timer are looked at once in WAIT_POLLS polls.
+constexpr int WAIT_POLLS = 32;
+
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t parity, volatile int *abort_flag,
                                           int *err) {
   if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long t0 = global_ns();
   for (;;) {
-    if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
+    for (int i = 0; i < WAIT_POLLS; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
     if (global_ns() - t0 > WAIT_NS) {
       *abort_flag = 1;
@@ -87,6 +97,32 @@ __device__ __forceinline__ bool warp_wait(unsigned long long *bar, uint32_t pari
   ok = __shfl_sync(0xffffffffu, ok, 0);
   __syncwarp();
   return ok != 0;
+}
+
+// The same wait by a whole warp that stays converged: every lane polls, and
+// all leave together (the slow path votes too).
+__device__ __forceinline__ bool warp_wait_all(unsigned long long *bar, uint32_t parity, volatile int *abort_flag,
+                                              int *err) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < WAIT_POLLS; ++i)
+      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const bool late = global_ns() - t0 > WAIT_NS;
+    if (late && !*abort_flag) {
+      *abort_flag = 1;
+      atomicOr(err, 2);
+    }
+    if (__any_sync(0xffffffffu, late || *abort_flag)) return false;
+  }
+}
+
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem() {

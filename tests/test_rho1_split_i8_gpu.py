@@ -114,3 +114,27 @@ def test_i8_through_the_reference_entry_points(via):
         r_o, g_o = oracle.rho1(q)
         assert normwise_rel(r.reshape(r_o.shape, order="F"), r_o) < TOL_SPLIT
         assert normwise_rel(g.reshape(g_o.shape, order="F"), g_o) < TOL_SPLIT
+
+
+@pytest.mark.parametrize("nc_range,np_range,T,n_active", [
+    ((1, 4), (1, 9), 1, 1),          # part of one K chunk, one 8-row group
+    ((31, 34), (63, 66), 2, 1),      # one and two chunks: half and whole stages
+    ((64, 65), (127, 130), 3, 3),    # two and three chunks, one and two point tiles
+    ((95, 98), (255, 258), 1, 1),    # three and four chunks, two and three point tiles
+    ((513, 545), (5, 40), 2, 2),     # rows longer than a CTA's pass of the packing
+])
+def test_i8_tile_edges_match_oracle(nc_range, np_range, T, n_active):
+    """Remainders of chunks, stages, rows and point tiles; the phi blocks once
+    on 32-byte boundaries and once at odd offsets (plain loads), bit-identical."""
+    p = synth.make_rho1_problem(T=T, seed=90 + nc_range[1], n_atoms=40, box=None, density=0.1, n_batches=6,
+                                np_range=np_range, nc_range=nc_range, with_bias=True, extra_full_points=13,
+                                empty_batches=2, pad_value=np.nan, n_active=n_active, exact_selection=False)
+    r, g = run_i8(p)
+    r_o, g_o = oracle.rho1(p)
+    assert normwise_rel(r, r_o) < TOL_SPLIT and normwise_rel(g, g_o) < TOL_SPLIT
+    assert np.array_equal(r_o == 0, r == 0)
+    p.wave = np.concatenate([[np.nan], p.wave])
+    p.gradient_wave = np.concatenate([[np.nan] * 3, p.gradient_wave])
+    p.i_batch_2_wave_offset = (p.i_batch_2_wave_offset + 1).astype(np.int32)
+    r1, g1 = run_i8(p)
+    assert np.array_equal(r, r1) and np.array_equal(g, g1)
