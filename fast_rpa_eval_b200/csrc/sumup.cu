@@ -51,7 +51,7 @@ namespace frpa {
 
 constexpr int SU_LMAX = FRPA_SUMUP_MAX_L;  // 8
 constexpr int SU_THREADS = 128;
-constexpr int SU_CHUNK = 8;      // centre records per shared-memory chunk (two buffers)
+constexpr int SU_CHUNK = 8;      // centre records per shared-memory chunk (two buffers) at the highest l
 
 // Near-field constants: Y_lm = K[l][m] Q_l^m(z) {C_m, S_m}; recursion
 // Q_l^m = RA[l][m] z Q_{l-1}^m - RB[l][m] Q_{l-2}^m; DF[m] = (2m-1)!!.
@@ -411,6 +411,9 @@ __device__ __forceinline__ int classify(const Box &b, const double *rec) {
 // zero (kelvin_masked_eval); an unsafe one takes a pass per l_atom_max.  (A box
 // per 32 points as well was slower: 7.9 ms below, and 6% on truncated radii.)
 // CODES: every record per pair, with the branch codes written.
+// The two record buffers hold as many records as fit (8 at l_max 8, 12 at 6, 32
+// below 4): fewer barriers, at which the warps wait for the one with the most
+// mixed records (8 for every l_max: 3% more on 2,000 to 100,000 points).
 // Measured, 500 atoms, 2 million points, l_max 6: 9.4 ms (two points per thread,
 // decisions per pair, near field inside) -> 7.7 ms, 70% of the FP64 peak (two
 // points per thread 8.7 ms, in the compiler's order 9.0 ms).
@@ -421,6 +424,7 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
                      double *__restrict__ dv, unsigned char *__restrict__ codes) {
   const int RS = rec_stride(L), CO = rec_coef_off(L);
   __shared__ __align__(16) double srec[2][SU_CHUNK * rec_stride(SU_LMAX)];
+  const int CH = min(32, (SU_CHUNK * rec_stride(SU_LMAX) / RS) & ~3);  // records per chunk
   __shared__ double part[SU_THREADS / 32][32 * PPT];
   __shared__ Box boxes[SU_THREADS / 32];  // read by the classification only: not worth registers
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.y;
@@ -455,17 +459,17 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
 
   const double *src = recs + (long long)RS * n_chp * t;
   auto load = [&](int c0, int buf) {  // records c0.. of this perturbation (RS is even: 16-byte copies)
-    const int n = min(SU_CHUNK, n_chp - c0) * RS / 2;
+    const int n = min(CH, n_chp - c0) * RS / 2;
     const double *from = src + (long long)RS * c0;
     for (int e = tid; e < n; e += SU_THREADS) cp_async_16(&srec[buf][2 * e], from + 2 * e, 16);
     cp_async_commit();
   };
   load(0, 0);
-  for (int c0 = 0, buf = 0; c0 < n_chp; c0 += SU_CHUNK, buf ^= 1) {
-    const int nch = min(SU_CHUNK, n_chp - c0);
+  for (int c0 = 0, buf = 0; c0 < n_chp; c0 += CH, buf ^= 1) {
+    const int nch = min(CH, n_chp - c0);
     cp_async_wait<0>();
     __syncthreads();  // this chunk is there; every warp is done with the other buffer
-    if (c0 + SU_CHUNK < n_chp) load(c0 + SU_CHUNK, buf ^ 1);
+    if (c0 + CH < n_chp) load(c0 + CH, buf ^ 1);
     if (!work) continue;
     const double *chunk = srec[buf];
     int cls_mine = CLS_MIXED;

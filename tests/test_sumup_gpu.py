@@ -105,6 +105,8 @@ def test_sumup_session_cu_host_matches_oracle():
     (7, 33, 1, 3, 6.0),         # one record less than a chunk, a warp and one lane
     (8, 129, 1, 4, 6.0),        # a whole chunk
     (9, 1000, 2, 8, 5.0),       # a chunk and one record; one point per thread, records over 4 warps
+    (33, 300, 1, 2, None),      # a chunk of the low degrees and one record
+    (25, 900, 2, 6, 6.0),       # two chunks of this degree and one record
     (20, 20_000, 4, 6, 6.0),    # two points per thread
     (16, 40_001, 4, 5, 6.0),    # four points per thread, records over 4 warps
     (3, 152_001, 4, 2, None),   # four points per thread, all records in one warp
