@@ -765,7 +765,8 @@ def run_frpa(args, ranks: Ranks):
                                    "(no collective on the forward path)")},
         "roofline": roofline,
         "clocks": clk,
-        "gpu_launches": args.steps * {_lib.RHO1_FP64: 1, _lib.RHO1_SPLIT_BF16: 2,
+        "gpu_launches": args.steps * {_lib.RHO1_FP64: 2,  # outputs cleared, rho1
+                                      _lib.RHO1_SPLIT_BF16: 2,
                                       _lib.RHO1_SPLIT_I8: 1 + 3 * i8_groups}[mode],
         "cpu_baseline": cpu,
         "e2e": e2e,

@@ -330,7 +330,9 @@ int frpa_rho1_bias_part2(const frpa_rho1_plan *plan, int T, int n_atoms, int j_a
  *   FRPA_TUNE_FP64_TILE_POINTS  64 (256 threads, up to 2 CTAs per SM) or 128
  *                               (512 threads, 1 CTA per SM: each gathered P1c
  *                               tile serves twice the points);
- *   FRPA_TUNE_FP64_CTAS_PER_SM  0 (as many as fit), 1, 2 or 3;
+ *   FRPA_TUNE_FP64_CTAS_PER_SM  0 (as many as fit), 1, 2 or 3 (neither FP64 key
+ *                               concerns plans of batches with at most 120
+ *                               functions, which have their own kernel);
  *   FRPA_TUNE_SPLIT_TILE_POINTS 16..128 points per split-BF16 work item;
  *   FRPA_TUNE_ORDER             0 largest items first, 1 batch order, 2 (the
  *                               default) batches grouped by a MinHash of their
@@ -364,8 +366,10 @@ int frpa_rho1_plan_get_tuning(const frpa_rho1_plan *plan, int key, int *value);
  * first_order_H (n_basis, n_basis, T) is accumulated into.  The per-batch
  * contributions are added as 128-bit fixed-point integers, so the result is
  * the same bits on every run whatever the order of the additions.  The
- * accumulator ((n_basis, n_basis, T) x 16 bytes, shared with the adjoint) is
- * allocated by the plan's first such call: make it before any stream capture.
+ * accumulator ((n_basis, n_basis, T) x 16 bytes) and the scratch for the
+ * points' A rows (at most 512 MiB, or one batch's if that is more), both shared
+ * with the adjoint, are allocated by the plan's first such call: make it before
+ * any stream capture.
  * Device flags (frpa_rho1_device_flags): bit 3 an atom's compute range
  * leaves its batch (clipped), bit 4 a non-finite input (result incomplete). */
 int frpa_rho1_first_order_h(const frpa_rho1_plan *plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,
@@ -379,7 +383,7 @@ int frpa_rho1_first_order_h(const frpa_rho1_plan *plan, int n_active, int n_atom
 /* Adjoint: dP1 (n_basis, n_basis, T) += d(sum g_rho . rho1 + sum g_grad . grad)/dP1.
  * g_rho (n_full_points, T) or NULL, g_grad like grad or NULL.  dP1 is NOT zeroed.
  * Same engine and accumulation as frpa_rho1_first_order_h: deterministic
- * (bit-identical from run to run); the first call allocates the accumulator. */
+ * (bit-identical from run to run); the first call allocates the same scratch. */
 int frpa_rho1_adjoint_p1(const frpa_rho1_plan *plan, int n_active, const double *wave, const double *gradient_wave,
                          const double *g_rho, const double *g_grad, double *dP1, void *stream);
 
