@@ -343,4 +343,29 @@ int rho1_first_order_h_run(Rho1Plan &plan, int n_active, int n_atoms, int j_atom
 
 struct SumupPlan;  // defined in sumup.cu
 
+// Launches a kernel that may start while its predecessor in the stream is still
+// running: it calls grid_wait() before it touches anything the predecessor
+// writes (or that its own outputs' readers may still use), and the predecessor
+// calls grid_release() when its dependents may come in.  The start-up of small
+// launches overlaps that way: the sum-up of 2,000 points, 20 atoms (three
+// launches) 32.5 -> 26.6 us, rho1 of 64 batches of 40-120 functions (two) 32.6 ->
+// 29.7 us.  The chain's first launch is an ordinary one, so everything queued
+// before it is complete.
+template <class... K, class... A>
+cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 }  // namespace frpa

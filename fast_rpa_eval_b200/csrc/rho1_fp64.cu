@@ -450,6 +450,7 @@ int rows_aligned16(const Rho1Plan &plan, const double *wave, const double *gwave
 __global__ void clear_outputs_kernel(long long n_rho, double *__restrict__ rho, long long n_grad,
                                      double *__restrict__ grad, int *__restrict__ counter) {
   const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  grid_release();
   if (first == 0) *counter = 0;
   for (long long e = first; e < n_rho; e += step) rho[e] = 0.0;
   for (long long e = first; e < n_grad; e += step) grad[e] = 0.0;

@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(THREADS, 1) rho1_small_kernel(const SmallParam
   auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory"); };
   const long long nb2 = (long long)P.n_basis * P.n_basis;
 
+  grid_wait();  // the cleared outputs and cursor
   for (int it = blockIdx.x; it < P.n_items;) {
     const Rho1WorkItem W = P.items[it];
     const int nc = W.nc, ncp = (nc + 3) & ~3, nb = (nc + 7) / 8, nMt = (nc + 63) / 64;
@@ -317,7 +318,8 @@ int rho1_small_launch(const Rho1Plan &plan, int n_active, const double *wave, co
   const SmallParams P{plan.d_items_small, plan.n_items_small, plan.T, n_active, plan.n_basis, plan.n_full_points,
                       plan.n_max_batch_size, plan.n_batches, plan.n_max_compute, plan.d_counter, plan.d_ib, plan.d_map,
                       wave, gwave, P1, bias, gbias, rho, grad};
-  rho1_small_kernel<<<std::min(n_sm, plan.n_items_small), THREADS, small_smem(plan.n_max_compute), stream>>>(P);
+  FRPA_CUDA_TRY(launch_chained(rho1_small_kernel, std::min(n_sm, plan.n_items_small), THREADS,
+                               small_smem(plan.n_max_compute), stream, P));
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
 }

@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(128)
                       double *__restrict__ recs, double4 *__restrict__ heads, int *__restrict__ err) {
   __shared__ double q_kept[(SU_LMAX + 1) * (SU_LMAX + 1)];
   const int slot = blockIdx.x, t = blockIdx.y, L2 = (L + 1) * (L + 1);
+  grid_release();
   if (slot < n_atoms && threadIdx.x == 0) {
     const int lh = lhmfd[slot + n_atoms * t];
     if (lh < 0 || lh > L || lh > lma) atomicOr(err, 1);
@@ -456,6 +457,8 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
 #pragma unroll
   for (int j = 0; j < PPT; ++j) any_live = any_live || live[j];
   const bool work = CODES || __any_sync(FULL, any_live);
+  grid_wait();  // the records; only the plan's points are read before
+  grid_release();
 
   const double *src = recs + (long long)RS * n_chp * t;
   auto load = [&](int c0, int buf) {  // records c0.. of this perturbation (RS is even: 16-byte copies)
@@ -610,6 +613,7 @@ __global__ void __launch_bounds__(32 * NF_MAX_SLICES)
                pz = valid ? pxyz[pt + 2LL * n_valid] : 0.0;
   const bool live = valid && isfinite(px) && isfinite(py) && isfinite(pz);
   const Box box = warp_box<1>(&px, &py, &pz, &live);
+  grid_wait();  // the far field's sums (and, before them, the records); only plan data is read before
   const int m8 = lane & 7, grp = lane >> 3;
   double v = 0.0;
   bool touched = false;
@@ -839,9 +843,9 @@ int launch_near(const SumupPlan &P, int n_active, const double *spline, double *
   switch (P.L) {
 #define FRPA_NEAR_CASE(LL)                                                                                           \
   case LL:                                                                                                           \
-    sumup_near_kernel<LL><<<grid, threads, smem, stream>>>(P.n_valid_points, P.n_full_points, P.d_pfull, P.d_pxyz,    \
-                                                           P.n_chp, P.n_atoms, P.n_hartree_grid, slices, P.d_recs,   \
-                                                           P.d_heads, spline, dv);                                   \
+    FRPA_CUDA_TRY(launch_chained(sumup_near_kernel<LL>, grid, threads, smem, stream, P.n_valid_points,               \
+                                 P.n_full_points, P.d_pfull, P.d_pxyz, P.n_chp, P.n_atoms, P.n_hartree_grid, slices, \
+                                 P.d_recs, P.d_heads, spline, dv));                                                  \
     break;
     FRPA_NEAR_CASE(0) FRPA_NEAR_CASE(1) FRPA_NEAR_CASE(2) FRPA_NEAR_CASE(3) FRPA_NEAR_CASE(4)
     FRPA_NEAR_CASE(5) FRPA_NEAR_CASE(6) FRPA_NEAR_CASE(7) FRPA_NEAR_CASE(8)
@@ -857,8 +861,9 @@ template <int PPT, bool CODES>
 int launch_far(const SumupPlan &P, int n_active, int slices, double *dv, unsigned char *codes, cudaStream_t stream) {
   const int groups = SU_THREADS / 32 / slices;  // point groups per CTA
   const dim3 grid(ceil_div(ceil_div(P.n_valid_points, 32 * PPT), groups), n_active);
-  sumup_far_kernel<PPT, CODES><<<grid, SU_THREADS, 0, stream>>>(P.n_valid_points, P.n_full_points, P.d_order,
-                                                                P.d_pfull, P.d_pxyz, P.n_chp, P.L, P.d_recs, slices, dv, codes);
+  FRPA_CUDA_TRY(launch_chained(sumup_far_kernel<PPT, CODES>, grid, SU_THREADS, 0, stream, P.n_valid_points,
+                               P.n_full_points, P.d_order, P.d_pfull, P.d_pxyz, P.n_chp, P.L, P.d_recs, slices, dv,
+                               codes));
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
 }

@@ -1,6 +1,7 @@
 """rho1 / grad rho1 on the GPU against the oracle (and the reference's own CPU code)."""
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from fast_rpa_eval_b200 import _lib, synth
@@ -176,3 +177,40 @@ def test_rho1_small_batches_match_oracle_and_the_general_kernel(nc_range, np_ran
     p.i_batch_2_wave_offset = (p.i_batch_2_wave_offset + 1).astype(np.int32)
     r1, g1 = rho1_device_run(_lib.Rho1Plan(p), p)
     assert np.array_equal(r, r1) and np.array_equal(g, g1)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_rho1_small_calls_in_a_row_equal_calls_one_by_one(captured):
+    """The launch that clears the outputs overlaps the start-up of the next;
+    calls queued without a wait, on alternating outputs and density matrices,
+    give the bits of separate calls."""
+    p = synth.make_rho1_problem(T=2, seed=79, n_atoms=10, n_batches=30, np_range=(40, 120), nc_range=(20, 100),
+                                with_bias=True, extra_full_points=13)
+    plan = _lib.Rho1Plan(p)
+    w, gw, bias, gbias = (dev(x) for x in (p.wave, p.gradient_wave, p.first_order_rho_bias_part2,
+                                           p.first_order_gradient_rho_bias))
+    P1 = [dev(p.first_order_density_matrix), dev(-0.3 * p.first_order_density_matrix)]
+
+    def outputs():
+        return [(torch.full((p.n_full_points * p.T,), 7.0, dtype=torch.float64, device="cuda"),
+                 torch.full((3 * p.n_max_batch_size * p.n_my_batches_work * p.T,), 7.0, dtype=torch.float64,
+                            device="cuda")) for _ in range(2)]
+
+    ref, out = outputs(), outputs()
+    for i in range(2):
+        plan.execute(p.T, w, gw, P1[i], bias, gbias, *ref[i])
+        torch.cuda.synchronize()
+
+    def queue():
+        for i in range(40):
+            plan.execute(p.T, w, gw, P1[i & 1], bias, gbias, *out[i & 1])
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            queue()
+        graph.replay()
+    else:
+        queue()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for r, o in zip(ref, out) for a, b in zip(r, o))

@@ -143,3 +143,32 @@ def test_sumup_extreme_records_match_generic_kernel(points):
     assert np.max(np.abs(fast - generic)[small]) < TOL * np.max(np.abs(generic[small]))
     big = ok & ~small
     assert np.all(np.abs(fast - generic)[big] < TOL * np.abs(generic[big]) * 1e2)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_sumup_calls_in_a_row_equal_calls_one_by_one(captured):
+    """The three launches of a call overlap their start-up; calls queued without
+    a wait, with other moments each time, give the bits of separate calls."""
+    p = synth.make_sumup_problem(n_atoms=20, n_points=3000, l_pot_max=4, T=2, seed=97, extra_full_points=5)
+    plan = _lib.SumupPlan(p)
+    a = [dev(p.l_hartree_max_far_distance, np.int32), dev(p.multipole_radius_sq), dev(p.outer_potential_radius)]
+    moments = [dev(p.multipole_moments), dev(-0.7 * p.multipole_moments)]
+    spline, na = dev(p.spline), p.j_atom_end - p.j_atom_begin + 1
+    dv = [dev(p.delta_v_hartree) for _ in range(2)]
+    for i in range(40):
+        plan.execute(na, *a, moments[i & 1], spline, dv[0])
+        torch.cuda.synchronize()
+
+    def queue():
+        for i in range(40):
+            plan.execute(na, *a, moments[i & 1], spline, dv[1])
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            queue()
+        graph.replay()
+    else:
+        queue()
+    torch.cuda.synchronize()
+    assert torch.equal(dv[0], dv[1])
