@@ -446,8 +446,7 @@ template <int PPT, bool CODES>
 __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
     sumup_far_kernel(int n_valid, int n_full, const int *__restrict__ order, const int *__restrict__ pfull,
                      const double *__restrict__ pxyz, const Box *__restrict__ pbox, int n_chp, int L,
-                     const double *__restrict__ recs, int slices,
-                     double *__restrict__ dv, unsigned char *__restrict__ codes) {
+                     const double *recs, int slices, double *dv, unsigned char *codes) {
   const int RS = rec_stride(L), CO = rec_coef_off(L);
   __shared__ __align__(16) double srec[2][SU_CHUNK * rec_stride(SU_LMAX)];
   const int CH = min(32, (SU_CHUNK * rec_stride(SU_LMAX) / RS) & ~3);  // records per chunk
@@ -615,8 +614,7 @@ template <int L>
 __global__ void __launch_bounds__(32 * NF_MAX_SLICES)
     sumup_near_kernel(int n_valid, int n_full, const int *__restrict__ pfull, const double *__restrict__ pxyz,
                       const Box *__restrict__ pbox, int n_chp, int n_atoms, int n_hartree_grid, int slices,
-                      const double *__restrict__ recs, const double4 *__restrict__ heads,
-                      const double *__restrict__ spline, double *__restrict__ dv) {
+                      const double *recs, const double4 *heads, const double *__restrict__ spline, double *dv) {
   constexpr int RS = rec_stride(L), L2 = (L + 1) * (L + 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_ra[L2], s_rb[L2], s_k[L2];  // (l, m) at l (L + 1) + m
