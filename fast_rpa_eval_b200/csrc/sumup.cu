@@ -305,16 +305,6 @@ __device__ double near_field(int lam, int L2, double dx, double dy, double dz, d
   return acc;
 }
 
-// 1/sqrt(x) for x > 0: the PTX approximation y (relative error below 1e-6) with
-// one third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2: within about one
-// ulp of 1 / sqrt(x); cheaper than the library's correctly rounded form.
-__device__ __forceinline__ double rsqrt_refined(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // l_atom_max at squared distance d2 (sum_up_whole_potential.cpp:404-411).
 __device__ __forceinline__ int lam_at(const double *opr, int lam0, double d2) {
   int l = lam0;
@@ -511,7 +501,7 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
 #pragma unroll
         for (int j = 0; j < PPT; ++j) {
           const double dx = px[j] - cx, dy = py[j] - cy, dz = pz[j] - cz;
-          rinv[j] = rsqrt_refined(fma(dz, dz, fma(dy, dy, dx * dx)));
+          rinv[j] = rsqrt(fma(dz, dz, fma(dy, dy, dx * dx)));
           const double ir2 = rinv[j] * rinv[j];
           ux[j] = dx * ir2;
           uy[j] = dy * ir2;
@@ -546,7 +536,7 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
         if (CODES && val)
           codes[vi + (long long)n_valid * ((c0 + s) + (long long)n_chp * t)] =
               (unsigned char)(is_near ? 1 + lam : (is_far ? 16 + lam : 0));
-        const double ri = is_far ? rsqrt_refined(d2) : 0.0;
+        const double ri = is_far ? rsqrt(d2) : 0.0;
         const double ir2 = ri * ri;
         const double ux = is_far ? dx * ir2 : 0.0, uy = is_far ? dy * ir2 : 0.0, uz = is_far ? dz * ir2 : 0.0;
         double P = 0.0, sum = 0.0;
@@ -1006,7 +996,7 @@ __device__ __forceinline__ void dcoef_pass(int n_valid, const int *__restrict__ 
     unsigned todo = __ballot_sync(FULL, is_far);
     if (!todo) continue;
     const int lam = lam_at(rec + R_OPR, lam0, d2);
-    const double ri = is_far ? rsqrt_refined(d2) : 0.0, ir2 = ri * ri;
+    const double ri = is_far ? rsqrt(d2) : 0.0, ir2 = ri * ri;
     const double gw = is_far ? P.g * ri : 0.0;
     const double ux = dx * ir2, uy = dy * ir2, uz = dz * ir2;
     // neighbouring points mostly share l_atom_max; each value present is one

@@ -172,3 +172,27 @@ def test_sumup_calls_in_a_row_equal_calls_one_by_one(captured):
         queue()
     torch.cuda.synchronize()
     assert torch.equal(dv[0], dv[1])
+
+
+def test_sumup_inverse_distance_of_a_point_charge():
+    """One centre with a monopole: delta_v is c / r.  Distances over the whole
+    far field, dense around powers of four in r^2, and the centre itself
+    (infinite, as in the table loop).  The points lie on the x axis, so r^2 has
+    one rounding (that of x x, repeated here) and the rest is one inverse square
+    root (CUDA: 1 ulp) and one multiplication (half an ulp): 2 ulp."""
+    p = synth.make_sumup_problem(n_atoms=1, n_points=5000, l_pot_max=0, seed=5, outer_radius=None)
+    rng = np.random.default_rng(5)
+    powers = 2.0 ** np.arange(-60, 14)
+    near_powers = np.concatenate([np.nextafter(powers, 0), powers, np.nextafter(powers, np.inf)])
+    x = np.concatenate([[0.0], near_powers, 10.0 ** rng.uniform(-19.5, 3.99, 5000 - 1 - near_powers.size)])
+    p.coords_center[:] = 0.0
+    p.coord_points[:] = 0.0
+    p.coord_points[0, p.i_valid_point_2_i_full_points_map] = x * rng.choice([-1.0, 1.0], x.size)
+    p.multipole_radius_sq[:] = 0.0
+    p.multipole_moments[:] = 1.0
+    p.delta_v_hartree[:] = 0.0
+    plan = _lib.SumupPlan(p)
+    v = run(plan, p)[p.i_valid_point_2_i_full_points_map, 0]
+    assert v[0] == np.inf == run(plan, p, generic=True)[p.i_valid_point_2_i_full_points_map[0], 0]
+    want = p.cc[0] / np.sqrt((x[1:] * x[1:]).astype(np.longdouble))
+    assert float(np.max(np.abs(v[1:] - want) / want)) < 2 * 2.0**-52
