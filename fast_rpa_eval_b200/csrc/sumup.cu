@@ -25,11 +25,11 @@
 //   loop.  The Horner degree is lam, specialised at compile time per warp-
 //   uniform lam (the l_max-specialised AOT kernels of the reference's
 //   task3_jit/version5, but derived from the runtime table rather than baked in).
-// * Near field, in a launch of its own after the far field's.  Real Y_lm by the
-//   associated-Legendre recursion fused with the Hermite spline dot, read
-//   straight from the caller's (L^2, 2, n_hartree_grid, atom, t) table (the two
-//   grid nodes needed are one contiguous 4 L^2 run), so the reference's
-//   per-call transpose is not needed.
+// * Near field, in a launch of its own after the far field's except for dense
+//   points around few centres.  Real Y_lm by the associated-Legendre recursion
+//   fused with the Hermite spline dot, read straight from the caller's
+//   (L^2, 2, n_hartree_grid, atom, t) table (the two grid nodes needed are one
+//   contiguous 4 L^2 run), so the reference's per-call transpose is not needed.
 // * Which pairs are near, far or skipped is decided for a warp's points at once
 //   wherever the box around them allows it (the points are in spatial order).
 // * Generic path.  When the fast path's preconditions do not hold (a
@@ -271,8 +271,8 @@ __device__ __forceinline__ NearGeom near_geometry(double dx, double dy, double d
   return G;
 }
 
-// Near field of one pair by one thread (generic path): Y_lm by recursion fused
-// with the Hermite spline dot.
+// Near field of one pair by one thread (generic path and dense points): Y_lm by
+// recursion fused with the Hermite spline dot.
 __device__ double near_field(int lam, int L2, double dx, double dy, double dz, double d2, double rgm, double linc,
                              int ngrid, const double *__restrict__ spl) {
   const NearGeom G = near_geometry(dx, dy, dz, d2, rgm, linc, ngrid);
@@ -303,6 +303,12 @@ __device__ double near_field(int lam, int L2, double dx, double dy, double dz, d
     }
   }
   return acc;
+}
+
+// The same as a call, so that its registers do not count against the far field's.
+__device__ __noinline__ double near_field_call(int lam, int L, const double *rec_near, double dx, double dy, double dz,
+                                               double d2, const double *__restrict__ spl) {
+  return near_field(lam, (L + 1) * (L + 1), dx, dy, dz, d2, rec_near[0], rec_near[1], (int)rec_near[2], spl);
 }
 
 // l_atom_max at squared distance d2 (sum_up_whole_potential.cpp:404-411).
@@ -395,12 +401,12 @@ __device__ __forceinline__ void box_distance(const Box &b, double cx, double cy,
 
 constexpr int CLS_SKIP = -1, CLS_MIXED = SU_LMAX + 1;  // 0..SU_LMAX: every point far with that l_atom_max
 
-// One record for one warp's box.
-__device__ __forceinline__ int classify(const Box &b, const double *rec) {
+// One record for one warp's box; near: this launch has the near field too.
+__device__ __forceinline__ int classify(const Box &b, const double *rec, bool near) {
   double n2, f2;
   box_distance(b, rec[R_X], rec[R_Y], rec[R_Z], &n2, &f2);
   const double mrs = rec[R_MRS];
-  if (n2 >= 1e8 || f2 < mrs) return CLS_SKIP;  // beyond the far field, or all near (the near-field launch's)
+  if (n2 >= 1e8 || (!near && f2 < mrs)) return CLS_SKIP;  // beyond the far field, or the near-field launch's
   if (!(n2 >= mrs) || !(f2 < 1e8)) return CLS_MIXED;
   // l_atom_max does not grow with the distance
   const int l0 = (int)rec[R_LAM0], l = lam_at(rec + R_OPR, l0, n2);
@@ -425,18 +431,22 @@ __device__ __forceinline__ int classify(const Box &b, const double *rec) {
 // largest l_atom_max present in which a lane's higher degrees are multiplied by
 // zero (kelvin_masked_eval); an unsafe one takes a pass per l_atom_max.  (A box
 // per 32 points as well was slower: 7.9 ms below, and 6% on truncated radii.)
+// NEAR: the near field too, each thread its own point's (near_inline says when).
 // CODES: every record per pair, with the branch codes written.
+// The sums go to delta_v as additions without a returned value (one per point, so
+// nothing depends on an order): a read before them was one latency more per CTA.
 // The two record buffers hold as many records as fit (8 at l_max 8, 12 at 6, 32
 // below 4): fewer barriers, at which the warps wait for the one with the most
 // mixed records (8 for every l_max: 3% more on 2,000 to 100,000 points).
 // Measured, 500 atoms, 2 million points, l_max 6: 9.4 ms (two points per thread,
 // decisions per pair, near field inside) -> 7.7 ms, 70% of the FP64 peak (two
 // points per thread 8.7 ms, in the compiler's order 9.0 ms).
-template <int PPT, bool CODES>
+template <int PPT, bool CODES, bool NEAR>
 __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
     sumup_far_kernel(int n_valid, int n_full, const int *__restrict__ order, const int *__restrict__ pfull,
                      const double *__restrict__ pxyz, const Box *__restrict__ pbox, int n_chp, int L,
-                     const double *recs, int slices, double *dv, unsigned char *codes) {
+                     const double *recs, int slices, double *dv, unsigned char *codes, const double *__restrict__ spline,
+                     int n_atoms, int n_hartree_grid) {
   const int RS = rec_stride(L), CO = rec_coef_off(L);
   __shared__ __align__(16) double srec[2][SU_CHUNK * rec_stride(SU_LMAX)];
   const int CH = min(32, (SU_CHUNK * rec_stride(SU_LMAX) / RS) & ~3);  // records per chunk
@@ -490,7 +500,7 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
     if (!work) continue;
     const double *chunk = srec[buf];
     int cls_mine = CLS_MIXED;
-    if (!CODES) cls_mine = lane < nch ? classify(boxes[warp], chunk + lane * RS) : CLS_SKIP;
+    if (!CODES) cls_mine = lane < nch ? classify(boxes[warp], chunk + lane * RS, NEAR) : CLS_SKIP;
     for (int s = slice; s < nch; s += slices) {
       const double *rec = chunk + s * RS;
       const int cls = CODES ? CLS_MIXED : __shfl_sync(FULL, cls_mine, s);
@@ -549,7 +559,11 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
             pend = false;
           }
         }
-        if (is_far) {
+        if (NEAR && is_near)
+          sum = near_field_call(lam, L, rec + R_RGM, dx, dy, dz, d2,
+                                spline + 2LL * (L + 1) * (L + 1) * n_hartree_grid *
+                                             ((long long)rec[R_ATOM] + (long long)n_atoms * t));
+        if (is_far || (NEAR && is_near)) {
 #pragma unroll
           for (int i = 0; i < PPT; ++i)
             if (j == i) v[i] += sum;
@@ -568,7 +582,7 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
   }
 #pragma unroll
   for (int j = 0; j < PPT; ++j)
-    if (live[j]) dv[full[j] + (long long)n_full * t] += v[j];
+    if (live[j]) atomicAdd(dv + full[j] + (long long)n_full * t, v[j]);
 }
 
 // -------------------------------------------------- near-field kernel ---
@@ -754,7 +768,7 @@ __global__ void __launch_bounds__(32 * NF_MAX_SLICES)
       }
     }
   }
-  if (touched) dv[pfull[pt] + (long long)n_full * t] += v;
+  if (touched) atomicAdd(dv + pfull[pt] + (long long)n_full * t, v);
 }
 
 // ------------------------------------------------------ generic kernel ---
@@ -868,21 +882,37 @@ int launch_near(const SumupPlan &P, int n_active, const double *spline, double *
   return FRPA_OK;
 }
 
-template <int PPT, bool CODES>
-int launch_far(const SumupPlan &P, int n_active, int slices, double *dv, unsigned char *codes, cudaStream_t stream) {
+template <int PPT, bool CODES, bool NEAR>
+int launch_far(const SumupPlan &P, int n_active, int slices, const double *spline, double *dv, unsigned char *codes,
+               cudaStream_t stream) {
   const int groups = SU_THREADS / 32 / slices;  // point groups per CTA
   const dim3 grid(ceil_div(ceil_div(P.n_valid_points, 32 * PPT), groups), n_active);
-  FRPA_CUDA_TRY(launch_chained(sumup_far_kernel<PPT, CODES>, grid, SU_THREADS, 0, stream, P.n_valid_points,
-                               P.n_full_points, P.d_order, P.d_pfull, P.d_pxyz, P.d_pbox, P.n_chp, P.L, P.d_recs, slices, dv,
-                               codes));
+  FRPA_CUDA_TRY(launch_chained(sumup_far_kernel<PPT, CODES, NEAR>, grid, SU_THREADS, 0, stream, P.n_valid_points,
+                               P.n_full_points, P.d_order, P.d_pfull, P.d_pxyz, P.d_pbox, P.n_chp, P.L, P.d_recs,
+                               slices, dv, codes, spline, P.n_atoms, P.n_hartree_grid));
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
+}
+
+// Where a warp's 32 points mostly share a centre's near sphere, each thread adds its
+// own near field in the far-field launch: the launch of its own (10 us and a chain of
+// latencies per group of points) pays only where a warp's near pairs are few or their
+// sums long.  Measured, us, own launch / inline:
+//   points per centre        1 centre                     10 centres      50 centres      200 centres
+//   l_max 4: 2,000, 16,000   21 / 12, 26 / 17 (2)         31 / 20, 72 / 51  106 / 91, 370 / 311  562 / 513 (2,000)
+//   l_max 2: 2,000, 16,000   18 / 13, 20 / 13 (2)         24 / 15, 51 / 35  75 / 60, 213 / 201   350 / 369 (2,000)
+//   l_max 5: 2,000, 64,000   - , 24 / 18                  43 / 32, 116 / 108 (8)  167 / 196 (2,000)
+//   l_max 6: 8,000, 64,000   26 / 19, 28 / 20             72 / 61, 134 / 159 (8)  312 / 397 (8,000)
+// (in brackets: at another number of centres, or the one size).
+bool near_inline(int L, int n_points, int n_centres) {
+  const int most = L <= 4 ? 128 : (L == 5 ? 16 : 1);
+  return n_centres <= most && n_points >= 2048LL * n_centres;
 }
 
 int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *dv, unsigned char *codes,
                 cudaStream_t stream) {
   if (codes) {
-    FRPA_TRY((launch_far<2, true>(P, n_active, 1, dv, codes, stream)));
+    FRPA_TRY((launch_far<2, true, false>(P, n_active, 1, spline, dv, codes, stream)));
     return launch_near(P, n_active, spline, dv, stream);
   }
   int n_sm = 148;
@@ -895,15 +925,18 @@ int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *
   auto warps = [&] { return (long long)ceil_div(P.n_valid_points, 32 * ppt) * n_active * slices; };
   while (warps() < want && slices < 4 && P.n_chp >= 4 * slices) slices *= 2;
   while (warps() < want && ppt > 1) ppt /= 2;
+  if (near_inline(P.L, P.n_valid_points, P.n_chp)) {
+    if (ppt > 1) return launch_far<2, false, true>(P, n_active, slices, spline, dv, nullptr, stream);
+    return launch_far<1, false, true>(P, n_active, slices, spline, dv, nullptr, stream);
+  }
   if (ppt == 4)
-    FRPA_TRY((launch_far<4, false>(P, n_active, slices, dv, nullptr, stream)));
+    FRPA_TRY((launch_far<4, false, false>(P, n_active, slices, spline, dv, nullptr, stream)));
   else if (ppt == 2)
-    FRPA_TRY((launch_far<2, false>(P, n_active, slices, dv, nullptr, stream)));
+    FRPA_TRY((launch_far<2, false, false>(P, n_active, slices, spline, dv, nullptr, stream)));
   else
-    FRPA_TRY((launch_far<1, false>(P, n_active, slices, dv, nullptr, stream)));
+    FRPA_TRY((launch_far<1, false, false>(P, n_active, slices, spline, dv, nullptr, stream)));
   return launch_near(P, n_active, spline, dv, stream);
 }
-
 
 // -------------------------------------------------------- adjoint (dQ) ---
 

@@ -196,3 +196,25 @@ def test_sumup_inverse_distance_of_a_point_charge():
     assert v[0] == np.inf == run(plan, p, generic=True)[p.i_valid_point_2_i_full_points_map[0], 0]
     want = p.cc[0] / np.sqrt((x[1:] * x[1:]).astype(np.longdouble))
     assert float(np.max(np.abs(v[1:] - want) / want)) < 2 * 2.0**-52
+
+
+@pytest.mark.parametrize("atoms,points,T,L,outer", [
+    (1, 2047, 1, 4, 3.0),      # the near field in its own launch
+    (1, 2048, 1, 4, 3.0),      # inline: one point per thread
+    (1, 2100, 2, 8, 3.0),      # the highest l; one centre at most
+    (2, 5000, 1, 6, None),     # own launch at this l
+    (16, 33_000, 1, 5, 4.0),   # the most centres of l 5, records over 4 warps
+    (17, 36_000, 1, 5, 4.0),   # one more
+    (128, 262_144, 1, 0, None),  # two points per thread, several chunks of records
+    (3, 152_001, 2, 1, 2.5),   # two points per thread, all records in one warp
+])
+def test_sumup_dense_points_match_oracle(atoms, points, T, L, outer):
+    """Both sides of the rule that puts the near field into the far field's
+    launch, with radii cut inside and outside the near sphere."""
+    p = synth.make_sumup_problem(n_atoms=atoms, n_points=points, l_pot_max=L, T=T, seed=120 + atoms, outer_radius=outer,
+                                 l_hartree_per_species=[L, max(0, L - 1), L, max(0, L - 2)], extra_full_points=5)
+    out = run(_lib.SumupPlan(p), p)
+    ref = oracle.sumup(p, n_threads=8)
+    assert delta_rel(out, ref, p.delta_v_hartree) < TOL
+    untouched = np.setdiff1d(np.arange(p.n_full_points), p.i_valid_point_2_i_full_points_map)
+    assert np.array_equal(out[untouched], p.delta_v_hartree[untouched])
