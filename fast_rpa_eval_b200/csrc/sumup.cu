@@ -432,7 +432,8 @@ __device__ __forceinline__ int classify(const Box &b, const double *rec, bool ne
 // zero (kelvin_masked_eval); an unsafe one takes a pass per l_atom_max.  (A box
 // per 32 points as well was slower: 7.9 ms below, and 6% on truncated radii.)
 // NEAR: the near field too, each thread its own point's (near_inline says when).
-// CODES: every record per pair, with the branch codes written.
+// CODES: the decisions are written as well, each where it is taken: the far field's
+// (and, if NEAR, the near field's) here, otherwise the near field's by its launch.
 // The sums go to delta_v as additions without a returned value (one per point, so
 // nothing depends on an order): a read before them was one latency more per CTA.
 // The two record buffers hold as many records as fit (8 at l_max 8, 12 at 6, 32
@@ -499,11 +500,17 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
     if (c0 + CH < n_chp) load(c0 + CH, buf ^ 1);
     if (!work) continue;
     const double *chunk = srec[buf];
-    int cls_mine = CLS_MIXED;
-    if (!CODES) cls_mine = lane < nch ? classify(boxes[warp], chunk + lane * RS, NEAR) : CLS_SKIP;
+    const int cls_mine = lane < nch ? classify(boxes[warp], chunk + lane * RS, NEAR) : CLS_SKIP;
     for (int s = slice; s < nch; s += slices) {
       const double *rec = chunk + s * RS;
-      const int cls = CODES ? CLS_MIXED : __shfl_sync(FULL, cls_mine, s);
+      const int cls = __shfl_sync(FULL, cls_mine, s);
+      if (CODES && cls != CLS_MIXED) {
+#pragma unroll
+        for (int j = 0; j < PPT; ++j)
+          if (valid[j])
+            codes[vidx[j] + (long long)n_valid * ((c0 + s) + (long long)n_chp * t)] =
+                (unsigned char)(live[j] && cls != CLS_SKIP ? 16 + cls : 0);
+      }
       if (cls == CLS_SKIP) continue;
       const double cx = rec[R_X], cy = rec[R_Y], cz = rec[R_Z];
       if (cls < CLS_MIXED) {
@@ -545,7 +552,7 @@ __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
         const bool is_near = val && d2 < mrs, is_far = val && !is_near && d2 < 1e8;
         if (CODES && val)
           codes[vi + (long long)n_valid * ((c0 + s) + (long long)n_chp * t)] =
-              (unsigned char)(is_near ? 1 + lam : (is_far ? 16 + lam : 0));
+              (unsigned char)(is_far ? 16 + lam : (NEAR && is_near ? 1 + lam : 0));
         const double ri = is_far ? rsqrt(d2) : 0.0;
         const double ir2 = ri * ri;
         const double ux = is_far ? dx * ir2 : 0.0, uy = is_far ? dy * ir2 : 0.0, uz = is_far ? dz * ir2 : 0.0;
@@ -614,11 +621,12 @@ struct NearWarp {
 // were slower (1.57 ms against 0.94 ms on 2 million points, 500 atoms).  Where the
 // points are few, 2 to 8 warps share 32 points and take the candidate centres in
 // turn (2,000 points, 20 atoms: 76 us with one).  Every sum has a fixed order.
-template <int L>
+template <int L, bool CODES>
 __global__ void __launch_bounds__(32 * NF_MAX_SLICES)
     sumup_near_kernel(int n_valid, int n_full, const int *__restrict__ pfull, const double *__restrict__ pxyz,
                       const Box *__restrict__ pbox, int n_chp, int n_atoms, int n_hartree_grid, int slices,
-                      const double *recs, const double4 *heads, const double *__restrict__ spline, double *dv) {
+                      const double *recs, const double4 *heads, const double *__restrict__ spline, double *dv,
+                      const int *__restrict__ order, unsigned char *codes) {
   constexpr int RS = rec_stride(L), L2 = (L + 1) * (L + 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_ra[L2], s_rb[L2], s_k[L2];  // (l, m) at l (L + 1) + m
@@ -661,7 +669,11 @@ __global__ void __launch_bounds__(32 * NF_MAX_SLICES)
         W.h[lane][1] = G.tb;
         W.h[lane][2] = G.tc;
         W.h[lane][3] = G.td;
-        W.lam[lane] = lam_at(rec + R_OPR, (int)rec[R_LAM0], d2);
+        const int lam = lam_at(rec + R_OPR, (int)rec[R_LAM0], d2);
+        W.lam[lane] = lam;
+        if (CODES)
+          codes[order[pt - lane + o] + (long long)n_valid * (W.slot[lane] + (long long)n_chp * t)] =
+              (unsigned char)(1 + lam);
         W.run[lane] = spline + (long long)2 * L2 *
                                    (n_hartree_grid * ((long long)rec[R_ATOM] + (long long)n_atoms * t) + G.i_spl - 1);
       }
@@ -855,7 +867,9 @@ int launch_prep(const SumupPlan &P, int n_active, const int *lhmfd, const double
   return FRPA_OK;
 }
 
-int launch_near(const SumupPlan &P, int n_active, const double *spline, double *dv, cudaStream_t stream) {
+template <bool CODES>
+int launch_near(const SumupPlan &P, int n_active, const double *spline, double *dv, unsigned char *codes,
+                cudaStream_t stream) {
   int n_sm = 148;
   FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, P.device));
   const int groups = ceil_div(P.n_valid_points, 32);
@@ -866,11 +880,11 @@ int launch_near(const SumupPlan &P, int n_active, const double *spline, double *
   const dim3 grid(ceil_div(groups, threads / 32 / slices), n_active);
   const size_t smem = (threads / 32) * sizeof(NearWarp);
   switch (P.L) {
-#define FRPA_NEAR_CASE(LL)                                                                                           \
-  case LL:                                                                                                           \
-    FRPA_CUDA_TRY(launch_chained(sumup_near_kernel<LL>, grid, threads, smem, stream, P.n_valid_points,               \
-                                 P.n_full_points, P.d_pfull, P.d_pxyz, P.d_pbox, P.n_chp, P.n_atoms, P.n_hartree_grid, slices, \
-                                 P.d_recs, P.d_heads, spline, dv));                                                  \
+#define FRPA_NEAR_CASE(LL)                                                                                        \
+  case LL:                                                                                                        \
+    FRPA_CUDA_TRY(launch_chained(sumup_near_kernel<LL, CODES>, grid, threads, smem, stream, P.n_valid_points,     \
+                                 P.n_full_points, P.d_pfull, P.d_pxyz, P.d_pbox, P.n_chp, P.n_atoms,              \
+                                 P.n_hartree_grid, slices, P.d_recs, P.d_heads, spline, dv, P.d_order, codes));   \
     break;
     FRPA_NEAR_CASE(0) FRPA_NEAR_CASE(1) FRPA_NEAR_CASE(2) FRPA_NEAR_CASE(3) FRPA_NEAR_CASE(4)
     FRPA_NEAR_CASE(5) FRPA_NEAR_CASE(6) FRPA_NEAR_CASE(7) FRPA_NEAR_CASE(8)
@@ -909,12 +923,9 @@ bool near_inline(int L, int n_points, int n_centres) {
   return n_centres <= most && n_points >= 2048LL * n_centres;
 }
 
+template <bool CODES>
 int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *dv, unsigned char *codes,
                 cudaStream_t stream) {
-  if (codes) {
-    FRPA_TRY((launch_far<2, true, false>(P, n_active, 1, spline, dv, codes, stream)));
-    return launch_near(P, n_active, spline, dv, stream);
-  }
   int n_sm = 148;
   FRPA_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, P.device));
   // four points per thread share every coefficient load; the fewer warps that
@@ -926,16 +937,16 @@ int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *
   while (warps() < want && slices < 4 && P.n_chp >= 4 * slices) slices *= 2;
   while (warps() < want && ppt > 1) ppt /= 2;
   if (near_inline(P.L, P.n_valid_points, P.n_chp)) {
-    if (ppt > 1) return launch_far<2, false, true>(P, n_active, slices, spline, dv, nullptr, stream);
-    return launch_far<1, false, true>(P, n_active, slices, spline, dv, nullptr, stream);
+    if (ppt > 1) return launch_far<2, CODES, true>(P, n_active, slices, spline, dv, codes, stream);
+    return launch_far<1, CODES, true>(P, n_active, slices, spline, dv, codes, stream);
   }
   if (ppt == 4)
-    FRPA_TRY((launch_far<4, false, false>(P, n_active, slices, spline, dv, nullptr, stream)));
+    FRPA_TRY((launch_far<4, CODES, false>(P, n_active, slices, spline, dv, codes, stream)));
   else if (ppt == 2)
-    FRPA_TRY((launch_far<2, false, false>(P, n_active, slices, spline, dv, nullptr, stream)));
+    FRPA_TRY((launch_far<2, CODES, false>(P, n_active, slices, spline, dv, codes, stream)));
   else
-    FRPA_TRY((launch_far<1, false, false>(P, n_active, slices, spline, dv, nullptr, stream)));
-  return launch_near(P, n_active, spline, dv, stream);
+    FRPA_TRY((launch_far<1, CODES, false>(P, n_active, slices, spline, dv, codes, stream)));
+  return launch_near<CODES>(P, n_active, spline, dv, codes, stream);
 }
 
 // -------------------------------------------------------- adjoint (dQ) ---
@@ -1491,7 +1502,8 @@ int sumup_execute(const SumupPlan *P, int n_active, int force_generic, const int
   if (n_active == 0 || P->n_valid_points == 0 || P->n_chp == 0) return FRPA_OK;
   if (P->fast && !force_generic) {
     FRPA_TRY(launch_prep(*P, n_active, lhmfd, mrs, opr, Q, stream));
-    return launch_fast(*P, n_active, spline, dv, codes, stream);
+    if (codes) return launch_fast<true>(*P, n_active, spline, dv, codes, stream);
+    return launch_fast<false>(*P, n_active, spline, dv, nullptr, stream);
   }
   sumup_multipole_c_kernel<<<dim3(P->n_atoms, n_active), 128, 0, stream>>>(
       P->n_atoms, P->L, P->L2, P->mc_dim, P->icc_dim0, P->lma, P->d_icc, P->d_ncc, P->d_cc, lhmfd, Q, P->d_mc,

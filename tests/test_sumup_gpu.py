@@ -218,3 +218,49 @@ def test_sumup_dense_points_match_oracle(atoms, points, T, L, outer):
     assert delta_rel(out, ref, p.delta_v_hartree) < TOL
     untouched = np.setdiff1d(np.arange(p.n_full_points), p.i_valid_point_2_i_full_points_map)
     assert np.array_equal(out[untouched], p.delta_v_hartree[untouched])
+
+
+@pytest.mark.parametrize("atoms,points,T,L", [
+    (9, 1000, 2, 8),       # one point per thread, records over 4 warps; centres shared by 8 near-field warps
+    (20, 20_000, 4, 6),    # two points per thread
+    (16, 40_001, 4, 5),    # four points per thread, records over 4 warps
+    (40, 160_000, 1, 5),   # four points per thread
+    (3, 7000, 1, 3),       # near field inline, one point per thread
+    (3, 152_001, 2, 2),    # near field inline, two points per thread
+])
+def test_sumup_branch_codes_are_those_of_the_plain_call(atoms, points, T, L):
+    """The codes are written by the launches of a call without codes (same bits of
+    delta_v) and equal the table loop's decisions, with points exactly at a near
+    radius, at an outer radius of every l and at the end of the far field, and the
+    next representable distances on both sides."""
+    p = synth.make_sumup_problem(n_atoms=atoms, n_points=points, l_pot_max=L, T=T, seed=140 + atoms, outer_radius=4.0,
+                                 l_hartree_per_species=[L, max(0, L - 1), L, max(0, L - 2)], extra_full_points=5)
+    rng = np.random.default_rng(atoms)
+    slot = 0
+    free = p.i_valid_point_2_i_full_points_map[rng.permutation(points)]
+
+    def at_distance(a, d):
+        """Three points on the x axis through centre a; the middle one's squared distance."""
+        nonlocal slot
+        c = p.coords_center[:, a]
+        x = c[0] + d
+        for v in (np.nextafter(x, -np.inf), x, np.nextafter(x, np.inf)):
+            p.coord_points[:, free[slot]] = (v, c[1], c[2])
+            slot += 1
+        return (x - c[0]) * (x - c[0])
+
+    for a in range(min(atoms, 6)):
+        for t in range(T):
+            p.multipole_radius_sq[a, t] = at_distance(a, rng.uniform(1.5, 2.5))
+            for l in range(1, L + 1):  # falling with l, around and outside the near sphere
+                p.outer_potential_radius[l, a, t] = at_distance(a, 1.0 + 6.0 * (L + 1 - l) / L * rng.uniform(0.9, 1.0))
+        at_distance(a, 1e4)
+        at_distance(a, -1e4)
+    assert slot < points
+    plan = _lib.SumupPlan(p)
+    out, codes = run(plan, p, codes=True)
+    ref, rcodes = oracle.sumup(p, branch_codes=True)
+    assert np.array_equal(codes, rcodes)
+    assert np.any(rcodes == 0) and np.any((rcodes > 0) & (rcodes < 16)) and np.any(rcodes >= 16)
+    assert np.array_equal(out, run(plan, p))
+    assert delta_rel(out, ref, p.delta_v_hartree) < TOL
