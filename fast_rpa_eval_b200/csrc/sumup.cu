@@ -1108,18 +1108,21 @@ __global__ void __launch_bounds__(SU_THREADS, 2)
     dcoef_pass<L, A1, L + 1>(n_valid, pfull, pxyz, rec, gt, p_begin, p_end, red, out);
 }
 
-// dQ of one atom and perturbation: its slots' coefficient gradients (point blocks
-// in order, then slots), back through the Kelvin conversion and cc to (l, m),
+constexpr int DQ_THREADS = 256;
+static_assert(DQ_THREADS >= kelvin_count(SU_LMAX), "a thread per coefficient");
+
+// dQ of one atom and perturbation: its slots' coefficient gradients (in a fixed
+// order), back through the Kelvin conversion and cc to (l, m),
 // where the forward kept the moment (l <= l_hartree_max_far_distance,
 // |Q| > 1e-10).  A warp per (l, m), lanes over its table rows.  Perturbations
 // past n_active get zeros.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(DQ_THREADS)
     sumup_dq_kernel(int n_atoms, int L, int n_chp, int n_coef, int n_active, int nz, const int *__restrict__ slot_ptr,
                     const int *__restrict__ slots, const int *__restrict__ lm_ptr, const int *__restrict__ lm_row,
                     const int *__restrict__ convT_ptr, const int *__restrict__ convT_k,
                     const double *__restrict__ convT_f, const double *__restrict__ cc, const int *__restrict__ lhmfd,
                     const double *__restrict__ Q, const double *__restrict__ part, double *__restrict__ dQ) {
-  __shared__ double dc[(SU_LMAX + 1) * (SU_LMAX + 2) * (SU_LMAX + 3) / 6];
+  __shared__ double dc[(SU_LMAX + 1) * (SU_LMAX + 2) * (SU_LMAX + 3) / 6], part_sum[DQ_THREADS];
   const int a = blockIdx.x, t = blockIdx.y, L2 = (L + 1) * (L + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double *out = dQ + (long long)L2 * (a + (long long)n_atoms * t);
@@ -1128,14 +1131,23 @@ __global__ void __launch_bounds__(256)
     return;
   }
   const long long stride = (long long)n_coef * n_chp * n_active;
-  for (int k = threadIdx.x; k < n_coef; k += blockDim.x) {
+  // up to 16 threads per coefficient, each a range of the point blocks
+  const int shares = min(16, DQ_THREADS / n_coef), share = threadIdx.x / n_coef, k = threadIdx.x - share * n_coef;
+  if (share < shares) {
+    const int z0 = nz * share / shares, z1 = nz * (share + 1) / shares;
     double s = 0.0;
     for (int q = slot_ptr[a]; q < slot_ptr[a + 1]; ++q) {
       const double *p = part + k + (long long)n_coef * (slots[q] + (long long)n_chp * t);
 #pragma unroll 8
-      for (int z = 0; z < nz; ++z) s += p[stride * z];
+      for (int z = z0; z < z1; ++z) s += p[stride * z];
     }
-    dc[k] = s;
+    part_sum[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < n_coef) {
+    double s = part_sum[threadIdx.x];
+    for (int i = 1; i < shares; ++i) s += part_sum[threadIdx.x + i * n_coef];
+    dc[threadIdx.x] = s;
   }
   __syncthreads();
   const int lh = min(max(lhmfd[a + n_atoms * t], 0), L);
@@ -1172,7 +1184,7 @@ int launch_dq(const SumupPlan &P, int n_active, const int *lhmfd, const double *
       return fail(FRPA_ERR_UNSUPPORTED, "sum-up adjoint: l_pot_max %d above %d", P.L, SU_LMAX);
   }
   FRPA_LAUNCH_CHECK();
-  sumup_dq_kernel<<<dim3(P.n_atoms, P.T), 256, 0, stream>>>(
+  sumup_dq_kernel<<<dim3(P.n_atoms, P.T), DQ_THREADS, 0, stream>>>(
       P.n_atoms, P.L, P.n_chp, P.n_coef, n_active, P.adj_nz, P.d_atom_slot_ptr, P.d_atom_slots, P.d_lm_ptr, P.d_lm_row,
       P.d_convT_ptr, P.d_convT_k, P.d_convT_f, P.d_cc, lhmfd, Q, P.d_dcoef_part, dQ);
   FRPA_LAUNCH_CHECK();
@@ -1446,11 +1458,14 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
   UP(d_convT_k, convT_k.data(), sizeof(int) * convT_k.size());
   UP(d_convT_f, convT_f.data(), sizeof(double) * convT_f.size());
   // adjoint: point blocks of 512 to 4096 points (more past 262,144 points, at most
-  // 64 blocks there), as small as still gives about 2,400 blocks; partials added in order
+  // 64 blocks there), as small as still gives about 2,400 blocks, but no more per
+  // centre than the chip takes at once (296: with few centres the last kernel's sum
+  // over a thousand of them took longer than the points); partials added in order
   {
     const long long pairs = (long long)P->n_valid_points * P->n_chp * T;
     const long long most = std::max(4096, ceil_div(P->n_valid_points, 64));
-    P->adj_pts = (int)((std::min(most, std::max(512LL, pairs / 2400)) + 127) / 128 * 128);
+    const long long least = std::max(512, ceil_div(P->n_valid_points, 296));
+    P->adj_pts = (int)((std::min(most, std::max(least, pairs / 2400)) + 127) / 128 * 128);
     P->adj_nz = std::max(1, ceil_div(P->n_valid_points, P->adj_pts));
   }
   std::vector<int> cnt(P->n_atoms + 1, 0), slots(std::max(1, P->n_chp));

@@ -166,3 +166,28 @@ def test_dQ_equals_unit_moment_potentials(L, T, points):
         v = oracle.sumup(p)
         # 1,300 terms of at most |g| |v| each, one rounding per operation
         assert abs(got[lm, a, t] - np.sum(g[:, t] * v[:, t])) < 1e-12 * scale
+
+
+@pytest.mark.parametrize("atoms,points,L", [(1, 200_000, 0), (1, 200_000, 2), (2, 70_001, 5), (1, 30_000, 8)])
+def test_dQ_few_centres_many_points(atoms, points, L):
+    """Few centres: many point blocks per centre, their partial sums shared out
+    over up to 16 threads a coefficient (one at l_max 8).  At most about 100
+    additions follow one another, so 1e-13 of the sum of the terms' magnitudes
+    leaves a factor of five over their rounding."""
+    p = synth.make_sumup_problem(n_atoms=atoms, n_points=points, l_pot_max=L, T=1, seed=70 + L, outer_radius=5.0)
+    g = np.random.default_rng(L).normal(size=(p.n_full_points, 1))
+    plan = _lib.SumupPlan(p)
+    dQ = torch.empty(p.multipole_moments.size, dtype=torch.float64, device="cuda")
+    p.multipole_moments[:] = np.where(np.abs(p.multipole_moments) > 1e-10, p.multipole_moments, 0.5)
+    plan.adjoint_q(1, dev(p.l_hartree_max_far_distance, np.int32), dev(p.multipole_radius_sq),
+                   dev(p.outer_potential_radius), dev(p.multipole_moments), dev(g), dQ)
+    torch.cuda.synchronize()
+    got = host(dQ, p.multipole_moments.shape)
+    p.spline[:] = 0.0  # the far field only
+    p.delta_v_hartree[:] = 0.0
+    for lm in sorted({0, (L + 1) ** 2 // 2, (L + 1) ** 2 - 1}):
+        for a in range(atoms):
+            p.multipole_moments[:] = 0.0
+            p.multipole_moments[lm, a, 0] = 1.0
+            terms = g[:, 0] * oracle.sumup(p, n_threads=8)[:, 0]
+            assert abs(got[lm, a, 0] - np.sum(terms)) < 1e-13 * np.sum(np.abs(terms))
