@@ -32,9 +32,10 @@ TUNE_FP64_CTAS_PER_SM = 2
 TUNE_SPLIT_TILE_POINTS = 3
 TUNE_ORDER = 4
 TUNE_SPLIT_I8_SCRATCH_MB = 5
+TUNE_FP64_SMALL = 6
 TUNINGS = {"fp64_tile_points": TUNE_FP64_TILE_POINTS, "fp64_ctas_per_sm": TUNE_FP64_CTAS_PER_SM,
            "split_tile_points": TUNE_SPLIT_TILE_POINTS, "order": TUNE_ORDER,
-           "split_i8_scratch_mb": TUNE_SPLIT_I8_SCRATCH_MB}
+           "split_i8_scratch_mb": TUNE_SPLIT_I8_SCRATCH_MB, "fp64_small": TUNE_FP64_SMALL}
 
 c_int = ctypes.c_int
 c_ll = ctypes.c_longlong
@@ -244,7 +245,9 @@ class Rho1Plan:
         """fp64_tile_points (64 | 128), fp64_ctas_per_sm (0..3),
         split_tile_points (16..128), order (0 largest first | 1 batch order |
         2 locality order, the default),
-        split_i8_scratch_mb (>= 1: packed-operand scratch per group of batches)."""
+        split_i8_scratch_mb (>= 1: packed-operand scratch per group of batches),
+        fp64_small (0 by estimated time, the default | 1 never | 2 always: the
+        kernel for plans of batches with at most 120 functions)."""
         for k, v in kw.items():
             check(lib().frpa_rho1_plan_set_tuning(self.handle, c_int(TUNINGS[k]), c_int(int(v))))
 

@@ -43,6 +43,18 @@ def space(mode: int) -> list[dict]:
     return FP64_SPACE if mode == _lib.RHO1_FP64 else SPLIT_SPACE
 
 
+SMALL_MAX_COMPUTE = 120  # most functions per batch of the FP64 kernel for small batches
+
+
+def candidates(prob, mode: int) -> list[dict]:
+    """The candidates that are different launches for this problem: plans of small
+    batches also have a kernel of their own, whose list the FP64 keys do not change."""
+    out = space(mode)
+    if mode == _lib.RHO1_FP64 and np.max(prob.n_compute_c_batches, initial=0) <= SMALL_MAX_COMPUTE:
+        out = [{"fp64_small": 2}] + [dict(c, fp64_small=1) for c in out]
+    return out
+
+
 def geometry_key(prob, mode: int, device_name: str = "") -> str:
     """Cache key: GPU name, mode, T and the batch shapes (n_compute, points)."""
     h = hashlib.sha1()
@@ -66,7 +78,7 @@ def _time_ms(run, reps: int) -> float:
 
 
 def tune_rho1(plan, prob, run, mode: int, reps: int = 2, cache_path: str | None = None) -> dict:
-    """Times ``run`` under each candidate of ``space(mode)``, leaves the fastest
+    """Times ``run`` under each of ``candidates(prob, mode)``, leaves the fastest
     applied to ``plan`` and returns {"choice", "ms", "timings", "cached"}."""
     import torch
 
@@ -81,7 +93,7 @@ def tune_rho1(plan, prob, run, mode: int, reps: int = 2, cache_path: str | None 
         plan.set_tuning(**cache[key]["choice"])
         return dict(cache[key], cached=True)
     timings = []
-    for cand in space(mode):
+    for cand in candidates(prob, mode):
         plan.set_tuning(**cand)
         timings.append((_time_ms(run, reps), cand))
     ms, best = min(timings, key=lambda x: x[0])

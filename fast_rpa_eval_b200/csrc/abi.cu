@@ -76,6 +76,11 @@ unsigned plan_use(int mode) {
   return PLAN_RHO1 | (mode == FRPA_RHO1_SPLIT_BF16 ? PLAN_SPLIT : mode == FRPA_RHO1_SPLIT_I8 ? PLAN_I8 : 0);
 }
 
+static int device_sms(int device) {
+  int n = 0;
+  return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+}
+
 static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D, unsigned use = PLAN_ALL) {
   *out = nullptr;
   FRPA_CHECK_ARG(D != nullptr, "rho1: null descriptor");
@@ -159,7 +164,7 @@ static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D, unsigned use
   P->h_batches = batches;
   P->h_ib = ibc;
   if (nc_max <= SMALL_MAX_NC && !items.empty()) {
-    rho1_small_build_items(batches, P->order, &small);
+    rho1_small_build_items(batches, T, device_sms(P->device), P->order, P->fp64_small, &small);
     P->n_items_small = (int)small.size();
     mem.array((void **)&P->d_items_small, small.data(), sizeof(Rho1WorkItem) * small.size());
     st = rho1_small_configure(P->device);
@@ -529,6 +534,10 @@ int frpa_rho1_plan_set_tuning(frpa_rho1_plan *plan, int key, int value) {
       FRPA_CHECK_ARG(value >= 0 && value <= 2, "rho1 tuning: order %d not 0, 1 or 2", value);
       P.order = value;
       break;
+    case FRPA_TUNE_FP64_SMALL:
+      FRPA_CHECK_ARG(value >= 0 && value <= 2, "rho1 tuning: kernel for small batches %d not 0, 1 or 2", value);
+      P.fp64_small = value;
+      break;
     case FRPA_TUNE_SPLIT_I8_SCRATCH_MB:
       FRPA_CHECK_ARG(value >= 1, "rho1 tuning: split-int8 scratch %d MiB not >= 1", value);
       P.i8_budget = (long long)value << 20;
@@ -542,8 +551,8 @@ int frpa_rho1_plan_set_tuning(frpa_rho1_plan *plan, int key, int value) {
                         &P.fp64_chunk_batches);
   rho1_split_build_items(P.h_batches, P.split_tile_points, P.order, &split);
   FRPA_TRY(replace_items(P, &P.d_items, &P.n_items, items));
-  if (P.n_items_small > 0) {
-    rho1_small_build_items(P.h_batches, P.order, &items);
+  if (P.n_max_compute <= SMALL_MAX_NC && P.n_items > 0) {
+    rho1_small_build_items(P.h_batches, P.T, device_sms(P.device), P.order, P.fp64_small, &items);
     FRPA_TRY(replace_items(P, &P.d_items_small, &P.n_items_small, items));
   }
   FRPA_TRY(replace_items(P, &P.d_items_split, &P.n_items_split, split));
@@ -558,6 +567,7 @@ int frpa_rho1_plan_get_tuning(const frpa_rho1_plan *plan, int key, int *value) {
     case FRPA_TUNE_FP64_CTAS_PER_SM: *value = P.fp64_ctas_per_sm; return FRPA_OK;
     case FRPA_TUNE_SPLIT_TILE_POINTS: *value = P.split_tile_points; return FRPA_OK;
     case FRPA_TUNE_ORDER: *value = P.order; return FRPA_OK;
+    case FRPA_TUNE_FP64_SMALL: *value = P.fp64_small; return FRPA_OK;
     case FRPA_TUNE_SPLIT_I8_SCRATCH_MB: *value = (int)(P.i8_budget >> 20); return FRPA_OK;
     default: return fail(FRPA_ERR_INVALID, "rho1 tuning: unknown key %d", key);
   }

@@ -234,7 +234,7 @@ struct Rho1Plan {
   int *d_counter = nullptr;   // persistent scheduler cursor
   int grid_fp64 = 0;
   // plans whose batches have at most SMALL_MAX_NC functions: the list of
-  // rho1_fp64_small.cu (empty otherwise)
+  // rho1_fp64_small.cu (empty otherwise, and where the general kernel is taken)
   Rho1WorkItem *d_items_small = nullptr;
   int n_items_small = 0;
   // adjoint and first-order H: work list in groups (first_order_h.cu), built
@@ -255,6 +255,7 @@ struct Rho1Plan {
   int fp64_tile_points = 64;   // 64 or 128 points per FP64 work item
   int fp64_ctas_per_sm = 0;    // 0: as many as fit
   int split_tile_points = 128; // <= 128 points per split-BF16 work item
+  int fp64_small = 0;          // kernel for small batches: 0 by estimated time, 1 never, 2 always
   int order = 2;               // 0: largest items first, 1: batch order, 2: locality key
   // the FP64 work list in FP64_CHUNKS pieces of consecutive batches (6%, 44%,
   // 44%, 6% of the cost): chunk c holds items [fp64_chunk_items[c], fp64_chunk_items[c + 1])
@@ -301,7 +302,8 @@ int rho1_fp64_launch_chunk(const Rho1Plan &plan, int chunk, int n_active, const 
                            cudaStream_t stream);
 int rho1_fp64_grid(int device);
 constexpr int SMALL_MAX_NC = 120;  // P1c, two phi tiles and a work1 tile fit one SM's shared memory
-void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int order, std::vector<Rho1WorkItem> *out);
+void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int n_sm, int order, int use,
+                            std::vector<Rho1WorkItem> *out);
 int rho1_small_configure(int device);
 int rho1_small_launch(const Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *P1,
                       const double *bias, const double *gbias, double *rho, double *grad, cudaStream_t stream);

@@ -1,7 +1,8 @@
 // Plain FP64 first-order density (rho1) and its gradient for plans whose batches
-// all have at most SMALL_MAX_NC compute functions and 16-byte aligned phi rows
-// (rho1_fp64.cu has the semantics and the kernel for everything else; the sums are
-// formed in the same order, so both give the same bits).
+// all have at most SMALL_MAX_NC compute functions and 16-byte aligned phi rows, where
+// that is the faster way (rho1_small_build_items; rho1_fp64.cu has the semantics and
+// the kernel for everything else; the sums are formed in the same order, so both give
+// the same bits).
 //
 // Such batches are short: the general kernel takes a handful of 32-wide K chunks
 // per row tile, each a memory latency behind a barrier, gathers P1c once per 64
@@ -244,52 +245,103 @@ __global__ void __launch_bounds__(THREADS, 1) rho1_small_kernel(const SmallParam
 
 constexpr int STEP = GROUPS * PTS;  // points of a pass of both groups
 
-// Measured times of an item's parts, in microseconds: its start with the P1c
-// gather, and a pass of both groups (the MMA part is nc^2 x 32 points at one SM's
-// 250 GFLOP/s of FP64 MMAs).
-static double item_time(int nc, int passes) { return 3.5 + passes * (1.5 + 2.6e-4 * nc * nc); }
+namespace {
 
-// Work items: whole batches where those are many; otherwise every batch in equal
-// parts of at most a time limit, the limit that makes the launch shortest (with no
-// more items than SMs the longest item, else the mean load of an SM and half the
-// longest item), taken largest first.
-void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int order, std::vector<Rho1WorkItem> *out) {
-  constexpr int SMS = 148;
-  auto parts_of = [](const Rho1WorkItem &b, double limit) {
-    const int steps = ceil_div(b.np, STEP);
-    int parts = 1;
-    while (parts < steps && item_time(b.nc, ceil_div(steps, parts)) > limit) ++parts;
-    return parts;
-  };
-  double limit = 1e30;
-  const bool few = batches.size() <= 4 * SMS;
-  if (few) {
-    double best = 1e30;
-    for (double l = 5.0; l < 300.0; l *= 1.4) {
-      double sum = 0.0, longest = 0.0;
-      int n = 0;
-      bool cut = false;
-      for (const Rho1WorkItem &b : batches) {
-        if (b.np == 0) continue;
-        const int parts = parts_of(b, l);
-        cut = cut || parts > 1;
-        const double t = item_time(b.nc, ceil_div(ceil_div(b.np, STEP), parts));
-        sum += parts * t;
-        longest = std::max(longest, t);
-        n += parts;
-      }
-      const double launch = n <= SMS ? longest : sum / SMS + 0.5 * longest;
-      if (launch < best) {
-        best = launch;
-        limit = l;
-      }
-      if (!cut) break;
-    }
+// The time of a persistent launch over items on `slots` SMs (or halves of one): with
+// no more items than slots the longest, else the mean load of a slot and part of the
+// longest item at the end.
+struct LaunchTime {
+  double sum = 0.0, longest = 0.0;
+  long long n = 0;
+  void add(long long count, double item) {
+    n += count;
+    sum += count * item;
+    longest = std::max(longest, item);
   }
+  double total(int slots, double tail) const {
+    return n <= slots ? longest : std::max(longest, sum / slots + tail * longest);
+  }
+};
+
+// Times in microseconds of an item's parts, fitted to both kernels' launches on 270
+// plans (4 to 6,000 batches of 1 to 120 functions and 4 to 1,000 points, some with one
+// batch of 2,000 or 20,000, one to four perturbations; rms error 9% each).  `cold` is
+// 1 where the arrays are much larger than L2 and goes to 0 with their size.
+//
+// This kernel: the item's start, and per perturbation the P1c gather and `steps`
+// passes of both groups (a batch of at most 16 points is one pass of one group).
+double item_time(int nc, int np, int T, int steps, double cold) {
+  const double nc2 = (double)nc * nc, pass = (1.27 * (1.0 + 0.35 * cold) + 4.3e-4 * nc2) * (np <= PTS ? 0.56 : 1.0);
+  return 0.96 + T * (0.69 + 2.0e-4 * nc2 + steps * pass);
+}
+// The general kernel: an item of at most 64 points, two CTAs per SM.
+double general_item_time(int nc, double points, int T, double cold) {
+  const int row_tiles = ceil_div(nc, 64);
+  return 0.1 + row_tiles * (4.9 * cold * (1.0 + 0.31 * (T - 1)) +
+                            T * (3.04 + 0.614 * (nc / 32.0 + 0.4) + 0.003 * points)) +
+         T * 1.13e-5 * points * nc * nc;
+}
+// The fewest parts whose time is at most `limit`.
+int parts_of(const Rho1WorkItem &b, int T, double cold, double limit) {
+  const int steps = ceil_div(b.np, STEP);
+  const double start = item_time(b.nc, b.np, T, 0, cold), step = item_time(b.nc, b.np, T, 1, cold) - start;
+  const int most = std::max(1, (int)std::min(1e9, (limit - start) / step));
+  return ceil_div(steps, std::min(steps, most));
+}
+
+}  // namespace
+
+// Work items: every batch in equal parts of at most a time limit, the limit that makes
+// the launch shortest (none, where the batches are many and alike).  Few items are
+// taken largest first.
+// use 0: no items, so that the general kernel is taken, where that one's launch is
+// shorter; 1: none; 2: always.  Which one is depends on how often P1c is gathered (per
+// item here, per 64 points there) and on what covers a gather (nothing here, the SM's
+// other CTA there).  Measured, us, general kernel / this one: 64 batches of 40-120
+// functions, 100-200 points 22 / 13 (148: 35 / 35 of 20-120; 2,000: 403 / 364);
+// 2,000 batches of 110-120 functions, 60-64 points 256 / 304, 8-16 points 159 / 142;
+// 600 batches of 16-24 functions, 250-400 points, four perturbations 309 / 385.  On the
+// 270 plans the choice costs 0.3% of the better kernel's time in the mean, 14% at most.
+void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int n_sm, int order, int use,
+                            std::vector<Rho1WorkItem> *out) {
   out->clear();
+  if (use == 1) return;
+  double bytes = 0.0;  // phi and grad phi, biases and grad rho1
+  int np_max = 0;
+  for (const Rho1WorkItem &b : batches) {
+    bytes += 32.0 * ((b.nc + 3) & ~3) * b.np;
+    np_max = std::max(np_max, b.np);
+  }
+  bytes += 64.0 * T * np_max * batches.size();
+  const double cold = std::min(1.0, bytes / 1e8);
+  double limit = 1e30, best = 1e30;
+  for (double l = 5.0; l < 1e9; l *= 1.4) {
+    LaunchTime launch;
+    bool cut = false;
+    for (const Rho1WorkItem &b : batches) {
+      if (b.np == 0) continue;
+      const int parts = parts_of(b, T, cold, l);
+      cut = cut || parts > 1;
+      launch.add(parts, item_time(b.nc, b.np, T, ceil_div(ceil_div(b.np, STEP), parts), cold));
+    }
+    const double t = 2.6 + launch.total(n_sm, 0.45);
+    if (t < best) {
+      best = t;
+      limit = l;
+    }
+    if (!cut) break;
+  }
+  if (use == 0) {
+    LaunchTime general;
+    for (const Rho1WorkItem &b : batches) {
+      const int tiles = ceil_div(b.np, 64);
+      if (tiles > 0) general.add(tiles, general_item_time(b.nc, (double)b.np / tiles, T, cold));
+    }
+    if (best > 1.03 * (4.1 + general.total(2 * n_sm, 0.67))) return;
+  }
   for (const Rho1WorkItem &b : batches) {
     if (b.np == 0) continue;
-    const int steps = ceil_div(b.np, STEP), parts = parts_of(b, limit);
+    const int steps = ceil_div(b.np, STEP), parts = parts_of(b, T, cold, limit);
     for (int k = 0, p0 = 0; k < parts; ++k) {  // the 32-point steps dealt out evenly
       const int w = STEP * (steps / parts + (k < steps % parts ? 1 : 0));
       out->push_back(Rho1WorkItem{b.batch, b.nc, b.np, p0, std::min(w, b.np - p0), b.ib_off, b.prefix, b.key,
@@ -297,7 +349,7 @@ void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int order,
       p0 += w;
     }
   }
-  rho1_order_items(out, few ? 0 : order);
+  rho1_order_items(out, (long long)out->size() <= 4LL * n_sm ? 0 : order);
 }
 
 // Shared-memory attribute of the kernel, once per device (outside any capture).

@@ -330,9 +330,20 @@ int frpa_rho1_bias_part2(const frpa_rho1_plan *plan, int T, int n_atoms, int j_a
  *   FRPA_TUNE_FP64_TILE_POINTS  64 (256 threads, up to 2 CTAs per SM) or 128
  *                               (512 threads, 1 CTA per SM: each gathered P1c
  *                               tile serves twice the points);
- *   FRPA_TUNE_FP64_CTAS_PER_SM  0 (as many as fit), 1, 2 or 3 (neither FP64 key
- *                               concerns plans of batches with at most 120
- *                               functions, which have their own kernel);
+ *   FRPA_TUNE_FP64_CTAS_PER_SM  0 (as many as fit), 1, 2 or 3;
+ *   FRPA_TUNE_FP64_SMALL        which kernel frpa_rho1_execute takes in the FP64
+ *                               mode for plans whose batches all have at most 120
+ *                               functions: 0 (the default) the one with the
+ *                               shorter estimated time, 1 the general kernel, 2
+ *                               the one for small batches (phi rows or arrays off
+ *                               16-byte boundaries always take the general one, as
+ *                               do the fused-bias and chunked host-buffer calls).
+ *                               The kernel for small batches cuts its own work
+ *                               items: the two FP64 keys above do not concern it
+ *                               (they do the general kernel and, the first, the
+ *                               bias producer's items), and FRPA_TUNE_ORDER only
+ *                               where it has more than four items per SM (fewer
+ *                               are always taken largest first);
  *   FRPA_TUNE_SPLIT_TILE_POINTS 16..128 points per split-BF16 work item;
  *   FRPA_TUNE_ORDER             0 largest items first, 1 batch order, 2 (the
  *                               default) batches grouped by a MinHash of their
@@ -350,7 +361,8 @@ enum {
   FRPA_TUNE_FP64_CTAS_PER_SM = 2,
   FRPA_TUNE_SPLIT_TILE_POINTS = 3,
   FRPA_TUNE_ORDER = 4,
-  FRPA_TUNE_SPLIT_I8_SCRATCH_MB = 5
+  FRPA_TUNE_SPLIT_I8_SCRATCH_MB = 5,
+  FRPA_TUNE_FP64_SMALL = 6
 };
 int frpa_rho1_plan_set_tuning(frpa_rho1_plan *plan, int key, int value);
 int frpa_rho1_plan_get_tuning(const frpa_rho1_plan *plan, int key, int *value);

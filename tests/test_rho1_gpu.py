@@ -214,3 +214,29 @@ def test_rho1_small_calls_in_a_row_equal_calls_one_by_one(captured):
         queue()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for r, o in zip(ref, out) for a, b in zip(r, o))
+
+
+@pytest.mark.parametrize("nc_range,np_range,n_batches,T,n_active,log", [
+    ((1, 3), (1, 9), 5, 1, 1, False),          # one row block, part of a pass
+    ((15, 18), (31, 34), 7, 2, 1, False),      # either side of two row blocks and of a 32-point pass
+    ((63, 66), (60, 98), 6, 3, 3, False),      # one and two row tiles, items of several passes
+    ((119, 120), (60, 64), 200, 2, 2, False),  # the largest this kernel takes, more items than SMs
+    ((20, 60), (2, 2000), 600, 1, 1, True),  # more than four rounds of SMs, the long batches in many parts
+])
+def test_rho1_both_kernels_for_small_batches_same_bits(nc_range, np_range, n_batches, T, n_active, log):
+    """Both kernels on the same arrays, whichever the estimated times would choose."""
+    p = synth.make_rho1_problem(T=T, seed=170 + nc_range[1], n_atoms=10, n_batches=n_batches, np_range=np_range,
+                                nc_range=nc_range, log_uniform=log, with_bias=True, extra_full_points=13,
+                                empty_batches=2, pad_value=np.nan, n_active=n_active)
+    plan = _lib.Rho1Plan(p)
+    out = []
+    for use in (1, 2, 0):
+        plan.set_tuning(fp64_small=use)
+        assert plan.tuning()["fp64_small"] == use
+        out.append(rho1_device_run(plan, p))
+    r_o, g_o = oracle.rho1(p, n_threads=8)
+    assert normwise_rel(out[0][0], r_o) < TOL_FP64 and normwise_rel(out[0][1], g_o) < TOL_FP64
+    for r, g in out[1:]:
+        assert np.array_equal(r, out[0][0]) and np.array_equal(g, out[0][1])
+    with pytest.raises(_lib.FrpaError):
+        plan.set_tuning(fp64_small=3)
