@@ -33,9 +33,11 @@ TUNE_SPLIT_TILE_POINTS = 3
 TUNE_ORDER = 4
 TUNE_SPLIT_I8_SCRATCH_MB = 5
 TUNE_FP64_SMALL = 6
+TUNE_H1_SCRATCH_MB = 7
 TUNINGS = {"fp64_tile_points": TUNE_FP64_TILE_POINTS, "fp64_ctas_per_sm": TUNE_FP64_CTAS_PER_SM,
            "split_tile_points": TUNE_SPLIT_TILE_POINTS, "order": TUNE_ORDER,
-           "split_i8_scratch_mb": TUNE_SPLIT_I8_SCRATCH_MB, "fp64_small": TUNE_FP64_SMALL}
+           "split_i8_scratch_mb": TUNE_SPLIT_I8_SCRATCH_MB, "fp64_small": TUNE_FP64_SMALL,
+           "h1_scratch_mb": TUNE_H1_SCRATCH_MB}
 
 c_int = ctypes.c_int
 c_ll = ctypes.c_longlong
@@ -247,7 +249,8 @@ class Rho1Plan:
         2 locality order, the default),
         split_i8_scratch_mb (>= 1: packed-operand scratch per group of batches),
         fp64_small (0 by estimated time, the default | 1 never | 2 always: the
-        kernel for plans of batches with at most 120 functions)."""
+        kernel for plans of batches with at most 120 functions),
+        h1_scratch_mb (>= 1: first-order H / adjoint scratch per group of batches)."""
         for k, v in kw.items():
             check(lib().frpa_rho1_plan_set_tuning(self.handle, c_int(TUNINGS[k]), c_int(int(v))))
 

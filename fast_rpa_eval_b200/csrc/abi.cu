@@ -62,7 +62,8 @@ int synth_basis_values(const frpa_rho1_desc *D, const double *points, int n_atom
 
 static void rho1_plan_free(Rho1Plan *P) {
   if (!P) return;
-  for (void *p : {(void *)P->d_items, (void *)P->d_items_small, (void *)P->d_items_split}) P->release(p);
+  for (void *p : {(void *)P->d_items, (void *)P->d_items_small, (void *)P->d_items_split, P->d_h1_items, P->d_h1_tiles})
+    P->release(p);
   cudaFree(P->d_h1_acc);
   cudaFree(P->arena);
   rho1_i8_free(P);
@@ -175,7 +176,7 @@ static int rho1_plan_build(Rho1Plan **out, const frpa_rho1_desc *D, unsigned use
     mem.array((void **)&P->d_items_split, split.data(), sizeof(Rho1WorkItem) * split.size());
   }
   if (use & PLAN_H1) {
-    rho1_h1_build_items(batches, &h1_items, &h1_tiles, &P->h1_groups, &P->h1_a_len);
+    rho1_h1_build_items(batches, P->h1_budget, &h1_items, &h1_tiles, &P->h1_groups, &P->h1_a_len);
     mem.array(&P->d_h1_items, h1_items.data(), h1_items.size());
     mem.array(&P->d_h1_tiles, h1_tiles.data(), h1_tiles.size());
   }
@@ -538,6 +539,11 @@ int frpa_rho1_plan_set_tuning(frpa_rho1_plan *plan, int key, int value) {
       FRPA_CHECK_ARG(value >= 0 && value <= 2, "rho1 tuning: kernel for small batches %d not 0, 1 or 2", value);
       P.fp64_small = value;
       break;
+    case FRPA_TUNE_H1_SCRATCH_MB:
+      FRPA_CHECK_ARG(value >= 1, "rho1 tuning: first-order H scratch %d MiB not >= 1", value);
+      FRPA_TRY(rho1_h1_rebuild(&P, (long long)value << 20));  // the next call allocates the scratch again
+      P.h1_budget = (long long)value << 20;
+      return FRPA_OK;
     case FRPA_TUNE_SPLIT_I8_SCRATCH_MB:
       FRPA_CHECK_ARG(value >= 1, "rho1 tuning: split-int8 scratch %d MiB not >= 1", value);
       P.i8_budget = (long long)value << 20;
@@ -568,6 +574,7 @@ int frpa_rho1_plan_get_tuning(const frpa_rho1_plan *plan, int key, int *value) {
     case FRPA_TUNE_SPLIT_TILE_POINTS: *value = P.split_tile_points; return FRPA_OK;
     case FRPA_TUNE_ORDER: *value = P.order; return FRPA_OK;
     case FRPA_TUNE_FP64_SMALL: *value = P.fp64_small; return FRPA_OK;
+    case FRPA_TUNE_H1_SCRATCH_MB: *value = (int)(P.h1_budget >> 20); return FRPA_OK;
     case FRPA_TUNE_SPLIT_I8_SCRATCH_MB: *value = (int)(P.i8_budget >> 20); return FRPA_OK;
     default: return fail(FRPA_ERR_INVALID, "rho1 tuning: unknown key %d", key);
   }

@@ -29,8 +29,9 @@
 // tiles whose widths are multiples of 8, and the 8-row blocks of a tile go round
 // the warps, so that a narrow tile loads all four tensor pipes.  The symmetric H
 // computes the tiles with j >= i only, each from both products.  Where A would
-// take more than H1_A_BYTES, the first pass only finds the bound, and groups of
-// batches that fit are then combined and multiplied in turn.  Measured, 1,600
+// take more than the plan's budget (512 MiB, less where that cannot be allocated),
+// the first pass only finds the bound, and groups of batches that fit are then
+// combined and multiplied in turn.  Measured, 1,600
 // batches of 100-200 points, n_compute 40-120, n_basis 4,000 (one B200): first-order
 // H 1.60 ms (A rebuilt in every tile from synchronous loads, 128-bit sums with a
 // carry) -> 0.59 ms; adjoint 1.21 -> 0.48 ms, of it first pass 0.16 (60% of the HBM
@@ -62,7 +63,6 @@ namespace {
 
 constexpr int TILE = 64, KC = 16, THREADS = 256;
 constexpr int LD = TILE + 4;  // [k = point][row]: stride = 4 (mod 16) doubles, conflict-free fragment loads
-constexpr long long H1_A_BYTES = 512LL << 20;  // scratch for A
 constexpr int EMAX_EMPTY = -2139062144;  // 0x80808080: no non-zero bound seen
 constexpr int H1_FLAG_NONFINITE = 16;    // device flag: a non-finite input reached the accumulation
 
@@ -521,9 +521,9 @@ __global__ void h1_finalize_kernel(long long n, ulonglong2 *__restrict__ acc_all
 
 // Groups of batches, in locality order (`key`, then cost, so that the entries
 // neighbouring batches share are added to while they are in L2), whose A fits
-// H1_A_BYTES: one item per batch (for the first pass), and per group its tiles,
-// those with j >= i first (the symmetric H takes only them).
-void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *items,
+// `budget` bytes (or one batch): one item per batch (for the first pass), and per
+// group its tiles, those with j >= i first (the symmetric H takes only them).
+void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, long long budget, std::vector<unsigned char> *items,
                          std::vector<unsigned char> *tile_list, std::vector<H1Group> *groups, long long *a_len) {
   std::vector<Rho1WorkItem> order;
   order.reserve(batches.size());
@@ -543,7 +543,7 @@ void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<u
     for (; b1 < order.size(); ++b1) {
       const Rho1WorkItem &b = order[b1];
       const long long need = (long long)((b.nc + 3) & ~3) * b.np;
-      if (b1 > b0 && (len + need) * (long long)sizeof(double) > H1_A_BYTES) break;
+      if (b1 > b0 && (len + need) * (long long)sizeof(double) > budget) break;
       const int w = (ceil_div(b.nc, ceil_div(b.nc, TILE)) + 7) / 8 * 8;
       for (int m0 = 0; m0 < b.nc; m0 += w)
         for (int n0 = 0; n0 < b.nc; n0 += w)
@@ -565,9 +565,41 @@ void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<u
   if (!tiles.empty()) memcpy(tile_list->data(), tiles.data(), tile_list->size());
 }
 
+// Groups for another budget: the scratch goes, and the lists are made and uploaded
+// again (synchronous; not inside a stream capture).
+int rho1_h1_rebuild(Rho1Plan *plan, long long budget) {
+  std::vector<unsigned char> items, tiles;
+  std::vector<H1Group> groups;
+  long long a_len = 0;
+  rho1_h1_build_items(plan->h_batches, budget, &items, &tiles, &groups, &a_len);
+  void *d_items = nullptr, *d_tiles = nullptr;
+  if (cudaMalloc(&d_items, std::max<size_t>(items.size(), 16)) != cudaSuccess ||
+      cudaMalloc(&d_tiles, std::max<size_t>(tiles.size(), 16)) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(d_items);
+    return fail(FRPA_ERR_OOM, "first-order H / adjoint: work list allocation failed");
+  }
+  if ((!items.empty() && cudaMemcpy(d_items, items.data(), items.size(), cudaMemcpyHostToDevice) != cudaSuccess) ||
+      (!tiles.empty() && cudaMemcpy(d_tiles, tiles.data(), tiles.size(), cudaMemcpyHostToDevice) != cudaSuccess)) {
+    cudaFree(d_items);
+    cudaFree(d_tiles);
+    return fail(FRPA_ERR_CUDA, "first-order H / adjoint: work list upload failed");
+  }
+  cudaFree(plan->d_h1_acc);
+  plan->d_h1_acc = nullptr;
+  plan->release(plan->d_h1_items);
+  plan->release(plan->d_h1_tiles);
+  plan->d_h1_items = d_items;
+  plan->d_h1_tiles = d_tiles;
+  plan->h1_groups = groups;
+  plan->h1_a_len = a_len;
+  return FRPA_OK;
+}
+
 // Scratch: the accumulator, two words per entry of (n_basis, n_basis, T), zero
 // between calls (the finalize pass clears what the tiles touched), the exponent
 // words, and A of one group; allocated by the first call (outside stream capture).
+// Where it does not fit, with groups of half the size, down to single batches.
 static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
   if (plan.d_h1_acc) return FRPA_OK;
   static PerDeviceOnce configured;
@@ -586,10 +618,15 @@ static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
                 "capturing a graph");
   const size_t n = (size_t)plan.n_basis * plan.n_basis * plan.T;
   const size_t words = 2 * sizeof(unsigned long long) * n, flags = (sizeof(int) * plan.T + 255) / 256 * 256;
-  const size_t bytes = words + flags + sizeof(double) * (size_t)plan.h1_a_len;
-  if (cudaMalloc((void **)&plan.d_h1_acc, bytes) != cudaSuccess) {
+  for (;;) {
+    const size_t a_bytes = sizeof(double) * (size_t)plan.h1_a_len, bytes = words + flags + a_bytes;
+    if (cudaMalloc((void **)&plan.d_h1_acc, bytes) == cudaSuccess) break;
+    cudaGetLastError();  // a refused allocation is no launch's error
     plan.d_h1_acc = nullptr;
-    return fail(FRPA_ERR_OOM, "first-order H / adjoint: %zu bytes of scratch could not be allocated", bytes);
+    const long long a_len = plan.h1_a_len;
+    if (a_bytes > 0) FRPA_TRY(rho1_h1_rebuild(&plan, (long long)a_bytes / 2));
+    if (plan.h1_a_len == a_len)
+      return fail(FRPA_ERR_OOM, "first-order H / adjoint: %zu bytes of scratch could not be allocated", bytes);
   }
   plan.h1_clean = false;
   return FRPA_OK;

@@ -241,6 +241,7 @@ struct Rho1Plan {
   // with the plan, and the scratch that the first call allocates: fixed-point
   // accumulator (zero between calls while h1_clean) and A of one group
   void *d_h1_items = nullptr, *d_h1_tiles = nullptr;
+  long long h1_budget = 512LL << 20;  // bytes of A per group
   std::vector<H1Group> h1_groups;
   long long h1_a_len = 0;
   bool h1_clean = false;
@@ -330,8 +331,9 @@ int rho1_bias_part2_launch(const Rho1Plan &plan, const int *h_atom_valid, const 
                            const double *gwave, const double *dm, double *bias, cudaStream_t stream);
 // First-order H and the rho1 adjoint (first_order_h.cu): deterministic
 // fixed-point accumulation into an (n_basis, n_basis, T) output.
-void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, std::vector<unsigned char> *items,
+void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, long long budget, std::vector<unsigned char> *items,
                          std::vector<unsigned char> *tile_list, std::vector<H1Group> *groups, long long *a_len);
+int rho1_h1_rebuild(Rho1Plan *plan, long long budget);
 int rho1_adjoint_run(Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *g_rho,
                      const double *g_grad, double *dP1, cudaStream_t stream);
 int rho1_first_order_h_run(Rho1Plan &plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,

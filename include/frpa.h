@@ -353,7 +353,10 @@ int frpa_rho1_bias_part2(const frpa_rho1_plan *plan, int T, int n_atoms, int j_a
  *                               batches in the split-int8 mode (default 4096;
  *                               the batches are packed and contracted group by
  *                               group, a batch larger than this is a group of
- *                               its own).
+ *                               its own);
+ *   FRPA_TUNE_H1_SCRATCH_MB     MiB of scratch for the points' A rows per group of
+ *                               batches in the first-order H and the adjoint
+ *                               (default 512; the next such call allocates again).
  * Results are unchanged by every setting.  Setting rebuilds and re-uploads the
  * work lists (synchronous: call it outside any stream capture). */
 enum {
@@ -362,7 +365,8 @@ enum {
   FRPA_TUNE_SPLIT_TILE_POINTS = 3,
   FRPA_TUNE_ORDER = 4,
   FRPA_TUNE_SPLIT_I8_SCRATCH_MB = 5,
-  FRPA_TUNE_FP64_SMALL = 6
+  FRPA_TUNE_FP64_SMALL = 6,
+  FRPA_TUNE_H1_SCRATCH_MB = 7
 };
 int frpa_rho1_plan_set_tuning(frpa_rho1_plan *plan, int key, int value);
 int frpa_rho1_plan_get_tuning(const frpa_rho1_plan *plan, int key, int *value);
@@ -376,12 +380,13 @@ int frpa_rho1_plan_get_tuning(const frpa_rho1_plan *plan, int key, int *value);
  * v_hartree_gradient and first_order_rho (n_full, T), v2rho2 (3, nmb, nb),
  * v2rhosigma and v2sigma2 (6, nmb, nb), partition_tab (n_full).
  * first_order_H (n_basis, n_basis, T) is accumulated into.  The per-batch
- * contributions are added as 128-bit fixed-point integers, so the result is
- * the same bits on every run whatever the order of the additions.  The
- * accumulator ((n_basis, n_basis, T) x 16 bytes) and the scratch for the
- * points' A rows (at most 512 MiB, or one batch's if that is more), both shared
- * with the adjoint, are allocated by the plan's first such call: make it before
- * any stream capture.
+ * contributions are added as 100-bit fixed-point integers in two 64-bit words,
+ * so the result is the same bits on every run whatever the order of the
+ * additions.  The accumulator ((n_basis, n_basis, T) x 16 bytes) and the scratch
+ * for the points' A rows (at most FRPA_TUNE_H1_SCRATCH_MB, or one batch's if that
+ * is more; less where that much cannot be allocated), both shared with the
+ * adjoint, are allocated by the plan's first such call: make it before any stream
+ * capture.
  * Device flags (frpa_rho1_device_flags): bit 3 an atom's compute range
  * leaves its batch (clipped), bit 4 a non-finite input (result incomplete). */
 int frpa_rho1_first_order_h(const frpa_rho1_plan *plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,

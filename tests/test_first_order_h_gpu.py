@@ -185,3 +185,86 @@ def test_adjoint_over_several_scratch_groups_equals_the_sum_of_its_parts():
     parts = run(halves[0]) + run(halves[1])
     assert float((whole - parts).abs().max()) < 1e-13 * float(parts.abs().max())
     assert float(parts.abs().max()) > 0
+
+
+def _adjoint_reference(p, gr, gg):
+    want = np.zeros((p.n_basis, p.n_basis, p.T))
+    for b in range(p.n_my_batches_work):
+        nc, npb, o = (int(v) for v in (p.n_compute_c_batches[b], p.n_point_batches[b], p.i_batch_2_wave_offset[b]))
+        ncp, pre = (nc + 3) // 4 * 4, int(p.n_point_batches_prefix_sum[b])
+        phi = p.wave[o:o + ncp * npb].reshape(npb, ncp)[:, :nc]
+        gphi = p.gradient_wave[3 * o:3 * (o + ncp * npb)].reshape(npb, 3, ncp)[:, :, :nc]
+        ib = p.i_basis_batches[:nc, b] - 1
+        for t in range(p.T):
+            a = 2.0 * np.einsum("kp,pki->pi", gg[:, :npb, b, t], gphi)
+            if t < p.j_atom_end - p.j_atom_begin + 1:
+                a += gr[p.i_valid_point_2_i_full_points_map[pre:pre + npb], t][:, None] * phi
+            want[np.ix_(ib, ib, [t])] += (a.T @ phi)[:, :, None]
+    return want
+
+
+@pytest.mark.parametrize("n_batches,np_range,nc_range,n_atoms,T,n_active", [
+    (60, (100, 200), (40, 120), 8, 2, 1),   # several batches a group, one perturbation of two active
+    (60, (100, 200), (40, 120), 8, 3, 3),
+    (5, (290, 310), (480, 500), 30, 1, 1),  # every batch a group of its own (more than 1 MiB each)
+])
+def test_scratch_groups_match_oracle_and_one_group(n_batches, np_range, nc_range, n_atoms, T, n_active):
+    """First-order H and the adjoint (g_rho and g_grad) with the points' A rows in
+    groups of 1 MiB, against the oracle and, bit for bit, against one group: the
+    scale and every contribution are the same.  At most 310 x 60 terms an entry."""
+    p = synth.make_rho1_problem(T=T, seed=300 + n_batches, n_atoms=n_atoms, box=None, density=0.037,
+                                n_batches=n_batches, np_range=np_range, nc_range=nc_range, pad_value=np.nan,
+                                with_bias=True, n_active=n_active)
+    xc = synth.first_order_h_inputs(p, seed=5, pad_value=np.nan)
+    rng = np.random.default_rng(n_batches)
+    v = np.asfortranarray(rng.normal(size=(p.n_full_points, T)))
+    gr = rng.normal(size=(p.n_full_points, T))
+    gg = rng.normal(size=(3, p.n_max_batch_size, p.n_my_batches_work, T))
+    plan = _lib.Rho1Plan(p)
+    assert plan.tuning()["h1_scratch_mb"] == 512
+    d, vd, pt, av = _device_inputs(p, xc, v)
+    w, gw, n = dev(p.wave), dev(p.gradient_wave), p.n_basis * p.n_basis * T
+    out = []
+    for mb in (512, 1, 2):
+        plan.set_tuning(h1_scratch_mb=mb)
+        H, dP1 = (torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(2))
+        for _ in range(2):  # the second call starts from the accumulator the first one left
+            plan.first_order_h(n_active, p.n_atoms, 1, 3, av, w, gw, d["hessian_wave"], d, vd, pt, H)
+            plan.adjoint_p1(n_active, w, gw, dev(gr), dev(gg), dP1)
+        out.append((H, dP1))
+    assert plan.device_flags() == 0
+    ref = oracle.first_order_h(p, v, use_reference=oracle.ref_available(T), xc=xc, j_coord=3)
+    want = _adjoint_reference(p, gr, gg)
+    assert normwise_rel(0.5 * host(out[0][0], ref.shape), ref) < TOL
+    assert normwise_rel(0.5 * host(out[0][1], want.shape), want) < TOL
+    for H, dP1 in out[1:]:
+        assert torch.equal(H, out[0][0]) and torch.equal(dP1, out[0][1])
+    with pytest.raises(_lib.FrpaError):
+        plan.set_tuning(h1_scratch_mb=0)
+
+
+def test_scratch_shrinks_where_it_cannot_be_allocated():
+    """With less free memory than one group's A rows take (170 MB), the call goes
+    through smaller groups; the accumulator alone (0.4 MB) always fits."""
+    p = synth.make_rho1_problem(T=1, seed=310, n_batches=1500, np_range=(150, 200), nc_range=(60, 100), eval_phi=False)
+    assert 8 * p.wave_len > 150 << 20
+    w = torch.empty(p.wave_len, dtype=torch.float64, device="cuda")
+    gw = torch.empty(3 * p.wave_len, dtype=torch.float64, device="cuda")
+    _lib.synth_basis_values(p, dev(np.asfortranarray(p.valid_points_xyz.T)), w, gw)
+    gr = dev(np.random.default_rng(3).normal(size=p.n_full_points))
+    out = [torch.zeros(p.n_basis * p.n_basis, dtype=torch.float64, device="cuda") for _ in range(2)]
+    plans = [_lib.Rho1Plan(p) for _ in range(2)]
+    plans[0].adjoint_p1(1, w, gw, gr, None, out[0])
+    torch.cuda.synchronize()
+    plans[0].close()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    filler = torch.empty(free - (100 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        plans[1].adjoint_p1(1, w, gw, gr, None, out[1])
+        torch.cuda.synchronize()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert plans[1].device_flags() == 0
+    assert torch.equal(out[0], out[1])
