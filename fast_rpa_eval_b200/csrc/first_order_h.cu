@@ -17,13 +17,13 @@
 // With g_rho = w v and no g_grad the adjoint is the first-order H with every
 // exchange-correlation term zero.
 //
-// Work, two passes per perturbation.  The first is bound by memory: it reads phi,
-// grad phi (and the Hessian rows of atom j) once, writes A in phi's layout to a
-// scratch array and finds the bound of the contributions that fixes the
-// accumulation's scale (below), which needs a pass over the inputs anyway.  The
-// second is one CTA per (i, j) tile of at most 64 x 64 of one batch: a plain
-// product of A and phi on the FP64 MMA (mma.sync m8n8k4, the only FP64 tensor
-// instruction of sm_100a), both streamed by asynchronous copies three or four
+// Work, two passes, over all perturbations at once where their scratch allows.  The
+// first is bound by memory: it reads phi, grad phi (and the Hessian rows of atom j)
+// once, writes A in phi's layout to a scratch array and finds the bound of the
+// contributions that fixes the accumulation's scale (below), which needs a pass over
+// the inputs anyway.  The second is one CTA per (i, j) tile of at most 64 x 64 of one
+// batch: a plain product of A and phi on the FP64 MMA (mma.sync m8n8k4, the only FP64
+// tensor instruction of sm_100a), both streamed by asynchronous copies three or four
 // stages of 16 points ahead, because batches are small (tens to some hundred
 // functions) and what counts is latency.  A batch's rows are split evenly into
 // tiles whose widths are multiples of 8, and the 8-row blocks of a tile go round
@@ -31,11 +31,11 @@
 // computes the tiles with j >= i only, each from both products.  Where A would
 // take more than the plan's budget (512 MiB, less where that cannot be allocated),
 // the first pass only finds the bound, and groups of batches that fit are then
-// combined and multiplied in turn.  Measured, 1,600
-// batches of 100-200 points, n_compute 40-120, n_basis 4,000 (one B200): first-order
-// H 1.60 ms (A rebuilt in every tile from synchronous loads, 128-bit sums with a
-// carry) -> 0.59 ms; adjoint 1.21 -> 0.48 ms, of it first pass 0.16 (60% of the HBM
-// bandwidth), tiles 0.25, last pass 0.05.
+// combined and multiplied in turn.  Measured, 1,600 batches of 100-200 points,
+// n_compute 40-120, n_basis 4,000 (one B200): first-order H 1.60 ms (A rebuilt in
+// every tile from synchronous loads, 128-bit sums with a carry) -> 0.60 ms; adjoint
+// 1.21 -> 0.43 ms, of it first pass 0.16 (60% of the HBM bandwidth), tiles 0.22,
+// last pass 0.05.
 //
 // Determinism.  Batches overlap in the output, so tiles of different batches
 // add into the same entries.  Every contribution is added as a 100-bit
@@ -94,7 +94,8 @@ struct H1Args {
   const double *g_rho, *g_grad;  // adjoint mode
   H1Inputs h;                     // first-order H mode
   ulonglong2 *acc;                // (n_basis, n_basis, T): low part, high part
-  double *A;                      // scratch: A(i, p) at a_off + p ncp + i
+  double *A;                      // scratch: A(i, p) at a_off + p ncp + i, the
+  long long a_stride;             // perturbations of one launch this far apart
   int *emax;                      // per perturbation
   int grad;       // grad phi enters A (always, except an adjoint without g_grad)
   int aligned16;  // phi, grad phi rows start on 16-byte boundaries
@@ -184,7 +185,7 @@ __device__ __forceinline__ double upper_bound(unsigned h) {
   return h == 0 ? 0.0 : (h >= 0x7ff00000u ? __hiloint2double(0x7ff00000, 0) : __hiloint2double((int)h + 1, 0));
 }
 
-// One block per batch of the list, perturbation t: A(i, p) to the scratch (WRITE)
+// One block per batch of the list, perturbation t = t0 + blockIdx.z: A(i, p) to the scratch (WRITE)
 // and, unless the scale is already known (BOUND), bound_b = sum_p max_i |A(i, p)|
 // max_j |phi_j(p)| (twice that for the symmetric H), of which the binary exponent
 // goes to an atomicMax.  The points' coefficients come first, a thread each; then
@@ -192,10 +193,11 @@ __device__ __forceinline__ double upper_bound(unsigned h) {
 // last 64 rows of a small batch).  gridDim.y blocks share a batch's points; each
 // bounds its own part and counts it gridDim.y times.
 template <bool WRITE, bool BOUND>
-__global__ void __launch_bounds__(THREADS) h1_combine_kernel(const H1Item *__restrict__ items, int t, H1Args a) {
+__global__ void __launch_bounds__(THREADS) h1_combine_kernel(const H1Item *__restrict__ items, int t0, H1Args a) {
   __shared__ double red[THREADS / 16];
   __shared__ PointCoef s_c[THREADS];
   const H1Item W = items[blockIdx.x];
+  const int t = t0 + blockIdx.z;
   const int nc = W.nc, ncp = (nc + 3) & ~3;
   const int part = (W.np + (int)gridDim.y - 1) / (int)gridDim.y;
   const int p_first = blockIdx.y * part, np = min(W.np, p_first + part);
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(THREADS) h1_combine_kernel(const H1Item *__res
       const double *phi = a.wave + W.wave_off + (long long)p * ncp;
       const double *gph = a.gwave + 3 * W.wave_off + 3LL * p * ncp;
       const double *hph = a.mode == 1 ? a.h.hessian + 6 * W.wave_off + 6LL * p * ncp : nullptr;
-      double *A = a.A + W.a_off + (long long)p * ncp;
+      double *A = a.A + a.a_stride * blockIdx.z + W.a_off + (long long)p * ncp;
       unsigned mp = 0, ma = 0;
       // two rows at a time (i even): a vector that starts below n_compute ends by ncp
 #pragma unroll 2
@@ -384,27 +386,38 @@ struct TileShape {
   static constexpr int SMEM = (int)sizeof(double) * STAGES * ARRAYS * KC * LD;
 };
 
-template <bool SYM>
+template <bool SYM, bool MANY>
 __global__ void __launch_bounds__(THREADS, TileShape<SYM>::CTAS)
-    h1_tile_kernel(const H1Item *__restrict__ items, const H1Tile *__restrict__ tiles, int n_tiles, int t, H1Args a) {
+    h1_tile_kernel(const H1Item *__restrict__ items, const H1Tile *__restrict__ tiles, int n_tiles, int t0, int n_t,
+                   H1Args a) {
   // a stage: A of the tile's i rows and phi of its j rows; if SYM, phi of the i rows and A of the j rows
   constexpr int STAGES = TileShape<SYM>::STAGES, ARRAYS = TileShape<SYM>::ARRAYS, BUF = KC * LD;
   extern __shared__ __align__(16) double smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 2, wn = warp & 3, g = lane >> 2, q = lane & 3;
-  const int emax = a.emax[t];
-  if (emax == EMAX_EMPTY) return;  // every contribution is zero
-  const FixedScale scale = make_scale(emax, a.n_batches);
-  ulonglong2 *entries = a.acc + (long long)a.n_basis * a.n_basis * t;
-
-  H1Tile tile = tiles[blockIdx.x];
-  for (int it = blockIdx.x; it < n_tiles; it += gridDim.x) {
+  // MANY: the tiles of perturbation t0, then of t0 + 1, ... (n_t of them)
+  int t = t0, emax = a.emax[t0];
+  if (!MANY && emax == EMAX_EMPTY) return;  // every contribution is zero
+  FixedScale scale = make_scale(emax, a.n_batches);
+  const int n_all = MANY ? n_tiles * n_t : n_tiles;
+  H1Tile tile = tiles[MANY ? blockIdx.x % n_tiles : blockIdx.x];
+  for (int it = blockIdx.x; it < n_all; it += gridDim.x) {
+    const int z = MANY ? it / n_tiles : 0;
     const H1Item W = items[tile.item];
     const int m0 = tile.m0, n0 = tile.n0, mw = min(W.w, W.nc - m0), nw = min(W.w, W.nc - n0);
-    if (it + (int)gridDim.x < n_tiles) tile = tiles[it + gridDim.x];
+    if (it + (int)gridDim.x < n_all) tile = tiles[MANY ? (it + gridDim.x) % n_tiles : it + gridDim.x];
+    if (MANY) {
+      if (t != t0 + z) {
+        t = t0 + z;
+        emax = a.emax[t];
+        scale = make_scale(emax, a.n_batches);
+      }
+      if (emax == EMAX_EMPTY) continue;
+    }
+    ulonglong2 *entries = a.acc + (long long)a.n_basis * a.n_basis * t;
     const int nc = W.nc, np = W.np, ncp = (nc + 3) & ~3;
     const bool diag = m0 == n0;
-    const double *phi = a.wave + W.wave_off, *amat = a.A + W.a_off;
+    const double *phi = a.wave + W.wave_off, *amat = a.A + a.a_stride * z + W.a_off;
     double acc[4][2][2];
 #pragma unroll
     for (int x = 0; x < 4; ++x)
@@ -598,16 +611,19 @@ int rho1_h1_rebuild(Rho1Plan *plan, long long budget) {
 
 // Scratch: the accumulator, two words per entry of (n_basis, n_basis, T), zero
 // between calls (the finalize pass clears what the tiles touched), the exponent
-// words, and A of one group; allocated by the first call (outside stream capture).
-// Where it does not fit, with groups of half the size, down to single batches.
+// words, and A of one group (of as many perturbations as the call takes at once);
+// allocated by the first call (outside stream capture).  Where it does not fit, with
+// fewer perturbations, then with groups of half the size, down to single batches.
 static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
   if (plan.d_h1_acc) return FRPA_OK;
   static PerDeviceOnce configured;
   FRPA_TRY(configured.run(plan.device, []() -> int {
-    FRPA_CUDA_TRY(cudaFuncSetAttribute(h1_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       TileShape<true>::SMEM));
-    FRPA_CUDA_TRY(cudaFuncSetAttribute(h1_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       TileShape<false>::SMEM));
+    for (auto kernel : {h1_tile_kernel<true, false>, h1_tile_kernel<true, true>})
+      FRPA_CUDA_TRY(
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TileShape<true>::SMEM));
+    for (auto kernel : {h1_tile_kernel<false, false>, h1_tile_kernel<false, true>})
+      FRPA_CUDA_TRY(
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TileShape<false>::SMEM));
     return FRPA_OK;
   }));
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -618,11 +634,24 @@ static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
                 "capturing a graph");
   const size_t n = (size_t)plan.n_basis * plan.n_basis * plan.T;
   const size_t words = 2 * sizeof(unsigned long long) * n, flags = (sizeof(int) * plan.T + 255) / 256 * 256;
+  // All perturbations in one launch each of the passes, while their A fits the budget:
+  // one at a time a small problem leaves most SMs idle and waits for a chain of launches
+  // per perturbation.  Measured, us, H / adjoint, four perturbations one at a time ->
+  // together: 20 batches of 20-120 functions 238 / 171 -> 75 / 61; 150: 473 / 268 ->
+  // 267 / 173; 1,600 batches of 40-120: 2,994 / 2,081 -> 2,796 / 1,990.
+  plan.h1_at_once = 1;
+  if (plan.h1_groups.size() == 1)
+    plan.h1_at_once = (int)std::max(
+        1LL, std::min<long long>(plan.T, plan.h1_budget / std::max(1LL, 8 * plan.h1_a_len)));
   for (;;) {
-    const size_t a_bytes = sizeof(double) * (size_t)plan.h1_a_len, bytes = words + flags + a_bytes;
+    const size_t a_bytes = sizeof(double) * (size_t)plan.h1_a_len, bytes = words + flags + a_bytes * plan.h1_at_once;
     if (cudaMalloc((void **)&plan.d_h1_acc, bytes) == cudaSuccess) break;
     cudaGetLastError();  // a refused allocation is no launch's error
     plan.d_h1_acc = nullptr;
+    if (plan.h1_at_once > 1) {
+      plan.h1_at_once /= 2;
+      continue;
+    }
     const long long a_len = plan.h1_a_len;
     if (a_bytes > 0) FRPA_TRY(rho1_h1_rebuild(&plan, (long long)a_bytes / 2));
     if (plan.h1_a_len == a_len)
@@ -633,10 +662,11 @@ static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
 }
 
 template <bool SYM>
-static int h1_tiles(const H1Item *items, const H1Tile *tiles, int n_tiles, int t, const H1Args &a, int n_sm,
+static int h1_tiles(const H1Item *items, const H1Tile *tiles, int n_tiles, int t, int n_t, const H1Args &a, int n_sm,
                     cudaStream_t stream) {
-  const int grid = std::min(n_tiles, n_sm * TileShape<SYM>::CTAS);
-  h1_tile_kernel<SYM><<<grid, THREADS, TileShape<SYM>::SMEM, stream>>>(items, tiles, n_tiles, t, a);
+  const int grid = (int)std::min<long long>((long long)n_tiles * n_t, n_sm * TileShape<SYM>::CTAS);
+  auto kernel = n_t > 1 ? h1_tile_kernel<SYM, true> : h1_tile_kernel<SYM, false>;
+  kernel<<<grid, THREADS, TileShape<SYM>::SMEM, stream>>>(items, tiles, n_tiles, t, n_t, a);
   FRPA_LAUNCH_CHECK();
   return FRPA_OK;
 }
@@ -670,6 +700,7 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
   if (h) a.h = *h;
   a.acc = acc;
   a.A = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(emax) + (sizeof(int) * plan.T + 255) / 256 * 256);
+  a.a_stride = plan.h1_a_len;
   a.emax = emax;
   a.err = plan.d_err;
   a.grad = mode == 1 || g_grad != nullptr;
@@ -681,7 +712,8 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
   const bool one_group = plan.h1_groups.size() == 1;
   // the adjoint's g_grad covers every perturbation, everything else the active ones
   const int n_t = mode == 0 && g_grad ? plan.T : std::max(0, n_active);
-  for (int t = 0; t < n_t; ++t) {
+  for (int t = 0, n = 1; t < n_t; t += n) {
+    n = std::min(plan.h1_at_once, n_t - t);  // more than 1 only with one group
     if (!one_group) {
       for (const H1Group &g : plan.h1_groups) {
         h1_combine_kernel<false, true><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
@@ -690,14 +722,14 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
     }
     for (const H1Group &g : plan.h1_groups) {
       if (one_group)
-        h1_combine_kernel<true, true><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
+        h1_combine_kernel<true, true><<<dim3(g.n_first, 2, n), THREADS, 0, stream>>>(items + g.first, t, a);
       else
         h1_combine_kernel<true, false><<<dim3(g.n_first, 2), THREADS, 0, stream>>>(items + g.first, t, a);
       FRPA_LAUNCH_CHECK();
       if (mode == 1)
-        FRPA_TRY(h1_tiles<true>(items, tiles + g.tiles, g.n_upper, t, a, n_sm, stream));
+        FRPA_TRY(h1_tiles<true>(items, tiles + g.tiles, g.n_upper, t, n, a, n_sm, stream));
       else
-        FRPA_TRY(h1_tiles<false>(items, tiles + g.tiles, g.n_tiles, t, a, n_sm, stream));
+        FRPA_TRY(h1_tiles<false>(items, tiles + g.tiles, g.n_tiles, t, n, a, n_sm, stream));
     }
   }
   if (n_t > 0) {

@@ -244,6 +244,7 @@ struct Rho1Plan {
   long long h1_budget = 512LL << 20;  // bytes of A per group
   std::vector<H1Group> h1_groups;
   long long h1_a_len = 0;
+  int h1_at_once = 1;  // perturbations per launch (the scratch holds A of each)
   bool h1_clean = false;
   unsigned long long *d_h1_acc = nullptr;
   // split-BF16 path: <= 128-point tiles, per-row P1 scales, device error flags
