@@ -786,6 +786,20 @@ void evaluate_first_order_h_reduce_memory_c_v2_(
   if (st == FRPA_OK) st = h2d(36, partition_tab, (size_t)nf, &pt, s);
   if (st == FRPA_OK) st = h2d(37, first_order_H_tile, nH, &H, s);
   if (st == FRPA_OK) st = h2d(38, atom_valid_n_compute_c_batches, nav, &av, s);
+  // A is kept between calls like the inputs' buffers (a tenth of theirs per
+  // perturbation, at most 512 MiB): allocated and freed with each call's plan it took
+  // 0.4 ms of 2.5.  Where it cannot be had, the plan allocates for smaller groups.
+  if (st == FRPA_OK && n_active > 0) {
+    const size_t a_bytes = rho1_h1_a_bytes(*P);
+    void *a = nullptr;
+    if (a_bytes > 0 && ensure(39, a_bytes, &a) == FRPA_OK) {
+      P->h1_a_lent = static_cast<double *>(a);
+      P->h1_a_lent_bytes = a_bytes;
+    } else if (a_bytes > 0) {
+      cudaGetLastError();
+      clear_error();
+    }
+  }
   frpa_rho1_plan handle{P};
   if (st == FRPA_OK)
     st = frpa_rho1_first_order_h(&handle, std::max(0, n_active), *n_atoms, *j_atom_begin, *j_coord, av, w, gw, hw, vs,

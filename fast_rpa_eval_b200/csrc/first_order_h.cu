@@ -609,11 +609,25 @@ int rho1_h1_rebuild(Rho1Plan *plan, long long budget) {
   return FRPA_OK;
 }
 
+// All perturbations in one launch each of the passes, while their A fits the budget:
+// one at a time a small problem leaves most SMs idle and waits for a chain of launches
+// per perturbation.  Measured, us, H / adjoint, four perturbations one at a time ->
+// together: 20 batches of 20-120 functions 238 / 171 -> 75 / 61; 150: 473 / 268 ->
+// 267 / 173; 1,600 batches of 40-120: 2,994 / 2,081 -> 2,796 / 1,990.
+size_t rho1_h1_a_bytes(Rho1Plan &plan) {
+  plan.h1_at_once = 1;
+  if (plan.h1_groups.size() == 1)
+    plan.h1_at_once = (int)std::max(
+        1LL, std::min<long long>(plan.T, plan.h1_budget / std::max(1LL, 8 * plan.h1_a_len)));
+  return sizeof(double) * (size_t)plan.h1_a_len * plan.h1_at_once;
+}
+
 // Scratch: the accumulator, two words per entry of (n_basis, n_basis, T), zero
 // between calls (the finalize pass clears what the tiles touched), the exponent
 // words, and A of one group (of as many perturbations as the call takes at once);
 // allocated by the first call (outside stream capture).  Where it does not fit, with
 // fewer perturbations, then with groups of half the size, down to single batches.
+// A caller's own buffer for A (h1_a_lent) is used where it is large enough.
 static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
   if (plan.d_h1_acc) return FRPA_OK;
   static PerDeviceOnce configured;
@@ -634,21 +648,18 @@ static int h1_scratch(Rho1Plan &plan, cudaStream_t stream) {
                 "capturing a graph");
   const size_t n = (size_t)plan.n_basis * plan.n_basis * plan.T;
   const size_t words = 2 * sizeof(unsigned long long) * n, flags = (sizeof(int) * plan.T + 255) / 256 * 256;
-  // All perturbations in one launch each of the passes, while their A fits the budget:
-  // one at a time a small problem leaves most SMs idle and waits for a chain of launches
-  // per perturbation.  Measured, us, H / adjoint, four perturbations one at a time ->
-  // together: 20 batches of 20-120 functions 238 / 171 -> 75 / 61; 150: 473 / 268 ->
-  // 267 / 173; 1,600 batches of 40-120: 2,994 / 2,081 -> 2,796 / 1,990.
-  plan.h1_at_once = 1;
-  if (plan.h1_groups.size() == 1)
-    plan.h1_at_once = (int)std::max(
-        1LL, std::min<long long>(plan.T, plan.h1_budget / std::max(1LL, 8 * plan.h1_a_len)));
+  const bool lent = plan.h1_a_lent_bytes >= rho1_h1_a_bytes(plan) && plan.h1_a_lent_bytes > 0;
   for (;;) {
-    const size_t a_bytes = sizeof(double) * (size_t)plan.h1_a_len, bytes = words + flags + a_bytes * plan.h1_at_once;
-    if (cudaMalloc((void **)&plan.d_h1_acc, bytes) == cudaSuccess) break;
+    const size_t a_bytes = lent ? 0 : sizeof(double) * (size_t)plan.h1_a_len;
+    const size_t bytes = words + flags + a_bytes * plan.h1_at_once;
+    if (cudaMalloc((void **)&plan.d_h1_acc, bytes) == cudaSuccess) {
+      unsigned char *own = reinterpret_cast<unsigned char *>(plan.d_h1_acc) + words + flags;
+      plan.h1_a = lent ? plan.h1_a_lent : reinterpret_cast<double *>(own);
+      break;
+    }
     cudaGetLastError();  // a refused allocation is no launch's error
     plan.d_h1_acc = nullptr;
-    if (plan.h1_at_once > 1) {
+    if (!lent && plan.h1_at_once > 1) {
       plan.h1_at_once /= 2;
       continue;
     }
@@ -699,7 +710,7 @@ static int h1_run(Rho1Plan &plan, int mode, int n_active, const double *wave, co
   a.g_grad = g_grad;
   if (h) a.h = *h;
   a.acc = acc;
-  a.A = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(emax) + (sizeof(int) * plan.T + 255) / 256 * 256);
+  a.A = plan.h1_a;
   a.a_stride = plan.h1_a_len;
   a.emax = emax;
   a.err = plan.d_err;

@@ -245,6 +245,9 @@ struct Rho1Plan {
   std::vector<H1Group> h1_groups;
   long long h1_a_len = 0;
   int h1_at_once = 1;  // perturbations per launch (the scratch holds A of each)
+  double *h1_a = nullptr;       // A: behind the accumulator, or a buffer lent by the caller
+  double *h1_a_lent = nullptr;  // (the host-array entry, which makes a plan per call)
+  size_t h1_a_lent_bytes = 0;
   bool h1_clean = false;
   unsigned long long *d_h1_acc = nullptr;
   // split-BF16 path: <= 128-point tiles, per-row P1 scales, device error flags
@@ -335,6 +338,7 @@ int rho1_bias_part2_launch(const Rho1Plan &plan, const int *h_atom_valid, const 
 void rho1_h1_build_items(const std::vector<Rho1WorkItem> &batches, long long budget, std::vector<unsigned char> *items,
                          std::vector<unsigned char> *tile_list, std::vector<H1Group> *groups, long long *a_len);
 int rho1_h1_rebuild(Rho1Plan *plan, long long budget);
+size_t rho1_h1_a_bytes(Rho1Plan &plan);
 int rho1_adjoint_run(Rho1Plan &plan, int n_active, const double *wave, const double *gwave, const double *g_rho,
                      const double *g_grad, double *dP1, cudaStream_t stream);
 int rho1_first_order_h_run(Rho1Plan &plan, int n_active, int n_atoms, int j_atom_begin, int j_coord,

@@ -243,6 +243,24 @@ def test_scratch_groups_match_oracle_and_one_group(n_batches, np_range, nc_range
         plan.set_tuning(h1_scratch_mb=0)
 
 
+def test_dropin_calls_of_alternating_sizes():
+    """The host-array entry keeps its device buffers, A among them, between calls:
+    smaller and larger problems in turn give the bits of their first call, and the
+    memory in use does not grow."""
+    cases = [_case(1, 171, n_batches=6), _case(3, 172, n_batches=40), _case(2, 173, n_batches=12)]
+    first, free = [], None
+    for turn in range(3):
+        for i, (p, xc, v) in enumerate(cases):
+            H = _lib.dropin_first_order_h(p, v, xc, j_coord=2)
+            if turn == 0:
+                first.append(H)
+                assert normwise_rel(H, _reference(p, v, xc, 2, 0.0)) < TOL
+            assert np.array_equal(H, first[i])
+        now = torch.cuda.mem_get_info()[0]
+        assert free is None or now == free
+        free = now if turn else None
+
+
 def test_scratch_shrinks_where_it_cannot_be_allocated():
     """With less free memory than one group's A rows take (170 MB), the call goes
     through smaller groups; the accumulator alone (0.4 MB) always fits."""
