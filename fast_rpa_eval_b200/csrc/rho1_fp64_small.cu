@@ -281,13 +281,20 @@ double general_item_time(int nc, double points, int T, double cold) {
                             T * (3.04 + 0.614 * (nc / 32.0 + 0.4) + 0.003 * points)) +
          T * 1.13e-5 * points * nc * nc;
 }
-// The fewest parts whose time is at most `limit`.
-int parts_of(const Rho1WorkItem &b, int T, double cold, double limit) {
-  const int steps = ceil_div(b.np, STEP);
-  const double start = item_time(b.nc, b.np, T, 0, cold), step = item_time(b.nc, b.np, T, 1, cold) - start;
-  const int most = std::max(1, (int)std::min(1e9, (limit - start) / step));
-  return ceil_div(steps, std::min(steps, most));
-}
+// A batch as the search for the limit sees it: time of a part = start + step x its steps.
+struct BatchTime {
+  int steps;
+  double start, step;
+  BatchTime(const Rho1WorkItem &b, int T, double cold)
+      : steps(ceil_div(b.np, STEP)),
+        start(item_time(b.nc, b.np, T, 0, cold)),
+        step(item_time(b.nc, b.np, T, 1, cold) - start) {}
+  // the fewest parts whose time is at most `limit`
+  int parts(double limit) const {
+    if (start + step * steps <= limit) return 1;
+    return ceil_div(steps, std::max(1, (int)((limit - start) / step)));
+  }
+};
 
 }  // namespace
 
@@ -314,15 +321,18 @@ void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int
   }
   bytes += 64.0 * T * np_max * batches.size();
   const double cold = std::min(1.0, bytes / 1e8);
+  std::vector<BatchTime> times;
+  times.reserve(batches.size());
+  for (const Rho1WorkItem &b : batches)
+    if (b.np > 0) times.emplace_back(b, T, cold);
   double limit = 1e30, best = 1e30;
   for (double l = 5.0; l < 1e9; l *= 1.4) {
     LaunchTime launch;
     bool cut = false;
-    for (const Rho1WorkItem &b : batches) {
-      if (b.np == 0) continue;
-      const int parts = parts_of(b, T, cold, l);
+    for (const BatchTime &b : times) {
+      const int parts = b.parts(l);
       cut = cut || parts > 1;
-      launch.add(parts, item_time(b.nc, b.np, T, ceil_div(ceil_div(b.np, STEP), parts), cold));
+      launch.add(parts, b.start + b.step * (parts == 1 ? b.steps : ceil_div(b.steps, parts)));
     }
     const double t = 2.6 + launch.total(n_sm, 0.45);
     if (t < best) {
@@ -339,9 +349,10 @@ void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int
     }
     if (best > 1.03 * (4.1 + general.total(2 * n_sm, 0.67))) return;
   }
+  size_t at = 0;
   for (const Rho1WorkItem &b : batches) {
     if (b.np == 0) continue;
-    const int steps = ceil_div(b.np, STEP), parts = parts_of(b, T, cold, limit);
+    const int steps = ceil_div(b.np, STEP), parts = times[at++].parts(limit);
     for (int k = 0, p0 = 0; k < parts; ++k) {  // the 32-point steps dealt out evenly
       const int w = STEP * (steps / parts + (k < steps % parts ? 1 : 0));
       out->push_back(Rho1WorkItem{b.batch, b.nc, b.np, p0, std::min(w, b.np - p0), b.ib_off, b.prefix, b.key,
