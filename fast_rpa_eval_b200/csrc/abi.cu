@@ -45,7 +45,7 @@ void clear_error() {
 
 // Declarations of the launchers implemented in the other translation units.
 struct SumupPlan;
-int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D);
+int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D, int (*lend)(size_t bytes, void **p) = nullptr);
 void sumup_plan_free(SumupPlan *P);
 int sumup_plan_is_fast(const SumupPlan *P);
 int sumup_execute(const SumupPlan *P, int n_active, int force_generic, const int *lhmfd, const double *mrs,
@@ -908,7 +908,9 @@ void sum_up_whole_potential_c_v3_atoms_full_points_j_atom_tile_(
   }
   if (check_lhmfd(l_hartree_max_far_distance, *n_atoms, T, *l_pot_max) != FRPA_OK) return;
   SumupPlan *P = nullptr;
-  if (sumup_plan_create(&P, &d) != FRPA_OK) return;
+  // the plan's memory is kept between calls like the other buffers: above what the
+  // driver hands out of its pools, an allocation and its release take 0.6 ms
+  if (sumup_plan_create(&P, &d, [](size_t bytes, void **p) { return ensure(40, bytes, p); }) != FRPA_OK) return;
   const int L2 = (*l_pot_max + 1) * (*l_pot_max + 1);
   const size_t na = (size_t)*n_atoms * T;
   cudaStream_t s = 0;

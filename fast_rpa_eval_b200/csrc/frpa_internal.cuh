@@ -106,7 +106,10 @@ inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b;
 // A plan's device memory, one allocation: arrays up to 256 KiB go up in one
 // copy, larger ones each from where they are (their sources have to live until
 // commit), workspaces are left as they come.  (One allocation and copy per array
-// made creating a small plan mostly driver calls.)
+// made creating a small plan mostly driver calls.  Above about 1.2 MB the driver maps
+// memory for an allocation, 0.6 ms with its release: a sum-up plan of 30 centres and
+// 20,000 points, whose arrays one by one came from its pools, takes 2.2 ms for 1.8; of
+// 64 points 0.06 for 0.29, of 50,000 points 4.8 for 5.0.)
 struct PlanMemory {
   static constexpr size_t STAGED = 256 << 10;
   struct Part {
@@ -133,9 +136,11 @@ struct PlanMemory {
     tail.push_back({dst, nullptr, tail_bytes, bytes});
     tail_bytes += padded(bytes);
   }
+  size_t total() const { return padded(host.size() + tail_bytes); }
+  // into *base, allocated here unless it is already there (with total() bytes)
   int commit(unsigned char **base, size_t *bytes) {
-    *bytes = padded(host.size() + tail_bytes);
-    if (cudaMalloc((void **)base, *bytes) != cudaSuccess) {
+    *bytes = total();
+    if (!*base && cudaMalloc((void **)base, *bytes) != cudaSuccess) {
       *base = nullptr;
       return fail(FRPA_ERR_OOM, "plan: allocation of %zu bytes failed", *bytes);
     }

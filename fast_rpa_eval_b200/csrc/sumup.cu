@@ -86,6 +86,7 @@ struct SumupPlan {
   int device = 0;
   unsigned char *arena = nullptr;  // the device allocation behind the pointers below
   size_t arena_bytes = 0;
+  bool arena_lent = false;  // the caller's
   int T = 1, L = 0, L2 = 1, lma = 0, icc_dim0 = 0, mc_dim = 0, hfla = 0;
   int n_full_points = 0, n_valid_points = 0, n_centers = 0, n_chp = 0, n_atoms = 0, n_species = 0;
   int n_hartree_grid = 0;
@@ -1237,13 +1238,14 @@ int sumup_upload_constants(int device) {
 
 void sumup_plan_free(SumupPlan *P) {
   if (!P) return;
-  cudaFree(P->arena);
+  if (!P->arena_lent) cudaFree(P->arena);
   delete P;
 }
 
 // Validates the constant inputs (every device access stays in bounds for any
 // per-call data once these hold) and uploads them.
-int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
+// lend: where given, provides the plan's memory (kept by the caller).
+int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D, int (*lend)(size_t bytes, void **p)) {
   *out = nullptr;
   FRPA_CHECK_ARG(D != nullptr, "sumup: null descriptor");
   const int L = D->l_pot_max, lma = D->l_max_analytic_multipole, T = D->atom_tile_size;
@@ -1492,6 +1494,10 @@ int sumup_plan_create(SumupPlan **out, const frpa_sumup_desc *D) {
   mem.space((void **)&P->d_recs, sizeof(double) * (size_t)P->rs * chp * T);
   mem.space((void **)&P->d_heads, sizeof(double4) * chp * T);
   mem.space((void **)&P->d_dcoef_part, sizeof(double) * (size_t)n_kelvin(L) * chp * T * P->adj_nz);
+  if (st == FRPA_OK && lend) {
+    P->arena_lent = true;
+    st = lend(mem.total(), (void **)&P->arena);
+  }
   if (st == FRPA_OK) st = mem.commit(&P->arena, &P->arena_bytes);
   if (st == FRPA_OK && P->n_valid_points > 0) {
     sumup_gather_points_kernel<<<std::min(1184, ceil_div(P->n_valid_points, 256)), 256>>>(

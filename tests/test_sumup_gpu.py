@@ -264,3 +264,24 @@ def test_sumup_branch_codes_are_those_of_the_plain_call(atoms, points, T, L):
     assert np.any(rcodes == 0) and np.any((rcodes > 0) & (rcodes < 16)) and np.any(rcodes >= 16)
     assert np.array_equal(out, run(plan, p))
     assert delta_rel(out, ref, p.delta_v_hartree) < TOL
+
+
+def test_sumup_dropin_calls_of_alternating_sizes():
+    """The host-array entry keeps its plan's memory between calls: smaller and
+    larger problems, l and tiles in turn give the bits of a plan of their own, and
+    the memory in use does not grow."""
+    cases = [synth.make_sumup_problem(n_atoms=a, n_points=n, l_pot_max=L, T=T, seed=200 + a, extra_full_points=3,
+                                      centers=c)
+             for a, n, L, T, c in ((5, 300, 4, 1, "identity"), (30, 20_000, 6, 2, "identity"), (9, 2000, 8, 1, "identity"),
+                                   (12, 900, 3, 1, "permuted"))]
+    free = None
+    for turn in range(3):
+        for p in cases:
+            out = _lib.dropin_sumup(p)
+            assert np.array_equal(out, run(_lib.SumupPlan(p), p))
+            if turn == 0:
+                assert delta_rel(out, oracle.sumup(p), p.delta_v_hartree) < TOL
+        torch.cuda.empty_cache()
+        now = torch.cuda.mem_get_info()[0]
+        assert free is None or now == free
+        free = now if turn else None
