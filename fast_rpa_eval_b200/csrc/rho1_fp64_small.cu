@@ -263,7 +263,7 @@ struct LaunchTime {
   }
 };
 
-// Times in microseconds of an item's parts, fitted to both kernels' launches on 270
+// Times in microseconds of an item's parts, fitted to both kernels' launches on 453
 // plans (4 to 6,000 batches of 1 to 120 functions and 4 to 1,000 points, some with one
 // batch of 2,000 or 20,000, one to four perturbations; rms error 9% each).  `cold` is
 // 1 where the arrays are much larger than L2 and goes to 0 with their size.
@@ -271,15 +271,15 @@ struct LaunchTime {
 // This kernel: the item's start, and per perturbation the P1c gather and `steps`
 // passes of both groups (a batch of at most 16 points is one pass of one group).
 double item_time(int nc, int np, int T, int steps, double cold) {
-  const double nc2 = (double)nc * nc, pass = (1.27 * (1.0 + 0.35 * cold) + 4.3e-4 * nc2) * (np <= PTS ? 0.56 : 1.0);
-  return 0.96 + T * (0.69 + 2.0e-4 * nc2 + steps * pass);
+  const double nc2 = (double)nc * nc, pass = (1.39 * (1.0 + 0.34 * cold) + 4.2e-4 * nc2) * (np <= PTS ? 0.58 : 1.0);
+  return 1.05 + T * (0.67 + 2.4e-4 * nc2 + steps * pass);
 }
 // The general kernel: an item of at most 64 points, two CTAs per SM.
 double general_item_time(int nc, double points, int T, double cold) {
   const int row_tiles = ceil_div(nc, 64);
-  return 0.1 + row_tiles * (4.9 * cold * (1.0 + 0.31 * (T - 1)) +
-                            T * (3.04 + 0.614 * (nc / 32.0 + 0.4) + 0.003 * points)) +
-         T * 1.13e-5 * points * nc * nc;
+  return 0.46 + row_tiles * (4.75 * cold * (1.0 + 0.37 * (T - 1)) +
+                             T * (3.04 + 0.6 * (nc / 32.0 + 0.33) + 0.0039 * points)) +
+         T * 1.17e-5 * points * nc * nc;
 }
 // A batch as the search for the limit sees it: time of a part = start + step x its steps.
 struct BatchTime {
@@ -308,7 +308,7 @@ struct BatchTime {
 // functions, 100-200 points 22 / 13 (148: 35 / 35 of 20-120; 2,000: 403 / 364);
 // 2,000 batches of 110-120 functions, 60-64 points 256 / 304, 8-16 points 159 / 142;
 // 600 batches of 16-24 functions, 250-400 points, four perturbations 309 / 385.  On the
-// 270 plans the choice costs 0.3% of the better kernel's time in the mean, 14% at most.
+// 453 plans the choice costs 0.2% of the better kernel's time in the mean, 15% at most.
 void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int n_sm, int order, int use,
                             std::vector<Rho1WorkItem> *out) {
   out->clear();
@@ -334,7 +334,7 @@ void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int
       cut = cut || parts > 1;
       launch.add(parts, b.start + b.step * (parts == 1 ? b.steps : ceil_div(b.steps, parts)));
     }
-    const double t = 2.6 + launch.total(n_sm, 0.45);
+    const double t = 2.2 + launch.total(n_sm, 0.44);
     if (t < best) {
       best = t;
       limit = l;
@@ -347,7 +347,7 @@ void rho1_small_build_items(const std::vector<Rho1WorkItem> &batches, int T, int
       const int tiles = ceil_div(b.np, 64);
       if (tiles > 0) general.add(tiles, general_item_time(b.nc, (double)b.np / tiles, T, cold));
     }
-    if (best > 1.03 * (4.1 + general.total(2 * n_sm, 0.67))) return;
+    if (best > 1.03 * (3.6 + general.total(2 * n_sm, 0.68))) return;
   }
   size_t at = 0;
   for (const Rho1WorkItem &b : batches) {
