@@ -380,7 +380,7 @@ def time_config5(K: int, W: int, ranks: Ranks, stream, fp64_peak: float, fma_pea
     out["adjoint_dP1"] = {"ms_per_call": ms, "tflops_fp64": gemm / (ms / 1e3) / 1e12,
                           "frac_of_measured_fp64_mma": gemm / (ms / 1e3) / 1e12 / fp64_peak / ranks.world,
                           "batches_per_rank": int(p.n_my_batches_work), "n_basis": int(p.n_basis),
-                          "accumulation": "128-bit fixed point, bit-identical across runs",
+                          "accumulation": "100-bit fixed point in two words, bit-identical across runs",
                           "ranks": ranks.world,
                           "collective": "NCCL all-reduce of dP1 after each call" if ranks.world > 1 else None}
     xc = {k: _dev(a) for k, a in synth.first_order_h_inputs(p, seed=6).items()}

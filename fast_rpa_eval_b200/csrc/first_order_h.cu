@@ -303,7 +303,7 @@ __host__ __device__ __forceinline__ int ceil_log2(long long n) {
 
 // The split of the fixed-point integer x = high 2^low + lowpart, |lowpart| <= 2^(low - 1):
 // the sum of 2 n_batches low parts stays below 2^62 and the sum of the high parts
-// below 2^62 (`bits` of the whole: 100 up to 2^23 batches); of a single
+// below 2^62 (`bits` of the whole: 100 up to 2^24 batches); of a single
 // contribution both parts are below 2^51.
 struct FixedPoint {
   int low, bits;

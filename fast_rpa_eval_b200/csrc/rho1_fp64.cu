@@ -573,9 +573,10 @@ int rho1_locality_key(const int *ib, int nc) {
   return (int)best;
 }
 
-// Work items of <= tile_points points (a batch's 8-point blocks split evenly), grouped into FP64_CHUNKS ranges of consecutive batches, each
-// range in the given order.  The ranges hold 6%, 44%, 44% and 6% of the cost
-// (nc^2 np): the host-buffer entry waits for the first range's biases before
+// Work items of <= tile_points points (a batch's 8-point blocks split evenly),
+// grouped into FP64_CHUNKS ranges of consecutive batches, each range in the given
+// order.  The ranges hold 6%, 44%, 44% and 6% of the cost (nc^2 np): the host-buffer
+// entry waits for the first range's biases before
 // any compute and for the last range's outputs after it, so those are small.
 void rho1_fp64_build_items(const std::vector<Rho1WorkItem> &batches, int tile_points, int order, int n_batches,
                            std::vector<Rho1WorkItem> *out, std::vector<int> *chunk_items,

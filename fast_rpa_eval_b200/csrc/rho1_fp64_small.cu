@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(THREADS, 1) rho1_small_kernel(const SmallParam
   const int g = lane >> 2, q = lane & 3;
   const int ld = small_ld(P.nc_max);
   // As[k][m]; per group Bs[2][n][k] and Ws[n][m]
-  double *As = smem, *Bs = As + ((P.nc_max + 3) & ~3) * ld + group * (2 * PTS * ld + PTS * LDW), *Ws = Bs + 2 * PTS * ld;
+  double *As = smem, *Bs = As + ((P.nc_max + 3) & ~3) * ld + group * (2 * PTS * ld + PTS * LDW);
+  double *Ws = Bs + 2 * PTS * ld;
   auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * GW) : "memory"); };
   const long long nb2 = (long long)P.n_basis * P.n_basis;
 

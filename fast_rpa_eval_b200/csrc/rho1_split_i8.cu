@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(PB_THREADS) i8_pack_b_kernel(const I8BTile *__
   __shared__ __align__(16) int s_ib[(FRPA_MAX_N_COMPUTE + 31) / 32 * 32];
   const I8BTile B = tiles[blockIdx.x];
   const int nc = B.nc;
-  for (int i = threadIdx.x; i < B.n_kc * I8_KC; i += PB_THREADS) s_ib[i] = i < nc ? __ldg(ib_all + B.ib_off + i) - 1 : 0;
+  for (int i = threadIdx.x; i < B.n_kc * I8_KC; i += PB_THREADS)
+    s_ib[i] = i < nc ? __ldg(ib_all + B.ib_off + i) - 1 : 0;
   __syncthreads();
   const int r = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = B.jn * I8_N + r;
@@ -824,7 +825,7 @@ int rho1_i8_launch(Rho1Plan &plan, int n_active, const double *wave, const doubl
     const int k = gi % sets, ni = g.item1 - g.item0, nt = g.tile1 - g.tile0;
     if (gi >= sets) FRPA_CUDA_TRY(cudaStreamWaitEvent(plan.i8_side, plan.i8_ev_done[k], 0));
     i8_pack_a_kernel<<<ni * PA_GROUPS, PA_THREADS, 0, plan.i8_side>>>(plan.d_i8_items + g.item0, wave, plan.d_i8_a[k],
-                                                          plan.d_i8_sa[k], P.wave_vec);
+                                                                      plan.d_i8_sa[k], P.wave_vec);
     FRPA_LAUNCH_CHECK();
     i8_pack_b_kernel<<<nt, PB_THREADS, 0, plan.i8_side>>>(plan.d_i8_tiles + g.tile0, plan.d_ib, P1, plan.d_rowmax,
                                                           plan.n_basis, plan.d_i8_b[k], plan.d_i8_sb[k]);

@@ -167,8 +167,9 @@ __global__ void __launch_bounds__(128)
                       const double *__restrict__ linc, const double *__restrict__ cc_xyz,
                       const double *__restrict__ mrs, const double *__restrict__ opr,
                       const int *__restrict__ lhmfd, const double *__restrict__ Q, const int *__restrict__ slot_of,
-                      const int *__restrict__ conv_ptr, const int *__restrict__ conv_lm, const double2 *__restrict__ conv_fc,
-                      double *__restrict__ recs, double4 *__restrict__ heads, int *__restrict__ err) {
+                      const int *__restrict__ conv_ptr, const int *__restrict__ conv_lm,
+                      const double2 *__restrict__ conv_fc, double *__restrict__ recs, double4 *__restrict__ heads,
+                      int *__restrict__ err) {
   __shared__ double q_kept[(SU_LMAX + 1) * (SU_LMAX + 1)];
   const int slot = blockIdx.x, t = blockIdx.y, L2 = (L + 1) * (L + 1);
   grid_release();
@@ -442,13 +443,14 @@ __device__ __forceinline__ int classify(const Box &b, const double *rec, bool ne
 // mixed records (8 for every l_max: 3% more on 2,000 to 100,000 points).
 // Measured, 500 atoms, 2 million points, l_max 6: 9.4 ms (two points per thread,
 // decisions per pair, near field inside) -> 7.7 ms, 70% of the FP64 peak (two
-// points per thread 8.7 ms, in the compiler's order 9.0 ms).
+// points per thread 8.7 ms, in the compiler's order 9.0 ms); with rsqrt() for the
+// inverse distances 2% more (l_max 4: 5%) than with a refinement written out here.
 template <int PPT, bool CODES, bool NEAR>
 __global__ void __launch_bounds__(SU_THREADS, PPT == 4 ? 4 : (PPT == 2 ? 5 : 6))
     sumup_far_kernel(int n_valid, int n_full, const int *__restrict__ order, const int *__restrict__ pfull,
                      const double *__restrict__ pxyz, const Box *__restrict__ pbox, int n_chp, int L,
-                     const double *recs, int slices, double *dv, unsigned char *codes, const double *__restrict__ spline,
-                     int n_atoms, int n_hartree_grid) {
+                     const double *recs, int slices, double *dv, unsigned char *codes,
+                     const double *__restrict__ spline, int n_atoms, int n_hartree_grid) {
   const int RS = rec_stride(L), CO = rec_coef_off(L);
   __shared__ __align__(16) double srec[2][SU_CHUNK * rec_stride(SU_LMAX)];
   const int CH = min(32, (SU_CHUNK * rec_stride(SU_LMAX) / RS) & ~3);  // records per chunk
@@ -798,7 +800,8 @@ __global__ void __launch_bounds__(SU_THREADS)
                          const double *__restrict__ mrs, const double *__restrict__ opr,
                          const int *__restrict__ ncc, const int *__restrict__ icc_packed,
                          const int *__restrict__ ijkmax, int mc_dim, const double *__restrict__ mc,
-                         const double *__restrict__ spline, double *__restrict__ dv, unsigned char *__restrict__ codes) {
+                         const double *__restrict__ spline, double *__restrict__ dv,
+                         unsigned char *__restrict__ codes) {
   const int iv = blockIdx.x * SU_THREADS + threadIdx.x;
   if (iv >= n_valid) return;
   const int f = map[iv];
