@@ -921,10 +921,19 @@ int launch_far(const SumupPlan &P, int n_active, int slices, const double *splin
 //   l_max 2: 2,000, 16,000   18 / 13, 20 / 13 (2)         24 / 15, 51 / 35  75 / 60, 213 / 201   350 / 369 (2,000)
 //   l_max 5: 2,000, 64,000   - , 24 / 18                  43 / 32, 116 / 108 (8)  167 / 196 (2,000)
 //   l_max 6: 8,000, 64,000   26 / 19, 28 / 20             72 / 61, 134 / 159 (8)  312 / 397 (8,000)
-// (in brackets: at another number of centres, or the one size).
-bool near_inline(int L, int n_points, int n_centres) {
+// (in brackets: at another number of centres, or the one size).  Above l_max 4 it also
+// pays around 2 to 8 centres while the points are enough for one warp to have its own
+// and few enough for about one round of warps, which the chain of latencies then sets:
+// 3 centres, 33,000 points each, l_max 6 58 / 43, l_max 8 87 / 65 (8,000 each: 29 / 39,
+// 43 / 60; 128,000 each: 72 / 80, 111 / 129); 8 centres, 16,000 each 92 / 70, 139 / 106
+// (32,000 each: 111 / 104, 164 / 157; 64,000 each: 134 / 159).  Not at l_max 7, whose
+// orders fill the own launch's eight lanes: 5 centres, 40,000 each 93 / 113.
+bool near_inline(int L, int n_points, int n_active, int n_centres) {
   const int most = L <= 4 ? 128 : (L == 5 ? 16 : 1);
-  return n_centres <= most && n_points >= 2048LL * n_centres;
+  if (n_centres <= most && n_points >= 2048LL * n_centres) return true;
+  if (L <= 4 && n_centres == 1) return true;  // 64 points: 10.6 / 8.3
+  const long long points = (long long)n_points * n_active;
+  return L != 7 && n_centres <= 8 && n_points >= 8192LL * n_centres && points >= 40000 && points <= 262144;
 }
 
 template <bool CODES>
@@ -940,7 +949,7 @@ int launch_fast(const SumupPlan &P, int n_active, const double *spline, double *
   auto warps = [&] { return (long long)ceil_div(P.n_valid_points, 32 * ppt) * n_active * slices; };
   while (warps() < want && slices < 4 && P.n_chp >= 4 * slices) slices *= 2;
   while (warps() < want && ppt > 1) ppt /= 2;
-  if (near_inline(P.L, P.n_valid_points, P.n_chp)) {
+  if (near_inline(P.L, P.n_valid_points, n_active, P.n_chp)) {
     if (ppt > 1) return launch_far<2, CODES, true>(P, n_active, slices, spline, dv, codes, stream);
     return launch_far<1, CODES, true>(P, n_active, slices, spline, dv, codes, stream);
   }

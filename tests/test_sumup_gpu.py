@@ -199,8 +199,14 @@ def test_sumup_inverse_distance_of_a_point_charge():
 
 
 @pytest.mark.parametrize("atoms,points,T,L,outer", [
-    (1, 2047, 1, 4, 3.0),      # the near field in its own launch
-    (1, 2048, 1, 4, 3.0),      # inline: one point per thread
+    (1, 64, 1, 2, 3.0),        # one centre at a low l: inline, few points
+    (2, 4095, 1, 4, 3.0),      # the near field in its own launch
+    (2, 4096, 1, 4, 3.0),      # inline: one point per thread
+    (8, 65_536, 1, 6, 3.0),    # the most centres above l 5, as few points each as that takes
+    (8, 65_535, 1, 6, 3.0),    # one point less
+    (4, 40_000, 1, 7, 3.0),    # not at this l
+    (2, 131_072, 2, 6, 3.0),   # as many points and perturbations as that takes
+    (2, 20_000, 2, 6, 3.0),    # as few
     (1, 2100, 2, 8, 3.0),      # the highest l; one centre at most
     (2, 5000, 1, 6, None),     # own launch at this l
     (16, 33_000, 1, 5, 4.0),   # the most centres of l 5, records over 4 warps
